@@ -1052,7 +1052,13 @@ void gradient_footprint(const Model& m, const eik_extra& ep, long long nrec, int
   const unsigned long long seedcap = refine ? std::max<unsigned long long>(win, 8) : 8;
   const unsigned long long nf = refine ? nfmax : 1;
   unsigned long long per = sizeof(SrcOut) + seedcap * (4 + 8) + N * (8 + 1 + 8 + 1) + sizeof(CoarseProblem) +
-                           std::max<unsigned long long>(N, nf) * (4 + 8 + 1 + 8 + 8) + 5 * 8;
+                           N * (4 + 8 + 8) + 5 * 8;
+  // brick state: traveltime, code, pending mask, front, flag and four list slots per brick
+  const unsigned long long bn = nd == 3 ? 512 : 256;
+  GridDesc wg = m.g;
+  for (int d = 0; d < nd; d++) wg.n[d] = (2 * ep.noderadius + 1) * ep.downscalefactor + 1;
+  const unsigned long long nbr = std::max(brick_nodes(m.g), refine ? brick_nodes(wg) : 0ull) / bn;
+  per += nbr * (bn * 9 + bn / 8 + 24) + 10 * 4;
   if (refine) per += nf * (8 + 1 + 1 + 4 + 4 + 1) + sizeof(CoarseProblem) + 8 * (4 + 8) + nf * (8 + 8 + 1) + 1;
   per += N * (8 + 8ull * nd + 8) + 8 + seedcap * 4 * 8 + nd * 8 + (refine ? nf * (8 + 8ull * nd) : 16) +
          sizeof(AdjProblem);
@@ -1162,6 +1168,11 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   GET(dap, AdjProblem, "adj_probs", nsrc);
   GET(dfb, ForwardBatch, "adj_fb", 1);
   GET(dwarn, uint32_t, "adj_warn", 1);
+  int32_t* astamp;
+  unsigned long long *alist0, *alist1;
+  GET(astamp, int32_t, "rs_stamp", nsrc * N);
+  GET(alist0, unsigned long long, "rs_list0", nsrc * N);
+  GET(alist1, unsigned long long, "rs_list1", nsrc * N);
 #undef GET
   std::vector<AdjProblem> hap(nsrc);
   for (int64_t s = 0; s < nsrc; s++) {
@@ -1179,10 +1190,12 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   CUDA_OK(ctx, cudaMemsetAsync(dwarn, 0, sizeof(uint32_t), st));
   CUDA_OK(ctx, cudaMemsetAsync(gsrc, 0, sizeof(double) * nsrc * nd, st));
   const CoarseProblem* dprobs = fw.sa.probs;
-  // the adjoint sweep reuses the forward's worklists; counts live in its round stamps
   AdjArgs aa;
   aa.sa = fw.sa;
   aa.ap = dap;
+  aa.sa.rs.stamp = astamp;
+  aa.sa.rs.list[0] = alist0;
+  aa.sa.rs.list[1] = alist1;
   aa.sa.rs.max_rounds = ctx->max_rounds > 0 ? ctx->max_rounds : (1 << 26);
   aa.sa.rs.rounds = fw.sa.rs.rounds + 1;  // the forward's count stays readable
   adj_rounds_init_kernel<<<1, 1, 0, st>>>(aa.sa);

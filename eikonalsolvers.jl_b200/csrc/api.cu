@@ -202,6 +202,8 @@ __global__ void problem_scale_kernel(CoarseProblem* dp, int nprob, const double*
   const double smin = *dsmin;
   dp[s].delta = gate * hmin * smin;
   dp[s].incmin = 0.999 * (2.0 / 3.0) * hmin * smin / sqrt((double)nd);
+  dp[s].linc = 0.999 * (2.0 / 3.0) * hmin / sqrt((double)nd);
+  dp[s].din = inner_window(nd, hmin * smin);
 }
 
 int model_create(eik_ctx* ctx, const eik_grid* grd, const double* vel, bool dev, eik_model_id* out) {
@@ -334,7 +336,8 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
       P.code = code + s * N;
       P.kL = kL + s * N;
       P.kd = kd + s * N;
-      P.delta = P.incmin = 0.0;  // set on the device from the model's smallest slowness
+      P.delta = P.incmin = P.linc = 0.0;  // set on the device from the model's smallest slowness
+      P.din = 0.0f;
       uniform_coeffs(P.g, &P.c1u, &P.c2u);
     }
   CoarseProblem* dp;
@@ -348,17 +351,32 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   sa.activations = ctr;
   sa.node_evals = ctr + 1;
   sa.abort_flag = (int32_t*)(ctr + 2);
-  // round-solver state, shared by the refined windows' solve and the coarse solve
+  // brick state, shared by the refined windows' solve and the coarse solve
   const long long rsn = nsrc * std::max<long long>(N, refine ? fb.nfmax : 1);
   if ((unsigned long long)rsn >= (1ull << 32))
     return fail(ctx, EIK_ERR_OUT_OF_BUDGET, "more than 2^32 node-sources in one call: split the sources");
-  GET(sa.rs.stamp, int32_t, "rs_stamp", rsn);
-  GET(sa.rs.tent, double, "rs_tent", rsn);
-  GET(sa.rs.dirty, uint8_t, "rs_dirty", rsn);
-  GET(sa.rs.list[0], unsigned long long, "rs_list0", rsn);
-  GET(sa.rs.list[1], unsigned long long, "rs_list1", rsn);
-  GET(sa.rs.nextmin, unsigned long long, "rs_nextmin", 3 * nsrc);
-  GET(sa.rs.thr, double, "rs_thr", 2 * nsrc);
+  const int bnodes = nd == 3 ? 512 : 256;  // nodes of a brick (brick.cuh)
+  unsigned long long cbricks = 1;          // bricks of the largest grid, and of a refined window
+  for (int i = 0; i < nmod; i++) cbricks = std::max(cbricks, brick_nodes(models[i]->g) / bnodes);
+  unsigned long long fbricks = 1;
+  if (refine) {
+    GridDesc wg = models[0]->g;
+    for (int d = 0; d < nd; d++) wg.n[d] = (2 * ep.noderadius + 1) * ep.downscalefactor + 1;
+    fbricks = brick_nodes(wg) / bnodes;
+  }
+  const unsigned long long nbr = (unsigned long long)nsrc * std::max(cbricks, fbricks);
+  GET(sa.bs.t, double, "br_t", nbr * bnodes);
+  GET(sa.bs.code, uint8_t, "br_code", nbr * bnodes);
+  GET(sa.bs.mask, unsigned, "br_mask", nbr * (bnodes / 32));
+  GET(sa.bs.front, unsigned, "br_front", nbr);
+  GET(sa.bs.listed, unsigned, "br_listed", nbr);
+  GET(sa.bs.lists, unsigned, "br_lists", 4 * nbr);
+  GET(sa.bs.ctr, unsigned, "br_ctr", 8);
+  GET(sa.bs.exam, unsigned, "br_exam", 4 * nsrc);
+  GET(sa.bs.marks, unsigned, "br_marks", 4 * nsrc);
+  GET(sa.bs.thr, float, "br_thr", 2 * nsrc);
+  sa.bs.listcap = nbr;
+  sa.bs.stride = (unsigned)cbricks;
   {
     unsigned int* rc32;
     GET(rc32, unsigned int, "rs_ctr", 32);
@@ -388,7 +406,6 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   // global solve (measured: 300x220 x 4 sources 27.7 -> 15.9 ms); in 3D the global solve is
   // faster (44^3 x 16: 33 vs 40 ms, and the refined windows), so only on request (2)
   const bool use_cluster = ctx->cluster_solve == 2 || (ctx->cluster_solve == 1 && nd == 2);
-  sa.rs.stride = (unsigned long long)N;
   sa.err = fb.err;
   sa.probs = dp;
   sa.max_activations = ~0ull;
@@ -411,7 +428,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   const void* hp_src = stage_host(ctx, hp.data(), sizeof(CoarseProblem) * nsrc);
   if (!hp_src) return fail(ctx, EIK_ERR_CUDA, "cudaMallocHost of a plan's staging copy failed");
   CUDA_OK(ctx, cudaMemcpyAsync(dp, hp_src, sizeof(CoarseProblem) * nsrc, cudaMemcpyHostToDevice, st));
-  const double gate = ctx->gate_for(work);
+  const double gate = ctx->gate_for(nd);
   const int sms = ctx->sms_for(work);
   // model i's slice of the per-source arrays, for the per-model start-up launches
   auto slice = [&](int i) {
@@ -468,7 +485,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
     }
     SolveArgs fsa = sa;
     fsa.probs = fprobs;
-    fsa.rs.stride = (unsigned long long)fb.nfmax;
+    fsa.bs.stride = (unsigned)fbricks;
     fsa.activations = sa.activations + 6;  // own counters: the coarse solve's stay separate
     fsa.node_evals = sa.activations + 7;
     fsa.rs.max_rounds = round_limit((long long)nd * ((2LL * ep.noderadius + 1) * ep.downscalefactor + 1));
@@ -479,10 +496,11 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
     if (in_cluster) {
       nlaunch += 2;
     } else {
-      launch_rounds_init(fsa, st);
-      launch_rounds_seed(fsa, fseed_lin, fseed_tt, fb.out, true, 8, st);
-      CUDA_OK(ctx, launch_coarse_solve(fsa, sms, ctx->ctas_per_sm, ctx->fwd_queue, st));
-      nlaunch += 3;
+      launch_bricks_init(fsa, st);
+      launch_bricks_seed(fsa, fseed_lin, fseed_tt, fb.out, true, 8, st);
+      CUDA_OK(ctx, launch_bricks_solve(fsa, ctx->brick_sms(nsrc * fbricks), st));
+      launch_bricks_store(fsa, st);
+      nlaunch += 5;
     }
     for (int i = 0; i < nmod; i++) {
       const int64_t o = src_off[i];
@@ -513,13 +531,15 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
     CUDA_OK(ctx, cudaGetLastError());
     nlaunch += 2;  // counters, solve
   } else {
-    launch_coarse_init(hp.data(), dp, (int)nsrc, fb, sa, st);
+    launch_bricks_init(sa, st);
+    launch_bricks_seed(sa, fb.seed_lin, fb.seed_tt, fb.out, false, fb.seedcap, st);
     CUDA_OK(ctx, cudaGetLastError());
     if (!ctx->capturing) cudaEventRecord(ctx->evk[2], st);
-    CUDA_OK(ctx, launch_coarse_solve(sa, sms, ctx->ctas_per_sm, ctx->fwd_queue, st));
+    CUDA_OK(ctx, launch_bricks_solve(sa, ctx->brick_sms(nsrc * cbricks), st));
     if (!ctx->capturing) cudaEventRecord(ctx->evk[3], st);
+    launch_bricks_store(sa, st);
     CUDA_OK(ctx, cudaGetLastError());
-    nlaunch += 4;  // coarse init, round init, seeds, solve
+    nlaunch += 5;  // counters, brick init, seeds, solve, store
   }
   fw->fb = fb;
   fw->sa = sa;

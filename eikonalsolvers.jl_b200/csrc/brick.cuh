@@ -1,0 +1,537 @@
+// Bricks of the forward round solver: layout, and the visit that settles one brick.
+//
+// A problem's grid is cut into bricks of 8x8x8 nodes (3D) or 16x16 (2D). The traveltimes are
+// kept brick by brick (a brick's nodes consecutive, x fastest), so a brick and the two layers
+// around it that its stencils read come in as 16-byte pieces whatever the grid's size. The
+// stencil reaches +-1 and +-2 along each axis: a brick reads only the bricks across its faces.
+// Bricks are therefore coloured like a checkerboard, and a round visits bricks of one colour
+// only: everything a visit reads outside its brick stands still while it runs, no write of a
+// round is read in the same round, and a visit needs no fence, flag or retry.
+//
+// One warp visits one brick. It copies the brick and its surroundings to shared memory,
+// evaluates the pending nodes there in the order of their fronts until none is left below the
+// round's threshold, and writes the brick back. A node is pending from the moment something
+// its rule may read has changed until it has been evaluated; the pending nodes of a brick are
+// a bit mask in global memory between visits. A node that changes makes the nodes whose
+// stencil reads it pending, in the warp's own brick (in shared memory) or in the brick across
+// a face (its mask, at the end of the visit).
+//
+// Why this shape: visited one by one from worklists, a node costs ~100 scattered sectors
+// (its neighbours, their codes and stamps, the relisting filter) and a round per layer of the
+// front. A brick visit reads ~10 KB in full sectors for ~200 evaluations and settles several
+// layers, so rounds are fewer (256^3 x 4 sources: 881 instead of 3970) and the evaluation chain
+// runs on shared memory. 8^3 nodes with one warp: a front crosses a brick in sheets of about 64
+// nodes, two warp-wide evaluations; larger bricks fill the lanes a little better but leave
+// fewer warps per SM to hide latency. Forward solve, worklists of nodes -> bricks, B200:
+// 256^3 x 4 420 -> 238 ms, 128^3 x 8 123 -> 79 ms, 64^3 x 32 48 -> 29 ms, 128^3 x 1 40 -> 28 ms,
+// 1024x640 x 64 196 -> 58 ms. What bounds it: the longest visit of a round while a round has
+// fewer bricks than the GPU has warps (a visit averages 30 us, the longest of a round 100 us);
+// DRAM and the FP64 pipe are idle (below 1 % and 3 %).
+#pragma once
+
+#include "kernels.cuh"
+#include "node.cuh"
+
+namespace eik {
+
+constexpr unsigned FULL_WARP = 0xffffffffu;
+constexpr unsigned PF_NONE = 0x7f800000u;  // +inf: no pending value
+
+// Brick geometry. Nodes are numbered x + BX*(y + BY*z); the shared-memory cube holds the brick
+// and two layers around it, x-pitch PY per row and PZ per plane, node (0,0,0) at ORG.
+template <int ND>
+struct Brick;
+template <>
+struct Brick<3> {
+  static constexpr int BX = 8, BY = 8, BZ = 8, NODES = 512, WORDS = 16, FACES = 6;
+  static constexpr int PY = 12, PZ = 144, ORG = 2 * 144 + 2 * 12 + 2, CUBE = 12 * 12 * 12;
+};
+template <>
+struct Brick<2> {
+  static constexpr int BX = 16, BY = 16, BZ = 1, NODES = 256, WORDS = 8, FACES = 4;
+  static constexpr int PY = 20, PZ = 0, ORG = 2 * 20 + 2, CUBE = 20 * 20;
+};
+
+// Number of bricks along an axis and in a problem, and the brick-ordered index of a node.
+template <int ND>
+EIK_HD int bricks_along(const GridDesc& g, int a) {
+  const int b = a == 0 ? Brick<ND>::BX : (a == 1 ? Brick<ND>::BY : Brick<ND>::BZ);
+  return (g.n[a] + b - 1) / b;
+}
+template <int ND>
+EIK_HD long long brick_count(const GridDesc& g) {
+  long long c = 1;
+  for (int a = 0; a < ND; a++) c *= bricks_along<ND>(g, a);
+  return c;
+}
+template <int ND>
+EIK_HD long long brick_node(const GridDesc& g, int i, int j, int k) {
+  typedef Brick<ND> B;
+  const int bi = i / B::BX, bj = j / B::BY, bk = ND == 3 ? k / B::BZ : 0;
+  const long long b = bi + (long long)bricks_along<ND>(g, 0) * (bj + (long long)bricks_along<ND>(g, 1) * bk);
+  return b * B::NODES + (i - bi * B::BX) + B::BX * ((j - bj * B::BY) + B::BY * (ND == 3 ? k - bk * B::BZ : 0));
+}
+
+// Shared memory of one warp. The list of a scan and the spherical coefficients (1/h^2 and
+// 9/(4h^2) of axes 1 and 2 per radial index of the brick) take corners of the cube that no
+// stencil reads in 3D: 20.9 KB a warp, 11 warps an SM.
+template <int ND>
+struct __align__(16) WarpMem {
+  typedef Brick<ND> B;
+  double cube[B::CUBE];                // traveltimes; sign bit: special key
+  double slow[B::NODES];
+  unsigned pf[B::NODES];               // pending front (float bits) or PF_NONE
+  uint8_t code[B::NODES];
+  unsigned face[B::FACES * B::WORDS];  // nodes made pending in the bricks across the faces
+  unsigned facemin[8];                 // and their smallest front
+  double extra[ND == 3 ? 2 : 48];
+  __device__ __forceinline__ uint16_t* list() {
+    return reinterpret_cast<uint16_t*>(ND == 3 ? cube : extra);  // 64 entries, 16 doubles
+  }
+  __device__ __forceinline__ double* coef() { return ND == 3 ? cube + 120 : extra + 16; }  // up to 32
+};
+// cube + 0..15 lie in the row y = -2 of the plane z = -2, cube + 120..151 in the rows y = 8, 9 of
+// that plane and y = -2 of the next: outside the layers that any stencil of the brick reads
+static_assert(Brick<3>::PZ == 144 && Brick<3>::PY == 12, "unused corners of the 3D cube");
+
+__device__ __forceinline__ unsigned front_bits(double v) {
+  // smallest float >= v, finite: a pending node is never lost to overflow
+  const float f = __double2float_ru(v);
+  return v < EIK_INF ? __float_as_uint(fminf(f, 3.402823466e38f)) : PF_NONE;
+}
+
+// 16 bytes through L2 only: the brick state is written by other SMs between rounds, and L1
+// may hold an older copy. (cp_async8 below goes through L1: for the slowness, which is constant.)
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+__device__ __forceinline__ bool sign_set(double v) { return __double2hiint(v) < 0; }
+
+// The order rule by full keys, for the nodes the fast rule leaves out (about one in a
+// thousand). Out of line; it reads the neighbourhood again from the cube, so that no array of
+// the visit has an address. t: the node in the cube; ok2: sides (bit slot(axis, side)) where
+// 2nd order is allowed; l: column-major node index; i: radial index.
+template <int ND>
+__device__ __noinline__ RuleOut rule_slow(const CoarseProblem& P, const double* t, unsigned ok2, long long l, int i,
+                                          double slow) {
+  typedef Brick<ND> B;
+  Nbhd nb;
+  nb_clear(nb);
+  node_dh(P.g, i, nb.dh);
+  nb.slow = slow;
+  nb.c1u = P.c1u;
+  nb.c2u = P.c2u;
+#pragma unroll
+  for (int a = 0; a < ND; a++) {
+    const long long st = a == 0 ? 1LL : (a == 1 ? (long long)P.g.n[0] : (long long)P.g.n[0] * P.g.n[1]);
+    const int cs = a == 0 ? 1 : (a == 1 ? B::PY : B::PZ);
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+      const long long l1 = s == 0 ? l + st : l - st, l2 = s == 0 ? l1 + st : l1 - st;
+      // an absent node is unreached: it is accepted by no group either way
+      const double r1 = t[s == 0 ? cs : -cs], r2 = ((ok2 >> slot(a, s)) & 1u) ? t[s == 0 ? 2 * cs : -2 * cs] : EIK_INF;
+      nb_put1(nb, a, s, fabs(r1), sign_set(r1) ? __ldcg(P.kL + l1) : r1, sign_set(r1) ? (int)__ldcg(P.kd + l1) : 0);
+      nb_put2(nb, a, s, fabs(r2), sign_set(r2) ? __ldcg(P.kL + l2) : r2, sign_set(r2) ? (int)__ldcg(P.kd + l2) : 0);
+    }
+  }
+  RuleOut o;
+  o.neg = false;
+  o.cd[0] = o.cd[1] = o.cd[2] = 0;
+  o.v = prefix_rule<ND>(nb, o.cd, &o.key, &o.neg);
+  return o;
+}
+
+// Copies brick b (of problem P, at brick coordinates bc, bricks nb per axis) and the layers
+// around it that exist to w.cube, the slowness to w.slow; positions outside the grid get +inf.
+template <int ND>
+__device__ __forceinline__ void load_brick(WarpMem<ND>& w, const BrickState& bs, const CoarseProblem& P, size_t b,
+                                           const int (&bc)[3], const int (&nb)[3], int lane) {
+  typedef Brick<ND> B;
+  const double* own = bs.t + b * B::NODES;
+  constexpr int ROWP = B::BX / 2;  // 16-byte pieces of a row
+#pragma unroll
+  for (int q = 0; q < B::NODES / 2; q += 32) {
+    const int e = q + lane, row = e / ROWP, xp = e % ROWP;
+    const int y = row % B::BY, z = row / B::BY;
+    cp_async16(&w.cube[B::ORG + z * B::PZ + y * B::PY + 2 * xp], own + 2 * e);
+  }
+  // layers across the faces: side 0 = +, side 1 = - (as slot())
+  const long long bst[3] = {1, nb[0], (long long)nb[0] * nb[1]};
+#pragma unroll
+  for (int a = 0; a < ND; a++)
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+      const bool have = s == 0 ? bc[a] + 1 < nb[a] : bc[a] > 0;
+      const double* src = s == 0 ? own + bst[a] * B::NODES : own - bst[a] * B::NODES;
+      // pairs of the two layers: along x one pair per row, else ROWP pairs per row of 2 rows
+      constexpr int PER = ND == 3 ? 64 : 16;
+      const int pieces = a == 0 ? B::BY * B::BZ : PER;
+#pragma unroll
+      for (int q = 0; q < (ND == 3 ? 64 : 16); q += 32) {
+        const int e = q + lane;
+        if (e < pieces) {
+          int ci, si;
+          if (a == 0) {
+            const int y = e % B::BY, z = e / B::BY;
+            ci = B::ORG + z * B::PZ + y * B::PY + (s == 0 ? B::BX : -2);
+            si = e * B::BX + (s == 0 ? 0 : B::BX - 2);
+          } else if (a == 1) {
+            const int z = e / (2 * ROWP), rr = (e / ROWP) & 1, xp = e % ROWP;
+            const int y = s == 0 ? rr : B::BY - 2 + rr;
+            ci = B::ORG + z * B::PZ + (s == 0 ? B::BY + rr : rr - 2) * B::PY + 2 * xp;
+            si = (z * B::BY + y) * B::BX + 2 * xp;
+          } else {
+            const int rr = e / (B::BY * ROWP), y = (e / ROWP) % B::BY, xp = e % ROWP;
+            const int z = s == 0 ? rr : B::BZ - 2 + rr;
+            ci = B::ORG + (s == 0 ? B::BZ + rr : rr - 2) * B::PZ + y * B::PY + 2 * xp;
+            si = (z * B::BY + y) * B::BX + 2 * xp;
+          }
+          if (have) {
+            cp_async16(&w.cube[ci], src + si);
+          } else {
+            w.cube[ci] = EIK_INF;
+            w.cube[ci + 1] = EIK_INF;
+          }
+        }
+      }
+    }
+  const GridDesc& g = P.g;
+  const int x0 = bc[0] * B::BX, y0 = bc[1] * B::BY, z0 = bc[2] * B::BZ;
+#pragma unroll
+  for (int q = 0; q < B::NODES; q += 32) {
+    const int e = q + lane, x = x0 + e % B::BX, y = y0 + (e / B::BX) % B::BY, z = z0 + e / (B::BX * B::BY);
+    if (x < g.n[0] && y < g.n[1] && z < g.n[2]) cp_async8(&w.slow[e], P.slow + lin3(g, x, y, z));
+  }
+}
+
+// Visit outcome counters of a warp (lane k < 7 holds outcome k).
+struct VisitTally {
+  unsigned n = 0;
+  __device__ __forceinline__ void add(unsigned oc, int lane) {
+    const unsigned b0 = __ballot_sync(FULL_WARP, oc & 1u), b1 = __ballot_sync(FULL_WARP, oc & 2u),
+                   b2 = __ballot_sync(FULL_WARP, oc & 4u);
+    if (lane < 7) {
+      const unsigned mk = ((lane & 1) ? b0 : ~b0) & ((lane & 2) ? b1 : ~b1) & ((lane & 4) ? b2 : ~b2);
+      n += (unsigned)__popc(mk);
+    }
+  }
+};
+
+// Evaluations a visit may start before it hands its pending nodes back to the next round: a
+// visit settles in a few dozen, and the bound keeps a schedule that alternates (the rule's
+// depth limit lets some transient keys do so) from holding the round.
+constexpr int VISIT_MAX_SCANS = 192;
+
+// Which steps -2, -1, +1, +2 along an axis stay within [lo, hi) from position p: bits 0..3 of
+// nibble p of the table, for positions 0..15 (low half: 0..7).
+__device__ __forceinline__ unsigned long long step_table(int lo, int hi) {
+  auto upto = [](int e) { return e <= 0 ? 0ull : (e >= 16 ? ~0ull : (1ull << (4 * e)) - 1ull); };
+  const unsigned long long one = 0x1111111111111111ull;
+  return (one & ~upto(lo + 2)) | ((one << 1) & ~upto(lo + 1)) | ((one << 2) & upto(hi - 1)) | ((one << 3) & upto(hi - 2));
+}
+
+// Settles brick b up to threshold T (a float-valued bound): returns the smallest pending front
+// left in it (float bits, PF_NONE if none), its mask written back. The fronts and masks for
+// the bricks across its faces are left in w.facemin / w.face for the caller to publish.
+template <int ND>
+__device__ __forceinline__ unsigned visit_brick(WarpMem<ND>& w, const BrickState& bs, const CoarseProblem& P, size_t b,
+                                                const int (&bc)[3], const int (&nb)[3], float T, int lane,
+                                                VisitTally& tally) {
+  typedef Brick<ND> B;
+  uint16_t* list = w.list();
+  double* coef = w.coef();
+  unsigned pend = 0u;
+  if (lane < B::WORDS) pend = __ldcg(bs.mask + b * B::WORDS + lane);
+  load_brick<ND>(w, bs, P, b, bc, nb, lane);
+  if (lane < B::NODES / 16) cp_async16(&w.code[lane * 16], bs.code + b * B::NODES + lane * 16);
+  for (int q = lane; q < B::FACES * B::WORDS; q += 32) w.face[q] = 0u;
+  if (lane < 8) w.facemin[lane] = PF_NONE;
+  // the problem's constants in registers: the visit's barriers would make the compiler read
+  // them from memory again at every step
+  const int n[3] = {P.g.n[0], P.g.n[1], P.g.n[2]};
+  const int x0[3] = {bc[0] * B::BX, bc[1] * B::BY, bc[2] * B::BZ};
+  double* const kL = P.kL;
+  uint8_t* const kd = P.kd;
+  const bool cart = P.c1u > 0.0;
+  if (!cart && lane < B::BX && x0[0] + lane < n[0]) {
+    double dh[3];
+    node_dh(P.g, x0[0] + lane, dh);
+#pragma unroll
+    for (int a = 1; a < ND; a++) {
+      coef[(lane * (ND - 1) + a - 1) * 2] = 1.0 / (dh[a] * dh[a]);
+      coef[(lane * (ND - 1) + a - 1) * 2 + 1] = 9.0 / (4.0 * (dh[a] * dh[a]));
+    }
+  }
+  const double h0 = P.g.spac[0];
+  const double c10 = cart ? P.c1u : 1.0 / (h0 * h0), c20 = cart ? P.c2u : 9.0 / (4.0 * (h0 * h0));
+  const double linc = P.linc;
+  const float din = P.din;
+  // steps that stay in the brick, and in the grid; whether 2nd order is allowed everywhere
+  unsigned long long tb[ND], tg[ND];
+  bool border = false;
+#pragma unroll
+  for (int a = 0; a < ND; a++) {
+    const int ext = a == 0 ? B::BX : (a == 1 ? B::BY : B::BZ), left = n[a] - x0[a];
+    tb[a] = step_table(0, min(ext, left));
+    tg[a] = step_table(x0[a] > 0 ? -2 : 0, left);
+    border = border || x0[a] == 0 || left < ext + 2;
+  }
+  cp_async_wait();
+  __syncwarp();
+  // fronts of the pending nodes: smallest neighbouring traveltime plus the least increment
+  // (from the high words, which is exact enough for an order, and for all nodes, which keeps
+  // the loads in flight)
+  const unsigned* hi = reinterpret_cast<const unsigned*>(w.cube) + 1;
+#pragma unroll 4
+  for (int k = 0; k < B::WORDS; k++) {
+    const unsigned word = __shfl_sync(FULL_WARP, pend, k);
+    const int q = 32 * k + lane;
+    const int ci = B::ORG + (q / (B::BX * B::BY)) * B::PZ + ((q / B::BX) % B::BY) * B::PY + q % B::BX;
+    auto t = [&](int off) { return hi[2 * (ci + off)] & 0x7fffffffu; };
+    unsigned pot = min(min(t(1), t(-1)), min(t(B::PY), t(-B::PY)));
+    if constexpr (ND == 3) pot = min(pot, min(t(B::PZ), t(-B::PZ)));
+    const unsigned f = front_bits(__hiloint2double((int)pot, 0) + linc * w.slow[q]);
+    w.pf[q] = ((word >> lane) & 1u) ? f : PF_NONE;
+  }
+  __syncwarp();
+  const unsigned Tb = __float_as_uint(T), below = (1u << lane) - 1u;
+  unsigned left = PF_NONE, leftmask = 0u;
+#pragma unroll 1
+  for (int it = 0;; it++) {
+    unsigned v[B::WORDS];
+    unsigned mn = PF_NONE;
+#pragma unroll
+    for (int k = 0; k < B::WORDS; k++) {
+      v[k] = w.pf[32 * k + lane];
+      mn = min(mn, v[k]);
+    }
+    mn = __reduce_min_sync(FULL_WARP, mn);
+    if (mn > Tb || mn == PF_NONE || it >= VISIT_MAX_SCANS) {
+      left = mn;
+#pragma unroll
+      for (int k = 0; k < B::WORDS; k++) {
+        const unsigned mm = __ballot_sync(FULL_WARP, v[k] != PF_NONE);
+        if (lane == k) leftmask = mm;
+      }
+      break;
+    }
+    // the nodes within the inner window above the smallest front, up to two warps of them
+    const float Tl = fminf(T, __fadd_ru(__uint_as_float(mn), din));
+    const unsigned Tlb = min(__float_as_uint(Tl), PF_NONE - 1u);
+    int cnt = 0;
+    unsigned sel[B::WORDS];
+#pragma unroll
+    for (int k = 0; k < B::WORDS; k++) sel[k] = __ballot_sync(FULL_WARP, v[k] <= Tlb);
+#pragma unroll
+    for (int k = 0; k < B::WORDS; k++) {
+      const int pos = cnt + __popc(sel[k] & below);
+      if (v[k] <= Tlb && pos < 64) list[pos] = (uint16_t)(32 * k + lane);
+      cnt += __popc(sel[k]);
+    }
+    cnt = min(cnt, 64);
+    __syncwarp();
+#pragma unroll 1
+    for (int c0 = 0; c0 < cnt; c0 += 32) {
+      const bool act = c0 + lane < cnt;
+      const unsigned uq = act ? (unsigned)list[c0 + lane] : 0u;
+      const int q = (int)uq, x = (int)(uq % B::BX), y = (int)((uq / B::BX) % B::BY), z = (int)(uq / (B::BX * B::BY));
+      const int ci = B::ORG + z * B::PZ + y * B::PY + x;
+      if (act) w.pf[q] = PF_NONE;
+      const double traw = w.cube[ci];
+      const double told = fabs(traw);
+      const double slow = w.slow[q];
+      double t1[ND][2], t2[ND][2];
+      int sgn = 0;
+      unsigned ok2 = 0xffu;
+#pragma unroll
+      for (int a = 0; a < ND; a++) {
+        const int st = a == 0 ? 1 : (a == 1 ? B::PY : B::PZ);
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+          const int sh = s == 0 ? st : -st;
+          t1[a][s] = w.cube[ci + sh];
+          t2[a][s] = w.cube[ci + 2 * sh];
+        }
+      }
+      if (border) {
+        // 2nd order needs the first neighbour off the border in every coordinate (isonbord)
+        const int gx[3] = {x0[0] + x, x0[1] + y, x0[2] + z};
+#pragma unroll
+        for (int a = 0; a < ND; a++) {
+          bool inner = true;
+#pragma unroll
+          for (int d = 0; d < ND; d++)
+            if (d != a) inner = inner && gx[d] >= 1 && gx[d] <= n[d] - 2;
+          if (!(inner && gx[a] + 1 <= n[a] - 2)) ok2 &= ~(1u << slot(a, 0));
+          if (!(inner && gx[a] - 1 >= 1)) ok2 &= ~(1u << slot(a, 1));
+        }
+#pragma unroll
+        for (int a = 0; a < ND; a++)
+#pragma unroll
+          for (int s = 0; s < 2; s++)
+            if (!((ok2 >> slot(a, s)) & 1u)) t2[a][s] = EIK_INF;
+      }
+#pragma unroll
+      for (int a = 0; a < ND; a++)
+#pragma unroll
+        for (int s = 0; s < 2; s++) sgn |= __double2hiint(t1[a][s]) | __double2hiint(t2[a][s]);
+      double Lold = told;
+      int dold = 0;
+      unsigned oc = VISIT_NONE;
+      if (act && sign_set(traw)) {
+        const long long l = (x0[0] + x) + (long long)n[0] * ((x0[1] + y) + (long long)n[1] * (x0[2] + z));
+        Lold = __ldcg(kL + l);
+        dold = (int)__ldcg(kd + l);
+        if (Lold == -EIK_INF) oc = VISIT_SOURCE;  // source points are fixed
+      }
+      const bool ev = act && oc == VISIT_NONE;
+      double nv;
+      int8_t cd[3] = {0, 0, 0};
+      bool done;
+      {
+        double c1[ND], c2[ND];
+        c1[0] = c10;
+        c2[0] = c20;
+#pragma unroll
+        for (int a = 1; a < ND; a++) {
+          c1[a] = c10;
+          c2[a] = c20;
+        }
+        if (!cart) {
+#pragma unroll
+          for (int a = 1; a < ND; a++) {
+            c1[a] = coef[(x * (ND - 1) + a - 1) * 2];
+            c2[a] = coef[(x * (ND - 1) + a - 1) * 2 + 1];
+          }
+        }
+        int8_t cf[ND];
+        if (!__any_sync(FULL_WARP, ev && sgn < 0)) {
+          done = prefix_rule_fast<ND, false>(t1, t2, t1, t2, c1, c2, slow, &nv, cf);
+        } else {
+          // special neighbours of some lane: the same with key levels
+          const long long l = (x0[0] + x) + (long long)n[0] * ((x0[1] + y) + (long long)n[1] * (x0[2] + z));
+          double L1[ND][2], L2[ND][2];
+#pragma unroll
+          for (int a = 0; a < ND; a++) {
+            const long long st = a == 0 ? 1LL : (a == 1 ? (long long)n[0] : (long long)n[0] * n[1]);
+#pragma unroll
+            for (int s = 0; s < 2; s++) {
+              const long long l1 = s == 0 ? l + st : l - st, l2 = s == 0 ? l1 + st : l1 - st;
+              L1[a][s] = sign_set(t1[a][s]) ? __ldcg(kL + l1) : t1[a][s];
+              L2[a][s] = sign_set(t2[a][s]) ? __ldcg(kL + l2) : t2[a][s];
+              t1[a][s] = fabs(t1[a][s]);
+              t2[a][s] = fabs(t2[a][s]);
+            }
+          }
+          done = prefix_rule_fast<ND, true>(t1, t2, L1, L2, c1, c2, slow, &nv, cf);
+        }
+#pragma unroll
+        for (int a = 0; a < ND; a++) cd[a] = cf[a];
+      }
+      double nL = nv;
+      int nd = 0;
+      if (ev && !done) {
+        const long long l = (x0[0] + x) + (long long)n[0] * ((x0[1] + y) + (long long)n[1] * (x0[2] + z));
+        const RuleOut o = rule_slow<ND>(P, &w.cube[ci], ok2, l, x0[0] + x, slow);
+        nv = o.v;
+        nL = o.key.L;
+        nd = o.key.d;
+#pragma unroll
+        for (int a = 0; a < 3; a++) cd[a] = o.cd[a];
+      }
+      __syncwarp();  // every lane has read before any writes
+      bool changed = false;
+      if (ev) {
+        const bool same = nv == told && nL == Lold && nd == dold;  // +inf equals +inf
+        const bool wait = !same && nv > (double)T && nv < EIK_INF && T < 3.402823466e38f;
+        changed = !same && !wait;
+        oc = same ? (nv < EIK_INF ? VISIT_SAME : VISIT_UNREACHED) : (wait ? VISIT_WAIT : VISIT_CHANGED);
+        if (wait) {
+          w.pf[q] = front_bits(nv);  // not final yet: the old value stands until the front is there
+        } else {
+          const bool spec = !(nL == nv && nd == 0);
+          w.cube[ci] = spec ? -nv : nv;
+          w.code[q] = pack_codes(cd, ND);
+          if (spec && changed) {
+            const long long l = (x0[0] + x) + (long long)n[0] * ((x0[1] + y) + (long long)n[1] * (x0[2] + z));
+            kL[l] = nL;
+            kd[l] = (uint8_t)nd;
+          }
+        }
+      }
+      tally.add(oc, lane);
+      __syncwarp();
+      // The nodes whose stencil reads a changed node become pending, except those whose own key
+      // is at most both its old and its new key: their rule never accepts it, so their value
+      // cannot change. An ordinary key (t, 0, t) is at most both when t is at most both levels;
+      // a special one (sign bit: largest as unsigned) is always taken. The node two steps away
+      // reads this one only beyond a reached node.
+      unsigned cm = 0u;
+      if (changed) {
+        const unsigned long long lim = (unsigned long long)__double_as_longlong(fmin(Lold, nL));
+#pragma unroll
+        for (int a = 0; a < ND; a++) {
+          const int st = a == 0 ? 1 : (a == 1 ? B::PY : B::PZ);
+          const unsigned long long m2 = __double_as_longlong(w.cube[ci - 2 * st]), m1 = __double_as_longlong(w.cube[ci - st]),
+                                   p1 = __double_as_longlong(w.cube[ci + st]), p2 = __double_as_longlong(w.cube[ci + 2 * st]);
+          const bool rm = ((unsigned)(m1 >> 32) & 0x7fffffffu) < 0x7ff00000u,
+                     rp = ((unsigned)(p1 >> 32) & 0x7fffffffu) < 0x7ff00000u;
+          cm |= (rm && m2 > lim ? 1u : 0u) << (4 * a) | (m1 > lim ? 2u : 0u) << (4 * a) |
+                (p1 > lim ? 4u : 0u) << (4 * a) | (rp && p2 > lim ? 8u : 0u) << (4 * a);
+        }
+        unsigned inb = 0u, ing = 0u;
+#pragma unroll
+        for (int a = 0; a < ND; a++) {
+          const int p = a == 0 ? x : (a == 1 ? y : z);
+          inb |= ((unsigned)(tb[a] >> (4 * p)) & 15u) << (4 * a);
+          ing |= ((unsigned)(tg[a] >> (4 * p)) & 15u) << (4 * a);
+        }
+        // their front: the least increment over the new value, at this node's slowness (an
+        // ordering only: a pending node is evaluated whatever its front was)
+        const unsigned fb = front_bits(nv + linc * slow);
+        const unsigned in = cm & inb;
+        cm &= ing & ~inb;
+#pragma unroll
+        for (int k = 0; k < 4 * ND; k++) {
+          const int a = k >> 2, j = k & 3;
+          const int qst = a == 0 ? 1 : (a == 1 ? B::BX : B::BX * B::BY);
+          if ((in >> k) & 1u) atomicMin(&w.pf[q + (j < 2 ? j - 2 : j - 1) * qst], fb);
+        }
+        while (cm) {
+          const int k = __ffs(cm) - 1, a = k >> 2, j = k & 3;
+          cm &= cm - 1u;
+          const int off = j < 2 ? j - 2 : j - 1;
+          const int ext = a == 0 ? B::BX : (a == 1 ? B::BY : B::BZ);
+          const int qst = a == 0 ? 1 : (a == 1 ? B::BX : B::BX * B::BY);
+          const int qj = q + (j < 2 ? off + ext : off - ext) * qst, f = 2 * a + (j < 2 ? 1 : 0);
+          atomicOr(&w.face[f * B::WORDS + (qj >> 5)], 1u << (qj & 31));
+          atomicMin(&w.facemin[f], fb);
+        }
+      }
+      __syncwarp();
+    }
+  }
+  // write back
+  double* own = bs.t + b * B::NODES;
+  constexpr int ROWP = B::BX / 2;
+#pragma unroll
+  for (int q = 0; q < B::NODES / 2; q += 32) {
+    const int e = q + lane, row = e / ROWP, xp = e % ROWP;
+    const int y = row % B::BY, z = row / B::BY;
+    *reinterpret_cast<double2*>(own + 2 * e) =
+        *reinterpret_cast<const double2*>(&w.cube[B::ORG + z * B::PZ + y * B::PY + 2 * xp]);
+  }
+  if (lane < B::NODES / 16)
+    *reinterpret_cast<uint4*>(bs.code + b * B::NODES + lane * 16) = *reinterpret_cast<const uint4*>(&w.code[lane * 16]);
+  if (lane < B::WORDS) bs.mask[b * B::WORDS + lane] = leftmask;
+  return left;
+}
+
+}  // namespace eik

@@ -1,415 +1,271 @@
 // Coarse-grid forward solve: the reference's heap-ordered FMM main loop
 // (ttFMM_core!, src/EikSolv/eikmainfwd.jl:427-823) restated as the fixed point of the
-// order rule of stencil.cuh and solved by a node-level worklist iteration.
+// order rule of stencil.cuh and solved by rounds of brick visits (brick.cuh).
 //
 // One cooperative persistent launch serves many problems (the sources of a call, or the
-// refined windows around them). It runs in rounds separated by a grid barrier. In round r
-// the warps take the round's worklist 32 entries at a time; a node whose potential is at
-// most the problem's threshold is evaluated, and when its value or key changes the nodes
-// whose stencil reads it are listed for round r+1; a node still above the threshold is
-// listed again with its pending front. The threshold follows the front (smallest pending
-// front + a round width of about one node's traveltime), so the rounds sweep the grid in
-// traveltime order. Every wait is bounded (global timer), the number of rounds is bounded;
-// both report through an error word instead of trapping.
+// refined windows around them). Rounds alternate between the two colours of bricks and are
+// separated by a grid barrier. Round r goes through the list of its colour; a brick whose
+// smallest pending front is at most its problem's threshold is visited by one warp, the
+// others stay listed. The threshold of problem p is (smallest pending front of p) + a window
+// of delta_p, never moving back, so the rounds sweep the grid in traveltime order. Every
+// wait is bounded (global timer), the number of rounds is bounded; both report through an
+// error word instead of trapping.
+#include <algorithm>
+
+#include "brick.cuh"
 #include "kernels.cuh"
-#include "node.cuh"
 #include "rounds.cuh"
 
 namespace eik {
 
-
-// Worklist entry: node id (problem * N + node) in the high word, a lower bound of the
-// node's pending front (float, rounded down) in the low word.
-__device__ __forceinline__ unsigned long long list_entry(unsigned int gid, double front) {
-  const float f = front < EIK_INF ? __double2float_rd(front) : __int_as_float(0x7f800000);
-  return ((unsigned long long)gid << 32) | (unsigned long long)__float_as_uint(f);
-}
-
-// Lists node gid for round r, once per round.
-__device__ __forceinline__ void list_node(const SolveArgs& a, int r, unsigned int gid, double front) {
-  if (atomicExch(a.rs.stamp + gid, r) != r) {
-    const unsigned int i = atomicAdd(a.rs.cnt + (r % 3), 1u);
-    a.rs.list[r & 1][i] = list_entry(gid, front);
-  }
-}
+// Warps per CTA, one CTA per SM: as many warps as their shared memory allows in 3D (20.9 KB
+// each), 16 in 2D (7 KB each) where a round seldom has more bricks per SM.
+template <int ND>
+constexpr int BRICK_WARPS = ND == 3 ? 11 : 16;
 
 // ----------------------------------------------------------------------- init --
-__global__ void coarse_init_kernel(const CoarseProblem* probs, int nprob, long long N) {
-  const long long tot = N * nprob;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot;
-       q += (long long)gridDim.x * blockDim.x) {
-    const int p = (int)(q / N);
-    const long long l = q - (long long)p * N;
-    probs[p].t[l] = EIK_INF;
-    probs[p].code[l] = CODE_NONE;
+__global__ void bricks_init_kernel(BrickState bs, unsigned nprob, int nodes, int words) {
+  const size_t nb = (size_t)bs.stride * nprob, t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x,
+               dt = (size_t)gridDim.x * blockDim.x;
+  const double2 inf2 = make_double2(EIK_INF, EIK_INF);
+  for (size_t q = t0; q < nb * nodes / 2; q += dt) reinterpret_cast<double2*>(bs.t)[q] = inf2;
+  const unsigned none = CODE_NONE * 0x01010101u;
+  for (size_t q = t0; q < nb * nodes / 16; q += dt)
+    reinterpret_cast<uint4*>(bs.code)[q] = make_uint4(none, none, none, none);
+  for (size_t q = t0; q < nb * words; q += dt) bs.mask[q] = 0u;
+  for (size_t q = t0; q < nb; q += dt) {
+    bs.front[q] = PF_NONE;
+    bs.listed[q] = 0u;
   }
+  for (size_t q = t0; q < 4 * (size_t)nprob; q += dt) {
+    bs.exam[q] = PF_NONE;
+    bs.marks[q] = PF_NONE;
+  }
+  for (size_t q = t0; q < 2 * (size_t)nprob; q += dt) bs.thr[q] = 0.0f;
+  if (t0 < 8) bs.ctr[t0] = 0u;
 }
 
-__global__ void rounds_init_kernel(SolveArgs a) {
-  const long long tot = (long long)a.rs.stride * a.nprob;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot;
-       q += (long long)gridDim.x * blockDim.x) {
-    a.rs.stamp[q] = -1;
-    a.rs.dirty[q] = 1;
-  }
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < 3LL * a.nprob;
-       q += (long long)gridDim.x * blockDim.x)
-    a.rs.nextmin[q] = (unsigned long long)__double_as_longlong(EIK_INF);
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < 2LL * a.nprob;
-       q += (long long)gridDim.x * blockDim.x)
-    a.rs.thr[q] = -EIK_INF;
-  if (blockIdx.x == 0 && threadIdx.x < 3) {
-    a.rs.cnt[threadIdx.x] = 0;
-    a.rs.grab[threadIdx.x] = 0;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    a.rs.bar[0] = 0;
-    a.rs.bar[1] = 0;
-    *a.rs.rounds = 0;
-    for (int k = 0; k < 7; k++) a.rs.visits[k] = 0;
-    *a.activations = 0;
-    *a.node_evals = 0;
-    *a.abort_flag = 0;
-  }
+__global__ void solve_counters_kernel(SolveArgs a) {
+  if (threadIdx.x != 0) return;
+  a.rs.bar[0] = 0;
+  a.rs.bar[1] = 0;
+  *a.rs.rounds = 0;
+  for (int k = 0; k < 7; k++) a.rs.visits[k] = 0;
+  *a.activations = 0;
+  *a.node_evals = 0;
+  *a.abort_flag = 0;
 }
 
 // Seeds: fixed traveltimes of the source points (coarse source box, coarse-coincident
 // accepted fine nodes, or the source box of a refined window); the nodes within two steps
-// of a seed start round 0, whose threshold is based on the smallest seed traveltime.
+// of a seed are pending at the start, with the seed's traveltime as their front.
 template <int ND>
 __global__ void seed_kernel(SolveArgs a, const int32_t* seed_lin, const double* seed_tt, const SrcOut* out,
                             int fine_corners, int seedcap) {
+  typedef Brick<ND> B;
   const int s = blockIdx.x;
   const CoarseProblem& P = a.probs[s];
+  const BrickState& bs = a.bs;
   const int ns = fine_corners ? out[s].nsrcf : out[s].nseeds;
+  const size_t base = (size_t)s * bs.stride;
   for (int q = threadIdx.x; q < ns; q += blockDim.x) {
     const long long l = seed_lin[(size_t)s * seedcap + q];
-    P.t[l] = seed_tt[(size_t)s * seedcap + q];
-    P.code[l] = (uint8_t)(CODE_NONE | CODE_SRC_BIT);
+    int c[3];
+    node_coords(P.g, l, c);
+    bs.t[base * B::NODES + brick_node<ND>(P.g, c[0], c[1], c[2])] = -fabs(seed_tt[(size_t)s * seedcap + q]);
     P.kL[l] = -EIK_INF;
     P.kd[l] = 0;
   }
   __syncthreads();
-  __threadfence();
   for (int q = threadIdx.x; q < ns; q += blockDim.x) {
-    const long long l = seed_lin[(size_t)s * seedcap + q];
-    const int i = (int)(l % P.g.n[0]);
-    const int j = (int)((l / P.g.n[0]) % P.g.n[1]);
-    const int k = (int)(l / ((long long)P.g.n[0] * P.g.n[1]));
-    const int c[3] = {i, j, k};
-    const double tt = seed_tt[(size_t)s * seedcap + q];
-    if (tt < EIK_INF) atomicMin(a.rs.nextmin + s, (unsigned long long)__double_as_longlong(tt));
-    const unsigned long long gbase = (unsigned long long)s * a.rs.stride;
+    int c[3];
+    node_coords(P.g, seed_lin[(size_t)s * seedcap + q], c);
+    const unsigned f = front_bits(fabs(seed_tt[(size_t)s * seedcap + q]));
+    if (f == PF_NONE) continue;
     for (int ax = 0; ax < ND; ax++)
       for (int d = -2; d <= 2; d++) {
         if (d == 0) continue;
         int p[3] = {c[0], c[1], c[2]};
         p[ax] += d;
         if (p[ax] < 0 || p[ax] >= P.g.n[ax]) continue;
-        list_node(a, 0, (unsigned int)(gbase + lin3(P.g, p[0], p[1], p[2])), tt);
+        const long long bn = brick_node<ND>(P.g, p[0], p[1], p[2]);
+        const size_t b = base + bn / B::NODES;
+        const int qn = (int)(bn % B::NODES);
+        atomicOr(bs.mask + b * B::WORDS + (qn >> 5), 1u << (qn & 31));
+        atomicMin(bs.front + b, f);
+        // pending of both colours: the visits of round 0 and (exam of round -1) of round 1
+        atomicMin(bs.marks + 3 * (size_t)a.nprob + s, f);
+        atomicMin(bs.exam + 3 * (size_t)a.nprob + s, f);
+        if (atomicExch(bs.listed + b, 1u) == 0u) {
+          const int col = (p[0] / B::BX + p[1] / B::BY + (ND == 3 ? p[2] / B::BZ : 0)) & 1;
+          bs.lists[(size_t)(2 * col) * bs.listcap + atomicAdd(bs.ctr + 2 * col, 1u)] = (unsigned)b;
+        }
       }
   }
 }
 
-#ifdef EIK_PHASE
-// tuning builds only: clock cycles per phase summed over warps (lane 0); 9..11: cycles of
-// the entry loads of a queue fill, and the counts of fill and evaluation steps
-__device__ unsigned long long eik_phase[12];
-extern "C" int eik_phase_read(unsigned long long* out) {
-  return (int)cudaMemcpyFromSymbol(out, eik_phase, sizeof(unsigned long long) * 12);
-}
-#define PH_T(v) const long long v = clock64()
-#define PH_ADD(k, t0) if ((threadIdx.x & 31) == 0) atomicAdd(&eik_phase[k], (unsigned long long)(clock64() - (t0)))
-#define PH_CNT(k) if ((threadIdx.x & 31) == 0) atomicAdd(&eik_phase[k], 1ull)
-#else
-#define PH_T(v)
-#define PH_ADD(k, t0)
-#define PH_CNT(k)
-#endif
-__device__ __forceinline__ double warp_min(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+// ---------------------------------------------------------------------- solve --
+__device__ __forceinline__ unsigned ld_vol(const unsigned* p) { return *(volatile const unsigned*)p; }
+
+// Threshold of problem p in round r: a window above its smallest pending front, which is the
+// smallest of what the last round's visits left, what the round before left on the other
+// colour, and what the last round put on other bricks. All three are complete when round r
+// starts and change again only after it.
+__device__ __forceinline__ float round_threshold(const BrickState& bs, int nprob, int p, int r, double delta) {
+  const unsigned* e1 = bs.exam + (size_t)((r + 3) & 3) * nprob;
+  const unsigned* e2 = bs.exam + (size_t)((r + 2) & 3) * nprob;
+  const unsigned* mk = bs.marks + (size_t)((r + 3) & 3) * nprob;
+  const float prev = __ldcg(bs.thr + (size_t)((r + 1) & 1) * nprob + p);
+  const unsigned m = min(min(__ldcg(e1 + p), __ldcg(e2 + p)), __ldcg(mk + p));
+  if (m == PF_NONE) return prev;
+  return fmaxf(prev, fminf(__double2float_ru((double)__uint_as_float(m) + delta), 3.402823466e38f));
 }
 
-__device__ __forceinline__ void atomic_min_pos(unsigned long long* p, double v) {
-  // traveltimes and potentials are >= 0: their bit patterns order as the values
-  if (v < EIK_INF && v < __longlong_as_double((long long)ld_volatile(p)))
-    atomicMin(p, (unsigned long long)__double_as_longlong(v));
-}
-
-// Forward coarse solve in rounds (one cooperative launch for all problems). Round r takes
-// the listed nodes; problem p only evaluates nodes whose potential (smallest neighbouring
-// traveltime) is at most T_p(r) = (smallest pending front of p after round r-1) + delta_p,
-// delta_p being about one node's traveltime at the largest velocity. The rounds thus
-// follow the front like a Dijkstra sweep with buckets one node wide. A node whose value or
-// key changed lists the nodes whose stencil reads it for the next round; a node below the
-// front is listed again. The result is the same fixed point as any other evaluation order.
-//
-// QUEUE selects how a warp works through its entries: true settles the visits whose front
-// still stands at once and queues the others in shared memory, evaluating them 32 at a time
-// (the lanes of a warp then run the long evaluation path together, and the later
-// evaluation sees more final neighbours); false evaluates each lane's entry in place. The
-// queue pays on large rounds; on small ones a warp left holding queued entries at the end
-// of a round keeps the others waiting at the barrier.
-//
-// MB is the number of resident CTAs per SM the register budget is sized for (4: 64
-// registers a thread, 3: 80, 2: 128); the launch's ctas_per_sm selects it. Fewer resident
-// warps with fewer spills pay on large launches, where every SM has work each round.
-template <int ND, bool QUEUE, int MB>
-__global__ void __launch_bounds__(SOLVE_THREADS, MB) coarse_rounds_kernel(SolveArgs a) {
-  const int lane = threadIdx.x & 31;
-  __shared__ unsigned long long wq[SOLVE_THREADS / 32][QUEUE ? 64 : 1];  // per-warp queue of entries to evaluate
-  __shared__ unsigned long long wv[SOLVE_THREADS / 32][8];  // per-warp visit counts by outcome
-  const unsigned long long N = a.rs.stride;  // node id = problem * stride + node
-  const unsigned N32 = (unsigned)N;            // node ids are 32-bit: so is the stride
-  unsigned long long* wvis = wv[threadIdx.x >> 5];
-  clear_visits(wvis, lane);
-#ifdef EIK_PHASE
-  VisitCount vk[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // lane cycles at 7..10: gates, node path, rule, relist filter
-#else
-  VisitCount* vk = nullptr;
-#endif
+template <int ND>
+__global__ void __launch_bounds__(BRICK_WARPS<ND> * 32, 1) brick_rounds_kernel(SolveArgs a) {
+  typedef Brick<ND> B;
+  extern __shared__ __align__(16) unsigned char brick_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  WarpMem<ND>& w = reinterpret_cast<WarpMem<ND>*>(brick_smem)[warp];
+  const BrickState bs = a.bs;
+  const unsigned nwarps = gridDim.x * BRICK_WARPS<ND>;
+  // consecutive entries go to different SMs
+  const unsigned gwarp = (unsigned)warp * gridDim.x + blockIdx.x;
+  VisitTally tally;
   int r = 0;
   for (; r < a.rs.max_rounds; r++) {
-    const int b3 = r % 3, nb3 = (r + 1) % 3;
-    const unsigned int n = *(volatile unsigned int*)(a.rs.cnt + b3);
-    if (n == 0) break;
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.activations, (unsigned long long)n);  // list entries
-    const unsigned long long* L = a.rs.list[r & 1];
-    unsigned long long* Lnext = a.rs.list[(r + 1) & 1];
-    const unsigned long long* nm = a.rs.nextmin + (size_t)b3 * a.nprob;
-    unsigned long long* nmn = a.rs.nextmin + (size_t)nb3 * a.nprob;
-    const double* thr_prev = a.rs.thr + (size_t)((r + 1) & 1) * a.nprob;  // thresholds of round r-1
-    double* thr_cur = a.rs.thr + (size_t)(r & 1) * a.nprob;
+    const int col = r & 1, ph = (r >> 1) & 1, nph = ph ^ 1, oph = ((r + 1) >> 1) & 1;
+    const unsigned n = ld_vol(bs.ctr + 2 * col + ph);
+    if (n == 0 && ld_vol(bs.ctr + 2 * (col ^ 1) + oph) == 0) break;  // no entry of either colour
+    unsigned* grab = bs.ctr + 4 + r % 3;
     if (blockIdx.x == 0)
       for (int p = threadIdx.x; p < a.nprob; p += blockDim.x)
-        thr_cur[p] = fmax(__ldcg(thr_prev + p), __longlong_as_double((long long)ld_volatile(nm + p)) + a.probs[p].delta);
-    if constexpr (QUEUE) {
-      // Visits whose front still stands (nothing they read has changed) are settled when
-      // taken; the others wait in a per-warp queue in shared memory and are evaluated 32 at a
-      // time, so that a warp's lanes run the long evaluation path together.
-      unsigned long long* q = wq[threadIdx.x >> 5];
-      int qn = 0;  // queued entries (warp-uniform)
-      bool more = true;
-      while (more || qn > 0) {
-        unsigned dirs = visit_code(VISIT_NONE);
-        double front = EIK_INF;
-        int prob = 0;
-        long long l = 0;
-        if (more && qn < 32) {
-          PH_T(tg);
-          unsigned int base = 0;
-          if (lane == 0) base = atomicAdd(a.rs.grab + b3, 32u);
-          base = __shfl_sync(0xffffffffu, base, 0);
-          PH_ADD(0, tg);
-          if (base >= n) {
-            more = false;
-            continue;
-          }
-          PH_T(tl);
-          PH_CNT(10);
-          const unsigned int idx = base + lane;
-          bool queue = false;
-          unsigned long long e = 0;
-          if (idx < n) {
-            e = __ldcg(L + idx);
-            const unsigned int gid = (unsigned int)(e >> 32);
-            const double ef = (double)__uint_as_float((unsigned int)e);
-            prob = (int)(gid / N32);
-            l = (long long)(gid - (unsigned long long)prob * N);
-            // threshold inputs and the dirty flag in one batch
-            const double tp = __ldcg(thr_prev + prob);
-            const unsigned long long nmv = ld_volatile(nm + prob);
-            const double del = a.probs[prob].delta;
-            const uint8_t dq = __ldcg(a.rs.dirty + gid);
-            const double T = fmax(tp, __longlong_as_double((long long)nmv) + del);
-            if (ef > T && ef < EIK_INF && !dq) {
-              front = ef;
-              dirs = (1u << DIR_SELF) | visit_code(VISIT_STANDS);
-            } else {
-              queue = true;
-            }
-          }
-          const unsigned qm = __ballot_sync(0xffffffffu, queue);
-          if (queue) q[qn + __popc(qm & ((1u << lane) - 1u))] = e;
-          qn += __popc(qm);
-          __syncwarp();
-          PH_ADD(9, tl);
-        } else {
-          PH_T(tp);
-          PH_CNT(11);
-          const int k = qn < 32 ? qn : 32;
-          if (lane < k) {
-            const unsigned long long e = q[qn - k + lane];
-            const unsigned int gid = (unsigned int)(e >> 32);
-            prob = (int)(gid / N32);
-            l = (long long)(gid - (unsigned long long)prob * N);
-            const CoarseProblem& P = a.probs[prob];
-            const double T = fmax(__ldcg(thr_prev + prob), __longlong_as_double((long long)ld_volatile(nm + prob)) + P.delta);
-            const unsigned long long gb = (unsigned long long)prob * N;
-            dirs = (ND == 3) ? process_node<3>(GlobalNodes{a, P, gb}, P, l, T, r, &front, vk)
-                             : process_node<2>(GlobalNodes{a, P, gb}, P, l, T, r, &front, vk);
-          }
-          qn -= k;
-          __syncwarp();
-          PH_ADD(1, tp);
-        }
-        count_visits(wvis, dirs, lane);
-        PH_T(ts);
-        // list the next round's nodes once each (per-node round stamps)
-        const CoarseProblem& P = a.probs[prob];
-        const unsigned long long gbase = (unsigned long long)prob * N;
-        unsigned keep = 0;
-        for (int k = 0; k <= DIR_SELF; k++) {
-          if (!((dirs >> k) & 1u)) continue;
-          const long long nl = dir_lin(P.g, l, k);
-          if (atomicExch(a.rs.stamp + gbase + nl, r + 1) != r + 1) keep |= 1u << k;
-        }
-        __syncwarp();
-        PH_ADD(2, ts);
-        PH_T(ta);
-        // warp-aggregated append: one atomic per 32 nodes
-        const int cntl = __popc(keep);
-        int incl = cntl;
-  #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        unsigned int wbase = 0;
-        if (lane == 0 && total) wbase = atomicAdd(a.rs.cnt + nb3, (unsigned int)total);
-        wbase = __shfl_sync(0xffffffffu, wbase, 0) + (unsigned int)(incl - cntl);
-        for (int k = 0; k <= DIR_SELF; k++) {
-          if (!((keep >> k) & 1u)) continue;
-          const long long nl = dir_lin(P.g, l, k);
-          Lnext[wbase++] = list_entry((unsigned int)(gbase + nl), front);
-        }
-        {
-          // one update per problem and warp: the lanes of a problem agree on their smallest front
-          const double fv = keep ? front : EIK_INF;
-          const unsigned grp = __match_any_sync(0xffffffffu, prob);
-          double gmin = fv;
-          for (unsigned m = grp; m; m &= m - 1) {
-            const int src = __ffs(m) - 1;
-            gmin = fmin(gmin, __shfl_sync(grp, fv, src));
-          }
-          if (lane == __ffs(grp) - 1) atomic_min_pos(nmn + prob, gmin);
-        }
-        __syncwarp();
-        PH_ADD(3, ta);
+        bs.thr[(size_t)(r & 1) * a.nprob + p] = round_threshold(bs, a.nprob, p, r, a.probs[p].delta);
+    const unsigned* L = bs.lists + (size_t)(2 * col + ph) * bs.listcap;
+    unsigned* Lkeep = bs.lists + (size_t)(2 * col + nph) * bs.listcap;
+    unsigned* Lother = bs.lists + (size_t)(2 * (col ^ 1) + oph) * bs.listcap;
+    // entries a warp takes at a time: one while a round has few, so that every warp gets some
+    const unsigned take = max(1u, min(8u, n / (4u * nwarps)));
+    unsigned base = gwarp * take;
+    while (base < n) {
+      unsigned b = 0;
+      unsigned f = PF_NONE;
+      float T = 0.0f;
+      int prob = 0;
+      const bool have = lane < take && base + lane < n;
+      if (have) {
+        b = __ldcg(L + base + lane);
+        f = __ldcg(bs.front + b);
+        prob = (int)(b / bs.stride);
+        T = round_threshold(bs, a.nprob, prob, r, a.probs[prob].delta);
       }
-    } else {
-      // every lane evaluates its own entry in place
-      for (;;) {
-        PH_T(tg);
-        unsigned int base = 0;
-        if (lane == 0) base = atomicAdd(a.rs.grab + b3, 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        PH_ADD(0, tg);
-        if (base >= n) break;
-        PH_T(tp);
-        const unsigned int idx = base + lane;
-        unsigned dirs = visit_code(VISIT_NONE);
-        double front = EIK_INF;
-        int prob = 0;
-        long long l = 0;
-        if (idx < n) {
-          const unsigned long long e = __ldcg(L + idx);
-          const unsigned int gid = (unsigned int)(e >> 32);
-          const double ef = (double)__uint_as_float((unsigned int)e);
-          prob = (int)(gid / N32);
-          l = (long long)(gid - (unsigned long long)prob * N);
-          const CoarseProblem& P = a.probs[prob];
-          // window of one round width above the smallest pending front, never moving back
-          // (its inputs and the dirty flag in one batch)
-          const double tp = __ldcg(thr_prev + prob);
-          const unsigned long long nmv = ld_volatile(nm + prob);
-          const double del = P.delta;
-          const uint8_t dq = __ldcg(a.rs.dirty + gid);
-          const double T = fmax(tp, __longlong_as_double((long long)nmv) + del);
-          const unsigned long long gb = (unsigned long long)prob * N;
-          if (ef > T && ef < EIK_INF && !dq) {
-            // still waiting and nothing it reads has changed: its front stands
-            front = ef;
-            dirs = (1u << DIR_SELF) | visit_code(VISIT_STANDS);
-          } else {
-            dirs = (ND == 3) ? process_node<3>(GlobalNodes{a, P, gb}, P, l, T, r, &front, vk)
-                             : process_node<2>(GlobalNodes{a, P, gb}, P, l, T, r, &front, vk);
+      const bool go = have && f <= __float_as_uint(T);
+      unsigned todo = __ballot_sync(FULL_WARP, go);
+      unsigned leftf = PF_NONE;  // per entry: smallest front still pending after this round
+      if (have && !go) leftf = f;
+      while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const unsigned vb = __shfl_sync(FULL_WARP, b, src);
+        const int vp = __shfl_sync(FULL_WARP, prob, src);
+        const float vT = __shfl_sync(FULL_WARP, T, src);
+        const CoarseProblem& P = a.probs[vp];
+        const unsigned lb = vb - (unsigned)vp * bs.stride;
+        const int nb[3] = {bricks_along<ND>(P.g, 0), bricks_along<ND>(P.g, 1),
+                           ND == 3 ? bricks_along<ND>(P.g, 2) : 1};
+        const int bc[3] = {(int)(lb % nb[0]), (int)((lb / nb[0]) % nb[1]), (int)(lb / ((unsigned)nb[0] * nb[1]))};
+        const unsigned left = visit_brick<ND>(w, bs, P, vb, bc, nb, vT, lane, tally);
+        if (lane == src) leftf = left;
+        if (lane == 0) {
+          bs.front[vb] = left;
+          if (left == PF_NONE) bs.listed[vb] = 0u;
+        }
+        // the bricks across the faces: pending bits, front, and a place in the other colour's list
+        __syncwarp();
+#pragma unroll
+        for (int q0 = 0; q0 < B::FACES * B::WORDS; q0 += 32) {
+          const int q = q0 + lane;
+          const unsigned bits = w.face[q];
+          if (bits) {
+            const int fc = q / B::WORDS, ax = fc >> 1;
+            const int st = ax == 0 ? 1 : (ax == 1 ? nb[0] : nb[0] * nb[1]);
+            const unsigned ob = (fc & 1) ? vb - st : vb + st;
+            atomicOr(bs.mask + (size_t)ob * B::WORDS + q % B::WORDS, bits);
           }
         }
-        __syncwarp();
-        PH_ADD(1, tp);
-        count_visits(wvis, dirs, lane);
-        PH_T(ts);
-        // list the next round's nodes once each (per-node round stamps)
-        const CoarseProblem& P = a.probs[prob];
-        const unsigned long long gbase = (unsigned long long)prob * N;
-        unsigned keep = 0;
-        for (int k = 0; k <= DIR_SELF; k++) {
-          if (!((dirs >> k) & 1u)) continue;
-          const long long nl = dir_lin(P.g, l, k);
-          if (atomicExch(a.rs.stamp + gbase + nl, r + 1) != r + 1) keep |= 1u << k;
+        if (lane < B::FACES && w.facemin[lane] != PF_NONE) {
+          const int ax = lane >> 1;
+          const int st = ax == 0 ? 1 : (ax == 1 ? nb[0] : nb[0] * nb[1]);
+          const unsigned ob = (lane & 1) ? vb - st : vb + st;
+          const unsigned fm = w.facemin[lane];
+          atomicMin(bs.front + ob, fm);
+          atomicMin(bs.marks + (size_t)(r & 3) * a.nprob + vp, fm);
+          if (atomicExch(bs.listed + ob, 1u) == 0u)
+            Lother[atomicAdd(bs.ctr + 2 * (col ^ 1) + oph, 1u)] = ob;
         }
         __syncwarp();
-        PH_ADD(2, ts);
-        PH_T(ta);
-        // warp-aggregated append: one atomic per 32 nodes
-        const int cntl = __popc(keep);
-        int incl = cntl;
-  #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        unsigned int wbase = 0;
-        if (lane == 0 && total) wbase = atomicAdd(a.rs.cnt + nb3, (unsigned int)total);
-        wbase = __shfl_sync(0xffffffffu, wbase, 0) + (unsigned int)(incl - cntl);
-        for (int k = 0; k <= DIR_SELF; k++) {
-          if (!((keep >> k) & 1u)) continue;
-          const long long nl = dir_lin(P.g, l, k);
-          Lnext[wbase++] = list_entry((unsigned int)(gbase + nl), front);
-        }
-        {
-          // one update per problem and warp: the lanes of a problem agree on their smallest front
-          const double fv = keep ? front : EIK_INF;
-          const unsigned grp = __match_any_sync(0xffffffffu, prob);
-          double gmin = fv;
-          for (unsigned m = grp; m; m &= m - 1) {
-            const int src = __ffs(m) - 1;
-            gmin = fmin(gmin, __shfl_sync(grp, fv, src));
-          }
-          if (lane == __ffs(grp) - 1) atomic_min_pos(nmn + prob, gmin);
-        }
-        __syncwarp();
-        PH_ADD(3, ta);
       }
+      // entries with something pending stay listed for their colour's next round
+      const bool keep = have && leftf != PF_NONE;
+      const unsigned km = __ballot_sync(FULL_WARP, keep);
+      if (km) {
+        unsigned at = 0;
+        if (lane == __ffs(km) - 1) at = atomicAdd(bs.ctr + 2 * col + nph, (unsigned)__popc(km));
+        at = __shfl_sync(FULL_WARP, at, __ffs(km) - 1);
+        if (keep) {
+          Lkeep[at + __popc(km & ((1u << lane) - 1u))] = b;
+          atomicMin(bs.exam + (size_t)(r & 3) * a.nprob + prob, leftf);
+        }
+      }
+      if (lane == 0) base = nwarps * take + atomicAdd(grab, take);
+      base = __shfl_sync(FULL_WARP, base, 0);
     }
-    // buffers of round r+2 (last used in round r-1)
+    // buffers that round r + 1 appends to or accumulates in (last read in round r - 1)
     if (blockIdx.x == 0) {
-      const int c3 = (r + 2) % 3;
       if (threadIdx.x == 0) {
-        a.rs.cnt[c3] = 0;
-        a.rs.grab[c3] = 0;
+        bs.ctr[2 * (col ^ 1) + (oph ^ 1)] = 0u;
+        bs.ctr[4 + (r + 2) % 3] = 0u;
       }
-      for (int p = threadIdx.x; p < a.nprob; p += blockDim.x)
-        a.rs.nextmin[(size_t)c3 * a.nprob + p] = (unsigned long long)__double_as_longlong(EIK_INF);
+      for (int p = threadIdx.x; p < a.nprob; p += blockDim.x) {
+        bs.exam[(size_t)((r + 1) & 3) * a.nprob + p] = PF_NONE;
+        bs.marks[(size_t)((r + 1) & 3) * a.nprob + p] = PF_NONE;
+      }
     }
-    PH_T(tb);
     if (!grid_barrier(a)) break;
-    PH_ADD(4, tb);
   }
-  flush_visits(wvis, a.rs.visits, a.node_evals, lane);
-#ifdef EIK_PHASE
-  for (int k = 7; k < 11; k++) atomicAdd(&eik_phase[k - 2], vk[k]);  // per lane
-#endif
+  if (lane < 7 && tally.n) {
+    atomicAdd(a.rs.visits + lane, (unsigned long long)tally.n);
+    atomicAdd(a.activations, (unsigned long long)tally.n);
+  }
+  const unsigned evals = __shfl_sync(FULL_WARP, tally.n, VISIT_WAIT) + __shfl_sync(FULL_WARP, tally.n, VISIT_SAME) +
+                         __shfl_sync(FULL_WARP, tally.n, VISIT_CHANGED);
+  if (lane == 0 && evals) atomicAdd(a.node_evals, (unsigned long long)evals);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *a.rs.rounds = r;
     if (r >= a.rs.max_rounds) {
       atomicOr(a.err, ERRB_NOT_CONVERGED);
       atomicExch(a.abort_flag, 1);
+    }
+  }
+}
+
+// Results in the problems' own arrays: column-major traveltimes, and codes with bit 7 for a
+// special key.
+template <int ND>
+__global__ void bricks_store_kernel(SolveArgs a) {
+  typedef Brick<ND> B;
+  for (int p = blockIdx.y; p < a.nprob; p += gridDim.y) {
+    const CoarseProblem& P = a.probs[p];
+    const GridDesc& g = P.g;
+    const size_t base = (size_t)p * a.bs.stride * B::NODES;
+    const unsigned long long N = (unsigned long long)npts(g);
+    for (unsigned long long l = blockIdx.x * blockDim.x + threadIdx.x; l < N; l += gridDim.x * blockDim.x) {
+      int c[3];
+      node_coords(g, (long long)l, c);
+      const size_t q = base + brick_node<ND>(g, c[0], c[1], c[2]);
+      const double t = a.bs.t[q];
+      P.t[l] = fabs(t);
+      P.code[l] = (uint8_t)((a.bs.code[q] & 0x7f) | (sign_set(t) ? CODE_SRC_BIT : 0));
     }
   }
 }
@@ -462,51 +318,47 @@ __global__ void picks_kernel(GridDesc g, const double* t, long long N, int nsrc,
 }
 
 // ------------------------------------------------------------------ launchers --
-void launch_coarse_init(const CoarseProblem* hprobs, const CoarseProblem* dprobs, int nprob,
-                        const ForwardBatch& fb, const SolveArgs& sa, cudaStream_t st) {
-  (void)hprobs;
-  // every problem's first stride nodes: its grid, and the padding up to the call's largest grid
-  coarse_init_kernel<<<1184, 256, 0, st>>>(dprobs, nprob, (long long)sa.rs.stride);
-  rounds_init_kernel<<<296, 256, 0, st>>>(sa);
-  launch_rounds_seed(sa, fb.seed_lin, fb.seed_tt, fb.out, false, fb.seedcap, st);
+unsigned long long brick_nodes(const GridDesc& g) {
+  return g.nd == 3 ? (unsigned long long)brick_count<3>(g) * Brick<3>::NODES
+                   : (unsigned long long)brick_count<2>(g) * Brick<2>::NODES;
 }
 
-void launch_rounds_init(const SolveArgs& sa, cudaStream_t st) { rounds_init_kernel<<<296, 256, 0, st>>>(sa); }
+void launch_bricks_init(const SolveArgs& sa, cudaStream_t st) {
+  solve_counters_kernel<<<1, 32, 0, st>>>(sa);
+  const int nodes = sa.nd == 3 ? Brick<3>::NODES : Brick<2>::NODES;
+  bricks_init_kernel<<<1184, 256, 0, st>>>(sa.bs, (unsigned)sa.nprob, nodes, nodes / 32);
+}
 
-void launch_rounds_seed(const SolveArgs& sa, const int32_t* seed_lin, const double* seed_tt, const SrcOut* out,
+void launch_bricks_seed(const SolveArgs& sa, const int32_t* seed_lin, const double* seed_tt, const SrcOut* out,
                         bool fine_corners, int seedcap, cudaStream_t st) {
   if (sa.nd == 3) seed_kernel<3><<<sa.nprob, 128, 0, st>>>(sa, seed_lin, seed_tt, out, fine_corners ? 1 : 0, seedcap);
   else seed_kernel<2><<<sa.nprob, 128, 0, st>>>(sa, seed_lin, seed_tt, out, fine_corners ? 1 : 0, seedcap);
 }
 
-template <int ND, bool QUEUE, int MB>
-static cudaError_t launch_solve_mb(const SolveArgs& sa, int nsm, int ctas_per_sm, cudaStream_t st) {
-  const size_t sm = 0;
-  int per = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, coarse_rounds_kernel<ND, QUEUE, MB>, SOLVE_THREADS, sm);
-  if (ctas_per_sm > 0 && ctas_per_sm < per) per = ctas_per_sm;
-  per = per < 1 ? 1 : per;
+template <int ND>
+static cudaError_t launch_bricks_solve_nd(const SolveArgs& sa, int nsm, cudaStream_t st) {
+  const size_t sm = sizeof(WarpMem<ND>) * BRICK_WARPS<ND>;
+  cudaError_t e = cudaFuncSetAttribute(brick_rounds_kernel<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
   SolveArgs args = sa;
   void* kargs[] = {&args};
   // cooperative: every CTA is resident, so the grid barrier between rounds cannot deadlock
-  return cudaLaunchCooperativeKernel((const void*)coarse_rounds_kernel<ND, QUEUE, MB>, dim3(nsm * per),
-                                     dim3(SOLVE_THREADS), kargs, sm, st);
+  return cudaLaunchCooperativeKernel((const void*)brick_rounds_kernel<ND>, dim3(nsm), dim3(BRICK_WARPS<ND> * 32),
+                                     kargs, sm, st);
 }
 
-template <int ND, bool QUEUE>
-static cudaError_t launch_solve_nd(const SolveArgs& sa, int nsm, int ctas_per_sm, cudaStream_t st) {
-  // 2 and 3 resident CTAs per SM take the register budget of that residency; else 4
-  if (ctas_per_sm == 2) return launch_solve_mb<ND, QUEUE, 2>(sa, nsm, ctas_per_sm, st);
-  if (ctas_per_sm == 3) return launch_solve_mb<ND, QUEUE, 3>(sa, nsm, ctas_per_sm, st);
-  return launch_solve_mb<ND, QUEUE, 4>(sa, nsm, ctas_per_sm, st);
+cudaError_t launch_bricks_solve(const SolveArgs& sa, int nsm, cudaStream_t st) {
+  return sa.nd == 3 ? launch_bricks_solve_nd<3>(sa, nsm, st) : launch_bricks_solve_nd<2>(sa, nsm, st);
 }
 
-cudaError_t launch_coarse_solve(const SolveArgs& sa, int nsm, int ctas_per_sm, int queue, cudaStream_t st) {
-  // automatic choice: the queue from 2^27 node-sources per launch (256^3 x 8 sources) up
-  const bool q = queue > 0 || (queue < 0 && (unsigned long long)sa.nprob * sa.rs.stride >= (1ull << 27));
-  if (sa.nd == 3)
-    return q ? launch_solve_nd<3, true>(sa, nsm, ctas_per_sm, st) : launch_solve_nd<3, false>(sa, nsm, ctas_per_sm, st);
-  return q ? launch_solve_nd<2, true>(sa, nsm, ctas_per_sm, st) : launch_solve_nd<2, false>(sa, nsm, ctas_per_sm, st);
+void launch_bricks_store(const SolveArgs& sa, cudaStream_t st) {
+  // blocks per problem: enough in all to fill the GPU, no more than a problem has nodes for
+  const unsigned long long nodes = (unsigned long long)sa.bs.stride * (sa.nd == 3 ? Brick<3>::NODES : Brick<2>::NODES);
+  const unsigned want = (unsigned)((nodes + 1023) / 1024);
+  const unsigned per = std::max(1u, std::min(want, std::max(8u, 2368u / (unsigned)sa.nprob)));
+  const dim3 grid(per, std::min(65535u, (unsigned)sa.nprob));
+  if (sa.nd == 3) bricks_store_kernel<3><<<grid, 256, 0, st>>>(sa);
+  else bricks_store_kernel<2><<<grid, 256, 0, st>>>(sa);
 }
 
 void launch_picks(const GridDesc& g, const double* t, long long N, int nsrc, const long long* recoff,

@@ -479,6 +479,8 @@ __global__ void fine_setup_kernel(ForwardBatch fb, CoarseProblem* fprobs, const 
   if (nfine > fb.nfmax) {
     atomicOr(fb.err, ERRB_HEAP_OVERFLOW);
     o.nsrcf = 0;
+    fprobs[s].g = g;  // a problem without nodes
+    for (int d = 0; d < 3; d++) fprobs[s].g.n[d] = 0;
     return;
   }
   const double* vel = fb.vel;
@@ -513,6 +515,8 @@ __global__ void fine_setup_kernel(ForwardBatch fb, CoarseProblem* fprobs, const 
   uniform_coeffs(gf, &P.c1u, &P.c2u);
   P.delta = gate * hmin * smin;
   P.incmin = 0.999 * (2.0 / 3.0) * hmin * smin / sqrt((double)gf.nd);
+  P.linc = 0.999 * (2.0 / 3.0) * hmin / sqrt((double)gf.nd);
+  P.din = inner_window(gf.nd, hmin * smin);
 }
 
 __global__ void fine_fill_kernel(ForwardBatch fb, const CoarseProblem* fprobs) {
@@ -527,9 +531,6 @@ __global__ void fine_fill_kernel(ForwardBatch fb, const CoarseProblem* fprobs) {
     const FineInfo& fi = fb.out[s].fine;
     const int i = (int)(l % gf.n[0]), j = (int)((l / gf.n[0]) % gf.n[1]), k = (int)(l / ((long long)gf.n[0] * gf.n[1]));
     const_cast<double*>(P.slow)[l] = fb.slow[fine_to_coarse(fb.g, fi, i, j, k)];
-    P.t[l] = EIK_INF;
-    P.code[l] = CODE_NONE;
-    P.kd[l] = 0;
     const size_t o = (size_t)s * fb.nfmax + l;
     fb.fine_status[o] = 0;
     fb.fine_onh[o] = 0;

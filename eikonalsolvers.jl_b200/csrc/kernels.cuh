@@ -63,6 +63,8 @@ struct CoarseProblem {
   uint8_t* kd;     // key depth of special nodes
   double delta;    // round width of the forward solve (traveltime units)
   double incmin;   // smallest increment of the local update over a neighbour: (2/3) h s_min / sqrt(nd)
+  double linc;     // the same per unit of slowness: (2/3) h / sqrt(nd), h the smallest spacing
+  float din;       // inner window of a brick visit (traveltime units)
   double c1u, c2u; // Cartesian grids: the local solver's coefficients 1/h^2 and 9/(4h^2); 0 otherwise
 };
 
@@ -78,22 +80,38 @@ EIK_HD void uniform_coeffs(const GridDesc& g, double* c1u, double* c2u) {
   }
 }
 
-// Worklists and thresholds of the round-synchronous forward solve. Nodes are numbered
-// globally over the problems of a call: problem * N + node.
+// Counters of the round-synchronous solves, and the worklists of the adjoint sweep, whose
+// nodes are numbered over the problems of a call: problem * N + node.
 struct RoundState {
-  int32_t* stamp;               // per node: last round it was listed for
-  double* tent;                 // per node: value of its last evaluation
-  uint8_t* dirty;               // per node: something it reads changed since that evaluation
-  unsigned long long* list[2];  // entries of the current and the next round (node id << 32 | front)
+  int32_t* stamp;               // adjoint, per node: dependants not final yet
+  unsigned long long* list[2];  // adjoint: entries of the current and the next round (node id << 32)
   unsigned int* cnt;            // [3] list length per round (mod 3)
   unsigned int* grab;           // [3] next list entry to take per round (mod 3)
-  unsigned long long* nextmin;  // [3][nprob] smallest pending potential (double bits)
-  double* thr;                  // [2][nprob] threshold of the previous / current round
   unsigned int* bar;            // [2] grid barrier: arrivals, generation
-  unsigned long long stride;    // node ids: problem * stride + node
   int32_t* rounds;              // rounds run
   unsigned long long* visits;   // [7] outcomes of the forward's list visits
   int32_t max_rounds;
+};
+
+// Inner window of a brick visit: the nodes evaluated together lie within this much of the
+// brick's smallest pending front. Narrower windows re-evaluate fewer nodes, wider ones fill
+// more lanes of a step; u is the least time across one node (smallest spacing x slowness).
+EIK_HD float inner_window(int nd, double u) { return (float)((nd == 3 ? 0.5 : 1.0) * u); }
+
+// State of the forward solve by bricks (brick.cuh): problem p's bricks are p * stride + b.
+struct BrickState {
+  double* t;            // traveltimes in brick order; sign bit: special key
+  uint8_t* code;        // derivative codes in brick order (low 7 bits)
+  unsigned* mask;       // pending nodes of each brick, one bit a node
+  unsigned* front;      // smallest pending front of each brick (float bits)
+  unsigned* listed;     // brick is in a list
+  unsigned* lists;      // [colour*2+phase][listcap]: bricks to visit
+  size_t listcap;
+  unsigned* ctr;        // cnt[colour*2+phase] at 0..3, grab[round % 3] at 4..6
+  unsigned* exam;       // [4][nprob] smallest front left by a round's visits (float bits)
+  unsigned* marks;      // [4][nprob] smallest front a round's visits put on other bricks
+  float* thr;           // [2][nprob] threshold of the previous / current round
+  unsigned stride;      // bricks per problem (the call's largest grid)
 };
 
 struct SolveArgs {
@@ -107,6 +125,7 @@ struct SolveArgs {
   int32_t* abort_flag;
   long long timeout_ns;
   RoundState rs;
+  BrickState bs;
 };
 
 
@@ -114,12 +133,15 @@ struct SolveArgs {
 void launch_srcbox(const ForwardBatch& fb, cudaStream_t st);
 void launch_fine(const ForwardBatch& fb, cudaStream_t st);
 size_t fine_smem_bytes(int heapcap);
-void launch_coarse_init(const CoarseProblem* hprobs, const CoarseProblem* dprobs, int nprob,
-                        const ForwardBatch& fb, const SolveArgs& sa, cudaStream_t st);
-// Round-solver state reset, and seeding from per-problem seed lists (fixed values).
-void launch_rounds_init(const SolveArgs& sa, cudaStream_t st);
-void launch_rounds_seed(const SolveArgs& sa, const int32_t* seed_lin, const double* seed_tt, const SrcOut* out,
+// Brick state reset, seeding from per-problem seed lists (fixed values), the solve, and the
+// results in the problems' own arrays (column-major traveltimes and codes).
+void launch_bricks_init(const SolveArgs& sa, cudaStream_t st);
+void launch_bricks_seed(const SolveArgs& sa, const int32_t* seed_lin, const double* seed_tt, const SrcOut* out,
                         bool fine_corners, int seedcap, cudaStream_t st);
+cudaError_t launch_bricks_solve(const SolveArgs& sa, int nsm, cudaStream_t st);
+void launch_bricks_store(const SolveArgs& sa, cudaStream_t st);
+// Nodes of a grid's bricks (the grid rounded up to whole bricks).
+unsigned long long brick_nodes(const GridDesc& g);
 // Refined start-up as a fixed point: window set-up, the fine problems' arrays, the
 // acceptance set at the reference's stop, and the exact heap replay for the sources
 // whose stop is decided by a tie (flags in fine_tie, nonzero = replay needed).
@@ -128,9 +150,6 @@ void launch_fine_setup(const ForwardBatch& fb, CoarseProblem* fprobs, const doub
                        cudaStream_t st);
 void launch_fine_select(const ForwardBatch& fb, const CoarseProblem* fprobs, uint8_t* fine_tie, cudaStream_t st);
 void launch_fine_replay(const ForwardBatch& fb, const uint8_t* fine_tie, cudaStream_t st);
-// ctas_per_sm: resident CTAs per SM of the persistent launch (0 = as many as fit);
-// queue: per-warp evaluation queue 1 = on, 0 = off, -1 = chosen by the launch's size
-cudaError_t launch_coarse_solve(const SolveArgs& sa, int nsm, int ctas_per_sm, int queue, cudaStream_t st);
 // The forward solve of small problems (every problem at most nmax nodes), one thread-block
 // cluster per problem with its state in distributed shared memory, seeds and counters
 // included (it replaces round init, seeding and launch_coarse_solve). *used = false when no

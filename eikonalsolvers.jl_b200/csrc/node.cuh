@@ -102,26 +102,6 @@ __device__ __forceinline__ long long dir_lin(const GridDesc& g, long long l, int
   return l + dir_off(k) * st;
 }
 
-// The round-solver state of problem P in global memory: node l at l (problem arrays) and at
-// gb + l (round-solver arrays, numbered over the problems of a launch).
-struct GlobalNodes {
-  const SolveArgs& a;
-  const CoarseProblem& P;
-  unsigned long long gb;
-  __device__ __forceinline__ uint8_t dirty(long long l) const { return __ldcg(a.rs.dirty + gb + l); }
-  __device__ __forceinline__ void set_dirty(long long l, uint8_t v) const { a.rs.dirty[gb + l] = v; }
-  __device__ __forceinline__ double tent(long long l) const { return __ldcg(a.rs.tent + gb + l); }
-  __device__ __forceinline__ void set_tent(long long l, double v) const { a.rs.tent[gb + l] = v; }
-  __device__ __forceinline__ uint8_t code(long long l) const { return __ldcg(P.code + l); }
-  __device__ __forceinline__ void set_code(long long l, uint8_t v) const { P.code[l] = v; }
-  __device__ __forceinline__ double t(long long l) const { return __ldcg(P.t + l); }
-  __device__ __forceinline__ void set_t(long long l, double v) const { P.t[l] = v; }
-  __device__ __forceinline__ int32_t stamp(long long l) const {
-    return *(volatile const int32_t*)(a.rs.stamp + gb + l);
-  }
-  __device__ __forceinline__ void fence() const { __threadfence(); }
-};
-
 // The order rule on a neighbourhood with special keys (source points, non-causal
 // acceptances), from the full keys of the immediate and distance-2 neighbours. Kept out of
 // line because it is rare; its inputs and outputs go by value, so that no array of the visit

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <string>
@@ -155,9 +156,9 @@ struct eik_ctx {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // whole call
   cudaEvent_t evk[6] = {};                    // start-up stage, coarse solve, adjoint solve
-  double round_gate = 0.0;  // forward round width in units of (smallest spacing x smallest slowness); 0 = by size
-  int ctas_per_sm = 0;       // resident CTAs per SM of the forward solve (0 = as many as fit)
-  int fwd_queue = -1;        // per-warp evaluation queue of the forward solve: -1 by size, 0 off, 1 on
+  double round_gate = 0.0;  // forward round width in units of (smallest spacing x smallest slowness); 0 = gate_for
+  int ctas_per_sm = 0;       // accepted, without effect (the forward solve has one CTA per SM)
+  int fwd_queue = -1;        // accepted, without effect
   int cluster_solve = 1;     // small problems in one thread-block cluster each: 1 in 2D, 2 in any dimension, 0 never
   int max_rounds = 0;        // round limit of the persistent solves (0 = the library's, see forward_multi)
   int retry = 0;             // a pipeline run again after the automatic round limit: wider rounds, limit 2^24
@@ -165,18 +166,24 @@ struct eik_ctx {
   double sm_fraction = 0.0; // share of the SMs the persistent (cooperative) solves use; 0 = by size
   double ray_room = 3.0;     // room of a ray in its first tracing pass, in straight-line lengths
   bool fine_replay = false; // refined start-up by exact heap replay for every source (else only on ties)
-  // Launch parameters of a call whose coarse solve has `work` node-sources: the values set
-  // on the context, else chosen by size. Small calls are bound by their rounds (each closed
-  // by a grid barrier over all resident CTAs), so they take wider rounds on fewer SMs.
-  static constexpr unsigned long long SMALL_WORK = 1ull << 22;
-  double gate_for(unsigned long long work) const {
-    const double g = round_gate > 0.0 ? round_gate : (work < SMALL_WORK ? 8.0 : 2.0);
+  // Round width of a call: the value set on the context, else by dimension (bricks: 128^3 x 8
+  // 2 / 4 / 6: 101 / 99 / 102 ms, 1024x640 x 64 4 / 8 / 16: 68 / 63 / 57 ms; flat around these).
+  double gate_for(int nd) const {
+    const double g = round_gate > 0.0 ? round_gate : (nd == 2 ? 8.0 : 6.0);
     return retry ? 1.5 * g : g;
   }
+  // SMs of the adjoint sweep of a call of `work` node-sources: small ones are bound by their
+  // rounds (each closed by a grid barrier over all resident CTAs) and take fewer.
+  static constexpr unsigned long long SMALL_WORK = 1ull << 22;
   int sms_for(unsigned long long work) const {
     const double f = sm_fraction > 0.0 ? sm_fraction : (work < SMALL_WORK ? 0.25 : 1.0);
     const int n = (int)(f * (double)nsm + 0.5);
     return n < 1 ? 1 : (n > nsm ? nsm : n);
+  }
+  // SMs of a forward solve over `bricks` bricks: a round visits one colour, so at most half.
+  int brick_sms(unsigned long long bricks) const {
+    const int cap = sm_fraction > 0.0 ? std::max(1, std::min(nsm, (int)(sm_fraction * (double)nsm + 0.5))) : nsm;
+    return (int)std::max<unsigned long long>(1, std::min<unsigned long long>(cap, (bricks + 1) / 2));
   }
   std::mutex mu;
   eik::Scratch scratch;

@@ -378,6 +378,198 @@ EIK_HD double prefix_rule_plain(const NbhdT& nb, int8_t* codes, Key* key_out, bo
   return EIK_INF;
 }
 
+// Fast form of the order rule: the value, codes and key (v, 0, v) of prefix_rule, bit for bit,
+// or false where it leaves the decision to the general rule. Traveltimes are +inf where the
+// neighbour is outside the grid, unreached or (t2) not allowed; c1, c2 are 1/h^2 and 9/(4h^2)
+// per axis. LEVELS: some neighbour has a special key, and L1, L2 hold the key levels (the
+// traveltime of an ordinary one); without it they are not read.
+//
+// An axis contributes through one side only, from the moment that side is accepted (its level),
+// so at most ND groups change the update. Whether the update of a group exceeds a later level
+// tn is the sign of q(tn) = sum ca (tn - x_a)^2 - slow^2 there (q < 0 strictly between the
+// roots of the quadratic; a group's own level has q < 0, so a later tn with q > 0 lies above
+// the larger root), which needs neither the square root nor the division: those, a chain of
+// dependent FP64 steps, run once per node instead of once per group. q is compared with a
+// margin far above its own rounding and the root's (an error of the root of about
+// eps alpha^(1/2) t^2 / slow, from the cancellation in beta^2 - 4 alpha gamma, moves q by
+// about eps alpha t^2; the margin takes 64 times that), so the decisions are those of the exact
+// values; inside the margin the general rule decides. Equal levels of different depth count as
+// one group: the groups between them are all continued when the last is (q only grows with
+// another axis).
+//
+// Mixed sides: an axis whose side 1 is the smaller and 1st order takes side 0's 2nd-order point
+// from the moment side 0 is accepted (the reference keeps it when side 1 replaces side 0, unless
+// side 1's own distance-2 node is accepted by then). When
+// that happens before the node's own acceptance on one axis, the groups from side 0's
+// traveltime on are decided again with the axis' new point.
+//
+// Left to the general rule: a value not above its group (non-causal), a negative discriminant,
+// mixed sides on several axes. With levels, also: source points; an axis with a special key
+// whose other side is accepted before the node; a 2nd-order point accepted after its 1st-order
+// one and before the node.
+template <int ND, bool LEVELS>
+EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2], const double (&L1)[ND][2],
+                             const double (&L2)[ND][2], const double (&c1)[ND], const double (&c2)[ND], double slow,
+                             double* v_out, int8_t* codes) {
+  const double s2 = slow * slow;
+  double m[ND], x[ND], ca[ND], lev[ND], mar = 0.0;
+  uint32_t second = 0u, side = 0u, late = 0u, keyed = 0u;
+  bool ok = true;
+  double first = EIK_INF;
+#pragma unroll
+  for (int a = 0; a < ND; a++) {
+    bool hi = t1[a][1] < t1[a][0];
+    if (LEVELS) {
+      const bool sp = L1[a][0] != t1[a][0] || L1[a][1] != t1[a][1] || L2[a][0] != t2[a][0] || L2[a][1] != t2[a][1];
+      if (sp) {
+        hi = L1[a][1] < L1[a][0];
+        keyed |= 1u << a;
+        const double lo = hi ? L1[a][1] : L1[a][0];
+        if (!(lo > -EIK_INF) || (L1[a][0] == L1[a][1] && lo < EIK_INF)) ok = false;
+      }
+    }
+    m[a] = hi ? t1[a][1] : t1[a][0];
+    const double p2 = hi ? t2[a][1] : t2[a][0];
+    lev[a] = LEVELS ? (hi ? L1[a][1] : L1[a][0]) : m[a];
+    bool u2 = p2 <= m[a] && m[a] < EIK_INF;
+    if (LEVELS) {
+      const double l2 = hi ? L2[a][1] : L2[a][0];
+      if (u2 && (l2 > lev[a] || (l2 == lev[a] && l2 != p2))) {  // at an equal level the depth decides
+        u2 = false;
+        late |= 1u << a;
+      }
+    }
+    x[a] = u2 ? (1.0 / 3.0) * (4.0 * m[a] - p2) : m[a];
+    ca[a] = u2 ? c2[a] : c1[a];
+    if (u2) second |= 1u << a;
+    if (hi) side |= 1u << a;
+    first = lev[a] < first ? lev[a] : first;
+    mar += c2[a];
+  }
+  mar *= 7.0e-15;
+#pragma unroll
+  for (int a = 0; a < ND; a++) codes[a] = 0;
+  if (!(first < EIK_INF)) {
+    *v_out = EIK_INF;
+    return ok;
+  }
+  // the axes in the order of their acceptance: group k is the first k of them
+  double sm[ND], sx[ND], sc[ND];
+#pragma unroll
+  for (int a = 0; a < ND; a++) {
+    sm[a] = lev[a];
+    sx[a] = x[a];
+    sc[a] = ca[a];
+  }
+#pragma unroll
+  for (int pass = 0; pass < ND - 1; pass++)
+#pragma unroll
+    for (int a = 0; a < ND - 1 - pass; a++) {
+      const bool sw = sm[a + 1] < sm[a];
+      const double tm = sm[a], tx = sx[a], tc = sc[a];
+      sm[a] = sw ? sm[a + 1] : tm;
+      sx[a] = sw ? sx[a + 1] : tx;
+      sc[a] = sw ? sc[a + 1] : tc;
+      sm[a + 1] = sw ? tm : sm[a + 1];
+      sx[a + 1] = sw ? tx : sx[a + 1];
+      sc[a + 1] = sw ? tc : sc[a + 1];
+    }
+  // straight-line: lanes of a warp end at different groups
+  double d = sm[0] - sx[0];
+  double q = sc[0] * (d * d);  // q + slow^2 of the group at its own level
+  ok = ok && q < s2 - (1e-9 * s2 + mar * (sm[0] * sm[0]));  // else the value may not lie above it
+  bool open = true;
+  double tg = sm[0];
+#pragma unroll
+  for (int g = 1; g < ND; g++) {
+    q = 0.0;
+#pragma unroll
+    for (int a = 0; a < g; a++) {
+      d = sm[g] - sx[a];
+      q = fma(sc[a], d * d, q);
+    }
+    const double band = 1e-9 * s2 + mar * (sm[g] * sm[g]);
+    open = open && sm[g] < EIK_INF && !(q > s2 + band);  // q above: the value is below group g, accepted
+    d = sm[g] - sx[g];
+    q = fma(sc[g], d * d, q);  // with axis g itself, at its own level
+    ok = ok && (!open || q < s2 - band);
+    tg = open ? sm[g] : tg;
+  }
+  auto root = [&](double* v) {
+    double alpha = 0.0, beta = 0.0, gamma = -s2;
+#pragma unroll
+    for (int a = 0; a < ND; a++) {
+      const bool in = lev[a] <= tg;
+      const double xa = in ? x[a] : 0.0, aa = in ? ca[a] : 0.0;
+      alpha += aa;  // an axis left out adds zero, which changes no bit
+      beta += (-2.0 * aa) * xa;
+      gamma += aa * (xa * xa);
+    }
+    const double sq = beta * beta - (4.0 * alpha) * gamma;
+    *v = (-beta + sqrt(sq)) / (2.0 * alpha);
+    return sq >= 0.0;
+  };
+  double v;
+  ok = root(&v) && ok;
+  uint32_t mixed = 0u;
+#pragma unroll
+  for (int a = 0; a < ND; a++) {
+    if ((((side & ~second) >> a) & 1u) && t1[a][0] < v && t2[a][0] <= t1[a][0] && t2[a][1] > t1[a][0])
+      mixed |= 1u << a;
+    if (LEVELS && ((keyed >> a) & 1u)) {
+      const bool hi = (side >> a) & 1u;
+      if ((hi ? L1[a][0] : L1[a][1]) <= v) ok = false;
+      if (((late >> a) & 1u) && (hi ? L2[a][1] : L2[a][0]) <= v) ok = false;
+    }
+  }
+  if (mixed) {
+    if (LEVELS || (mixed & (mixed - 1u))) return false;
+    double keep = EIK_INF;  // side 1's own 2nd-order point must stay unaccepted
+#pragma unroll
+    for (int a = 0; a < ND; a++)
+      if ((mixed >> a) & 1u) {
+        x[a] = (1.0 / 3.0) * (4.0 * m[a] - t2[a][0]);
+        ca[a] = c2[a];
+        tg = t1[a][0];
+        keep = t2[a][1];
+      }
+    open = true;
+#pragma unroll
+    for (int g = 0; g < ND; g++) {
+      double tn = EIK_INF, qn = 0.0;
+      q = 0.0;
+#pragma unroll
+      for (int a = 0; a < ND; a++) {
+        d = tg - x[a];
+        if (lev[a] <= tg) q = fma(ca[a], d * d, q);
+        else if (lev[a] < tn) tn = lev[a];
+      }
+      ok = ok && (!open || q < s2 - (1e-9 * s2 + mar * (tg * tg)));
+#pragma unroll
+      for (int a = 0; a < ND; a++) {
+        d = tn - x[a];
+        if (lev[a] <= tg) qn = fma(ca[a], d * d, qn);
+      }
+      const double band = 1e-9 * s2 + mar * (tn * tn);
+      open = open && tn < EIK_INF && !(qn > s2 + band);
+      ok = ok && (!open || qn < s2 - band);
+      tg = open ? tn : tg;
+    }
+    ok = root(&v) && ok && keep > v;
+#pragma unroll
+    for (int a = 0; a < ND; a++)
+      if ((((side & ~second & ~mixed) >> a) & 1u) && t1[a][0] < v && t2[a][0] <= t1[a][0] && t2[a][1] > t1[a][0])
+        ok = false;
+  }
+#pragma unroll
+  for (int a = 0; a < ND; a++) {
+    const int sh = ((side >> a) & 1u) ? 1 : -1;
+    codes[a] = (int8_t)(lev[a] <= tg ? (((second >> a) & 1u) ? 2 * sh : sh) : 0);
+  }
+  *v_out = v;
+  return ok;
+}
+
 // Packed derivative codes: one byte per node, (c0+2) + 5*(c1+2) + 25*(c2+2) in the low
 // 7 bits; bit 7 marks a source point (traveltime fixed by the initialisation).
 EIK_HD uint8_t pack_codes(const int8_t* c, int nd) {

@@ -126,11 +126,11 @@ void* eik_ctx_stream(eik_ctx* ctx);
  * smallest slowness); "sm_fraction" = share of the SMs that the persistent solve kernels of
  * this context occupy, in (0, 1] (contexts whose calls overlap on one GPU, as in a serving
  * loop, each take a share so that their solves can be resident together). For both, 0 (the
- * default) = chosen per call by its size: calls of fewer than 2^22 node-sources (nsrc x grid
- * nodes) take round_gate 8 on a quarter of the SMs, larger ones round_gate 2 on all of them; "ctas_per_sm" = resident CTAs per SM of the forward solve, an integer, 0 (the
- * default) = as many as fit; "fwd_queue" = how the forward solve's warps work through their
- * entries: 1 = evaluations queued per warp and run 32 at a time, 0 = each in place, -1 (the
- * default) = the queue from 2^27 node-sources per launch up; "ray_room" = room of a ray in
+ * default) = the library's: round_gate 8 in 2D and 6 in 3D; all SMs, but no more than a forward
+ * solve has work for and a quarter of them for the adjoint of calls of fewer than 2^22
+ * node-sources (nsrc x grid nodes); "ctas_per_sm" (an integer in [0, 32]) and "fwd_queue" (-1,
+ * 0 or 1) are accepted and checked, and without effect: the forward solve keeps one block per
+ * SM, sized by its shared memory; "ray_room" = room of a ray in
  * the single tracing pass, in multiples of its straight-line length (default 3; rays that
  * outgrow it are traced again); "fine_replay" = 1 replays the refined start-up's heap for every
  * source instead of only where an exact tie decides its stop (default 0); "max_rounds" = round
