@@ -549,42 +549,52 @@ __device__ double fine_gdt_of(const GridDesc& gf, const double* tt, const uint8_
   return 2.0 * tmp1;
 }
 
-// Fine node states during the adjoint: 2 accepted, 3 accepted with a final λ.
-constexpr uint8_t FST_FINAL = 3;
-
-// Σ_r Jf[r, l] λf_r over the accepted fine nodes whose stencil contains l; *ready is
-// false while one of them has no final λ yet.
-__device__ double fine_downsum(const GridDesc& gf, const uint8_t* st, const uint8_t* code, const double* fgdt,
-                               long long nfmax, const double* lamf, long long l, bool* ready) {
-  const int c[3] = {(int)(l % gf.n[0]), (int)((l / gf.n[0]) % gf.n[1]), (int)(l / ((long long)gf.n[0] * gf.n[1]))};
-  double sum = 0.0;
-  *ready = true;
-  for (int ax = 0; ax < gf.nd; ax++)
-    for (int dl = -2; dl <= 2; dl++) {
-      if (dl == 0) continue;
-      int pr[3] = {c[0], c[1], c[2]};
-      pr[ax] += dl;
-      if (pr[ax] < 0 || pr[ax] >= gf.n[ax]) continue;
-      const long long lr = lin3(gf, pr[0], pr[1], pr[2]);
-      const uint8_t sr = st[lr];
-      if (sr < 2) continue;
-      int8_t cd[3];
-      unpack_codes(code[lr], cd);
-      const int cc = cd[ax];
-      if (cc == 0) continue;
-      const int ac = cc < 0 ? -cc : cc;
-      const int sg = cc > 0 ? -1 : 1;
-      const int p = -dl * sg;
-      if (p < 1 || p > ac) continue;
-      if (sr != FST_FINAL) {
-        *ready = false;
-        return 0.0;
-      }
-      double dh[3];
-      node_dh(gf, pr[0], dh);
-      const double J = fgdt[(long long)ax * nfmax + lr] * ((double)sg * dcoeff(ac, p, dh[ax]));
-      sum += J * lamf[lr];
+// The accepted fine nodes whose stencil contains node l: bit 4*axis + {0: -2, 1: -1, 2: +1, 3: +2}
+// of the result for the node at that offset. st[r] == 2: accepted.
+__device__ __forceinline__ unsigned fine_dependants(const GridDesc& gf, const uint8_t* st, const uint8_t* code,
+                                                    const int* c, long long l) {
+  unsigned dep = 0u;
+  uint8_t sv[12], cv[12];
+#pragma unroll
+  for (int k = 0; k < 12; k++) {
+    const int ax = k >> 2;
+    sv[k] = 0;
+    cv[k] = CODE_NONE;
+    if (ax < gf.nd && c[ax] + dir_off(k) >= 0 && c[ax] + dir_off(k) < gf.n[ax]) {
+      const long long lr = dir_lin(gf, l, k);
+      sv[k] = st[lr];
+      cv[k] = code[lr];
     }
+  }
+#pragma unroll
+  for (int k = 0; k < 12; k++) {
+    if (sv[k] != 2) continue;
+    int8_t cd[3];
+    unpack_codes(cv[k], cd);
+    const int cc = cd[k >> 2];
+    const int p = -dir_off(k) * (cc > 0 ? -1 : 1);
+    if (cc != 0 && p >= 1 && p <= (cc < 0 ? -cc : cc)) dep |= 1u << k;
+  }
+  return dep;
+}
+
+// Σ_r Jf[r, l] λf_r over the dependants of l, in the order of their bits (axis, then offset).
+__device__ __forceinline__ double fine_downsum(const GridDesc& gf, const uint8_t* code, const double* fgdt,
+                                               long long nfmax, const double* lamf, const int* c, long long l,
+                                               unsigned dep) {
+  double sum = 0.0;
+  for (; dep; dep &= dep - 1u) {
+    const int k = __ffs(dep) - 1, ax = k >> 2, dl = dir_off(k);
+    const long long lr = dir_lin(gf, l, k);
+    int8_t cd[3];
+    unpack_codes(code[lr], cd);
+    const int cc = cd[ax];
+    const int ac = cc < 0 ? -cc : cc, sg = cc > 0 ? -1 : 1;
+    double dh[3];
+    node_dh(gf, c[0] + (ax == 0 ? dl : 0), dh);
+    const double J = fgdt[(long long)ax * nfmax + lr] * ((double)sg * dcoeff(ac, -dl * sg, dh[ax]));
+    sum += J * __ldcg(lamf + lr);
+  }
   return sum;
 }
 
@@ -607,15 +617,21 @@ __device__ double fine_diag(const GridDesc& gf, const uint8_t* code, const doubl
 }
 
 // Source-region terms T2Va + T1Va (eikmaingrad.jl:428-479) and the source-location
-// gradient (eikmaingrad.jl:362-399); one warp per source.
+// gradient (eikmaingrad.jl:362-399); one CTA per source.
 // With refinement the reference solves the fine adjoint for one right-hand side per coarse
 // source point and contracts the results with z = ∂ψ∂up_∂up∂us + ∂ψ_∂u_s
 // (computestuff_finegrid!, calc_duh_dva_finegrid!, eikmaingrad.jl:540-741). By linearity
 // the same numbers come from ONE fine adjoint solve with right-hand side -z on the
-// coarse-coincident fine nodes, done here in reverse fine FMM order, 32 positions at a time.
-__global__ void __launch_bounds__(32) adj_srcterm_kernel(SrcTermArgs sa) {
+// coarse-coincident fine nodes, done here in reverse fine FMM order, SRCTERM_THREADS
+// positions at a time: a node is computed once its dependants are (their λ carries the state,
+// LAM_PENDING_BITS before). Consecutive positions lie all over the front, so most of a window is
+// ready at once and the rest within a few steps; a step costs its chain of L2 reads, which is
+// why a CTA of 512 threads and not a warp: 16 -> 2.0 ms per call at the default window
+// (36^3 fine nodes), whatever the number of sources.
+constexpr int SRCTERM_THREADS = 512;
+__global__ void __launch_bounds__(SRCTERM_THREADS) adj_srcterm_kernel(SrcTermArgs sa) {
   const int s = blockIdx.x;
-  const int lane = threadIdx.x;
+  const int tid = threadIdx.x;
   const ForwardBatch& fb = *sa.fb;
   const SrcOut& o = fb.out[s];
   const GridDesc& g = sa.g;
@@ -627,11 +643,11 @@ __global__ void __launch_bounds__(32) adj_srcterm_kernel(SrcTermArgs sa) {
   const bool wantvel = sa.whichgrad == 1 || sa.whichgrad == 3;
   const bool wantsrc = sa.whichgrad == 2 || sa.whichgrad == 3;
   if (!sa.refine) {
-    for (int k = lane; k < o.nseeds; k += 32) {
+    for (int k = tid; k < o.nseeds; k += SRCTERM_THREADS) {
       const double dd = (-o.distcorn[k]) * (1.0 / (o.velcorn[k] * o.velcorn[k]));
       gnode[k] = dd * y[k] + dd * dpsi[k];
     }
-    if (wantsrc && lane == 0) {
+    if (wantsrc && tid == 0) {
       double gs[3] = {0.0, 0.0, 0.0}, gs2[3] = {0.0, 0.0, 0.0};
       for (int k = 0; k < o.nseeds; k++) {
         double xyz[3], der[3];
@@ -648,11 +664,12 @@ __global__ void __launch_bounds__(32) adj_srcterm_kernel(SrcTermArgs sa) {
     return;
   }
   __shared__ double qcorn[8];
-  GridDesc gf;
-  fine_grid_of(g, o.fine, &gf);
+  __shared__ GridDesc gf;
+  if (tid == 0) fine_grid_of(g, o.fine, &gf);
+  __syncthreads();
   const long long nfmax = fb.nfmax;
   const double* tt = fb.fine_tt + (size_t)s * nfmax;
-  uint8_t* st = fb.fine_status + (size_t)s * nfmax;
+  const uint8_t* st = fb.fine_status + (size_t)s * nfmax;
   const uint8_t* code = fb.fine_code + (size_t)s * nfmax;
   const int32_t* order = fb.fine_order + (size_t)s * nfmax;
   const uint8_t* onh = fb.fine_onh + (size_t)s * nfmax;
@@ -661,74 +678,85 @@ __global__ void __launch_bounds__(32) adj_srcterm_kernel(SrcTermArgs sa) {
   double* fgdt = sa.fine_gdt + (size_t)s * g.nd * nfmax;
   const int nacc = o.nacc, nsf = o.nsrcf;
   // rows of the fine system and the coarse-point numbering (FMM order of the h points)
+  __shared__ int wcount[SRCTERM_THREADS / 32];
+  const int lane = tid & 31, warp = tid >> 5;
   int run = 0;
-  for (int b = 0; b < nacc; b += 32) {
-    const int p = b + lane;
+  for (int b = 0; b < nacc; b += SRCTERM_THREADS) {
+    const int p = b + tid;
     long long l = 0;
     bool h = false;
     if (p < nacc) {
       l = order[p];
-      lamf[l] = 0.0;
+      lamf[l] = p >= nsf ? __longlong_as_double((long long)LAM_PENDING_BITS) : 0.0;
       for (int a = 0; a < g.nd; a++) fgdt[(long long)a * nfmax + l] = (p >= nsf) ? fine_gdt_of(gf, tt, code, l, a) : 0.0;
       h = onh[l] != 0;
     }
     const unsigned m = __ballot_sync(0xffffffffu, h);
-    if (p < nacc) hk[l] = h ? run + __popc(m & ((1u << lane) - 1u)) : -1;
-    run += __popc(m);
+    if (lane == 0) wcount[warp] = __popc(m);
+    __syncthreads();
+    int at = run;
+    for (int w = 0; w < SRCTERM_THREADS / 32; w++) {
+      if (w < warp) at += wcount[w];
+      run += wcount[w];
+    }
+    if (p < nacc) hk[l] = h ? at + __popc(m & ((1u << lane) - 1u)) : -1;
+    __syncthreads();
   }
-  __syncwarp();
   // reverse sweep: the largest unfinished position of a window is always ready
-  for (int b = nacc - 1; b >= nsf; b -= 32) {
-    const int p = b - lane;
-    const long long l = (p >= nsf) ? order[p] : -1;
+  for (int b = nacc - 1; b >= nsf; b -= SRCTERM_THREADS) {
+    const int p = b - tid;
     bool done = p < nsf;
-    for (int round = 0; round <= 32; round++) {
-      double nv = 0.0;
-      bool go = false;
+    long long l = 0;
+    int c[3] = {0, 0, 0};
+    unsigned dep = 0u;
+    double rhs = 0.0, diag = 1.0;
+    if (!done) {
+      l = order[p];
+      node_coords(gf, l, c);
+      dep = fine_dependants(gf, st, code, c, l);
+      const int k = hk[l];
+      rhs = (k >= 0) ? -(y[k] + dpsi[k]) : 0.0;
+      diag = fine_diag(gf, code, fgdt, nfmax, l);
+    }
+    for (int step = 0; step <= SRCTERM_THREADS; step++) {
       if (!done) {
-        bool ready;
-        const double sum = fine_downsum(gf, st, code, fgdt, nfmax, lamf, l, &ready);
+        bool ready = true;
+        for (unsigned m = dep; m && ready; m &= m - 1u)
+          ready = !lam_pending(__ldcg(lamf + dir_lin(gf, l, __ffs(m) - 1)));
         if (ready) {
-          const int k = hk[l];
-          const double rhs = (k >= 0) ? -(y[k] + dpsi[k]) : 0.0;
-          nv = (rhs - sum) / fine_diag(gf, code, fgdt, nfmax, l);
-          go = true;
+          // nodes of the window are computed from final values only, whenever they see them
+          __stcg(lamf + l, (rhs - fine_downsum(gf, code, fgdt, nfmax, lamf, c, l, dep)) / diag);
+          done = true;
         }
       }
-      __syncwarp();
-      if (go) {
-        lamf[l] = nv;
-        st[l] = FST_FINAL;
-        done = true;
-      }
-      __syncwarp();
-      if (__all_sync(0xffffffffu, done)) break;
+      if (__syncthreads_and(done)) break;
     }
   }
   // per source-box corner: (∂g/∂τ_s)ᵀ λf + H_Aᵀ z
-  if (lane < nsf) {
-    const long long l = order[lane];
-    bool ready;
-    const double sum = fine_downsum(gf, st, code, fgdt, nfmax, lamf, l, &ready);
+  if (tid < nsf) {
+    const long long l = order[tid];
+    int c[3];
+    node_coords(gf, l, c);
+    const double sum = fine_downsum(gf, code, fgdt, nfmax, lamf, c, l, fine_dependants(gf, st, code, c, l));
     const int k = hk[l];
-    qcorn[lane] = sum + ((k >= 0) ? (y[k] + dpsi[k]) : 0.0);
+    qcorn[tid] = sum + ((k >= 0) ? (y[k] + dpsi[k]) : 0.0);
   }
-  __syncwarp();
+  __syncthreads();
   if (wantvel) {
     // duh_dwq contracted with z, then summed onto the nearest coarse node of each accepted
     // fine node (dwq_dva, eikmaingrad.jl:716-738): here in place in lamf
-    for (int p = lane; p < nacc; p += 32) {
+    for (int p = tid; p < nacc; p += SRCTERM_THREADS) {
       const long long l = order[p];
       if (p < nsf) {
         const double dd = (-o.distcorn[p]) * (1.0 / (o.velcorn[p] * o.velcorn[p]));
-        lamf[l] = dd * qcorn[p];
+        __stcg(lamf + l, dd * qcorn[p]);
       } else {
         const double v = sa.vel[fine_nn_coarse(g, o.fine, l, gf)];
-        lamf[l] = 2.0 * lamf[l] / (v * v * v);
+        __stcg(lamf + l, 2.0 * __ldcg(lamf + l) / (v * v * v));
       }
     }
-    __syncwarp();
-    for (int k = lane; k < o.nseeds; k += 32) {
+    __syncthreads();
+    for (int k = tid; k < o.nseeds; k += SRCTERM_THREADS) {
       const long long cl = fb.seed_lin[(size_t)s * fb.seedcap + k];
       const int c[3] = {(int)(cl % g.n[0]), (int)((cl / g.n[0]) % g.n[1]), (int)(cl / ((long long)g.n[0] * g.n[1]))};
       int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
@@ -745,14 +773,14 @@ __global__ void __launch_bounds__(32) adj_srcterm_kernel(SrcTermArgs sa) {
           for (int fx = lo[0]; fx <= hi[0]; fx++) {
             if (fine_nn_axis(o.fine, fx) != c[0] - o.fine.ijk1[0]) continue;
             const long long lf = lin3(gf, fx, fy, fz);
-            if (st[lf] >= 2) acc += lamf[lf];
+            if (st[lf] >= 2) acc += __ldcg(lamf + lf);
           }
         }
       }
       gnode[k] = acc;
     }
   }
-  if (wantsrc && lane == 0) {
+  if (wantsrc && tid == 0) {
     double gsv[3] = {0.0, 0.0, 0.0};
     for (int k = 0; k < nsf; k++) {
       double xyz[3], der[3];
@@ -1240,7 +1268,7 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   ta.fine_gdt = fgdt;
   ta.warn = dwarn;
   adj_ysrc_kernel<<<(int)nsrc, 128, 0, st>>>(ta);
-  adj_srcterm_kernel<<<(int)nsrc, 32, 0, st>>>(ta);
+  adj_srcterm_kernel<<<(int)nsrc, SRCTERM_THREADS, 0, st>>>(ta);
   if (wantvel) {
     adj_field_kernel<<<ctx->nsm * 8, 256, 0, st>>>(ta, N);
     adj_carry_kernel<<<(int)nsrc, 64, 0, st>>>(ta, ep.radiussmoothgradsrc, carry);
