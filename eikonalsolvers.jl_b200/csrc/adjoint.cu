@@ -6,7 +6,7 @@
 // The reference assembles the derivative matrices in FMM order and back-substitutes the
 // upper-triangular system Jᵀλ = -P_Bᵀr with a sparse solver. Here the same system is solved
 // where it lives: row i of J couples node i with the <= 2*nd*2 nodes whose stencil codes
-// point at it, so λ_i = (b_i - Σ_r J[r,i] λ_r) / J[i,i] is computed by a tile dataflow the
+// point at it, so λ_i = (b_i - Σ_r J[r,i] λ_r) / J[i,i] is computed by a brick dataflow the
 // moment every downstream λ_r is final (one evaluation per node, no sparse matrices).
 // The refined-grid chain rule (the reference's dense N_h x N_acc products) is collapsed by
 // linearity into one fine-grid adjoint solve with right-hand side -H_Bᵀz per source.
@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/eikcuda.h"
+#include "brick.cuh"
 #include "node.cuh"
 #include "rounds.cuh"
 #include "runtime.hpp"
@@ -29,14 +30,16 @@ __device__ __forceinline__ bool lam_pending(double v) {
 }
 
 struct AdjProblem {
-  double* lam;   // N: adjoint variable (then the per-source gradient field)
-  double* gdt;   // ND x N: 2*(D_a t) of every node's own stencil
-  double* rhs;   // N
+  double* lam;  // N, column-major: right-hand side at the receivers' nodes during the sweep, then
+                // the per-source gradient field
 };
 
+// The sweep's state, in brick order (brick.cuh), beside the forward's traveltimes.
 struct AdjArgs {
   SolveArgs sa;
   const AdjProblem* ap;
+  double* lam;     // λ, LAM_PENDING_BITS before; 0 at source points and outside the grid
+  uint32_t* info;  // per node, see adj_info_kernel
 };
 
 // Stencil coefficients of the derivative matrices (setcoeffderiv!, eikmaingrad.jl:1042-1090;
@@ -52,69 +55,78 @@ __device__ __forceinline__ bool is_source(const CoarseProblem& P, long long l) {
 }
 
 // ------------------------------------------------------------ per-node preparation --
-// Also counts, for every node, the nodes whose stencil reads it (its dependants in Jᵀλ = b)
-// and lists the nodes without any for round 0 of the solve.
-__global__ void adj_prep_kernel(const CoarseProblem* probs, const AdjProblem* ap, int nprob, long long N,
-                                SolveArgs sa) {
-  const long long tot = N * nprob;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot; q += (long long)gridDim.x * blockDim.x) {
-    const int s = (int)(q / N);
-    const long long l = q - (long long)s * N;
-    const CoarseProblem& P = probs[s];
-    const AdjProblem& A = ap[s];
+// What the sweep needs of a node in one word: its own codes (bits 0-6), whether it has no
+// unknown (source points, positions outside the grid: bit 7), and its dependants, the nodes
+// whose stencil reads it: per axis six bits from bit 8 + 6*axis, {far -: 1 bit, near -: 2 bits,
+// near +: 2 bits, far +: 1 bit}; a near dependant (one step away) is of 1st or 2nd order (1, 2),
+// a far one of 2nd order. INFO_RHS marks nodes with a right-hand side (adj_recv_kernel).
+constexpr uint32_t INFO_FIXED = 1u << 7, INFO_RHS = 1u << 26;
+__device__ __forceinline__ unsigned info_near(uint32_t f, int ax, bool plus) {
+  return (f >> (8 + 6 * ax + (plus ? 3 : 1))) & 3u;
+}
+__device__ __forceinline__ bool info_far(uint32_t f, int ax, bool plus) { return (f >> (8 + 6 * ax + (plus ? 5 : 0))) & 1u; }
+constexpr uint32_t INFO_DEPS = 0x3ffffu << 8;
+
+// Lists the bricks that hold a node without dependants for the first round of their colour.
+// copy_t: the forward left its traveltimes in the problems' own arrays only.
+template <int ND>
+__global__ void adj_info_kernel(AdjArgs aa, int copy_t) {
+  typedef Brick<ND> B;
+  const BrickState& bs = aa.sa.bs;
+  const size_t total = (size_t)bs.stride * aa.sa.nprob * B::NODES;
+  // every 32 consecutive nodes belong to one brick
+  for (size_t id = blockIdx.x * (size_t)blockDim.x + threadIdx.x; id < total; id += (size_t)gridDim.x * blockDim.x) {
+    const unsigned b = (unsigned)(id / B::NODES), q = (unsigned)(id % B::NODES);
+    const unsigned p = b / bs.stride, lb = b - p * bs.stride;
+    const CoarseProblem& P = aa.sa.probs[p];
     const GridDesc& g = P.g;
-    const bool src = is_source(P, l);
-    A.lam[l] = src ? 0.0 : __longlong_as_double((long long)LAM_PENDING_BITS);
-    A.rhs[l] = 0.0;
-    const int i = (int)(l % g.n[0]), j = (int)((l / g.n[0]) % g.n[1]), k = (int)(l / ((long long)g.n[0] * g.n[1]));
-    int8_t cd[3];
-    unpack_codes(P.code[l], cd);
-    double dh[3];
-    node_dh(g, i, dh);
-    for (int a = 0; a < g.nd; a++) {
-      double v = 0.0;
-      if (!src && cd[a] != 0) {
-        const int ac = cd[a] < 0 ? -cd[a] : cd[a];
-        const int sg = cd[a] > 0 ? -1 : 1;
-        double tmp1 = 0.0;
-        for (int p = ac; p >= 0; p--) {  // the reference sums in ascending FMM column order
-          int c[3] = {i, j, k};
-          c[a] += sg * p;
-          tmp1 += ((double)sg * dcoeff(ac, p, dh[a])) * P.t[lin3(g, c[0], c[1], c[2])];
-        }
-        v = 2.0 * tmp1;
+    const unsigned nb0 = (unsigned)bricks_along<ND>(g, 0), nb1 = (unsigned)bricks_along<ND>(g, 1);
+    const unsigned bx = lb % nb0, by = (lb / nb0) % nb1, bz = lb / (nb0 * nb1);
+    const int c[3] = {(int)(bx * B::BX + q % B::BX), (int)(by * B::BY + (q / B::BX) % B::BY),
+                      (int)(bz * B::BZ + q / (B::BX * B::BY))};
+    uint32_t f = INFO_FIXED | CODE_NONE;
+    double lam = 0.0;
+    if (c[0] < g.n[0] && c[1] < g.n[1] && c[2] < g.n[2]) {
+      const long long l = lin3(g, c[0], c[1], c[2]);
+      const uint8_t cb = P.code[l];
+      if (copy_t) bs.t[id] = P.t[l];
+      f = cb & 0x7fu;
+      if (cb == (uint8_t)(CODE_NONE | CODE_SRC_BIT)) f |= INFO_FIXED;  // no other special node has these codes
+      else lam = __longlong_as_double((long long)LAM_PENDING_BITS);
+      uint8_t cv[4 * ND];
+#pragma unroll
+      for (int k = 0; k < 4 * ND; k++) {
+        const int ax = k >> 2, at = c[ax] + dir_off(k);
+        cv[k] = at >= 0 && at < g.n[ax] ? P.code[dir_lin(g, l, k)] : (uint8_t)CODE_NONE;
       }
-      A.gdt[(long long)a * N + l] = v;
+#pragma unroll
+      for (int k = 0; k < 4 * ND; k++) {
+        const int ax = k >> 2, j = k & 3, dl = dir_off(k);
+        int8_t cd[3];
+        unpack_codes(cv[k], cd);
+        const int cc = cd[ax];
+        const int ac = cc < 0 ? -cc : cc, pt = -dl * (cc > 0 ? -1 : 1);
+        if (cc == 0 || pt < 1 || pt > ac) continue;
+        // j = 0, 3: far (pt = 2 = ac); j = 1, 2: near, of order ac
+        f |= (j == 0 ? 1u : (j == 1 ? (unsigned)ac << 1 : (j == 2 ? (unsigned)ac << 3 : 1u << 5))) << (8 + 6 * ax);
+      }
     }
-    int ndep = 0;
-    for (int ax = 0; ax < g.nd; ax++)
-      for (int dl = -2; dl <= 2; dl++) {
-        if (dl == 0) continue;
-        int pr[3] = {i, j, k};
-        pr[ax] += dl;
-        if (pr[ax] < 0 || pr[ax] >= g.n[ax]) continue;
-        int8_t cr[3];
-        unpack_codes(P.code[lin3(g, pr[0], pr[1], pr[2])], cr);
-        const int cc = cr[ax];
-        if (cc == 0) continue;
-        const int ac = cc < 0 ? -cc : cc;
-        const int p = -dl * (cc > 0 ? -1 : 1);
-        if (p >= 1 && p <= ac) ndep++;
-      }
-    sa.rs.stamp[q] = ndep;
-    if (ndep == 0 && !src) {
-      const unsigned int at = atomicAdd(sa.rs.cnt, 1u);
-      sa.rs.list[0][at] = (unsigned long long)q << 32;
+    aa.info[id] = f;
+    aa.lam[id] = lam;
+    const bool root = !(f & (INFO_FIXED | INFO_DEPS));
+    const unsigned act = __activemask();
+    if (__any_sync(act, root) && (threadIdx.x & 31) == __ffs(act) - 1 && atomicExch(bs.listed + b, 1u) == 0u) {
+      const unsigned col = (bx + by + bz) & 1u;
+      bs.lists[(size_t)(2 * col) * bs.listcap + atomicAdd(bs.ctr + 2 * col, 1u)] = b;
     }
   }
 }
 
 // J[r, i] for node r = i + delta*e_a if r's stencil contains i, else 0 (and *is_down=false).
-__device__ __forceinline__ double jcoef(const GridDesc& g, const uint8_t* code, const double* gdt, long long N,
-                                        int a, int delta, long long lr, int ir, bool* is_down) {
+__device__ __forceinline__ double jcoef(const CoarseProblem& P, int a, int delta, long long lr, int ir, bool* is_down) {
   *is_down = false;
   int8_t cd[3];
-  unpack_codes(code[lr], cd);
+  unpack_codes(P.code[lr], cd);
   const int c = cd[a];
   if (c == 0) return 0.0;
   const int ac = c < 0 ? -c : c;
@@ -123,27 +135,12 @@ __device__ __forceinline__ double jcoef(const GridDesc& g, const uint8_t* code, 
   if (p < 1 || p > ac) return 0.0;
   *is_down = true;
   double dh[3];
-  node_dh(g, ir, dh);
-  return gdt[(long long)a * N + lr] * ((double)sg * dcoeff(ac, p, dh[a]));
-}
-
-__device__ __forceinline__ double jdiag(const GridDesc& g, const uint8_t* code, const double* gdt, long long N,
-                                        long long l, int i) {
-  int8_t cd[3];
-  unpack_codes(code[l], cd);
-  double dh[3];
-  node_dh(g, i, dh);
-  double s = 0.0;
-  bool first = true;
-  for (int a = 0; a < g.nd; a++) {
-    if (cd[a] == 0) continue;
-    const int ac = cd[a] < 0 ? -cd[a] : cd[a];
-    const int sg = cd[a] > 0 ? -1 : 1;
-    const double v = gdt[(long long)a * N + l] * ((double)sg * dcoeff(ac, 0, dh[a]));
-    s = first ? v : s + v;
-    first = false;
-  }
-  return s;
+  node_dh(P.g, ir, dh);
+  const long long st = a == 0 ? 1LL : (a == 1 ? (long long)P.g.n[0] : (long long)P.g.n[0] * P.g.n[1]);
+  double tmp1 = 0.0;
+  for (int m = ac; m >= 0; m--)  // the reference sums in ascending FMM column order
+    tmp1 += ((double)sg * dcoeff(ac, m, dh[a])) * P.t[lr + sg * m * st];
+  return (2.0 * tmp1) * ((double)sg * dcoeff(ac, p, dh[a]));
 }
 
 // --------------------------------------------------------- receivers: misfit, rhs --
@@ -157,6 +154,8 @@ struct RecvArgs {
   const double* pickobs;
   const double* stdobs;
   const ForwardBatch* fb;
+  uint32_t* info;   // adjoint words in brick order: INFO_RHS is set at the receivers' nodes
+  size_t stride;    // brick-ordered nodes of a source
   double* misfit;   // nsrc
   double* dpsi;     // nsrc x seedcap: ∂ψ/∂u_s per source point
 };
@@ -212,194 +211,318 @@ __device__ int seed_index(const ForwardBatch& fb, int s, long long node) {
   return -1;
 }
 
-// One thread per source, receivers in order (deterministic sums).
-__global__ void adj_recv_kernel(RecvArgs ra) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ra.nsrc) return;
+// One warp per source. The receivers' interpolation runs one receiver a lane; the sums go over
+// the receivers in order (deterministic), a receiver's corners (distinct nodes) one a lane.
+// With one thread per source every read and sum was a dependent round trip: 2.2 ms for 400
+// receivers a source.
+__global__ void __launch_bounds__(32) adj_recv_kernel(RecvArgs ra) {
+  const int s = blockIdx.x, lane = threadIdx.x;
   const GridDesc& g = ra.g;
   const CoarseProblem& P = ra.probs[s];
-  const AdjProblem& A = ra.ap[s];
+  double* rhs = ra.ap[s].lam;
   const ForwardBatch& fb = *ra.fb;
   double* dpsi = ra.dpsi + (size_t)s * fb.seedcap;
-  for (int k = 0; k < fb.out[s].nseeds; k++) dpsi[k] = 0.0;
-  double misf = 0.0;
-  for (long long r = ra.recoff[s]; r < ra.recoff[s + 1]; r++) {
+  uint32_t* info = ra.info + (size_t)s * ra.stride;
+  __shared__ double scoef[32][9];
+  __shared__ long long snode[32][9];  // node, or -2 - k for source point k
+  for (int k = lane; k < fb.out[s].nseeds; k += 32) __stcg(dpsi + k, 0.0);
+  const long long r0 = ra.recoff[s], r1 = ra.recoff[s + 1];
+  for (long long r = r0 + lane; r < r1; r += 32) {
     double coeff[8];
     long long node[8];
     const int nc = interp_corners(g, ra.rec + r * g.nd, coeff, node);
-    double pick = 0.0;
-    for (int c = 0; c < nc; c++) pick += coeff[c] * P.t[node[c]];
-    const double pd = pick - ra.pickobs[r];
-    const double sd2 = ra.stdobs[r] * ra.stdobs[r];
-    misf += (pd * pd) / sd2;
-    const double fact = pd / sd2;
     for (int c = 0; c < nc; c++) {
-      if (is_source(P, node[c])) {
-        const int k = seed_index(fb, s, node[c]);
-        if (k >= 0) dpsi[k] += coeff[c] * fact;
-      } else {
-        A.rhs[node[c]] += (-coeff[c]) * fact;
-      }
+      int x[3];
+      node_coords(g, node[c], x);
+      const long long q = g.nd == 3 ? brick_node<3>(g, x[0], x[1], x[2]) : brick_node<2>(g, x[0], x[1], x[2]);
+      if (info[q] & INFO_FIXED) continue;
+      atomicOr(info + q, INFO_RHS);
+      __stcg(rhs + node[c], 0.0);
     }
   }
-  ra.misfit[s] = misf;
+  __syncwarp();
+  double misf = 0.0;
+  for (long long rb = r0; rb < r1; rb += 32) {
+    const long long r = rb + lane;
+    double term = 0.0, fact = 0.0;
+    const int nc = g.nd == 3 ? 8 : 4;
+    if (r < r1) {
+      double coeff[8];
+      long long node[8];
+      interp_corners(g, ra.rec + r * g.nd, coeff, node);
+      double pick = 0.0;
+      for (int c = 0; c < nc; c++) pick += coeff[c] * P.t[node[c]];
+      const double pd = pick - ra.pickobs[r];
+      const double sd2 = ra.stdobs[r] * ra.stdobs[r];
+      term = (pd * pd) / sd2;
+      fact = pd / sd2;
+      for (int c = 0; c < nc; c++) {
+        scoef[lane][c] = coeff[c];
+        snode[lane][c] = is_source(P, node[c]) ? -2 - (long long)seed_index(fb, s, node[c]) : node[c];
+      }
+    }
+    __syncwarp();
+    const int m = (int)min(32LL, r1 - rb);
+    for (int i = 0; i < m; i++) {
+      misf += __shfl_sync(0xffffffffu, term, i);
+      const double fi = __shfl_sync(0xffffffffu, fact, i);
+      if (lane < nc) {
+        const long long node = snode[i][lane];
+        if (node >= 0) __stcg(rhs + node, __ldcg(rhs + node) + (-scoef[i][lane]) * fi);
+        else if (node < -1) __stcg(dpsi + (-2 - node), __ldcg(dpsi + (-2 - node)) + scoef[i][lane] * fi);
+      }
+      __syncwarp();
+    }
+  }
+  if (lane == 0) ra.misfit[s] = misf;
 }
 
 // ------------------------------------------------------------- adjoint solve --
-// Jᵀλ = b in topological order of the stencil graph (Kahn): round r takes the nodes whose
-// dependants are all final, computes
+// Jᵀλ = b by bricks, in the order its dependences allow: a node's
 //   λ_i = (b_i − Σ_{r reads i} J[r,i] λ_r) / J[i,i]
-// pulling the dependants' λ in a fixed order (deterministic), then releases the nodes its
-// own stencil reads; a node whose dependant count drops to zero is listed for the next
-// round. Every node is computed exactly once, after everything it depends on.
-__global__ void adj_rounds_init_kernel(SolveArgs a) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  for (int k = 0; k < 3; k++) {
-    a.rs.cnt[k] = 0;
-    a.rs.grab[k] = 0;
+// is computed once the λ of every node that reads it is final, each node exactly once. As in the
+// forward solve (brick.cuh) a brick reads only the bricks across its faces and a round visits one
+// colour, so what a visit reads outside its brick stands still. A visit counts the pending
+// dependants of its brick's pending nodes, works off the nodes that have none, releasing the
+// nodes their stencils read, until none is left, and lists the bricks across the faces that
+// those stencils reach. The coefficients J come from the traveltimes and codes on the spot. The
+// terms of a node are subtracted in a fixed order (axis, then offset -2, -1, +1, +2).
+//
+// Why bricks: as worklist rounds over all nodes the sweep took one grid barrier and a chain of
+// scattered L2 reads per level of the dependence graph (1185 levels at 256^3, 1930 at 1024x640)
+// and a pass that stored 2 (D_a t) per axis; a visit takes the levels inside its brick from shared
+// memory (128^3: 80 rounds, 3.2 visits a brick). Sweep and preparation, worklists -> bricks, B200:
+// 256^3 x 4 54 -> 31 ms, 1024x640 x 64 47 -> 9 ms, 300x220 x 4 6.0 -> 1.4 ms, 64^3 x 32 8.0 -> 5.4 ms.
+template <int ND>
+struct __align__(16) AdjMem {
+  typedef Brick<ND> B;
+  double t[B::CUBE];
+  double lam[B::CUBE];
+  uint32_t info[B::NODES];
+  unsigned cnt[B::NODES];    // pending dependants of a pending node; CNT_FIXED otherwise
+  uint16_t queue[B::NODES];  // nodes ready to compute
+  double extra[ND == 3 ? 2 : 64];
+  unsigned tail;
+  // spherical grids: 1/h, 3/(2h), 4/(2h), 1/(2h) of axis 1 (and 2) per radial index of the brick, in
+  // corners of the cube that no stencil reads (brick.cuh)
+  __device__ __forceinline__ double* coef(int ax) { return ND == 3 ? t + (ax == 1 ? 120 : 1560) : extra; }
+};
+// t + 1560..1607 lie in the rows y = 8, 9 of the plane z = 8 and y = -2, -1 of the next
+constexpr unsigned CNT_FIXED = 0x40000000u;
+// 32.8 KB a warp in 3D: 7 warps an SM; 9.5 KB in 2D
+template <int ND>
+constexpr int ADJ_WARPS = ND == 3 ? 7 : 16;
+
+__device__ __forceinline__ bool pending_hi(double v) { return (unsigned)__double2hiint(v) == (unsigned)(LAM_PENDING_BITS >> 32); }
+
+// Visits brick b; returns the faces (bit 2*axis + (0: +, 1: -)) its computed nodes' stencils reach.
+template <int ND>
+__device__ __forceinline__ unsigned adj_visit(AdjMem<ND>& w, const AdjArgs& aa, int prob, size_t b, const int (&bc)[3],
+                                              const int (&nb)[3], int lane) {
+  typedef Brick<ND> B;
+  const CoarseProblem& P = aa.sa.probs[prob];
+  load_cube<ND>(w.t, aa.sa.bs.t, b, bc, nb, EIK_INF, lane);
+  load_cube<ND>(w.lam, aa.lam, b, bc, nb, 0.0, lane);
+#pragma unroll
+  for (int q = 0; q < B::NODES / 4; q += 32)
+    if (q + lane < B::NODES / 4) cp_async16(&w.info[4 * (q + lane)], aa.info + b * B::NODES + 4 * (q + lane));
+  const int n[3] = {P.g.n[0], P.g.n[1], P.g.n[2]};
+  const int x0[3] = {bc[0] * B::BX, bc[1] * B::BY, bc[2] * B::BZ};
+  const bool cart = P.c1u > 0.0;
+  const double h0 = P.g.spac[0];
+  const double k0[4] = {1.0 / h0, 3.0 / (2.0 * h0), 4.0 / (2.0 * h0), 1.0 / (2.0 * h0)};
+  if (!cart && lane < B::BX && x0[0] + lane < n[0]) {
+    double dh[3];
+    node_dh(P.g, x0[0] + lane, dh);
+#pragma unroll
+    for (int a = 1; a < ND; a++) {
+      double* k = w.coef(a) + 4 * lane;
+      k[0] = 1.0 / dh[a];
+      k[1] = 3.0 / (2.0 * dh[a]);
+      k[2] = 4.0 / (2.0 * dh[a]);
+      k[3] = 1.0 / (2.0 * dh[a]);
+    }
   }
-  a.rs.bar[0] = 0;
-  a.rs.bar[1] = 0;
-  *a.rs.rounds = 0;
-  *a.abort_flag = 0;
+  const double* rhs = aa.ap[prob].lam;
+  if (lane == 0) w.tail = 0u;
+  cp_async_wait();
+  __syncwarp();
+  // pending dependants of the pending nodes; the nodes that have none are ready
+  int tail = 0;
+#pragma unroll 2
+  for (int k = 0; k < B::WORDS; k++) {
+    const int q = 32 * k + lane;
+    const int ci = B::ORG + (q / (B::BX * B::BY)) * B::PZ + ((q / B::BX) % B::BY) * B::PY + q % B::BX;
+    const bool pend = pending_hi(w.lam[ci]);
+    unsigned cnt = CNT_FIXED;
+    if (__any_sync(FULL_WARP, pend)) {
+      const uint32_t f = w.info[q];
+      unsigned c = 0u;
+#pragma unroll
+      for (int a = 0; a < ND; a++) {
+        const int st = a == 0 ? 1 : (a == 1 ? B::PY : B::PZ);
+        if (info_far(f, a, false) && pending_hi(w.lam[ci - 2 * st])) c++;
+        if (info_near(f, a, false) && pending_hi(w.lam[ci - st])) c++;
+        if (info_near(f, a, true) && pending_hi(w.lam[ci + st])) c++;
+        if (info_far(f, a, true) && pending_hi(w.lam[ci + 2 * st])) c++;
+      }
+      if (pend) cnt = c;
+      const unsigned rm = __ballot_sync(FULL_WARP, cnt == 0u);
+      if (cnt == 0u) w.queue[tail + __popc(rm & ((1u << lane) - 1u))] = (uint16_t)q;
+      tail += __popc(rm);
+    }
+    w.cnt[q] = cnt;
+  }
+  if (lane == 0) w.tail = (unsigned)tail;
+  __syncwarp();
+  if (tail == 0) return 0u;  // nothing to do yet
+  unsigned faces = 0u;
+  int head = 0;
+#pragma unroll 1
+  while (head < tail) {
+    const bool act = head + lane < tail;
+    const unsigned q = act ? (unsigned)w.queue[head + lane] : 0u;
+    const int x = (int)(q % B::BX), y = (int)((q / B::BX) % B::BY), z = (int)(q / (B::BX * B::BY));
+    const int ci = B::ORG + z * B::PZ + y * B::PY + x;
+    const uint32_t f = act ? w.info[q] : 0u;
+    int8_t cm[3];
+    unpack_codes((uint8_t)(f & 0x7fu), cm);
+    double sum = 0.0, dg = 0.0;
+    if (f & INFO_RHS)
+      sum = __ldcg(rhs + ((x0[0] + x) + (long long)n[0] * ((x0[1] + y) + (long long)n[1] * (x0[2] + z))));
+    bool first = true;
+#pragma unroll
+    for (int a = 0; a < ND; a++) {
+      const int st = a == 0 ? 1 : (a == 1 ? B::PY : B::PZ);
+      double k[4];
+#pragma unroll
+      for (int m = 0; m < 4; m++) k[m] = (a == 0 || cart) ? k0[m] : w.coef(a)[4 * x + m];
+      double tv[5];
+#pragma unroll
+      for (int m = 0; m < 5; m++) tv[m] = fabs(w.t[ci + (m - 2) * st]);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        // dependant at offset dl; its stencil runs towards this node (sign sg)
+        const int dl = j < 2 ? j - 2 : j - 1;
+        const double sg = dl > 0 ? -1.0 : 1.0;
+        const int is = dl > 0 ? -1 : 1;
+        const unsigned order = (j == 0 || j == 3) ? (info_far(f, a, j == 3) ? 2u : 0u) : info_near(f, a, j == 2);
+        if (order) {
+          const bool near = j == 1 || j == 2;
+          const int r = 2 + dl;  // index of the dependant in tv
+          double tmp1, J;
+          if (order == 1u) {
+            tmp1 = 0.0 + (sg * k[0]) * tv[r + is];
+            tmp1 += (sg * -k[0]) * tv[r];
+            J = (2.0 * tmp1) * (sg * k[0]);
+          } else {
+            tmp1 = 0.0 + (sg * -k[3]) * tv[r + 2 * is];
+            tmp1 += (sg * k[2]) * tv[r + is];
+            tmp1 += (sg * -k[1]) * tv[r];
+            J = (2.0 * tmp1) * (sg * (near ? k[2] : -k[3]));
+          }
+          sum -= J * w.lam[ci + dl * st];
+        }
+      }
+      if (cm[a] != 0) {
+        const int ac = cm[a] < 0 ? -cm[a] : cm[a];
+        const double sg = cm[a] > 0 ? -1.0 : 1.0;
+        const double p0 = tv[2], p1 = cm[a] > 0 ? tv[1] : tv[3], p2 = cm[a] > 0 ? tv[0] : tv[4];
+        double tmp1, v;
+        if (ac == 1) {
+          tmp1 = 0.0 + (sg * k[0]) * p1;
+          tmp1 += (sg * -k[0]) * p0;
+          v = (2.0 * tmp1) * (sg * -k[0]);
+        } else {
+          tmp1 = 0.0 + (sg * -k[3]) * p2;
+          tmp1 += (sg * k[2]) * p1;
+          tmp1 += (sg * -k[1]) * p0;
+          v = (2.0 * tmp1) * (sg * -k[1]);
+        }
+        dg = first ? v : dg + v;
+        first = false;
+      }
+    }
+    if (act) {
+      w.lam[ci] = sum / dg;
+      // release the nodes this node's stencil reads
+#pragma unroll
+      for (int a = 0; a < ND; a++) {
+        const int ac = cm[a] < 0 ? -cm[a] : cm[a], sgn = cm[a] > 0 ? -1 : 1;
+        const int pos = a == 0 ? x : (a == 1 ? y : z), ext = a == 0 ? B::BX : (a == 1 ? B::BY : B::BZ);
+        const int qst = a == 0 ? 1 : (a == 1 ? B::BX : B::BX * B::BY);
+#pragma unroll
+        for (int p = 1; p <= 2; p++) {
+          if (p > ac) continue;
+          const int at = pos + sgn * p;
+          if (at >= 0 && at < ext) {
+            const unsigned qt = q + (unsigned)(sgn * p * qst);
+            if (atomicSub(&w.cnt[qt], 1u) == 1u) w.queue[atomicAdd(&w.tail, 1u)] = (uint16_t)qt;
+          } else {
+            faces |= 1u << (2 * a + (sgn > 0 ? 0 : 1));
+          }
+        }
+      }
+    }
+    head = min(head + 32, tail);
+    __syncwarp();
+    tail = (int)*(volatile unsigned*)&w.tail;
+    __syncwarp();
+  }
+  double* own = aa.lam + b * B::NODES;
+  constexpr int ROWP = B::BX / 2;
+#pragma unroll
+  for (int q = 0; q < B::NODES / 2; q += 32) {
+    const int e = q + lane, row = e / ROWP, xp = e % ROWP;
+    const int y = row % B::BY, z = row / B::BY;
+    *reinterpret_cast<double2*>(own + 2 * e) =
+        *reinterpret_cast<const double2*>(&w.lam[B::ORG + z * B::PZ + y * B::PY + 2 * xp]);
+  }
+  return __reduce_or_sync(FULL_WARP, faces);
 }
 
-// The node's solve is a chain of dependent L2 round trips; its loads go out in batches: the
-// codes of the node and of the 4*ND nodes that may read it (with the right-hand side), then
-// per axis the coefficient and λ of the dependants on that axis. The terms are subtracted
-// in the same fixed order as they would be one by one (axis, then offset -2, -1, +1, +2).
-// Everything read here was written before this node was listed (the forward's codes and
-// coefficients, and the dependants' λ, each released only after its store and a fence).
 template <int ND>
-__device__ void adj_node(const AdjArgs& aa, int prob, long long l, unsigned long long gb, unsigned int* rel) {
+__global__ void __launch_bounds__(ADJ_WARPS<ND> * 32, 1) adj_rounds_kernel(AdjArgs aa) {
+  typedef Brick<ND> B;
+  extern __shared__ __align__(16) unsigned char adj_smem[];
   const SolveArgs& a = aa.sa;
-  const CoarseProblem& P = a.probs[prob];
-  const AdjProblem& A = aa.ap[prob];
-  const GridDesc& g = P.g;
-  const long long N = npts(g);
-  int c[3];
-  node_coords(g, l, c);
-  long long nl[ND][4];
-  uint8_t ncode[ND][4];
-#pragma unroll
-  for (int ax = 0; ax < ND; ax++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int dl = j < 2 ? j - 2 : j - 1;
-      nl[ax][j] = -1;
-      if (c[ax] + dl < 0 || c[ax] + dl >= g.n[ax]) continue;
-      int pr[3] = {c[0], c[1], c[2]};
-      pr[ax] += dl;
-      nl[ax][j] = lin3(g, pr[0], pr[1], pr[2]);
-    }
-  const uint8_t cb = P.code[l];
-  const double rhs = A.rhs[l];
-#pragma unroll
-  for (int ax = 0; ax < ND; ax++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) ncode[ax][j] = nl[ax][j] >= 0 ? P.code[nl[ax][j]] : (uint8_t)CODE_NONE;
-  int8_t cm[3];
-  unpack_codes(cb, cm);
-  if ((cb & CODE_SRC_BIT) && P.kL[l] == -EIK_INF) return;  // source points: no unknown
-  double sum = rhs;
-  double dh[3];
-  double gself[ND];
-#pragma unroll
-  for (int ax = 0; ax < ND; ax++) gself[ax] = A.gdt[(long long)ax * N + l];
-#pragma unroll
-  for (int ax = 0; ax < ND; ax++) {
-    double gv[4], lv[4];
-    int pp[4], acc4[4], sg4[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int dl = j < 2 ? j - 2 : j - 1;
-      pp[j] = 0;
-      if (nl[ax][j] < 0) continue;
-      int8_t cd[3];
-      unpack_codes(ncode[ax][j], cd);
-      const int cc = cd[ax];
-      if (cc == 0) continue;
-      const int ac = cc < 0 ? -cc : cc;
-      const int sg = cc > 0 ? -1 : 1;
-      const int p = -dl * sg;
-      if (p < 1 || p > ac) continue;
-      pp[j] = p;
-      acc4[j] = ac;
-      sg4[j] = sg;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      gv[j] = pp[j] ? A.gdt[(long long)ax * N + nl[ax][j]] : 0.0;
-      lv[j] = pp[j] ? __ldcg(A.lam + nl[ax][j]) : 0.0;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      if (!pp[j]) continue;
-      const int dl = j < 2 ? j - 2 : j - 1;
-      node_dh(g, c[0] + (ax == 0 ? dl : 0), dh);
-      const double J = gv[j] * ((double)sg4[j] * dcoeff(acc4[j], pp[j], dh[ax]));
-      sum -= J * lv[j];
-    }
-  }
-  node_dh(g, c[0], dh);
-  double dg = 0.0;
-  bool first = true;
-#pragma unroll
-  for (int ax = 0; ax < ND; ax++) {
-    if (cm[ax] == 0) continue;
-    const int ac = cm[ax] < 0 ? -cm[ax] : cm[ax];
-    const int sg = cm[ax] > 0 ? -1 : 1;
-    const double v = gself[ax] * ((double)sg * dcoeff(ac, 0, dh[ax]));
-    dg = first ? v : dg + v;
-    first = false;
-  }
-  A.lam[l] = sum / dg;
-  __threadfence();
-  // release the nodes this node's stencil reads
-#pragma unroll
-  for (int ax = 0; ax < ND; ax++) {
-    const int ac = cm[ax] < 0 ? -cm[ax] : cm[ax];
-    const int sg = cm[ax] > 0 ? -1 : 1;
-    for (int p = 1; p <= ac; p++) {
-      int q[3] = {c[0], c[1], c[2]};
-      q[ax] += sg * p;
-      const long long lu = lin3(g, q[0], q[1], q[2]);
-      if (atomicSub(a.rs.stamp + gb + lu, 1) == 1) rel[2 * ax + p - 1] = (unsigned int)(gb + lu);
-    }
-  }
-}
-
-template <int ND>
-__global__ void __launch_bounds__(SOLVE_THREADS) adj_rounds_kernel(AdjArgs aa) {
-  const SolveArgs& a = aa.sa;
-  const int lane = threadIdx.x & 31;
-  const unsigned long long N = (unsigned long long)npts(a.probs[0].g);
+  const BrickState& bs = a.bs;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  AdjMem<ND>& w = reinterpret_cast<AdjMem<ND>*>(adj_smem)[warp];
+  const unsigned nwarps = gridDim.x * ADJ_WARPS<ND>;
+  const unsigned gwarp = (unsigned)warp * gridDim.x + blockIdx.x;  // consecutive entries go to different SMs
   int r = 0;
   for (; r < a.rs.max_rounds; r++) {
-    const int b3 = r % 3;
-    const unsigned int n = *(volatile unsigned int*)(a.rs.cnt + b3);
-    if (n == 0) break;
-    const unsigned long long* L = a.rs.list[r & 1];
-    for (;;) {
-      unsigned int base = 0;
-      if (lane == 0) base = atomicAdd(a.rs.grab + b3, 32u);
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (base >= n) break;
-      const unsigned int idx = base + lane;
-      unsigned int rel[6] = {~0u, ~0u, ~0u, ~0u, ~0u, ~0u};
-      if (idx < n) {
-        const unsigned int gid = (unsigned int)(__ldcg(L + idx) >> 32);
-        const int prob = (int)(gid / N);
-        const unsigned long long gb = (unsigned long long)prob * N;
-        adj_node<ND>(aa, prob, (long long)(gid - gb), gb, rel);
+    // lists and phases as in the forward rounds (brick_rounds_kernel); a brick is listed for its
+    // colour's next round by its neighbours only
+    const int col = r & 1, ph = (r >> 1) & 1, oph = ((r + 1) >> 1) & 1;
+    const unsigned n = *(volatile unsigned*)(bs.ctr + 2 * col + ph);
+    if (n == 0 && *(volatile unsigned*)(bs.ctr + 2 * (col ^ 1) + oph) == 0) break;
+    const unsigned* L = bs.lists + (size_t)(2 * col + ph) * bs.listcap;
+    unsigned* Lother = bs.lists + (size_t)(2 * (col ^ 1) + oph) * bs.listcap;
+    unsigned idx = gwarp;
+    while (idx < n) {
+      const unsigned b = __ldcg(L + idx);
+      const int prob = (int)(b / bs.stride);
+      const GridDesc& g = a.probs[prob].g;
+      const unsigned lb = b - (unsigned)prob * bs.stride;
+      const int nb[3] = {bricks_along<ND>(g, 0), bricks_along<ND>(g, 1), ND == 3 ? bricks_along<ND>(g, 2) : 1};
+      const int bc[3] = {(int)(lb % nb[0]), (int)((lb / nb[0]) % nb[1]), (int)(lb / ((unsigned)nb[0] * nb[1]))};
+      if (lane == 0) bs.listed[b] = 0u;
+      const unsigned faces = adj_visit<ND>(w, aa, prob, b, bc, nb, lane);
+      if (lane < B::FACES && ((faces >> lane) & 1u)) {
+        const int ax = lane >> 1;
+        const int st = ax == 0 ? 1 : (ax == 1 ? nb[0] : nb[0] * nb[1]);
+        const unsigned ob = (lane & 1) ? b - st : b + st;  // in the grid: a stencil reads grid nodes only
+        if (atomicExch(bs.listed + ob, 1u) == 0u) Lother[atomicAdd(bs.ctr + 2 * (col ^ 1) + oph, 1u)] = ob;
       }
-#pragma unroll
-      for (int k = 0; k < 2 * ND; k++) warp_append(a, r + 1, rel[k] != ~0u, rel[k]);
+      __syncwarp();
+      if (lane == 0) idx = nwarps + atomicAdd(bs.ctr + 4 + r % 3, 1u);
+      idx = __shfl_sync(FULL_WARP, idx, 0);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-      const int c3 = (r + 2) % 3;
-      a.rs.cnt[c3] = 0;
-      a.rs.grab[c3] = 0;
+      bs.ctr[2 * (col ^ 1) + (oph ^ 1)] = 0u;
+      bs.ctr[4 + (r + 2) % 3] = 0u;
     }
     if (!grid_barrier(a)) break;
   }
@@ -412,14 +535,17 @@ __global__ void __launch_bounds__(SOLVE_THREADS) adj_rounds_kernel(AdjArgs aa) {
   }
 }
 
-__global__ void adj_check_kernel(const AdjProblem* ap, int nprob, long long N, uint32_t* err) {
-  const long long tot = N * nprob;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot; q += (long long)gridDim.x * blockDim.x) {
-    const int s = (int)(q / N);
-    const double v = ap[s].lam[q - (long long)s * N];
-    if (lam_pending(v)) atomicOr(err, ERRB_ADJ_NOT_CONVERGED);
-    else if (!(fabs(v) <= 1.7976931348623157e308)) atomicOr(err, ERRB_SINGULAR);
-  }
+__global__ void adj_init_kernel(AdjArgs aa) {
+  const BrickState& bs = aa.sa.bs;
+  const size_t nb = (size_t)bs.stride * aa.sa.nprob;
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < nb; q += (size_t)gridDim.x * blockDim.x)
+    bs.listed[q] = 0u;
+  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+  for (int k = 0; k < 8; k++) bs.ctr[k] = 0u;
+  aa.sa.rs.bar[0] = 0;
+  aa.sa.rs.bar[1] = 0;
+  *aa.sa.rs.rounds = 0;
+  *aa.sa.abort_flag = 0;
 }
 
 // ------------------------------------------------------ source-region contributions --
@@ -436,6 +562,8 @@ struct SrcTermArgs {
   const AdjProblem* ap;
   const ForwardBatch* fb;
   const double* vel;
+  const double* lam;    // λ in brick order, stride nodes per source
+  size_t stride;
   const double* coordsrc;
   const double* dpsi;   // nsrc x seedcap: ∂ψ/∂u_s
   double* ysrc;         // nsrc x seedcap: ∂ψ/∂u_p ∂u_p/∂u_s
@@ -481,9 +609,8 @@ __global__ void adj_ysrc_kernel(SrcTermArgs sa) {
   const int s = blockIdx.x;
   const ForwardBatch& fb = *sa.fb;
   const CoarseProblem& P = sa.probs[s];
-  const AdjProblem& A = sa.ap[s];
+  const double* lam = sa.lam + (size_t)s * sa.stride;
   const GridDesc& g = sa.g;
-  const long long N = npts(g);
   for (int k = threadIdx.x; k < fb.out[s].nseeds; k += blockDim.x) {
     const long long l = fb.seed_lin[(size_t)s * fb.seedcap + k];
     const int c[3] = {(int)(l % g.n[0]), (int)((l / g.n[0]) % g.n[1]), (int)(l / ((long long)g.n[0] * g.n[1]))};
@@ -497,8 +624,9 @@ __global__ void adj_ysrc_kernel(SrcTermArgs sa) {
         const long long lr = lin3(g, pr[0], pr[1], pr[2]);
         if (is_source(P, lr)) continue;
         bool down;
-        const double J = jcoef(g, P.code, A.gdt, N, ax, dl, lr, pr[0], &down);
-        if (down) y += J * A.lam[lr];
+        const double J = jcoef(P, ax, dl, lr, pr[0], &down);
+        if (down)
+          y += J * lam[g.nd == 3 ? brick_node<3>(g, pr[0], pr[1], pr[2]) : brick_node<2>(g, pr[0], pr[1], pr[2])];
       }
     sa.ysrc[(size_t)s * fb.seedcap + k] = y;
   }
@@ -794,16 +922,23 @@ __global__ void __launch_bounds__(SRCTERM_THREADS) adj_srcterm_kernel(SrcTermArg
 }
 
 // ------------------------------------------------------------- gradient assembly --
-// Per-source field G_s: 2λ/v³ off the source points (eikmaingrad.jl:417-423).
-__global__ void adj_field_kernel(SrcTermArgs sa, long long N) {
-  const long long tot = N * sa.nsrc;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot; q += (long long)gridDim.x * blockDim.x) {
-    const int s = (int)(q / N);
-    const long long l = q - (long long)s * N;
-    const AdjProblem& A = sa.ap[s];
-    if (is_source(sa.probs[s], l)) continue;
+// Checks every λ and, for velocity gradients, writes the per-source field G_s: 2λ/v³ off the
+// source points (eikmaingrad.jl:417-423), 0 on them until adj_srcnodes_kernel.
+template <int ND>
+__global__ void adj_field_kernel(SrcTermArgs sa, long long N, int want, uint32_t* err) {
+  const unsigned long long tot = (unsigned long long)N * sa.nsrc;
+  for (unsigned long long q = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; q < tot;
+       q += (unsigned long long)gridDim.x * blockDim.x) {
+    const int s = (int)(q / (unsigned long long)N);
+    const long long l = (long long)(q - (unsigned long long)s * N);
+    int c[3];
+    node_coords(sa.g, l, c);
+    const double lam = sa.lam[(size_t)s * sa.stride + brick_node<ND>(sa.g, c[0], c[1], c[2])];
+    if (lam_pending(lam)) atomicOr(err, ERRB_ADJ_NOT_CONVERGED);
+    else if (!(fabs(lam) <= 1.7976931348623157e308)) atomicOr(err, ERRB_SINGULAR);
+    if (!want) continue;
     const double v = sa.vel[l];
-    A.lam[l] = 2.0 * A.lam[l] / (v * v * v);
+    sa.ap[s].lam[l] = is_source(sa.probs[s], l) ? 0.0 : 2.0 * lam / (v * v * v);
   }
 }
 
@@ -993,15 +1128,15 @@ __global__ void adj_sum_kernel(const AdjProblem* ap, int nsrc, int s0, const int
 void sum_state_advance(SumState* ss, int nsrc, int s0, const int32_t* gstart);
 
 template <int ND>
-static cudaError_t launch_adj_solve(const AdjArgs& aa, int nsm, cudaStream_t st) {
-  int per = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, adj_rounds_kernel<ND>, SOLVE_THREADS, 0);
-  per = per < 1 ? 1 : per;
+static cudaError_t launch_adj_solve(const AdjArgs& aa, int sms, cudaStream_t st) {
+  const size_t sm = sizeof(AdjMem<ND>) * ADJ_WARPS<ND>;
+  cudaError_t e = cudaFuncSetAttribute(adj_rounds_kernel<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
   AdjArgs args = aa;
   void* kargs[] = {&args};
   // cooperative: every CTA is resident, so the grid barrier between rounds cannot deadlock
-  return cudaLaunchCooperativeKernel((const void*)adj_rounds_kernel<ND>, dim3(nsm * per), dim3(SOLVE_THREADS),
-                                     kargs, 0, st);
+  return cudaLaunchCooperativeKernel((const void*)adj_rounds_kernel<ND>, dim3(sms), dim3(ADJ_WARPS<ND> * 32), kargs, sm,
+                                     st);
 }
 
 }  // namespace eik
@@ -1079,16 +1214,16 @@ void gradient_footprint(const Model& m, const eik_extra& ep, long long nrec, int
   }
   const unsigned long long seedcap = refine ? std::max<unsigned long long>(win, 8) : 8;
   const unsigned long long nf = refine ? nfmax : 1;
-  unsigned long long per = sizeof(SrcOut) + seedcap * (4 + 8) + N * (8 + 1 + 8 + 1) + sizeof(CoarseProblem) +
-                           N * (4 + 8 + 8) + 5 * 8;
-  // brick state: traveltime, code, pending mask, front, flag and four list slots per brick
+  unsigned long long per = sizeof(SrcOut) + seedcap * (4 + 8) + N * (8 + 1 + 8 + 1) + sizeof(CoarseProblem);
+  // brick state: traveltime, code, pending mask, front, flag and four list slots per brick; the
+  // adjoint's λ and node words
   const unsigned long long bn = nd == 3 ? 512 : 256;
   GridDesc wg = m.g;
   for (int d = 0; d < nd; d++) wg.n[d] = (2 * ep.noderadius + 1) * ep.downscalefactor + 1;
   const unsigned long long nbr = std::max(brick_nodes(m.g), refine ? brick_nodes(wg) : 0ull) / bn;
-  per += nbr * (bn * 9 + bn / 8 + 24) + 10 * 4;
+  per += nbr * (bn * 9 + bn / 8 + 24) + 10 * 4 + brick_nodes(m.g) * (8 + 4);
   if (refine) per += nf * (8 + 1 + 1 + 4 + 4 + 1) + sizeof(CoarseProblem) + 8 * (4 + 8) + nf * (8 + 8 + 1) + 1;
-  per += N * (8 + 8ull * nd + 8) + 8 + seedcap * 4 * 8 + nd * 8 + (refine ? nf * (8 + 8ull * nd) : 16) +
+  per += N * 8 + 8 + seedcap * 4 * 8 + nd * 8 + (refine ? nf * (8 + 8ull * nd) : 16) +
          sizeof(AdjProblem);
   per += 3ull * nd * 8 + 8 + 4;  // coordinates, receiver offsets, source-location gradient, group start
   const bool smoothing = (whichgrad == 1 || whichgrad == 3) && ep.smoothgradkern > 0;
@@ -1169,13 +1304,15 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   if (!var) return rc == EIK_ERR_OUT_OF_BUDGET                                       \
                      ? fail(ctx, rc, "scratch '%s' exceeds the HBM budget", name)    \
                      : fail(ctx, rc, "cudaMalloc of scratch '%s' failed", name);
-  double *lam, *gdt, *rhs, *misf, *dpsi, *ysrc, *gnode, *gsrc, *flam, *fgdt, *carry, *gsum, *gw;
+  double *lam, *blam, *misf, *dpsi, *ysrc, *gnode, *gsrc, *flam, *fgdt, *carry, *gsum, *gw;
   AdjProblem* dap;
   ForwardBatch* dfb;
   uint32_t* dwarn;
   GET(lam, double, "adj_lam", nsrc * N);
-  GET(gdt, double, "adj_gdt", nsrc * N * nd);
-  GET(rhs, double, "adj_rhs", nsrc * N);
+  const size_t bstride = (size_t)brick_nodes(m.g);  // brick-ordered nodes of a source
+  uint32_t* binfo;
+  GET(blam, double, "adj_blam", nsrc * bstride);
+  GET(binfo, uint32_t, "adj_info", nsrc * bstride);
   GET(misf, double, "adj_misf", nsrc);
   GET(dpsi, double, "adj_dpsi", nsrc * fw.fb.seedcap);
   GET(ysrc, double, "adj_ysrc", nsrc * fw.fb.seedcap);
@@ -1196,17 +1333,10 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   GET(dap, AdjProblem, "adj_probs", nsrc);
   GET(dfb, ForwardBatch, "adj_fb", 1);
   GET(dwarn, uint32_t, "adj_warn", 1);
-  int32_t* astamp;
-  unsigned long long *alist0, *alist1;
-  GET(astamp, int32_t, "rs_stamp", nsrc * N);
-  GET(alist0, unsigned long long, "rs_list0", nsrc * N);
-  GET(alist1, unsigned long long, "rs_list1", nsrc * N);
 #undef GET
   std::vector<AdjProblem> hap(nsrc);
   for (int64_t s = 0; s < nsrc; s++) {
     hap[s].lam = lam + s * N;
-    hap[s].gdt = gdt + s * N * nd;
-    hap[s].rhs = rhs + s * N;
   }
   const void* hap_src = stage_host(ctx, hap.data(), sizeof(AdjProblem) * nsrc);
   const void* fb_src = stage_host(ctx, &fw.fb, sizeof(ForwardBatch));
@@ -1221,13 +1351,14 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   AdjArgs aa;
   aa.sa = fw.sa;
   aa.ap = dap;
-  aa.sa.rs.stamp = astamp;
-  aa.sa.rs.list[0] = alist0;
-  aa.sa.rs.list[1] = alist1;
+  aa.lam = blam;
+  aa.info = binfo;
   aa.sa.rs.max_rounds = ctx->max_rounds > 0 ? ctx->max_rounds : (1 << 26);
   aa.sa.rs.rounds = fw.sa.rs.rounds + 1;  // the forward's count stays readable
-  adj_rounds_init_kernel<<<1, 1, 0, st>>>(aa.sa);
-  adj_prep_kernel<<<2 * ctx->nsm * 8, 256, 0, st>>>(dprobs, dap, (int)nsrc, N, aa.sa);
+  adj_init_kernel<<<ctx->nsm, 256, 0, st>>>(aa);
+  const int copy_t = fw.in_bricks ? 0 : 1;
+  if (nd == 3) adj_info_kernel<3><<<ctx->nsm * 8, 256, 0, st>>>(aa, copy_t);
+  else adj_info_kernel<2><<<ctx->nsm * 8, 256, 0, st>>>(aa, copy_t);
   RecvArgs ra;
   ra.g = m.g;
   ra.nsrc = (int)nsrc;
@@ -1238,13 +1369,15 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   ra.pickobs = d_po;
   ra.stdobs = d_so;
   ra.fb = dfb;
+  ra.info = binfo;
+  ra.stride = bstride;
   ra.misfit = misf;
   ra.dpsi = dpsi;
-  adj_recv_kernel<<<(int)((nsrc + 63) / 64), 64, 0, st>>>(ra);
+  adj_recv_kernel<<<(int)nsrc, 32, 0, st>>>(ra);
   if (!ctx->capturing) cudaEventRecord(ctx->evk[4], st);
-  CUDA_OK(ctx, nd == 3 ? launch_adj_solve<3>(aa, fw.sms, st) : launch_adj_solve<2>(aa, fw.sms, st));
+  const int asms = ctx->brick_sms((unsigned long long)nsrc * aa.sa.bs.stride);
+  CUDA_OK(ctx, nd == 3 ? launch_adj_solve<3>(aa, asms, st) : launch_adj_solve<2>(aa, asms, st));
   if (!ctx->capturing) cudaEventRecord(ctx->evk[5], st);
-  adj_check_kernel<<<ctx->nsm * 8, 256, 0, st>>>(dap, (int)nsrc, N, fw.fb.err);
   CUDA_OK(ctx, cudaGetLastError());
   SrcTermArgs ta;
   ta.g = m.g;
@@ -1259,6 +1392,8 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   ta.ap = dap;
   ta.fb = dfb;
   ta.vel = m.vel;
+  ta.lam = blam;
+  ta.stride = bstride;
   ta.coordsrc = d_cs;
   ta.dpsi = dpsi;
   ta.ysrc = ysrc;
@@ -1269,8 +1404,9 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   ta.warn = dwarn;
   adj_ysrc_kernel<<<(int)nsrc, 128, 0, st>>>(ta);
   adj_srcterm_kernel<<<(int)nsrc, SRCTERM_THREADS, 0, st>>>(ta);
+  if (nd == 3) adj_field_kernel<3><<<ctx->nsm * 8, 256, 0, st>>>(ta, N, wantvel ? 1 : 0, fw.fb.err);
+  else adj_field_kernel<2><<<ctx->nsm * 8, 256, 0, st>>>(ta, N, wantvel ? 1 : 0, fw.fb.err);
   if (wantvel) {
-    adj_field_kernel<<<ctx->nsm * 8, 256, 0, st>>>(ta, N);
     adj_carry_kernel<<<(int)nsrc, 64, 0, st>>>(ta, ep.radiussmoothgradsrc, carry);
     adj_srcnodes_kernel<<<(int)nsrc, 128, 0, st>>>(ta, carry);
     if (ep.radiussmoothgradsrc > 0) adj_smooth_kernel<<<(int)nsrc, 256, 0, st>>>(ta, ep.radiussmoothgradsrc);
@@ -1324,7 +1460,7 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   tail.dwarn = dwarn;
   tail.arounds = aa.sa.rs.rounds;
   tail.launches = 7 + (d_misfit ? 1 : 0) +
-                  (wantvel ? 3 + (ep.radiussmoothgradsrc > 0 ? 1 : 0) + (d_gradvel ? 1 : 0) : 0) +
+                  (wantvel ? 2 + (ep.radiussmoothgradsrc > 0 ? 1 : 0) + (d_gradvel ? 1 : 0) : 0) +
                   (smoothing ? (int)nout : 0);
   if (tail_out) *tail_out = tail;
   if (ctx->capturing) return EIK_OK;  // read back after each replay of the captured graph

@@ -274,11 +274,9 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   const int64_t nsrc = src_off[nmod];
   const int nd = models[0]->g.nd;
   long long N = 0;  // stride: the largest grid
-  unsigned long long work = 0;
   for (int i = 0; i < nmod; i++) {
     if (models[i]->g.nd != nd) return fail(ctx, EIK_ERR_ASSERT, "models of one call have one dimension");
     N = std::max<long long>(N, models[i]->N);
-    work += (unsigned long long)(src_off[i + 1] - src_off[i]) * (unsigned long long)models[i]->N;
   }
   cudaStream_t st = ctx->stream;
   Scratch& S = ctx->scratch;
@@ -380,8 +378,6 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   {
     unsigned int* rc32;
     GET(rc32, unsigned int, "rs_ctr", 32);
-    sa.rs.cnt = rc32;
-    sa.rs.grab = rc32 + 3;
     sa.rs.bar = rc32 + 6;
     sa.rs.rounds = (int32_t*)(rc32 + 8);
     sa.rs.visits = reinterpret_cast<unsigned long long*>(rc32 + 12);  // 8-byte aligned: 7 counters
@@ -429,7 +425,6 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   if (!hp_src) return fail(ctx, EIK_ERR_CUDA, "cudaMallocHost of a plan's staging copy failed");
   CUDA_OK(ctx, cudaMemcpyAsync(dp, hp_src, sizeof(CoarseProblem) * nsrc, cudaMemcpyHostToDevice, st));
   const double gate = ctx->gate_for(nd);
-  const int sms = ctx->sms_for(work);
   // model i's slice of the per-source arrays, for the per-model start-up launches
   auto slice = [&](int i) {
     ForwardBatch f = fb;
@@ -530,6 +525,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
     if (!ctx->capturing) cudaEventRecord(ctx->evk[3], st);
     CUDA_OK(ctx, cudaGetLastError());
     nlaunch += 2;  // counters, solve
+    fw->in_bricks = false;
   } else {
     launch_bricks_init(sa, st);
     launch_bricks_seed(sa, fb.seed_lin, fb.seed_tt, fb.out, false, fb.seedcap, st);
@@ -540,6 +536,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
     launch_bricks_store(sa, st);
     CUDA_OK(ctx, cudaGetLastError());
     nlaunch += 5;  // counters, brick init, seeds, solve, store
+    fw->in_bricks = true;
   }
   fw->fb = fb;
   fw->sa = sa;
@@ -552,7 +549,6 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   fw->fine_tie = (refine && !ctx->fine_replay) ? ftie : nullptr;
   fw->launches = nlaunch;
   fw->gate = gate;
-  fw->sms = sms;
   if (stats) stats->launches += nlaunch;
   return EIK_OK;
 }

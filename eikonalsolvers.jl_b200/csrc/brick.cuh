@@ -148,19 +148,19 @@ __device__ __noinline__ RuleOut rule_slow(const CoarseProblem& P, const double* 
   return o;
 }
 
-// Copies brick b (of problem P, at brick coordinates bc, bricks nb per axis) and the layers
-// around it that exist to w.cube, the slowness to w.slow; positions outside the grid get +inf.
+// Copies brick b (at brick coordinates bc, bricks nb per axis) of a brick-ordered array and the
+// layers around it that exist to a cube; positions across the grid's faces get `outside`.
 template <int ND>
-__device__ __forceinline__ void load_brick(WarpMem<ND>& w, const BrickState& bs, const CoarseProblem& P, size_t b,
-                                           const int (&bc)[3], const int (&nb)[3], int lane) {
+__device__ __forceinline__ void load_cube(double* cube, const double* array, size_t b, const int (&bc)[3],
+                                          const int (&nb)[3], double outside, int lane) {
   typedef Brick<ND> B;
-  const double* own = bs.t + b * B::NODES;
+  const double* own = array + b * B::NODES;
   constexpr int ROWP = B::BX / 2;  // 16-byte pieces of a row
 #pragma unroll
   for (int q = 0; q < B::NODES / 2; q += 32) {
     const int e = q + lane, row = e / ROWP, xp = e % ROWP;
     const int y = row % B::BY, z = row / B::BY;
-    cp_async16(&w.cube[B::ORG + z * B::PZ + y * B::PY + 2 * xp], own + 2 * e);
+    cp_async16(&cube[B::ORG + z * B::PZ + y * B::PY + 2 * xp], own + 2 * e);
   }
   // layers across the faces: side 0 = +, side 1 = - (as slot())
   const long long bst[3] = {1, nb[0], (long long)nb[0] * nb[1]};
@@ -194,21 +194,14 @@ __device__ __forceinline__ void load_brick(WarpMem<ND>& w, const BrickState& bs,
             si = (z * B::BY + y) * B::BX + 2 * xp;
           }
           if (have) {
-            cp_async16(&w.cube[ci], src + si);
+            cp_async16(&cube[ci], src + si);
           } else {
-            w.cube[ci] = EIK_INF;
-            w.cube[ci + 1] = EIK_INF;
+            cube[ci] = outside;
+            cube[ci + 1] = outside;
           }
         }
       }
     }
-  const GridDesc& g = P.g;
-  const int x0 = bc[0] * B::BX, y0 = bc[1] * B::BY, z0 = bc[2] * B::BZ;
-#pragma unroll
-  for (int q = 0; q < B::NODES; q += 32) {
-    const int e = q + lane, x = x0 + e % B::BX, y = y0 + (e / B::BX) % B::BY, z = z0 + e / (B::BX * B::BY);
-    if (x < g.n[0] && y < g.n[1] && z < g.n[2]) cp_async8(&w.slow[e], P.slow + lin3(g, x, y, z));
-  }
 }
 
 // Visit outcome counters of a warp (lane k < 7 holds outcome k).
@@ -249,7 +242,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND>& w, const BrickState
   double* coef = w.coef();
   unsigned pend = 0u;
   if (lane < B::WORDS) pend = __ldcg(bs.mask + b * B::WORDS + lane);
-  load_brick<ND>(w, bs, P, b, bc, nb, lane);
+  load_cube<ND>(w.cube, bs.t, b, bc, nb, EIK_INF, lane);
   if (lane < B::NODES / 16) cp_async16(&w.code[lane * 16], bs.code + b * B::NODES + lane * 16);
   for (int q = lane; q < B::FACES * B::WORDS; q += 32) w.face[q] = 0u;
   if (lane < 8) w.facemin[lane] = PF_NONE;
@@ -257,6 +250,12 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND>& w, const BrickState
   // them from memory again at every step
   const int n[3] = {P.g.n[0], P.g.n[1], P.g.n[2]};
   const int x0[3] = {bc[0] * B::BX, bc[1] * B::BY, bc[2] * B::BZ};
+#pragma unroll
+  for (int q = 0; q < B::NODES; q += 32) {
+    const int e = q + lane, x = x0[0] + e % B::BX, y = x0[1] + (e / B::BX) % B::BY, z = x0[2] + e / (B::BX * B::BY);
+    if (x < n[0] && y < n[1] && z < n[2])
+      cp_async8(&w.slow[e], P.slow + (x + (long long)n[0] * (y + (long long)n[1] * z)));
+  }
   double* const kL = P.kL;
   uint8_t* const kd = P.kd;
   const bool cart = P.c1u > 0.0;

@@ -80,16 +80,11 @@ EIK_HD void uniform_coeffs(const GridDesc& g, double* c1u, double* c2u) {
   }
 }
 
-// Counters of the round-synchronous solves, and the worklists of the adjoint sweep, whose
-// nodes are numbered over the problems of a call: problem * N + node.
+// Counters of the round-synchronous solves.
 struct RoundState {
-  int32_t* stamp;               // adjoint, per node: dependants not final yet
-  unsigned long long* list[2];  // adjoint: entries of the current and the next round (node id << 32)
-  unsigned int* cnt;            // [3] list length per round (mod 3)
-  unsigned int* grab;           // [3] next list entry to take per round (mod 3)
-  unsigned int* bar;            // [2] grid barrier: arrivals, generation
-  int32_t* rounds;              // rounds run
-  unsigned long long* visits;   // [7] outcomes of the forward's list visits
+  unsigned int* bar;           // [2] grid barrier: arrivals, generation
+  int32_t* rounds;             // rounds run
+  unsigned long long* visits;  // [7] outcomes of the forward's visits
   int32_t max_rounds;
 };
 

@@ -1,12 +1,10 @@
 // Round-synchronous sweeps in one cooperative launch (forward and adjoint solves): the
-// grid barrier between rounds and the warp-aggregated append to a round's worklist.
+// grid barrier between rounds.
 #pragma once
 
 #include "kernels.cuh"
 
 namespace eik {
-
-constexpr int SOLVE_THREADS = 256;  // threads per CTA of the round kernels
 
 __device__ __forceinline__ unsigned long long ld_volatile(const unsigned long long* p) {
   return *(volatile const unsigned long long*)p;
@@ -55,18 +53,6 @@ __device__ __forceinline__ bool grid_barrier(const SolveArgs& a) {
   }
   __syncthreads();
   return s_ok != 0;
-}
-
-// Appends val for every lane of the warp with have set to the worklist of round r, one
-// atomic per warp. All 32 lanes must call it.
-__device__ __forceinline__ void warp_append(const SolveArgs& a, int r, bool have, unsigned int val) {
-  const unsigned m = __ballot_sync(0xffffffffu, have);
-  if (!m) return;
-  const int lane = threadIdx.x & 31;
-  unsigned int base = 0;
-  if (lane == 0) base = atomicAdd(a.rs.cnt + (r % 3), (unsigned int)__popc(m));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (have) a.rs.list[r & 1][base + __popc(m & ((1u << lane) - 1u))] = (unsigned long long)val << 32;
 }
 
 }  // namespace eik

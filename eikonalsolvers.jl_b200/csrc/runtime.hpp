@@ -74,7 +74,7 @@ struct ForwardState {
   const uint8_t* fine_tie = nullptr;  // per-source replay flags of the refined start-up (device)
   int launches = 0;                   // kernels the forward stage launched
   double gate = 2.0;                  // round width used (units of smallest spacing x slowness)
-  int sms = 1;                        // SMs of the persistent solves of this call
+  bool in_bricks = true;              // the coarse traveltimes are in brick order too (SolveArgs::bs)
   std::vector<SrcOut> host_out;
 };
 
@@ -172,15 +172,7 @@ struct eik_ctx {
     const double g = round_gate > 0.0 ? round_gate : (nd == 2 ? 8.0 : 6.0);
     return retry ? 1.5 * g : g;
   }
-  // SMs of the adjoint sweep of a call of `work` node-sources: small ones are bound by their
-  // rounds (each closed by a grid barrier over all resident CTAs) and take fewer.
-  static constexpr unsigned long long SMALL_WORK = 1ull << 22;
-  int sms_for(unsigned long long work) const {
-    const double f = sm_fraction > 0.0 ? sm_fraction : (work < SMALL_WORK ? 0.25 : 1.0);
-    const int n = (int)(f * (double)nsm + 0.5);
-    return n < 1 ? 1 : (n > nsm ? nsm : n);
-  }
-  // SMs of a forward solve over `bricks` bricks: a round visits one colour, so at most half.
+  // SMs of a solve over `bricks` bricks: a round visits one colour, so at most half.
   int brick_sms(unsigned long long bricks) const {
     const int cap = sm_fraction > 0.0 ? std::max(1, std::min(nsm, (int)(sm_fraction * (double)nsm + 0.5))) : nsm;
     return (int)std::max<unsigned long long>(1, std::min<unsigned long long>(cap, (bricks + 1) / 2));
