@@ -23,10 +23,10 @@
 // runs on shared memory. 8^3 nodes with one warp: a front crosses a brick in sheets of about 64
 // nodes, two warp-wide evaluations; larger bricks fill the lanes a little better but leave
 // fewer warps per SM to hide latency. Forward solve, worklists of nodes -> bricks, B200:
-// 256^3 x 4 420 -> 238 ms, 128^3 x 8 123 -> 79 ms, 64^3 x 32 48 -> 29 ms, 128^3 x 1 40 -> 28 ms,
-// 1024x640 x 64 196 -> 58 ms. What bounds it: the longest visit of a round while a round has
-// fewer bricks than the GPU has warps (a visit averages 30 us, the longest of a round 100 us);
-// DRAM and the FP64 pipe are idle (below 1 % and 3 %).
+// 256^3 x 4 420 -> 151 ms, 128^3 x 8 123 -> 54 ms, 64^3 x 32 48 -> 20 ms, 128^3 x 1 40 -> 21 ms,
+// 1024x640 x 64 196 -> 53 ms. What bounds it: the longest visit of a round while a round has
+// fewer bricks than the GPU has warps (256^3 x 4: a visit averages 27 us, the longest of a round
+// 130 us); DRAM and the FP64 pipe are idle (below 1 % and 3 %).
 #pragma once
 
 #include "kernels.cuh"
@@ -114,37 +114,118 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 
 __device__ __forceinline__ bool sign_set(double v) { return __double2hiint(v) < 0; }
 
-// The order rule by full keys, for the nodes the fast rule leaves out (about one in a
-// thousand). Out of line; it reads the neighbourhood again from the cube, so that no array of
-// the visit has an address. t: the node in the cube; ok2: sides (bit slot(axis, side)) where
-// 2nd order is allowed; l: column-major node index; i: radial index.
+// key_le without branches.
+__device__ __forceinline__ bool key_le_flat(const Key& a, const Key& b) {
+  const bool deep = (a.d < b.d) | ((a.d == b.d) & ((a.L == -EIK_INF) | (a.t <= b.t)));
+  return (a.L < b.L) | ((a.L == b.L) & deep);
+}
+
+// The order rule by full keys, for the nodes the fast rule leaves out (about one in a thousand,
+// but clustered), by the whole warp: prefix_rule (stencil.cuh) goes through the groups of equal
+// keys one after the other; here the nodes take 2*ND lanes each, lane j the group of immediate
+// neighbour j, and the rule's result is read off the groups' outcomes: the first one, in the
+// order of the keys, at which the rule ends, or the one before a depth limit. One lane going
+// through the groups took 14 000 cycles, which made the bricks where such nodes cluster the
+// longest visits of a round (with the fast rule taking non-causal and mixed nodes: 256^3 x 4 forward
+// 238 -> 151 ms).
+//
+// Called by all lanes; a lane's inputs are those of its node (the same in the node's 2*ND lanes),
+// and so is what it returns. t: the node in the cube; ok2: sides (bit slot) where 2nd order is
+// allowed; l: column-major node index; i: radial index; active: the lane has a node.
 template <int ND>
 __device__ __noinline__ RuleOut rule_slow(const CoarseProblem& P, const double* t, unsigned ok2, long long l, int i,
-                                          double slow) {
+                                          double slow, bool active, int lane) {
   typedef Brick<ND> B;
-  Nbhd nb;
-  nb_clear(nb);
+  constexpr int G = 2 * ND;
+  const int j = lane % G, base = lane - j;
+  // the keys of immediate neighbour j and of the node beyond it
+  const int a0 = j >> 1;
+  const long long st = a0 == 0 ? 1LL : (a0 == 1 ? (long long)P.g.n[0] : (long long)P.g.n[0] * P.g.n[1]);
+  const int cs = a0 == 0 ? 1 : (a0 == 1 ? B::PY : B::PZ), sh = (j & 1) ? -1 : 1;
+  double v1 = active ? t[sh * cs] : EIK_INF, v2 = active && ((ok2 >> j) & 1u) ? t[2 * sh * cs] : EIK_INF;
+  const bool s1 = sign_set(v1), s2 = sign_set(v2);
+  const double l1 = s1 ? __ldcg(P.kL + l + sh * st) : v1, l2 = s2 ? __ldcg(P.kL + l + 2 * sh * st) : v2;
+  const int d1 = s1 ? (int)__ldcg(P.kd + l + sh * st) : 0, d2 = s2 ? (int)__ldcg(P.kd + l + 2 * sh * st) : 0;
+  v1 = fabs(v1);
+  v2 = fabs(v2);
+  const Key kg{l1, d1, v1};
+  const bool reached = key_reached(kg);
+  NbhdM nb;
+  double L[G];
+  int d[G];
+  unsigned acc = 0u;
+  int rank = 0;
+#pragma unroll
+  for (int k = 0; k < G; k++) {
+    const int from = min(base + k, 31);
+    const Key kn{__shfl_sync(FULL_WARP, l1, from), __shfl_sync(FULL_WARP, d1, from), __shfl_sync(FULL_WARP, v1, from)};
+    const Key km{__shfl_sync(FULL_WARP, l2, from), __shfl_sync(FULL_WARP, d2, from), __shfl_sync(FULL_WARP, v2, from)};
+    acc |= (unsigned)key_le_flat(kn, kg) << k | (unsigned)key_le_flat(km, kg) << (6 + k);
+    rank += !key_le_flat(kg, kn);
+    nb.t1[k >> 1][k & 1] = kn.t;
+    nb.t2[k >> 1][k & 1] = km.t;
+    L[k] = kn.L;
+    d[k] = kn.d;
+  }
   node_dh(P.g, i, nb.dh);
   nb.slow = slow;
   nb.c1u = P.c1u;
   nb.c2u = P.c2u;
+  int8_t cd[3] = {0, 0, 0};
+  bool neg = false;
+  double v = EIK_INF;
+  if (reached) v = update_at_g<ND>(nb, acc, cd, &neg);
+  const bool above = v > kg.L;
+  const Key mine = above ? key_normal(v) : Key{kg.L, kg.d + 1, v};
+  // the next group: the smallest rank above this one's (equal keys share a rank)
+  int next = 7;
+  Key kn = key_unreached();
 #pragma unroll
-  for (int a = 0; a < ND; a++) {
-    const long long st = a == 0 ? 1LL : (a == 1 ? (long long)P.g.n[0] : (long long)P.g.n[0] * P.g.n[1]);
-    const int cs = a == 0 ? 1 : (a == 1 ? B::PY : B::PZ);
-#pragma unroll
-    for (int s = 0; s < 2; s++) {
-      const long long l1 = s == 0 ? l + st : l - st, l2 = s == 0 ? l1 + st : l1 - st;
-      // an absent node is unreached: it is accepted by no group either way
-      const double r1 = t[s == 0 ? cs : -cs], r2 = ((ok2 >> slot(a, s)) & 1u) ? t[s == 0 ? 2 * cs : -2 * cs] : EIK_INF;
-      nb_put1(nb, a, s, fabs(r1), sign_set(r1) ? __ldcg(P.kL + l1) : r1, sign_set(r1) ? (int)__ldcg(P.kd + l1) : 0);
-      nb_put2(nb, a, s, fabs(r2), sign_set(r2) ? __ldcg(P.kL + l2) : r2, sign_set(r2) ? (int)__ldcg(P.kd + l2) : 0);
+  for (int k = 0; k < G; k++) {
+    const int rk = __shfl_sync(FULL_WARP, reached ? rank : 7, min(base + k, 31));
+    if (rk > rank && rk < next) {
+      next = rk;
+      kn = Key{L[k], d[k], nb.t1[k >> 1][k & 1]};
     }
   }
+  // how the rule leaves this group: 2 at the depth limit, 1 with this group's value, 0 onwards
+  const int event = !reached ? 0 : (!above && kg.d >= EIK_MAX_DEPTH && rank > 0) ? 2 : (next == 7 || key_le(mine, kn)) ? 1 : 0;
+  int first = 8, pick = -1, before = -1, brank = -1, fev = 0;
+#pragma unroll
+  for (int k = 0; k < G; k++) {
+    const int code = __shfl_sync(FULL_WARP, reached ? rank * 4 + event : 32, min(base + k, 31));
+    const int rk = code >> 2, ek = code & 3;
+    if (ek && rk < first) {
+      first = rk;
+      fev = ek;
+      pick = k;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < G; k++) {
+    const int rk = __shfl_sync(FULL_WARP, reached ? rank : 8, min(base + k, 31));
+    if (rk < first && rk > brank) {
+      brank = rk;
+      before = k;
+    }
+  }
+  if (fev == 2) pick = before;
+  const int from = min(base + max(pick, 0), 31);
+  const int packed = ((int)(uint8_t)cd[0]) | ((int)(uint8_t)cd[1] << 8) | ((int)(uint8_t)cd[2] << 16);
   RuleOut o;
+  o.v = __shfl_sync(FULL_WARP, v, from);
+  o.key.L = __shfl_sync(FULL_WARP, mine.L, from);
+  o.key.d = __shfl_sync(FULL_WARP, mine.d, from);
+  const int pc = __shfl_sync(FULL_WARP, packed, from);
   o.neg = false;
-  o.cd[0] = o.cd[1] = o.cd[2] = 0;
-  o.v = prefix_rule<ND>(nb, o.cd, &o.key, &o.neg);
+  if (pick < 0) {
+    o.v = EIK_INF;
+    o.key.L = EIK_INF;
+    o.key.d = 0;
+  }
+  o.key.t = o.v;
+#pragma unroll
+  for (int a = 0; a < 3; a++) o.cd[a] = pick < 0 ? (int8_t)0 : (int8_t)(pc >> (8 * a));
   return o;
 }
 
@@ -391,7 +472,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND>& w, const BrickState
         if (Lold == -EIK_INF) oc = VISIT_SOURCE;  // source points are fixed
       }
       const bool ev = act && oc == VISIT_NONE;
-      double nv;
+      double nv, nL;
       int8_t cd[3] = {0, 0, 0};
       bool done;
       {
@@ -412,7 +493,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND>& w, const BrickState
         }
         int8_t cf[ND];
         if (!__any_sync(FULL_WARP, ev && sgn < 0)) {
-          done = prefix_rule_fast<ND, false>(t1, t2, t1, t2, c1, c2, slow, &nv, cf);
+          done = prefix_rule_fast<ND, false>(t1, t2, t1, t2, c1, c2, slow, &nv, &nL, cf);
         } else {
           // special neighbours of some lane: the same with key levels
           const long long l = (x0[0] + x) + (long long)n[0] * ((x0[1] + y) + (long long)n[1] * (x0[2] + z));
@@ -429,21 +510,40 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND>& w, const BrickState
               t2[a][s] = fabs(t2[a][s]);
             }
           }
-          done = prefix_rule_fast<ND, true>(t1, t2, L1, L2, c1, c2, slow, &nv, cf);
+          done = prefix_rule_fast<ND, true>(t1, t2, L1, L2, c1, c2, slow, &nv, &nL, cf);
         }
 #pragma unroll
         for (int a = 0; a < ND; a++) cd[a] = cf[a];
       }
-      double nL = nv;
-      int nd = 0;
-      if (ev && !done) {
-        const long long l = (x0[0] + x) + (long long)n[0] * ((x0[1] + y) + (long long)n[1] * (x0[2] + z));
-        const RuleOut o = rule_slow<ND>(P, &w.cube[ci], ok2, l, x0[0] + x, slow);
-        nv = o.v;
-        nL = o.key.L;
-        nd = o.key.d;
+      int nd = nL == nv ? 0 : 1;
+      for (unsigned sl = __ballot_sync(FULL_WARP, ev && !done); sl;) {
+        // the next 32 / (2*ND) of them, 2*ND lanes each
+        constexpr int G = 2 * ND, PAR = 32 / G;
+        unsigned mine = sl;
+        for (int k = 0; k < lane / G; k++) mine &= mine - 1u;
+        const bool has = mine != 0u && lane < PAR * G;
+        const int src = has ? __ffs(mine) - 1 : 0;
+        const int sq = __shfl_sync(FULL_WARP, q, src), sci = __shfl_sync(FULL_WARP, ci, src);
+        const unsigned sok = __shfl_sync(FULL_WARP, ok2, src);
+        const double ss = __shfl_sync(FULL_WARP, slow, src);
+        const int sx = x0[0] + sq % B::BX;
+        const long long l = sx + (long long)n[0] * ((x0[1] + (sq / B::BX) % B::BY) + (long long)n[1] * (x0[2] + sq / (B::BX * B::BY)));
+        const RuleOut o = rule_slow<ND>(P, &w.cube[sci], sok, l, sx, ss, has, lane);
+        // back to the node's own lane
+        const int place = __popc(sl & below);
+        const bool take = ((sl >> lane) & 1u) && place < PAR;
+        const int from = take ? place * G : 0;
+        const double rv = __shfl_sync(FULL_WARP, o.v, from), rL = __shfl_sync(FULL_WARP, o.key.L, from);
+        const int rd = __shfl_sync(FULL_WARP, o.key.d, from);
+        const int rc = __shfl_sync(FULL_WARP, (o.cd[0] + 2) | (o.cd[1] + 2) << 4 | (o.cd[2] + 2) << 8, from);
+        if (take) {
+          nv = rv;
+          nL = rL;
+          nd = rd;
 #pragma unroll
-        for (int a = 0; a < 3; a++) cd[a] = o.cd[a];
+          for (int a = 0; a < 3; a++) cd[a] = (int8_t)(((rc >> (4 * a)) & 15) - 2);
+        }
+        for (int k = 0; k < PAR && sl; k++) sl &= sl - 1u;
       }
       __syncwarp();  // every lane has read before any writes
       bool changed = false;

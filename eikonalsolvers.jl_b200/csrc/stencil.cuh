@@ -378,8 +378,20 @@ EIK_HD double prefix_rule_plain(const NbhdT& nb, int8_t* codes, Key* key_out, bo
   return EIK_INF;
 }
 
-// Fast form of the order rule: the value, codes and key (v, 0, v) of prefix_rule, bit for bit,
-// or false where it leaves the decision to the general rule. Traveltimes are +inf where the
+// A neighbourhood for one group of the prefix rule, whose accepted nodes are given as a mask: bit
+// slot(axis, side) for distance 1, 6 + that for distance 2.
+struct NbhdM {
+  double t1[3][2];
+  double t2[3][2];
+  double dh[3];
+  double slow;
+  double c1u, c2u;
+};
+EIK_HD bool acc1(const NbhdM&, int a, int l, unsigned T) { return (T >> slot(a, l)) & 1u; }
+EIK_HD bool acc2(const NbhdM&, int a, int l, unsigned T) { return (T >> (6 + slot(a, l))) & 1u; }
+
+// Fast form of the order rule: the value, codes and key of prefix_rule, bit for bit (key level
+// in L_out; the depth is 0 when it equals the value, else 1), or false where it leaves the decision to the general rule. Traveltimes are +inf where the
 // neighbour is outside the grid, unreached or (t2) not allowed; c1, c2 are 1/h^2 and 9/(4h^2)
 // per axis. LEVELS: some neighbour has a special key, and L1, L2 hold the key levels (the
 // traveltime of an ordinary one); without it they are not read.
@@ -403,14 +415,16 @@ EIK_HD double prefix_rule_plain(const NbhdT& nb, int8_t* codes, Key* key_out, bo
 // that happens before the node's own acceptance on one axis, the groups from side 0's
 // traveltime on are decided again with the axis' new point.
 //
-// Left to the general rule: a value not above its group (non-causal), a negative discriminant,
-// mixed sides on several axes. With levels, also: source points; an axis with a special key
+// A value not above its group (non-causal) ends the rule: its key is (group, 1, value).
+//
+// Left to the general rule: a negative discriminant, mixed sides on several axes or with a
+// non-causal value. With levels, also: a non-causal value; source points; an axis with a special key
 // whose other side is accepted before the node; a 2nd-order point accepted after its 1st-order
 // one and before the node.
 template <int ND, bool LEVELS>
 EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2], const double (&L1)[ND][2],
                              const double (&L2)[ND][2], const double (&c1)[ND], const double (&c2)[ND], double slow,
-                             double* v_out, int8_t* codes) {
+                             double* v_out, double* L_out, int8_t* codes) {
   const double s2 = slow * slow;
   double m[ND], x[ND], ca[ND], lev[ND], mar = 0.0;
   uint32_t second = 0u, side = 0u, late = 0u, keyed = 0u;
@@ -450,7 +464,7 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
 #pragma unroll
   for (int a = 0; a < ND; a++) codes[a] = 0;
   if (!(first < EIK_INF)) {
-    *v_out = EIK_INF;
+    *v_out = *L_out = EIK_INF;
     return ok;
   }
   // the axes in the order of their acceptance: group k is the first k of them
@@ -477,8 +491,8 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
   // straight-line: lanes of a warp end at different groups
   double d = sm[0] - sx[0];
   double q = sc[0] * (d * d);  // q + slow^2 of the group at its own level
-  ok = ok && q < s2 - (1e-9 * s2 + mar * (sm[0] * sm[0]));  // else the value may not lie above it
-  bool open = true;
+  // a group the value may not lie above ends the rule there (checked on the exact value below)
+  bool below = !(q < s2 - (1e-9 * s2 + mar * (sm[0] * sm[0]))), open = !below;
   double tg = sm[0];
 #pragma unroll
   for (int g = 1; g < ND; g++) {
@@ -490,10 +504,14 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
     }
     const double band = 1e-9 * s2 + mar * (sm[g] * sm[g]);
     open = open && sm[g] < EIK_INF && !(q > s2 + band);  // q above: the value is below group g, accepted
+    ok = ok && (!open || q < s2 - band);
     d = sm[g] - sx[g];
     q = fma(sc[g], d * d, q);  // with axis g itself, at its own level
-    ok = ok && (!open || q < s2 - band);
     tg = open ? sm[g] : tg;
+    if (open && !(q < s2 - band)) {
+      below = true;
+      open = false;
+    }
   }
   auto root = [&](double* v) {
     double alpha = 0.0, beta = 0.0, gamma = -s2;
@@ -511,10 +529,13 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
   };
   double v;
   ok = root(&v) && ok;
+  if (below && (LEVELS || !(v < tg))) ok = false;
+  const double reach = below ? tg : v;  // neighbours up to here are accepted before the node
   uint32_t mixed = 0u;
 #pragma unroll
   for (int a = 0; a < ND; a++) {
-    if ((((side & ~second) >> a) & 1u) && t1[a][0] < v && t2[a][0] <= t1[a][0] && t2[a][1] > t1[a][0])
+    if ((((side & ~second) >> a) & 1u) && (below ? t1[a][0] <= reach : t1[a][0] < reach) && t2[a][0] <= t1[a][0] &&
+        t2[a][1] > t1[a][0])
       mixed |= 1u << a;
     if (LEVELS && ((keyed >> a) & 1u)) {
       const bool hi = (side >> a) & 1u;
@@ -523,8 +544,8 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
     }
   }
   if (mixed) {
-    if (LEVELS || (mixed & (mixed - 1u))) return false;
-    double keep = EIK_INF;  // side 1's own 2nd-order point must stay unaccepted
+    if (LEVELS || below || (mixed & (mixed - 1u))) return false;
+    double keep = EIK_INF;  // side 1's own distance-2 node must stay unaccepted up to the last group
 #pragma unroll
     for (int a = 0; a < ND; a++)
       if ((mixed >> a) & 1u) {
@@ -555,11 +576,13 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
       ok = ok && (!open || qn < s2 - band);
       tg = open ? tn : tg;
     }
-    ok = root(&v) && ok && keep > v;
+    ok = root(&v) && ok;
 #pragma unroll
-    for (int a = 0; a < ND; a++)
+    for (int a = 0; a < ND; a++) {
+      if ((t1[a][0] < v && t1[a][0] >= keep) || (t1[a][1] < v && t1[a][1] >= keep)) ok = false;
       if ((((side & ~second & ~mixed) >> a) & 1u) && t1[a][0] < v && t2[a][0] <= t1[a][0] && t2[a][1] > t1[a][0])
         ok = false;
+    }
   }
 #pragma unroll
   for (int a = 0; a < ND; a++) {
@@ -567,6 +590,7 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
     codes[a] = (int8_t)(lev[a] <= tg ? (((second >> a) & 1u) ? 2 * sh : sh) : 0);
   }
   *v_out = v;
+  *L_out = below ? tg : v;
   return ok;
 }
 

@@ -65,13 +65,13 @@ static void run(long long cases, unsigned long long seed, bool specials) {
     int8_t cr[3] = {0, 0, 0}, cf[ND];
     Key key;
     bool neg = false;
-    double vf;
+    double vf, Lf;
     const double v = prefix_rule<ND>(nb, cr, &key, &neg);
-    const bool ok = special ? prefix_rule_fast<ND, true>(t1, t2, L1, L2, c1, c2, nb.slow, &vf, cf)
-                            : prefix_rule_fast<ND, false>(t1, t2, t1, t2, c1, c2, nb.slow, &vf, cf);
+    const bool ok = special ? prefix_rule_fast<ND, true>(t1, t2, L1, L2, c1, c2, nb.slow, &vf, &Lf, cf)
+                            : prefix_rule_fast<ND, false>(t1, t2, t1, t2, c1, c2, nb.slow, &vf, &Lf, cf);
     if (!ok) continue;
     decided++;
-    if (std::memcmp(&v, &vf, 8) || std::memcmp(&key.L, &vf, 8) || key.d != 0 || neg || std::memcmp(cr, cf, ND)) differing++;
+    if (std::memcmp(&v, &vf, 8) || std::memcmp(&key.L, &Lf, 8) || key.d != (Lf == vf ? 0 : 1) || neg || std::memcmp(cr, cf, ND)) differing++;
   }
   std::printf("%lld %lld\n", decided, differing);
 }
