@@ -23,10 +23,10 @@
 // runs on shared memory. 8^3 nodes with one warp: a front crosses a brick in sheets of about 64
 // nodes, two warp-wide evaluations; larger bricks fill the lanes a little better but leave
 // fewer warps per SM to hide latency. Forward solve, worklists of nodes -> bricks, B200:
-// 256^3 x 4 420 -> 151 ms, 128^3 x 8 123 -> 54 ms, 64^3 x 32 48 -> 20 ms, 128^3 x 1 40 -> 21 ms,
-// 1024x640 x 64 196 -> 53 ms. What bounds it: the longest visit of a round while a round has
-// fewer bricks than the GPU has warps (256^3 x 4: a visit averages 27 us, the longest of a round
-// 130 us); DRAM and the FP64 pipe are idle (below 1 % and 3 %).
+// 256^3 x 4 420 -> 122 ms, 128^3 x 8 123 -> 45 ms, 64^3 x 32 48 -> 16 ms, 128^3 x 1 40 -> 19 ms,
+// 1024x640 x 64 196 -> 44 ms. What bounds it: the longest visit of a round while a round has
+// fewer bricks than the GPU has warps (256^3 x 4: a visit averages 25 us, the longest of a round
+// 90 us); DRAM and the FP64 pipe are idle (below 1 % and 3 %).
 #pragma once
 
 #include "kernels.cuh"
@@ -298,10 +298,13 @@ struct VisitTally {
   }
 };
 
-// Evaluations a visit may start before it hands its pending nodes back to the next round: a
-// visit settles in a few dozen, and the bound keeps a schedule that alternates (the rule's
-// depth limit lets some transient keys do so) from holding the round.
-constexpr int VISIT_MAX_SCANS = 192;
+// Scans (steps of up to two warps of nodes) of a visit before it hands its pending nodes back
+// to the next round of its colour. A visit needs about eight; a few need a hundred and would
+// hold up the round: 256^3 x 4 at 8 / 12 / 16 / 24 / 192 scans: 140 / 126 / 122 / 129 / 150 ms, 64^3 x
+// 32 18.2 / 16.6 / 17.0 / 19.4 / 20.5 ms, 1024x640 x 64 61 / 53 / 49 / 44 / 53 ms. It also ends a visit in
+// which values alternate (the rule's depth limit lets some transient keys do so).
+template <int ND>
+constexpr int VISIT_MAX_SCANS = ND == 3 ? 16 : 24;
 
 // Which steps -2, -1, +1, +2 along an axis stay within [lo, hi) from position p: bits 0..3 of
 // nibble p of the table, for positions 0..15 (low half: 0..7).
@@ -393,7 +396,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND>& w, const BrickState
       mn = min(mn, v[k]);
     }
     mn = __reduce_min_sync(FULL_WARP, mn);
-    if (mn > Tb || mn == PF_NONE || it >= VISIT_MAX_SCANS) {
+    if (mn > Tb || mn == PF_NONE || it >= VISIT_MAX_SCANS<ND>) {
       left = mn;
 #pragma unroll
       for (int k = 0; k < B::WORDS; k++) {
