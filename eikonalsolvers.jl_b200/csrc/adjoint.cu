@@ -68,10 +68,9 @@ __device__ __forceinline__ bool info_far(uint32_t f, int ax, bool plus) { return
 constexpr uint32_t INFO_DEPS = 0x3ffffu << 8;
 
 // Lists the bricks that hold a node without dependants for the first round of their colour.
-// copy_t: the forward left its traveltimes in the problems' own arrays only.
-template <int ND>
-__global__ void adj_info_kernel(AdjArgs aa, int copy_t) {
-  typedef Brick<ND> B;
+template <int ND, bool SMALL>
+__global__ void adj_info_kernel(AdjArgs aa) {
+  typedef Brick<ND, SMALL> B;
   const BrickState& bs = aa.sa.bs;
   const size_t total = (size_t)bs.stride * aa.sa.nprob * B::NODES;
   // every 32 consecutive nodes belong to one brick
@@ -80,7 +79,7 @@ __global__ void adj_info_kernel(AdjArgs aa, int copy_t) {
     const unsigned p = b / bs.stride, lb = b - p * bs.stride;
     const CoarseProblem& P = aa.sa.probs[p];
     const GridDesc& g = P.g;
-    const unsigned nb0 = (unsigned)bricks_along<ND>(g, 0), nb1 = (unsigned)bricks_along<ND>(g, 1);
+    const unsigned nb0 = (unsigned)bricks_along<ND, SMALL>(g, 0), nb1 = (unsigned)bricks_along<ND, SMALL>(g, 1);
     const unsigned bx = lb % nb0, by = (lb / nb0) % nb1, bz = lb / (nb0 * nb1);
     const int c[3] = {(int)(bx * B::BX + q % B::BX), (int)(by * B::BY + (q / B::BX) % B::BY),
                       (int)(bz * B::BZ + q / (B::BX * B::BY))};
@@ -89,7 +88,6 @@ __global__ void adj_info_kernel(AdjArgs aa, int copy_t) {
     if (c[0] < g.n[0] && c[1] < g.n[1] && c[2] < g.n[2]) {
       const long long l = lin3(g, c[0], c[1], c[2]);
       const uint8_t cb = P.code[l];
-      if (copy_t) bs.t[id] = P.t[l];
       f = cb & 0x7fu;
       if (cb == (uint8_t)(CODE_NONE | CODE_SRC_BIT)) f |= INFO_FIXED;  // no other special node has these codes
       else lam = __longlong_as_double((long long)LAM_PENDING_BITS);
@@ -156,6 +154,7 @@ struct RecvArgs {
   const ForwardBatch* fb;
   uint32_t* info;   // adjoint words in brick order: INFO_RHS is set at the receivers' nodes
   size_t stride;    // brick-ordered nodes of a source
+  int small;        // small bricks
   double* misfit;   // nsrc
   double* dpsi;     // nsrc x seedcap: ∂ψ/∂u_s per source point
 };
@@ -234,7 +233,7 @@ __global__ void __launch_bounds__(32) adj_recv_kernel(RecvArgs ra) {
     for (int c = 0; c < nc; c++) {
       int x[3];
       node_coords(g, node[c], x);
-      const long long q = g.nd == 3 ? brick_node<3>(g, x[0], x[1], x[2]) : brick_node<2>(g, x[0], x[1], x[2]);
+      const long long q = brick_node(g, ra.small != 0, x[0], x[1], x[2]);
       if (info[q] & INFO_FIXED) continue;
       atomicOr(info + q, INFO_RHS);
       __stcg(rhs + node[c], 0.0);
@@ -293,9 +292,9 @@ __global__ void __launch_bounds__(32) adj_recv_kernel(RecvArgs ra) {
 // and a pass that stored 2 (D_a t) per axis; a visit takes the levels inside its brick from shared
 // memory (128^3: 80 rounds, 3.2 visits a brick). Sweep and preparation, worklists -> bricks, B200:
 // 256^3 x 4 54 -> 31 ms, 1024x640 x 64 47 -> 9 ms, 300x220 x 4 6.0 -> 1.4 ms, 64^3 x 32 8.0 -> 5.4 ms.
-template <int ND>
+template <int ND, bool SMALL>
 struct __align__(16) AdjMem {
-  typedef Brick<ND> B;
+  typedef Brick<ND, SMALL> B;
   double t[B::CUBE];
   double lam[B::CUBE];
   uint32_t info[B::NODES];
@@ -304,25 +303,24 @@ struct __align__(16) AdjMem {
   double extra[ND == 3 ? 2 : 64];
   unsigned tail;
   // spherical grids: 1/h, 3/(2h), 4/(2h), 1/(2h) of axis 1 (and 2) per radial index of the brick, in
-  // corners of the cube that no stencil reads (brick.cuh)
-  __device__ __forceinline__ double* coef(int ax) { return ND == 3 ? t + (ax == 1 ? 120 : 1560) : extra; }
+  // free runs of the cube (brick.cuh)
+  __device__ __forceinline__ double* coef(int ax) { return ND == 3 ? t + (ax == 1 ? B::FREE1 : B::FREE2) : extra; }
 };
-// t + 1560..1607 lie in the rows y = 8, 9 of the plane z = 8 and y = -2, -1 of the next
 constexpr unsigned CNT_FIXED = 0x40000000u;
-// 32.8 KB a warp in 3D: 7 warps an SM; 9.5 KB in 2D
-template <int ND>
-constexpr int ADJ_WARPS = ND == 3 ? 7 : 16;
+// 32.8 KB a warp in 3D: 7 warps an SM; 9.5 KB in 2D, 9 KB and 3.4 KB with small bricks
+template <int ND, bool SMALL>
+constexpr int ADJ_WARPS = ND == 3 && !SMALL ? 7 : 16;
 
 __device__ __forceinline__ bool pending_hi(double v) { return (unsigned)__double2hiint(v) == (unsigned)(LAM_PENDING_BITS >> 32); }
 
 // Visits brick b; returns the faces (bit 2*axis + (0: +, 1: -)) its computed nodes' stencils reach.
-template <int ND>
-__device__ __forceinline__ unsigned adj_visit(AdjMem<ND>& w, const AdjArgs& aa, int prob, size_t b, const int (&bc)[3],
+template <int ND, bool SMALL>
+__device__ __forceinline__ unsigned adj_visit(AdjMem<ND, SMALL>& w, const AdjArgs& aa, int prob, size_t b, const int (&bc)[3],
                                               const int (&nb)[3], int lane) {
-  typedef Brick<ND> B;
+  typedef Brick<ND, SMALL> B;
   const CoarseProblem& P = aa.sa.probs[prob];
-  load_cube<ND>(w.t, aa.sa.bs.t, b, bc, nb, EIK_INF, lane);
-  load_cube<ND>(w.lam, aa.lam, b, bc, nb, 0.0, lane);
+  load_cube<ND, SMALL>(w.t, aa.sa.bs.t, b, bc, nb, EIK_INF, lane);
+  load_cube<ND, SMALL>(w.lam, aa.lam, b, bc, nb, 0.0, lane);
 #pragma unroll
   for (int q = 0; q < B::NODES / 4; q += 32)
     if (q + lane < B::NODES / 4) cp_async16(&w.info[4 * (q + lane)], aa.info + b * B::NODES + 4 * (q + lane));
@@ -481,15 +479,15 @@ __device__ __forceinline__ unsigned adj_visit(AdjMem<ND>& w, const AdjArgs& aa, 
   return __reduce_or_sync(FULL_WARP, faces);
 }
 
-template <int ND>
-__global__ void __launch_bounds__(ADJ_WARPS<ND> * 32, 1) adj_rounds_kernel(AdjArgs aa) {
-  typedef Brick<ND> B;
+template <int ND, bool SMALL>
+__global__ void __launch_bounds__(ADJ_WARPS<ND, SMALL> * 32, 1) adj_rounds_kernel(AdjArgs aa) {
+  typedef Brick<ND, SMALL> B;
   extern __shared__ __align__(16) unsigned char adj_smem[];
   const SolveArgs& a = aa.sa;
   const BrickState& bs = a.bs;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  AdjMem<ND>& w = reinterpret_cast<AdjMem<ND>*>(adj_smem)[warp];
-  const unsigned nwarps = gridDim.x * ADJ_WARPS<ND>;
+  AdjMem<ND, SMALL>& w = reinterpret_cast<AdjMem<ND, SMALL>*>(adj_smem)[warp];
+  const unsigned nwarps = gridDim.x * ADJ_WARPS<ND, SMALL>;
   const unsigned gwarp = (unsigned)warp * gridDim.x + blockIdx.x;  // consecutive entries go to different SMs
   int r = 0;
   for (; r < a.rs.max_rounds; r++) {
@@ -506,10 +504,10 @@ __global__ void __launch_bounds__(ADJ_WARPS<ND> * 32, 1) adj_rounds_kernel(AdjAr
       const int prob = (int)(b / bs.stride);
       const GridDesc& g = a.probs[prob].g;
       const unsigned lb = b - (unsigned)prob * bs.stride;
-      const int nb[3] = {bricks_along<ND>(g, 0), bricks_along<ND>(g, 1), ND == 3 ? bricks_along<ND>(g, 2) : 1};
+      const int nb[3] = {bricks_along<ND, SMALL>(g, 0), bricks_along<ND, SMALL>(g, 1), ND == 3 ? bricks_along<ND, SMALL>(g, 2) : 1};
       const int bc[3] = {(int)(lb % nb[0]), (int)((lb / nb[0]) % nb[1]), (int)(lb / ((unsigned)nb[0] * nb[1]))};
       if (lane == 0) bs.listed[b] = 0u;
-      const unsigned faces = adj_visit<ND>(w, aa, prob, b, bc, nb, lane);
+      const unsigned faces = adj_visit<ND, SMALL>(w, aa, prob, b, bc, nb, lane);
       if (lane < B::FACES && ((faces >> lane) & 1u)) {
         const int ax = lane >> 1;
         const int st = ax == 0 ? 1 : (ax == 1 ? nb[0] : nb[0] * nb[1]);
@@ -564,6 +562,7 @@ struct SrcTermArgs {
   const double* vel;
   const double* lam;    // λ in brick order, stride nodes per source
   size_t stride;
+  int small;            // small bricks
   const double* coordsrc;
   const double* dpsi;   // nsrc x seedcap: ∂ψ/∂u_s
   double* ysrc;         // nsrc x seedcap: ∂ψ/∂u_p ∂u_p/∂u_s
@@ -626,7 +625,7 @@ __global__ void adj_ysrc_kernel(SrcTermArgs sa) {
         bool down;
         const double J = jcoef(P, ax, dl, lr, pr[0], &down);
         if (down)
-          y += J * lam[g.nd == 3 ? brick_node<3>(g, pr[0], pr[1], pr[2]) : brick_node<2>(g, pr[0], pr[1], pr[2])];
+          y += J * lam[brick_node(g, sa.small != 0, pr[0], pr[1], pr[2])];
       }
     sa.ysrc[(size_t)s * fb.seedcap + k] = y;
   }
@@ -924,7 +923,7 @@ __global__ void __launch_bounds__(SRCTERM_THREADS) adj_srcterm_kernel(SrcTermArg
 // ------------------------------------------------------------- gradient assembly --
 // Checks every λ and, for velocity gradients, writes the per-source field G_s: 2λ/v³ off the
 // source points (eikmaingrad.jl:417-423), 0 on them until adj_srcnodes_kernel.
-template <int ND>
+template <int ND, bool SMALL>
 __global__ void adj_field_kernel(SrcTermArgs sa, long long N, int want, uint32_t* err) {
   const unsigned long long tot = (unsigned long long)N * sa.nsrc;
   for (unsigned long long q = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; q < tot;
@@ -933,7 +932,7 @@ __global__ void adj_field_kernel(SrcTermArgs sa, long long N, int want, uint32_t
     const long long l = (long long)(q - (unsigned long long)s * N);
     int c[3];
     node_coords(sa.g, l, c);
-    const double lam = sa.lam[(size_t)s * sa.stride + brick_node<ND>(sa.g, c[0], c[1], c[2])];
+    const double lam = sa.lam[(size_t)s * sa.stride + brick_node<ND, SMALL>(sa.g, c[0], c[1], c[2])];
     if (lam_pending(lam)) atomicOr(err, ERRB_ADJ_NOT_CONVERGED);
     else if (!(fabs(lam) <= 1.7976931348623157e308)) atomicOr(err, ERRB_SINGULAR);
     if (!want) continue;
@@ -1127,15 +1126,15 @@ __global__ void adj_sum_kernel(const AdjProblem* ap, int nsrc, int s0, const int
 // The group state after sources s0 .. s0+nsrc-1 (the same steps as the sums, on the host).
 void sum_state_advance(SumState* ss, int nsrc, int s0, const int32_t* gstart);
 
-template <int ND>
+template <int ND, bool SMALL>
 static cudaError_t launch_adj_solve(const AdjArgs& aa, int sms, cudaStream_t st) {
-  const size_t sm = sizeof(AdjMem<ND>) * ADJ_WARPS<ND>;
-  cudaError_t e = cudaFuncSetAttribute(adj_rounds_kernel<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const size_t sm = sizeof(AdjMem<ND, SMALL>) * ADJ_WARPS<ND, SMALL>;
+  cudaError_t e = cudaFuncSetAttribute(adj_rounds_kernel<ND, SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   AdjArgs args = aa;
   void* kargs[] = {&args};
   // cooperative: every CTA is resident, so the grid barrier between rounds cannot deadlock
-  return cudaLaunchCooperativeKernel((const void*)adj_rounds_kernel<ND>, dim3(sms), dim3(ADJ_WARPS<ND> * 32), kargs, sm,
+  return cudaLaunchCooperativeKernel((const void*)adj_rounds_kernel<ND, SMALL>, dim3(sms), dim3(ADJ_WARPS<ND, SMALL> * 32), kargs, sm,
                                      st);
 }
 
@@ -1215,13 +1214,19 @@ void gradient_footprint(const Model& m, const eik_extra& ep, long long nrec, int
   const unsigned long long seedcap = refine ? std::max<unsigned long long>(win, 8) : 8;
   const unsigned long long nf = refine ? nfmax : 1;
   unsigned long long per = sizeof(SrcOut) + seedcap * (4 + 8) + N * (8 + 1 + 8 + 1) + sizeof(CoarseProblem);
-  // brick state: traveltime, code, pending mask, front, flag and four list slots per brick; the
-  // adjoint's λ and node words
-  const unsigned long long bn = nd == 3 ? 512 : 256;
+  // brick state: traveltime, code, pending mask, front, flag and four list slots per brick, the
+  // larger of both brick sizes; the adjoint's λ and node words
   GridDesc wg = m.g;
   for (int d = 0; d < nd; d++) wg.n[d] = (2 * ep.noderadius + 1) * ep.downscalefactor + 1;
-  const unsigned long long nbr = std::max(brick_nodes(m.g), refine ? brick_nodes(wg) : 0ull) / bn;
-  per += nbr * (bn * 9 + bn / 8 + 24) + 10 * 4 + brick_nodes(m.g) * (8 + 4);
+  unsigned long long nodes = 0, cnodes = 0, nbr = 0;
+  for (int small = 0; small < 2; small++) {
+    const unsigned long long cb = brick_number(m.g, small != 0), fb = refine ? brick_number(wg, small != 0) : 0ull;
+    const unsigned long long bn = brick_size(nd, small != 0);
+    nodes = std::max(nodes, std::max(cb, fb) * bn);
+    cnodes = std::max(cnodes, cb * bn);
+    nbr = std::max(nbr, std::max(cb, fb));
+  }
+  per += nodes * 9 + nodes / 8 + nbr * 24 + 10 * 4 + cnodes * (8 + 4);
   if (refine) per += nf * (8 + 1 + 1 + 4 + 4 + 1) + sizeof(CoarseProblem) + 8 * (4 + 8) + nf * (8 + 8 + 1) + 1;
   per += N * 8 + 8 + seedcap * 4 * 8 + nd * 8 + (refine ? nf * (8 + 8ull * nd) : 16) +
          sizeof(AdjProblem);
@@ -1309,7 +1314,8 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   ForwardBatch* dfb;
   uint32_t* dwarn;
   GET(lam, double, "adj_lam", nsrc * N);
-  const size_t bstride = (size_t)brick_nodes(m.g);  // brick-ordered nodes of a source
+  const bool small = fw.sa.bs.small != 0;
+  const size_t bstride = (size_t)fw.sa.bs.stride * brick_size(nd, small);  // brick-ordered nodes of a source
   uint32_t* binfo;
   GET(blam, double, "adj_blam", nsrc * bstride);
   GET(binfo, uint32_t, "adj_info", nsrc * bstride);
@@ -1356,9 +1362,9 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   aa.sa.rs.max_rounds = ctx->max_rounds > 0 ? ctx->max_rounds : (1 << 26);
   aa.sa.rs.rounds = fw.sa.rs.rounds + 1;  // the forward's count stays readable
   adj_init_kernel<<<ctx->nsm, 256, 0, st>>>(aa);
-  const int copy_t = fw.in_bricks ? 0 : 1;
-  if (nd == 3) adj_info_kernel<3><<<ctx->nsm * 8, 256, 0, st>>>(aa, copy_t);
-  else adj_info_kernel<2><<<ctx->nsm * 8, 256, 0, st>>>(aa, copy_t);
+  auto info = [&](auto kernel) { kernel<<<ctx->nsm * 8, 256, 0, st>>>(aa); };
+  if (nd == 3) small ? info(adj_info_kernel<3, true>) : info(adj_info_kernel<3, false>);
+  else small ? info(adj_info_kernel<2, true>) : info(adj_info_kernel<2, false>);
   RecvArgs ra;
   ra.g = m.g;
   ra.nsrc = (int)nsrc;
@@ -1371,12 +1377,14 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   ra.fb = dfb;
   ra.info = binfo;
   ra.stride = bstride;
+  ra.small = small ? 1 : 0;
   ra.misfit = misf;
   ra.dpsi = dpsi;
   adj_recv_kernel<<<(int)nsrc, 32, 0, st>>>(ra);
   if (!ctx->capturing) cudaEventRecord(ctx->evk[4], st);
   const int asms = ctx->brick_sms((unsigned long long)nsrc * aa.sa.bs.stride);
-  CUDA_OK(ctx, nd == 3 ? launch_adj_solve<3>(aa, asms, st) : launch_adj_solve<2>(aa, asms, st));
+  CUDA_OK(ctx, nd == 3 ? (small ? launch_adj_solve<3, true>(aa, asms, st) : launch_adj_solve<3, false>(aa, asms, st))
+                       : (small ? launch_adj_solve<2, true>(aa, asms, st) : launch_adj_solve<2, false>(aa, asms, st)));
   if (!ctx->capturing) cudaEventRecord(ctx->evk[5], st);
   CUDA_OK(ctx, cudaGetLastError());
   SrcTermArgs ta;
@@ -1394,6 +1402,7 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   ta.vel = m.vel;
   ta.lam = blam;
   ta.stride = bstride;
+  ta.small = small ? 1 : 0;
   ta.coordsrc = d_cs;
   ta.dpsi = dpsi;
   ta.ysrc = ysrc;
@@ -1404,8 +1413,9 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
   ta.warn = dwarn;
   adj_ysrc_kernel<<<(int)nsrc, 128, 0, st>>>(ta);
   adj_srcterm_kernel<<<(int)nsrc, SRCTERM_THREADS, 0, st>>>(ta);
-  if (nd == 3) adj_field_kernel<3><<<ctx->nsm * 8, 256, 0, st>>>(ta, N, wantvel ? 1 : 0, fw.fb.err);
-  else adj_field_kernel<2><<<ctx->nsm * 8, 256, 0, st>>>(ta, N, wantvel ? 1 : 0, fw.fb.err);
+  auto field = [&](auto kernel) { kernel<<<ctx->nsm * 8, 256, 0, st>>>(ta, N, wantvel ? 1 : 0, fw.fb.err); };
+  if (nd == 3) small ? field(adj_field_kernel<3, true>) : field(adj_field_kernel<3, false>);
+  else small ? field(adj_field_kernel<2, true>) : field(adj_field_kernel<2, false>);
   if (wantvel) {
     adj_carry_kernel<<<(int)nsrc, 64, 0, st>>>(ta, ep.radiussmoothgradsrc, carry);
     adj_srcnodes_kernel<<<(int)nsrc, 128, 0, st>>>(ta, carry);

@@ -196,14 +196,14 @@ const void* stage_host(eik_ctx* ctx, const void* src, size_t bytes) {
 // Round width and lower-bound increment of every coarse problem from the model's smallest
 // slowness, read on the device (the expressions and their order are the host's).
 __global__ void problem_scale_kernel(CoarseProblem* dp, int nprob, const double* dsmin, double gate, double hmin,
-                                     int nd) {
+                                     int nd, int small) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nprob) return;
   const double smin = *dsmin;
   dp[s].delta = gate * hmin * smin;
   dp[s].incmin = 0.999 * (2.0 / 3.0) * hmin * smin / sqrt((double)nd);
   dp[s].linc = 0.999 * (2.0 / 3.0) * hmin / sqrt((double)nd);
-  dp[s].din = inner_window(nd, hmin * smin);
+  dp[s].din = inner_window(nd, small != 0, hmin * smin);
 }
 
 int model_create(eik_ctx* ctx, const eik_grid* grd, const double* vel, bool dev, eik_model_id* out) {
@@ -257,6 +257,27 @@ int err_to_rc(eik_ctx* ctx, uint32_t e) {
     return fail(ctx, EIK_ERR_NOT_CONVERGED, "iteration limit reached (error word 0x%x)", e);
   if (e & ERRB_SINGULAR) return fail(ctx, EIK_ERR_ERROR, "SingularException in the adjoint solve");
   return fail(ctx, EIK_ERR_UNSUPPORTED, "refined-grid capacity exceeded (error word 0x%x)", e);
+}
+
+// Largest solve (nodes over all problems) whose reset, seeds and store are fused into it.
+constexpr long long FUSE_NODES = 1LL << 20;
+
+// Large bricks (8^3, 16^2) that a front across a grid touches at a time, about: the mean area of
+// its faces (3D), its mean side (2D). Measured visits of a round are half of that on average.
+static double front_bricks(const GridDesc& g) {
+  const double a = g.n[0], b = g.n[1], c = g.n[2];
+  return g.nd == 3 ? (a * b + b * c + a * c) / (3.0 * 64.0) : (a + b) / 16.0;
+}
+
+// Small bricks for solves whose rounds leave most of the GPU's warps without a large brick: a
+// round then lasts as long as its longest visit, which a small brick shortens. Large ones cost
+// less per node once the rounds fill the GPU. Small / large bricks, forward solve, by front:
+// 64 (64^3 x 1) 4.6 / 7.5 ms, 256 (128^3 x 1) 12.9 / 19.0, 1024 (256^3 x 1) 48 / 59, 2048 (64^3 x 32)
+// 15.0 / 16.0, 2048 (128^3 x 8) 37 / 45, 4096 (256^3 x 4) 138 / 127; 2D 130 (300x220 x 4) 6.0 / 7.3,
+// 6656 (1024x640 x 64) 38 / 42.
+static bool small_bricks(const eik_ctx* ctx, int nd, double front) {
+  if (ctx->brick_size > 0) return ctx->brick_size == 1;
+  return front < (nd == 3 ? 3000.0 : 8000.0);
 }
 
 // -------------------------------------------------------------- forward pipeline --
@@ -353,19 +374,21 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   const long long rsn = nsrc * std::max<long long>(N, refine ? fb.nfmax : 1);
   if ((unsigned long long)rsn >= (1ull << 32))
     return fail(ctx, EIK_ERR_OUT_OF_BUDGET, "more than 2^32 node-sources in one call: split the sources");
-  const int bnodes = nd == 3 ? 512 : 256;  // nodes of a brick (brick.cuh)
-  unsigned long long cbricks = 1;          // bricks of the largest grid, and of a refined window
-  for (int i = 0; i < nmod; i++) cbricks = std::max(cbricks, brick_nodes(models[i]->g) / bnodes);
-  unsigned long long fbricks = 1;
-  if (refine) {
-    GridDesc wg = models[0]->g;
-    for (int d = 0; d < nd; d++) wg.n[d] = (2 * ep.noderadius + 1) * ep.downscalefactor + 1;
-    fbricks = brick_nodes(wg) / bnodes;
-  }
+  // brick sizes of the coarse grids and of the refined windows, chosen separately
+  GridDesc wg = models[0]->g;
+  for (int d = 0; d < nd; d++) wg.n[d] = (2 * ep.noderadius + 1) * ep.downscalefactor + 1;
+  double cfront = 0.0;
+  for (int i = 0; i < nmod; i++) cfront += (double)(src_off[i + 1] - src_off[i]) * front_bricks(models[i]->g);
+  const bool csmall = small_bricks(ctx, nd, cfront), fsmall = small_bricks(ctx, nd, (double)nsrc * front_bricks(wg));
+  unsigned long long cbricks = 1, fbricks = 1;  // bricks of the largest grid, and of a refined window
+  for (int i = 0; i < nmod; i++) cbricks = std::max(cbricks, brick_number(models[i]->g, csmall));
+  if (refine) fbricks = brick_number(wg, fsmall);
   const unsigned long long nbr = (unsigned long long)nsrc * std::max(cbricks, fbricks);
-  GET(sa.bs.t, double, "br_t", nbr * bnodes);
-  GET(sa.bs.code, uint8_t, "br_code", nbr * bnodes);
-  GET(sa.bs.mask, unsigned, "br_mask", nbr * (bnodes / 32));
+  const unsigned long long bnodes =
+      (unsigned long long)nsrc * std::max(cbricks * brick_size(nd, csmall), refine ? fbricks * brick_size(nd, fsmall) : 1);
+  GET(sa.bs.t, double, "br_t", bnodes);
+  GET(sa.bs.code, uint8_t, "br_code", bnodes);
+  GET(sa.bs.mask, unsigned, "br_mask", bnodes / 32 + 1);
   GET(sa.bs.front, unsigned, "br_front", nbr);
   GET(sa.bs.listed, unsigned, "br_listed", nbr);
   GET(sa.bs.lists, unsigned, "br_lists", 4 * nbr);
@@ -375,6 +398,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   GET(sa.bs.thr, float, "br_thr", 2 * nsrc);
   sa.bs.listcap = nbr;
   sa.bs.stride = (unsigned)cbricks;
+  sa.bs.small = csmall ? 1 : 0;
   {
     unsigned int* rc32;
     GET(rc32, unsigned int, "rs_ctr", 32);
@@ -398,10 +422,9 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
     diam = std::max(diam, d);
   }
   sa.rs.max_rounds = round_limit(diam);
-  // small problems in thread-block clusters: in 2D by default (1), where it is faster than the
-  // global solve (measured: 300x220 x 4 sources 27.7 -> 15.9 ms); in 3D the global solve is
-  // faster (44^3 x 16: 33 vs 40 ms, and the refined windows), so only on request (2)
-  const bool use_cluster = ctx->cluster_solve == 2 || (ctx->cluster_solve == 1 && nd == 2);
+  // one launch for the reset, seeds, solve and store of a small solve (up to FUSE_NODES nodes in
+  // all): in 2D by default (1), in any dimension on request (2), never (0)
+  const bool fuse = ctx->cluster_solve == 2 || (ctx->cluster_solve == 1 && nd == 2);
   sa.err = fb.err;
   sa.probs = dp;
   sa.max_activations = ~0ull;
@@ -424,7 +447,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   const void* hp_src = stage_host(ctx, hp.data(), sizeof(CoarseProblem) * nsrc);
   if (!hp_src) return fail(ctx, EIK_ERR_CUDA, "cudaMallocHost of a plan's staging copy failed");
   CUDA_OK(ctx, cudaMemcpyAsync(dp, hp_src, sizeof(CoarseProblem) * nsrc, cudaMemcpyHostToDevice, st));
-  const double gate = ctx->gate_for(nd);
+  const double gate = ctx->gate_for(nd, csmall);
   // model i's slice of the per-source arrays, for the per-model start-up launches
   auto slice = [&](int i) {
     ForwardBatch f = fb;
@@ -457,7 +480,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
     double hmin = dh[0];
     for (int a = 1; a < nd; a++) hmin = std::min(hmin, dh[a]);
     problem_scale_kernel<<<(int)((ni + 127) / 128), 128, 0, st>>>(dp + src_off[i], (int)ni, models[i]->dstat + 2,
-                                                                  gate, hmin, nd);
+                                                                  gate, hmin, nd, csmall ? 1 : 0);
     nlaunch += 1;
   }
   CUDA_OK(ctx, cudaMemsetAsync(fb.err, 0, sizeof(uint32_t) * 4, st));
@@ -474,26 +497,25 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
     for (int i = 0; i < nmod; i++) {
       const int64_t o = src_off[i];
       if (src_off[i + 1] == o) continue;
-      launch_fine_setup(slice(i), fprobs + o, models[i]->dstat + 2, gate, fseed_lin + o * 8, fseed_tt + o * 8,
+      launch_fine_setup(slice(i), fprobs + o, models[i]->dstat + 2, ctx->gate_for(nd, fsmall), fsmall, fseed_lin + o * 8, fseed_tt + o * 8,
                         fslow + o * fb.nfmax, fkL + o * fb.nfmax, fkd + o * fb.nfmax, st);
       nlaunch += 2;
     }
     SolveArgs fsa = sa;
     fsa.probs = fprobs;
     fsa.bs.stride = (unsigned)fbricks;
+    fsa.bs.small = fsmall ? 1 : 0;
     fsa.activations = sa.activations + 6;  // own counters: the coarse solve's stay separate
     fsa.node_evals = sa.activations + 7;
     fsa.rs.max_rounds = round_limit((long long)nd * ((2LL * ep.noderadius + 1) * ep.downscalefactor + 1));
-    // the windows are small: one thread-block cluster each when the GPU has room for it
-    bool in_cluster = false;
-    if (use_cluster)
-      CUDA_OK(ctx, launch_cluster_solve(fsa, fb.nfmax, fseed_lin, fseed_tt, fb.out, true, 8, st, &in_cluster));
-    if (in_cluster) {
-      nlaunch += 2;
+    const int fsms = ctx->brick_sms(nsrc * fbricks);
+    if (fuse && nsrc * fb.nfmax <= FUSE_NODES) {
+      CUDA_OK(ctx, launch_bricks_fused(fsa, fseed_lin, fseed_tt, fb.out, true, 8, fsms, st));
+      nlaunch += 2;  // counters, everything else
     } else {
       launch_bricks_init(fsa, st);
       launch_bricks_seed(fsa, fseed_lin, fseed_tt, fb.out, true, 8, st);
-      CUDA_OK(ctx, launch_bricks_solve(fsa, ctx->brick_sms(nsrc * fbricks), st));
+      CUDA_OK(ctx, launch_bricks_solve(fsa, fsms, st));
       launch_bricks_store(fsa, st);
       nlaunch += 5;
     }
@@ -516,28 +538,23 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   }
   if (!ctx->capturing) cudaEventRecord(ctx->evk[1], st);
   CUDA_OK(ctx, cudaGetLastError());
-  if (use_cluster && cluster_solve_fits(sa, N)) {
-    // small grids: one thread-block cluster per source, init and seeds included
+  const int csms = ctx->brick_sms(nsrc * cbricks);
+  if (fuse && nsrc * N <= FUSE_NODES) {
     if (!ctx->capturing) cudaEventRecord(ctx->evk[2], st);
-    bool in_cluster = false;
-    CUDA_OK(ctx, launch_cluster_solve(sa, N, fb.seed_lin, fb.seed_tt, fb.out, false, fb.seedcap, st, &in_cluster));
-    if (!in_cluster) return fail(ctx, EIK_ERR_CUDA, "the cluster solve could not be launched");
+    CUDA_OK(ctx, launch_bricks_fused(sa, fb.seed_lin, fb.seed_tt, fb.out, false, fb.seedcap, csms, st));
     if (!ctx->capturing) cudaEventRecord(ctx->evk[3], st);
-    CUDA_OK(ctx, cudaGetLastError());
-    nlaunch += 2;  // counters, solve
-    fw->in_bricks = false;
+    nlaunch += 2;  // counters, everything else
   } else {
     launch_bricks_init(sa, st);
     launch_bricks_seed(sa, fb.seed_lin, fb.seed_tt, fb.out, false, fb.seedcap, st);
     CUDA_OK(ctx, cudaGetLastError());
     if (!ctx->capturing) cudaEventRecord(ctx->evk[2], st);
-    CUDA_OK(ctx, launch_bricks_solve(sa, ctx->brick_sms(nsrc * cbricks), st));
+    CUDA_OK(ctx, launch_bricks_solve(sa, csms, st));
     if (!ctx->capturing) cudaEventRecord(ctx->evk[3], st);
     launch_bricks_store(sa, st);
-    CUDA_OK(ctx, cudaGetLastError());
     nlaunch += 5;  // counters, brick init, seeds, solve, store
-    fw->in_bricks = true;
   }
+  CUDA_OK(ctx, cudaGetLastError());
   fw->fb = fb;
   fw->sa = sa;
   fw->t = t;
@@ -700,6 +717,12 @@ int eik_ctx_set_param(eik_ctx* ctx, const char* name, double value) {
     if (!(value == 0.0 || value == 1.0 || value == 2.0))
       return fail(ctx, EIK_ERR_ASSERT, "cluster_solve must be 0, 1 or 2");
     ctx->cluster_solve = (int)value;
+    return EIK_OK;
+  }
+  if (std::strcmp(name, "brick_size") == 0) {
+    if (!(value == 0.0 || value == 1.0 || value == 2.0))
+      return fail(ctx, EIK_ERR_ASSERT, "brick_size must be 0 (automatic), 1 (small) or 2 (large)");
+    ctx->brick_size = (int)value;
     return EIK_OK;
   }
   if (std::strcmp(name, "max_rounds") == 0) {

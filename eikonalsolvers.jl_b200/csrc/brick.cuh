@@ -38,46 +38,54 @@ constexpr unsigned FULL_WARP = 0xffffffffu;
 constexpr unsigned PF_NONE = 0x7f800000u;  // +inf: no pending value
 
 // Brick geometry. Nodes are numbered x + BX*(y + BY*z); the shared-memory cube holds the brick
-// and two layers around it, x-pitch PY per row and PZ per plane, node (0,0,0) at ORG.
-template <int ND>
-struct Brick;
-template <>
-struct Brick<3> {
-  static constexpr int BX = 8, BY = 8, BZ = 8, NODES = 512, WORDS = 16, FACES = 6;
-  static constexpr int PY = 12, PZ = 144, ORG = 2 * 144 + 2 * 12 + 2, CUBE = 12 * 12 * 12;
-};
-template <>
-struct Brick<2> {
-  static constexpr int BX = 16, BY = 16, BZ = 1, NODES = 256, WORDS = 8, FACES = 4;
-  static constexpr int PY = 20, PZ = 0, ORG = 2 * 20 + 2, CUBE = 20 * 20;
+// and two layers around it, x-pitch PY per row and PZ per plane, node (0,0,0) at ORG. Small
+// bricks (4x4x4, 8x8) shorten the chain of steps of a round and are for solves whose rounds have
+// fewer large bricks than the GPU has warps (small_bricks in api.cu).
+template <int ND, bool SMALL>
+struct Brick {
+  static constexpr int BX = ND == 3 ? (SMALL ? 4 : 8) : (SMALL ? 8 : 16);
+  static constexpr int BY = BX, BZ = ND == 3 ? BX : 1;
+  static constexpr int NODES = BX * BY * BZ, WORDS = NODES / 32, FACES = 2 * ND;
+  static constexpr int PY = BX + 4, PZ = ND == 3 ? PY * PY : 0;
+  static constexpr int ORG = 2 * PZ + 2 * PY + 2, CUBE = ND == 3 ? PY * PY * PY : PY * PY;
+  // Runs of the 3D cube that no stencil of the brick reads: two rows of PY before the brick's
+  // in the plane z = -2, and four rows between the brick's rows of the planes z = -2, -1 and
+  // z = BZ, BZ + 1 (each plane's last two rows and the next one's first two).
+  static constexpr int FREE0 = 0, FREE1 = PZ - 2 * PY, FREE2 = (BZ + 3) * PZ - 2 * PY;
 };
 
 // Number of bricks along an axis and in a problem, and the brick-ordered index of a node.
-template <int ND>
+template <int ND, bool SMALL>
 EIK_HD int bricks_along(const GridDesc& g, int a) {
-  const int b = a == 0 ? Brick<ND>::BX : (a == 1 ? Brick<ND>::BY : Brick<ND>::BZ);
+  typedef Brick<ND, SMALL> B;
+  const int b = a == 0 ? B::BX : (a == 1 ? B::BY : B::BZ);
   return (g.n[a] + b - 1) / b;
 }
-template <int ND>
+template <int ND, bool SMALL>
 EIK_HD long long brick_count(const GridDesc& g) {
   long long c = 1;
-  for (int a = 0; a < ND; a++) c *= bricks_along<ND>(g, a);
+  for (int a = 0; a < ND; a++) c *= bricks_along<ND, SMALL>(g, a);
   return c;
 }
-template <int ND>
+template <int ND, bool SMALL>
 EIK_HD long long brick_node(const GridDesc& g, int i, int j, int k) {
-  typedef Brick<ND> B;
+  typedef Brick<ND, SMALL> B;
   const int bi = i / B::BX, bj = j / B::BY, bk = ND == 3 ? k / B::BZ : 0;
-  const long long b = bi + (long long)bricks_along<ND>(g, 0) * (bj + (long long)bricks_along<ND>(g, 1) * bk);
+  const long long b =
+      bi + (long long)bricks_along<ND, SMALL>(g, 0) * (bj + (long long)bricks_along<ND, SMALL>(g, 1) * bk);
   return b * B::NODES + (i - bi * B::BX) + B::BX * ((j - bj * B::BY) + B::BY * (ND == 3 ? k - bk * B::BZ : 0));
+}
+EIK_HD long long brick_node(const GridDesc& g, bool small, int i, int j, int k) {
+  if (g.nd == 3) return small ? brick_node<3, true>(g, i, j, k) : brick_node<3, false>(g, i, j, k);
+  return small ? brick_node<2, true>(g, i, j, k) : brick_node<2, false>(g, i, j, k);
 }
 
 // Shared memory of one warp. The list of a scan and the spherical coefficients (1/h^2 and
-// 9/(4h^2) of axes 1 and 2 per radial index of the brick) take corners of the cube that no
-// stencil reads in 3D: 20.9 KB a warp, 11 warps an SM.
-template <int ND>
+// 9/(4h^2) of axes 1 and 2 per radial index of the brick) take free runs of the cube in 3D:
+// 20.9 KB a warp, 11 warps an SM (small bricks: 5.0 KB).
+template <int ND, bool SMALL>
 struct __align__(16) WarpMem {
-  typedef Brick<ND> B;
+  typedef Brick<ND, SMALL> B;
   double cube[B::CUBE];                // traveltimes; sign bit: special key
   double slow[B::NODES];
   unsigned pf[B::NODES];               // pending front (float bits) or PF_NONE
@@ -86,13 +94,12 @@ struct __align__(16) WarpMem {
   unsigned facemin[8];                 // and their smallest front
   double extra[ND == 3 ? 2 : 48];
   __device__ __forceinline__ uint16_t* list() {
-    return reinterpret_cast<uint16_t*>(ND == 3 ? cube : extra);  // 64 entries, 16 doubles
+    return reinterpret_cast<uint16_t*>(ND == 3 ? cube + B::FREE0 : extra);  // 64 entries, 16 doubles
   }
-  __device__ __forceinline__ double* coef() { return ND == 3 ? cube + 120 : extra + 16; }  // up to 32
+  __device__ __forceinline__ double* coef() { return ND == 3 ? cube + B::FREE1 : extra + 16; }  // up to 32
 };
-// cube + 0..15 lie in the row y = -2 of the plane z = -2, cube + 120..151 in the rows y = 8, 9 of
-// that plane and y = -2 of the next: outside the layers that any stencil of the brick reads
-static_assert(Brick<3>::PZ == 144 && Brick<3>::PY == 12, "unused corners of the 3D cube");
+static_assert(2 * Brick<3, true>::PY >= 16 && 4 * Brick<3, true>::PY >= 4 * 4 && 4 * Brick<3, false>::PY >= 4 * 8,
+              "the free runs hold the list and the coefficients");
 
 __device__ __forceinline__ unsigned front_bits(double v) {
   // smallest float >= v, finite: a pending node is never lost to overflow
@@ -132,10 +139,10 @@ __device__ __forceinline__ bool key_le_flat(const Key& a, const Key& b) {
 // Called by all lanes; a lane's inputs are those of its node (the same in the node's 2*ND lanes),
 // and so is what it returns. t: the node in the cube; ok2: sides (bit slot) where 2nd order is
 // allowed; l: column-major node index; i: radial index; active: the lane has a node.
-template <int ND>
+template <int ND, bool SMALL>
 __device__ __noinline__ RuleOut rule_slow(const CoarseProblem& P, const double* t, unsigned ok2, long long l, int i,
                                           double slow, bool active, int lane) {
-  typedef Brick<ND> B;
+  typedef Brick<ND, SMALL> B;
   constexpr int G = 2 * ND;
   const int j = lane % G, base = lane - j;
   // the keys of immediate neighbour j and of the node beyond it
@@ -231,10 +238,10 @@ __device__ __noinline__ RuleOut rule_slow(const CoarseProblem& P, const double* 
 
 // Copies brick b (at brick coordinates bc, bricks nb per axis) of a brick-ordered array and the
 // layers around it that exist to a cube; positions across the grid's faces get `outside`.
-template <int ND>
+template <int ND, bool SMALL>
 __device__ __forceinline__ void load_cube(double* cube, const double* array, size_t b, const int (&bc)[3],
                                           const int (&nb)[3], double outside, int lane) {
-  typedef Brick<ND> B;
+  typedef Brick<ND, SMALL> B;
   const double* own = array + b * B::NODES;
   constexpr int ROWP = B::BX / 2;  // 16-byte pieces of a row
 #pragma unroll
@@ -252,10 +259,9 @@ __device__ __forceinline__ void load_cube(double* cube, const double* array, siz
       const bool have = s == 0 ? bc[a] + 1 < nb[a] : bc[a] > 0;
       const double* src = s == 0 ? own + bst[a] * B::NODES : own - bst[a] * B::NODES;
       // pairs of the two layers: along x one pair per row, else ROWP pairs per row of 2 rows
-      constexpr int PER = ND == 3 ? 64 : 16;
-      const int pieces = a == 0 ? B::BY * B::BZ : PER;
+      const int pieces = a == 0 ? B::BY * B::BZ : (a == 1 ? 2 * ROWP * B::BZ : 2 * ROWP * B::BY);
 #pragma unroll
-      for (int q = 0; q < (ND == 3 ? 64 : 16); q += 32) {
+      for (int q = 0; q < pieces; q += 32) {
         const int e = q + lane;
         if (e < pieces) {
           int ci, si;
@@ -303,7 +309,7 @@ struct VisitTally {
 // hold up the round: 256^3 x 4 at 8 / 12 / 16 / 24 / 192 scans: 140 / 126 / 122 / 129 / 150 ms, 64^3 x
 // 32 18.2 / 16.6 / 17.0 / 19.4 / 20.5 ms, 1024x640 x 64 61 / 53 / 49 / 44 / 53 ms. It also ends a visit in
 // which values alternate (the rule's depth limit lets some transient keys do so).
-template <int ND>
+template <int ND, bool SMALL>
 constexpr int VISIT_MAX_SCANS = ND == 3 ? 16 : 24;
 
 // Which steps -2, -1, +1, +2 along an axis stay within [lo, hi) from position p: bits 0..3 of
@@ -317,16 +323,16 @@ __device__ __forceinline__ unsigned long long step_table(int lo, int hi) {
 // Settles brick b up to threshold T (a float-valued bound): returns the smallest pending front
 // left in it (float bits, PF_NONE if none), its mask written back. The fronts and masks for
 // the bricks across its faces are left in w.facemin / w.face for the caller to publish.
-template <int ND>
-__device__ __forceinline__ unsigned visit_brick(WarpMem<ND>& w, const BrickState& bs, const CoarseProblem& P, size_t b,
+template <int ND, bool SMALL>
+__device__ __forceinline__ unsigned visit_brick(WarpMem<ND, SMALL>& w, const BrickState& bs, const CoarseProblem& P, size_t b,
                                                 const int (&bc)[3], const int (&nb)[3], float T, int lane,
                                                 VisitTally& tally) {
-  typedef Brick<ND> B;
+  typedef Brick<ND, SMALL> B;
   uint16_t* list = w.list();
   double* coef = w.coef();
   unsigned pend = 0u;
   if (lane < B::WORDS) pend = __ldcg(bs.mask + b * B::WORDS + lane);
-  load_cube<ND>(w.cube, bs.t, b, bc, nb, EIK_INF, lane);
+  load_cube<ND, SMALL>(w.cube, bs.t, b, bc, nb, EIK_INF, lane);
   if (lane < B::NODES / 16) cp_async16(&w.code[lane * 16], bs.code + b * B::NODES + lane * 16);
   for (int q = lane; q < B::FACES * B::WORDS; q += 32) w.face[q] = 0u;
   if (lane < 8) w.facemin[lane] = PF_NONE;
@@ -396,7 +402,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND>& w, const BrickState
       mn = min(mn, v[k]);
     }
     mn = __reduce_min_sync(FULL_WARP, mn);
-    if (mn > Tb || mn == PF_NONE || it >= VISIT_MAX_SCANS<ND>) {
+    if (mn > Tb || mn == PF_NONE || it >= VISIT_MAX_SCANS<ND, SMALL>) {
       left = mn;
 #pragma unroll
       for (int k = 0; k < B::WORDS; k++) {
@@ -531,7 +537,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND>& w, const BrickState
         const double ss = __shfl_sync(FULL_WARP, slow, src);
         const int sx = x0[0] + sq % B::BX;
         const long long l = sx + (long long)n[0] * ((x0[1] + (sq / B::BX) % B::BY) + (long long)n[1] * (x0[2] + sq / (B::BX * B::BY)));
-        const RuleOut o = rule_slow<ND>(P, &w.cube[sci], sok, l, sx, ss, has, lane);
+        const RuleOut o = rule_slow<ND, SMALL>(P, &w.cube[sci], sok, l, sx, ss, has, lane);
         // back to the node's own lane
         const int place = __popc(sl & below);
         const bool take = ((sl >> lane) & 1u) && place < PAR;

@@ -19,12 +19,13 @@
 namespace eik {
 
 // Warps per CTA, one CTA per SM: as many warps as their shared memory allows in 3D (20.9 KB
-// each), 16 in 2D (7 KB each) where a round seldom has more bricks per SM.
-template <int ND>
-constexpr int BRICK_WARPS = ND == 3 ? 11 : 16;
+// each; 12 of small bricks, at 168 registers a thread), 16 in 2D (7 KB each) where a round seldom
+// has more bricks per SM.
+template <int ND, bool SMALL>
+constexpr int BRICK_WARPS = ND == 3 ? (SMALL ? 12 : 11) : 16;
 
 // ----------------------------------------------------------------------- init --
-__global__ void bricks_init_kernel(BrickState bs, unsigned nprob, int nodes, int words) {
+__device__ __forceinline__ void bricks_init(const BrickState& bs, unsigned nprob, int nodes, int words) {
   const size_t nb = (size_t)bs.stride * nprob, t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x,
                dt = (size_t)gridDim.x * blockDim.x;
   const double2 inf2 = make_double2(EIK_INF, EIK_INF);
@@ -44,6 +45,9 @@ __global__ void bricks_init_kernel(BrickState bs, unsigned nprob, int nodes, int
   for (size_t q = t0; q < 2 * (size_t)nprob; q += dt) bs.thr[q] = 0.0f;
   if (t0 < 8) bs.ctr[t0] = 0u;
 }
+__global__ void bricks_init_kernel(BrickState bs, unsigned nprob, int nodes, int words) {
+  bricks_init(bs, nprob, nodes, words);
+}
 
 __global__ void solve_counters_kernel(SolveArgs a) {
   if (threadIdx.x != 0) return;
@@ -59,20 +63,28 @@ __global__ void solve_counters_kernel(SolveArgs a) {
 // Seeds: fixed traveltimes of the source points (coarse source box, coarse-coincident
 // accepted fine nodes, or the source box of a refined window); the nodes within two steps
 // of a seed are pending at the start, with the seed's traveltime as their front.
-template <int ND>
-__global__ void seed_kernel(SolveArgs a, const int32_t* seed_lin, const double* seed_tt, const SrcOut* out,
-                            int fine_corners, int seedcap) {
-  typedef Brick<ND> B;
-  const int s = blockIdx.x;
+struct SeedArgs {
+  const int32_t* lin;  // nprob x cap
+  const double* tt;
+  const SrcOut* out;
+  int32_t fine_corners, cap;
+};
+// Problem s by one CTA.
+template <int ND, bool SMALL>
+__device__ __forceinline__ void seed_problem(const SolveArgs& a, const SeedArgs& sd, int s) {
+  typedef Brick<ND, SMALL> B;
+  const int32_t* seed_lin = sd.lin;
+  const double* seed_tt = sd.tt;
+  const int seedcap = sd.cap;
   const CoarseProblem& P = a.probs[s];
   const BrickState& bs = a.bs;
-  const int ns = fine_corners ? out[s].nsrcf : out[s].nseeds;
+  const int ns = sd.fine_corners ? sd.out[s].nsrcf : sd.out[s].nseeds;
   const size_t base = (size_t)s * bs.stride;
   for (int q = threadIdx.x; q < ns; q += blockDim.x) {
     const long long l = seed_lin[(size_t)s * seedcap + q];
     int c[3];
     node_coords(P.g, l, c);
-    bs.t[base * B::NODES + brick_node<ND>(P.g, c[0], c[1], c[2])] = -fabs(seed_tt[(size_t)s * seedcap + q]);
+    bs.t[base * B::NODES + brick_node<ND, SMALL>(P.g, c[0], c[1], c[2])] = -fabs(seed_tt[(size_t)s * seedcap + q]);
     P.kL[l] = -EIK_INF;
     P.kd[l] = 0;
   }
@@ -88,7 +100,7 @@ __global__ void seed_kernel(SolveArgs a, const int32_t* seed_lin, const double* 
         int p[3] = {c[0], c[1], c[2]};
         p[ax] += d;
         if (p[ax] < 0 || p[ax] >= P.g.n[ax]) continue;
-        const long long bn = brick_node<ND>(P.g, p[0], p[1], p[2]);
+        const long long bn = brick_node<ND, SMALL>(P.g, p[0], p[1], p[2]);
         const size_t b = base + bn / B::NODES;
         const int qn = (int)(bn % B::NODES);
         atomicOr(bs.mask + b * B::WORDS + (qn >> 5), 1u << (qn & 31));
@@ -101,6 +113,30 @@ __global__ void seed_kernel(SolveArgs a, const int32_t* seed_lin, const double* 
           bs.lists[(size_t)(2 * col) * bs.listcap + atomicAdd(bs.ctr + 2 * col, 1u)] = (unsigned)b;
         }
       }
+  }
+}
+
+template <int ND, bool SMALL>
+__global__ void seed_kernel(SolveArgs a, SeedArgs sd) {
+  seed_problem<ND, SMALL>(a, sd, blockIdx.x);
+}
+
+// Results in the problems' own arrays: column-major traveltimes, and codes with bit 7 for a
+// special key. Problem p by the threads t0, t0 + dt, ...
+template <int ND, bool SMALL>
+__device__ __forceinline__ void store_problem(const SolveArgs& a, int p, unsigned t0, unsigned dt) {
+  typedef Brick<ND, SMALL> B;
+  const CoarseProblem& P = a.probs[p];
+  const GridDesc& g = P.g;
+  const size_t base = (size_t)p * a.bs.stride * B::NODES;
+  const unsigned long long N = (unsigned long long)npts(g);
+  for (unsigned long long l = t0; l < N; l += dt) {
+    int c[3];
+    node_coords(g, (long long)l, c);
+    const size_t q = base + brick_node<ND, SMALL>(g, c[0], c[1], c[2]);
+    const double t = __ldcg(a.bs.t + q);
+    P.t[l] = fabs(t);
+    P.code[l] = (uint8_t)((__ldcg(a.bs.code + q) & 0x7f) | (sign_set(t) ? CODE_SRC_BIT : 0));
   }
 }
 
@@ -121,17 +157,28 @@ __device__ __forceinline__ float round_threshold(const BrickState& bs, int nprob
   return fmaxf(prev, fminf(__double2float_ru((double)__uint_as_float(m) + delta), 3.402823466e38f));
 }
 
-template <int ND>
-__global__ void __launch_bounds__(BRICK_WARPS<ND> * 32, 1) brick_rounds_kernel(SolveArgs a) {
-  typedef Brick<ND> B;
+// FUSED: the reset, the seeds and the store are part of the launch (small solves, where each
+// launch of its own costs as much as its work).
+template <int ND, bool SMALL, bool FUSED>
+__global__ void __launch_bounds__(BRICK_WARPS<ND, SMALL> * 32, 1) brick_rounds_kernel(SolveArgs a, SeedArgs sd) {
+  typedef Brick<ND, SMALL> B;
   extern __shared__ __align__(16) unsigned char brick_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  WarpMem<ND>& w = reinterpret_cast<WarpMem<ND>*>(brick_smem)[warp];
+  WarpMem<ND, SMALL>& w = reinterpret_cast<WarpMem<ND, SMALL>*>(brick_smem)[warp];
   const BrickState bs = a.bs;
-  const unsigned nwarps = gridDim.x * BRICK_WARPS<ND>;
+  const unsigned nwarps = gridDim.x * BRICK_WARPS<ND, SMALL>;
   // consecutive entries go to different SMs
   const unsigned gwarp = (unsigned)warp * gridDim.x + blockIdx.x;
   VisitTally tally;
+  if (FUSED) {
+    bricks_init(bs, (unsigned)a.nprob, B::NODES, B::WORDS);
+    if (!grid_barrier(a)) return;
+    for (int s = blockIdx.x; s < a.nprob; s += gridDim.x) {
+      seed_problem<ND, SMALL>(a, sd, s);
+      __syncthreads();
+    }
+    if (!grid_barrier(a)) return;
+  }
   int r = 0;
   for (; r < a.rs.max_rounds; r++) {
     const int col = r & 1, ph = (r >> 1) & 1, nph = ph ^ 1, oph = ((r + 1) >> 1) & 1;
@@ -171,10 +218,10 @@ __global__ void __launch_bounds__(BRICK_WARPS<ND> * 32, 1) brick_rounds_kernel(S
         const float vT = __shfl_sync(FULL_WARP, T, src);
         const CoarseProblem& P = a.probs[vp];
         const unsigned lb = vb - (unsigned)vp * bs.stride;
-        const int nb[3] = {bricks_along<ND>(P.g, 0), bricks_along<ND>(P.g, 1),
-                           ND == 3 ? bricks_along<ND>(P.g, 2) : 1};
+        const int nb[3] = {bricks_along<ND, SMALL>(P.g, 0), bricks_along<ND, SMALL>(P.g, 1),
+                           ND == 3 ? bricks_along<ND, SMALL>(P.g, 2) : 1};
         const int bc[3] = {(int)(lb % nb[0]), (int)((lb / nb[0]) % nb[1]), (int)(lb / ((unsigned)nb[0] * nb[1]))};
-        const unsigned left = visit_brick<ND>(w, bs, P, vb, bc, nb, vT, lane, tally);
+        const unsigned left = visit_brick<ND, SMALL>(w, bs, P, vb, bc, nb, vT, lane, tally);
         if (lane == src) leftf = left;
         if (lane == 0) {
           bs.front[vb] = left;
@@ -185,7 +232,7 @@ __global__ void __launch_bounds__(BRICK_WARPS<ND> * 32, 1) brick_rounds_kernel(S
 #pragma unroll
         for (int q0 = 0; q0 < B::FACES * B::WORDS; q0 += 32) {
           const int q = q0 + lane;
-          const unsigned bits = w.face[q];
+          const unsigned bits = q < B::FACES * B::WORDS ? w.face[q] : 0u;
           if (bits) {
             const int fc = q / B::WORDS, ax = fc >> 1;
             const int st = ax == 0 ? 1 : (ax == 1 ? nb[0] : nb[0] * nb[1]);
@@ -240,6 +287,10 @@ __global__ void __launch_bounds__(BRICK_WARPS<ND> * 32, 1) brick_rounds_kernel(S
   const unsigned evals = __shfl_sync(FULL_WARP, tally.n, VISIT_WAIT) + __shfl_sync(FULL_WARP, tally.n, VISIT_SAME) +
                          __shfl_sync(FULL_WARP, tally.n, VISIT_CHANGED);
   if (lane == 0 && evals) atomicAdd(a.node_evals, (unsigned long long)evals);
+  // every visit ended before the barrier that closed the last round
+  if (FUSED)
+    for (int p = 0; p < a.nprob; p++)
+      store_problem<ND, SMALL>(a, p, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *a.rs.rounds = r;
     if (r >= a.rs.max_rounds) {
@@ -249,25 +300,10 @@ __global__ void __launch_bounds__(BRICK_WARPS<ND> * 32, 1) brick_rounds_kernel(S
   }
 }
 
-// Results in the problems' own arrays: column-major traveltimes, and codes with bit 7 for a
-// special key.
-template <int ND>
+template <int ND, bool SMALL>
 __global__ void bricks_store_kernel(SolveArgs a) {
-  typedef Brick<ND> B;
-  for (int p = blockIdx.y; p < a.nprob; p += gridDim.y) {
-    const CoarseProblem& P = a.probs[p];
-    const GridDesc& g = P.g;
-    const size_t base = (size_t)p * a.bs.stride * B::NODES;
-    const unsigned long long N = (unsigned long long)npts(g);
-    for (unsigned long long l = blockIdx.x * blockDim.x + threadIdx.x; l < N; l += gridDim.x * blockDim.x) {
-      int c[3];
-      node_coords(g, (long long)l, c);
-      const size_t q = base + brick_node<ND>(g, c[0], c[1], c[2]);
-      const double t = a.bs.t[q];
-      P.t[l] = fabs(t);
-      P.code[l] = (uint8_t)((a.bs.code[q] & 0x7f) | (sign_set(t) ? CODE_SRC_BIT : 0));
-    }
-  }
+  for (int p = blockIdx.y; p < a.nprob; p += gridDim.y)
+    store_problem<ND, SMALL>(a, p, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // ------------------------------------------------------------------ picks --
@@ -318,47 +354,70 @@ __global__ void picks_kernel(GridDesc g, const double* t, long long N, int nsrc,
 }
 
 // ------------------------------------------------------------------ launchers --
-unsigned long long brick_nodes(const GridDesc& g) {
-  return g.nd == 3 ? (unsigned long long)brick_count<3>(g) * Brick<3>::NODES
-                   : (unsigned long long)brick_count<2>(g) * Brick<2>::NODES;
+int brick_size(int nd, bool small) {
+  return nd == 3 ? (small ? Brick<3, true>::NODES : Brick<3, false>::NODES)
+                 : (small ? Brick<2, true>::NODES : Brick<2, false>::NODES);
+}
+unsigned long long brick_number(const GridDesc& g, bool small) {
+  if (g.nd == 3) return (unsigned long long)(small ? brick_count<3, true>(g) : brick_count<3, false>(g));
+  return (unsigned long long)(small ? brick_count<2, true>(g) : brick_count<2, false>(g));
 }
 
 void launch_bricks_init(const SolveArgs& sa, cudaStream_t st) {
   solve_counters_kernel<<<1, 32, 0, st>>>(sa);
-  const int nodes = sa.nd == 3 ? Brick<3>::NODES : Brick<2>::NODES;
+  const int nodes = brick_size(sa.nd, sa.bs.small);
   bricks_init_kernel<<<1184, 256, 0, st>>>(sa.bs, (unsigned)sa.nprob, nodes, nodes / 32);
 }
 
 void launch_bricks_seed(const SolveArgs& sa, const int32_t* seed_lin, const double* seed_tt, const SrcOut* out,
                         bool fine_corners, int seedcap, cudaStream_t st) {
-  if (sa.nd == 3) seed_kernel<3><<<sa.nprob, 128, 0, st>>>(sa, seed_lin, seed_tt, out, fine_corners ? 1 : 0, seedcap);
-  else seed_kernel<2><<<sa.nprob, 128, 0, st>>>(sa, seed_lin, seed_tt, out, fine_corners ? 1 : 0, seedcap);
+  const SeedArgs sd{seed_lin, seed_tt, out, fine_corners ? 1 : 0, seedcap};
+  auto go = [&](auto kernel) { kernel<<<sa.nprob, 128, 0, st>>>(sa, sd); };
+  if (sa.nd == 3) sa.bs.small ? go(seed_kernel<3, true>) : go(seed_kernel<3, false>);
+  else sa.bs.small ? go(seed_kernel<2, true>) : go(seed_kernel<2, false>);
 }
 
-template <int ND>
-static cudaError_t launch_bricks_solve_nd(const SolveArgs& sa, int nsm, cudaStream_t st) {
-  const size_t sm = sizeof(WarpMem<ND>) * BRICK_WARPS<ND>;
-  cudaError_t e = cudaFuncSetAttribute(brick_rounds_kernel<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+template <int ND, bool SMALL, bool FUSED>
+static cudaError_t launch_bricks_solve_nd(const SolveArgs& sa, const SeedArgs& sd, int nsm, cudaStream_t st) {
+  const void* kernel = (const void*)brick_rounds_kernel<ND, SMALL, FUSED>;
+  const size_t sm = sizeof(WarpMem<ND, SMALL>) * BRICK_WARPS<ND, SMALL>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   SolveArgs args = sa;
-  void* kargs[] = {&args};
+  SeedArgs seeds = sd;
+  void* kargs[] = {&args, &seeds};
   // cooperative: every CTA is resident, so the grid barrier between rounds cannot deadlock
-  return cudaLaunchCooperativeKernel((const void*)brick_rounds_kernel<ND>, dim3(nsm), dim3(BRICK_WARPS<ND> * 32),
-                                     kargs, sm, st);
+  return cudaLaunchCooperativeKernel(kernel, dim3(nsm), dim3(BRICK_WARPS<ND, SMALL> * 32), kargs, sm, st);
+}
+
+template <bool FUSED>
+static cudaError_t launch_bricks_any(const SolveArgs& sa, const SeedArgs& sd, int nsm, cudaStream_t st) {
+  if (sa.nd == 3)
+    return sa.bs.small ? launch_bricks_solve_nd<3, true, FUSED>(sa, sd, nsm, st)
+                       : launch_bricks_solve_nd<3, false, FUSED>(sa, sd, nsm, st);
+  return sa.bs.small ? launch_bricks_solve_nd<2, true, FUSED>(sa, sd, nsm, st)
+                     : launch_bricks_solve_nd<2, false, FUSED>(sa, sd, nsm, st);
 }
 
 cudaError_t launch_bricks_solve(const SolveArgs& sa, int nsm, cudaStream_t st) {
-  return sa.nd == 3 ? launch_bricks_solve_nd<3>(sa, nsm, st) : launch_bricks_solve_nd<2>(sa, nsm, st);
+  return launch_bricks_any<false>(sa, SeedArgs{}, nsm, st);
+}
+
+cudaError_t launch_bricks_fused(const SolveArgs& sa, const int32_t* seed_lin, const double* seed_tt, const SrcOut* out,
+                                bool fine_corners, int seedcap, int nsm, cudaStream_t st) {
+  solve_counters_kernel<<<1, 32, 0, st>>>(sa);
+  return launch_bricks_any<true>(sa, SeedArgs{seed_lin, seed_tt, out, fine_corners ? 1 : 0, seedcap}, nsm, st);
 }
 
 void launch_bricks_store(const SolveArgs& sa, cudaStream_t st) {
   // blocks per problem: enough in all to fill the GPU, no more than a problem has nodes for
-  const unsigned long long nodes = (unsigned long long)sa.bs.stride * (sa.nd == 3 ? Brick<3>::NODES : Brick<2>::NODES);
+  const unsigned long long nodes = (unsigned long long)sa.bs.stride * brick_size(sa.nd, sa.bs.small);
   const unsigned want = (unsigned)((nodes + 1023) / 1024);
   const unsigned per = std::max(1u, std::min(want, std::max(8u, 2368u / (unsigned)sa.nprob)));
   const dim3 grid(per, std::min(65535u, (unsigned)sa.nprob));
-  if (sa.nd == 3) bricks_store_kernel<3><<<grid, 256, 0, st>>>(sa);
-  else bricks_store_kernel<2><<<grid, 256, 0, st>>>(sa);
+  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(sa); };
+  if (sa.nd == 3) sa.bs.small ? go(bricks_store_kernel<3, true>) : go(bricks_store_kernel<3, false>);
+  else sa.bs.small ? go(bricks_store_kernel<2, true>) : go(bricks_store_kernel<2, false>);
 }
 
 void launch_picks(const GridDesc& g, const double* t, long long N, int nsrc, const long long* recoff,

@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
 // node) does the heap's internal order decide; those sources are replayed exactly.
 
 // Window, fine source box, the fine problem of the round solver, its slowness and seeds.
-__global__ void fine_setup_kernel(ForwardBatch fb, CoarseProblem* fprobs, const double* dsmin, double gate,
+__global__ void fine_setup_kernel(ForwardBatch fb, CoarseProblem* fprobs, const double* dsmin, double gate, int small,
                                   int32_t* fseed_lin, double* fseed_tt, double* fslow, double* fkL, uint8_t* fkd) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= fb.nsrc) return;
@@ -516,7 +516,7 @@ __global__ void fine_setup_kernel(ForwardBatch fb, CoarseProblem* fprobs, const 
   P.delta = gate * hmin * smin;
   P.incmin = 0.999 * (2.0 / 3.0) * hmin * smin / sqrt((double)gf.nd);
   P.linc = 0.999 * (2.0 / 3.0) * hmin / sqrt((double)gf.nd);
-  P.din = inner_window(gf.nd, hmin * smin);
+  P.din = inner_window(gf.nd, small != 0, hmin * smin);
 }
 
 __global__ void fine_fill_kernel(ForwardBatch fb, const CoarseProblem* fprobs) {
@@ -784,10 +784,10 @@ __global__ void __launch_bounds__(SEL_THREADS) fine_select_kernel(ForwardBatch f
   }
 }
 
-void launch_fine_setup(const ForwardBatch& fb, CoarseProblem* fprobs, const double* dsmin, double gate,
+void launch_fine_setup(const ForwardBatch& fb, CoarseProblem* fprobs, const double* dsmin, double gate, bool small,
                        int32_t* fseed_lin, double* fseed_tt, double* fine_slow, double* fine_kL, uint8_t* fine_kd,
                        cudaStream_t st) {
-  fine_setup_kernel<<<(fb.nsrc + 63) / 64, 64, 0, st>>>(fb, fprobs, dsmin, gate, fseed_lin, fseed_tt, fine_slow,
+  fine_setup_kernel<<<(fb.nsrc + 63) / 64, 64, 0, st>>>(fb, fprobs, dsmin, gate, small ? 1 : 0, fseed_lin, fseed_tt, fine_slow,
                                                          fine_kL, fine_kd);
   fine_fill_kernel<<<592, 256, 0, st>>>(fb, fprobs);
 }

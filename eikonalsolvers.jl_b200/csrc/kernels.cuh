@@ -91,7 +91,8 @@ struct RoundState {
 // Inner window of a brick visit: the nodes evaluated together lie within this much of the
 // brick's smallest pending front. Narrower windows re-evaluate fewer nodes, wider ones fill
 // more lanes of a step; u is the least time across one node (smallest spacing x slowness).
-EIK_HD float inner_window(int nd, double u) { return (float)((nd == 3 ? 0.5 : 1.0) * u); }
+// 3D, 0.35 / 0.5 / 0.75 u with small bricks: 64^3 x 32 15.2 / 14.9 / 14.5 ms; large ones 0.5 u.
+EIK_HD float inner_window(int nd, bool small, double u) { return (float)((nd == 3 ? (small ? 0.75 : 0.5) : 1.0) * u); }
 
 // State of the forward solve by bricks (brick.cuh): problem p's bricks are p * stride + b.
 struct BrickState {
@@ -107,6 +108,7 @@ struct BrickState {
   unsigned* marks;      // [4][nprob] smallest front a round's visits put on other bricks
   float* thr;           // [2][nprob] threshold of the previous / current round
   unsigned stride;      // bricks per problem (the call's largest grid)
+  int32_t small;        // small bricks
 };
 
 struct SolveArgs {
@@ -134,24 +136,21 @@ void launch_bricks_init(const SolveArgs& sa, cudaStream_t st);
 void launch_bricks_seed(const SolveArgs& sa, const int32_t* seed_lin, const double* seed_tt, const SrcOut* out,
                         bool fine_corners, int seedcap, cudaStream_t st);
 cudaError_t launch_bricks_solve(const SolveArgs& sa, int nsm, cudaStream_t st);
+// All four in one launch after the counters' (reset, seeds, solve, store), for small solves.
+cudaError_t launch_bricks_fused(const SolveArgs& sa, const int32_t* seed_lin, const double* seed_tt, const SrcOut* out,
+                                bool fine_corners, int seedcap, int nsm, cudaStream_t st);
 void launch_bricks_store(const SolveArgs& sa, cudaStream_t st);
-// Nodes of a grid's bricks (the grid rounded up to whole bricks).
-unsigned long long brick_nodes(const GridDesc& g);
+// Nodes of a brick, and bricks of a grid (rounded up to whole ones).
+int brick_size(int nd, bool small);
+unsigned long long brick_number(const GridDesc& g, bool small);
 // Refined start-up as a fixed point: window set-up, the fine problems' arrays, the
 // acceptance set at the reference's stop, and the exact heap replay for the sources
 // whose stop is decided by a tie (flags in fine_tie, nonzero = replay needed).
-void launch_fine_setup(const ForwardBatch& fb, CoarseProblem* fprobs, const double* dsmin, double gate,
+void launch_fine_setup(const ForwardBatch& fb, CoarseProblem* fprobs, const double* dsmin, double gate, bool small,
                        int32_t* fseed_lin, double* fseed_tt, double* fine_slow, double* fine_kL, uint8_t* fine_kd,
                        cudaStream_t st);
 void launch_fine_select(const ForwardBatch& fb, const CoarseProblem* fprobs, uint8_t* fine_tie, cudaStream_t st);
 void launch_fine_replay(const ForwardBatch& fb, const uint8_t* fine_tie, cudaStream_t st);
-// The forward solve of small problems (every problem at most nmax nodes), one thread-block
-// cluster per problem with its state in distributed shared memory, seeds and counters
-// included (it replaces round init, seeding and launch_coarse_solve). *used = false when no
-// cluster of this GPU holds such a problem (nothing launched: use the global solve).
-cudaError_t launch_cluster_solve(const SolveArgs& sa, long long nmax, const int32_t* seed_lin, const double* seed_tt,
-                                 const SrcOut* out, bool fine_corners, int seedcap, cudaStream_t st, bool* used);
-bool cluster_solve_fits(const SolveArgs& sa, long long nmax);
 void launch_picks(const GridDesc& g, const double* t, long long N, int nsrc, const long long* recoff,
                   const double* rec, double* picks, cudaStream_t st);
 // Gaussian smoothing of a gradient field (smoothgradkern = l, odd): weights on the host,

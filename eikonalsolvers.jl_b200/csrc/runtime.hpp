@@ -74,7 +74,6 @@ struct ForwardState {
   const uint8_t* fine_tie = nullptr;  // per-source replay flags of the refined start-up (device)
   int launches = 0;                   // kernels the forward stage launched
   double gate = 2.0;                  // round width used (units of smallest spacing x slowness)
-  bool in_bricks = true;              // the coarse traveltimes are in brick order too (SolveArgs::bs)
   std::vector<SrcOut> host_out;
 };
 
@@ -159,17 +158,19 @@ struct eik_ctx {
   double round_gate = 0.0;  // forward round width in units of (smallest spacing x smallest slowness); 0 = gate_for
   int ctas_per_sm = 0;       // accepted, without effect (the forward solve has one CTA per SM)
   int fwd_queue = -1;        // accepted, without effect
-  int cluster_solve = 1;     // small problems in one thread-block cluster each: 1 in 2D, 2 in any dimension, 0 never
+  int cluster_solve = 1;     // small solves in one launch: 1 in 2D, 2 in any dimension, 0 never
+  int brick_size = 0;        // bricks of the forward and adjoint solves: 0 by the call's size, 1 small, 2 large
   int max_rounds = 0;        // round limit of the persistent solves (0 = the library's, see forward_multi)
   int retry = 0;             // a pipeline run again after the automatic round limit: wider rounds, limit 2^24
   int auto_round_limit = 0;  // the automatic round limit of a first run (0 = by the grid's diameter)
   double sm_fraction = 0.0; // share of the SMs the persistent (cooperative) solves use; 0 = by size
   double ray_room = 3.0;     // room of a ray in its first tracing pass, in straight-line lengths
   bool fine_replay = false; // refined start-up by exact heap replay for every source (else only on ties)
-  // Round width of a call: the value set on the context, else by dimension (bricks: 128^3 x 8
-  // 2 / 4 / 6: 101 / 99 / 102 ms, 1024x640 x 64 4 / 8 / 16: 68 / 63 / 57 ms; flat around these).
-  double gate_for(int nd) const {
-    const double g = round_gate > 0.0 ? round_gate : (nd == 2 ? 8.0 : 6.0);
+  // Round width of a call: the value set on the context, else by dimension and brick size (forward
+  // solve, 3D small bricks 6 / 8 / 12: 128^3 x 8 37.4 / 36.3 / 36.6 ms; large 4 / 6: 256^3 x 4 127 / 122;
+  // 2D small 16 / 24 / 32: 300x220 x 4 6.1 / 5.3 / 5.0; large 8 / 16 / 24: 1024x640 x 64 44 / 42 / 43).
+  double gate_for(int nd, bool small) const {
+    const double g = round_gate > 0.0 ? round_gate : (nd == 2 ? (small ? 24.0 : 16.0) : (small ? 8.0 : 6.0));
     return retry ? 1.5 * g : g;
   }
   // SMs of a solve over `bricks` bricks: a round visits one colour, so at most half.

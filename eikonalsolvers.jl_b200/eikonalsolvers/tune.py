@@ -3,10 +3,9 @@
 The forward solve's result is the unique fixed point of the FMM order rule, so its launch
 parameters change only how much work it takes to get there: the round width
 (``round_gate``, in units of smallest spacing x smallest slowness: wider rounds mean fewer
-grid barriers but more nodes evaluated before their inputs are final) and the number of
-resident CTAs per SM of the persistent launch (``ctas_per_sm``: more CTAs hide more memory
-latency, fewer leave each thread more registers and less barrier traffic). The best pair
-depends on the grid size, the number of sources in flight and the GPU.
+grid barriers but more nodes evaluated before their inputs are final; ``ctas_per_sm`` has no
+effect on the solve by bricks and is kept at 0). The best width depends on the grid size, the
+number of sources in flight and the GPU.
 
 ``Tuner.tune`` times every candidate pair on the caller's own workload (a traveltime call,
 the forward being most of a gradient call too), checks that every candidate returned the
@@ -30,7 +29,7 @@ from typing import Dict, Iterable, Optional, Sequence
 
 import numpy as np
 
-DEFAULT_CANDIDATES: Dict[str, Sequence[float]] = {"round_gate": (1.0, 2.0, 3.0), "ctas_per_sm": (2, 3, 4)}
+DEFAULT_CANDIDATES: Dict[str, Sequence[float]] = {"round_gate": (4.0, 8.0, 16.0, 24.0), "ctas_per_sm": (0,)}
 SHIPPED_TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuned_b200.json")
 
 

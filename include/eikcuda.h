@@ -126,9 +126,8 @@ void* eik_ctx_stream(eik_ctx* ctx);
  * smallest slowness); "sm_fraction" = share of the SMs that the persistent solve kernels of
  * this context occupy, in (0, 1] (contexts whose calls overlap on one GPU, as in a serving
  * loop, each take a share so that their solves can be resident together). For both, 0 (the
- * default) = the library's: round_gate 8 in 2D and 6 in 3D; all SMs, but no more than a forward
- * solve has work for and a quarter of them for the adjoint of calls of fewer than 2^22
- * node-sources (nsrc x grid nodes); "ctas_per_sm" (an integer in [0, 32]) and "fwd_queue" (-1,
+ * default) = the library's: round_gate by dimension and brick size; all SMs, but no more than a
+ * solve has work for; "ctas_per_sm" (an integer in [0, 32]) and "fwd_queue" (-1,
  * 0 or 1) are accepted and checked, and without effect: the forward solve keeps one block per
  * SM, sized by its shared memory; "ray_room" = room of a ray in
  * the single tracing pass, in multiples of its straight-line length (default 3; rays that
@@ -140,10 +139,11 @@ void* eik_ctx_stream(eik_ctx* ctx);
  * diameter (the sum of its sizes) plus 65 536, and a call whose forward solve reaches that
  * limit runs once more with wider rounds and a limit of 2^24 (eik_stats.retries; the result
  * does not depend on the schedule), 2^26 for the adjoint; "auto_round_limit" = that
- * automatic limit of a first run, an integer, 0 (the default) = by the grid's diameter; "cluster_solve" = how problems
- * small enough for one thread-block cluster's shared memory (the refined windows, grids up to
- * ~97 000 nodes) are solved: 1 (the default) = 2D ones in one cluster each (faster there),
- * 2 = in any dimension, 0 = always the persistent global solve. Returns EIK_ERR_ASSERT for an unknown name or a value out of
+ * automatic limit of a first run, an integer, 0 (the default) = by the grid's diameter; "cluster_solve" = whether a
+ * small forward solve (up to 2^20 node-sources; the refined windows, small grids) resets its
+ * state, sets its seeds, solves and stores its results in one launch: 1 (the default) = in 2D, 2 =
+ * in any dimension, 0 = never; "brick_size" = bricks of the forward solve and of the adjoint's: 0
+ * (the default) = by the call's size, 1 = 4x4x4 / 8x8 nodes, 2 = 8x8x8 / 16x16. Returns EIK_ERR_ASSERT for an unknown name or a value out of
  * range. */
 int eik_ctx_set_param(eik_ctx* ctx, const char* name, double value);
 
