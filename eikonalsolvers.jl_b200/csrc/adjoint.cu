@@ -359,10 +359,10 @@ __device__ __forceinline__ unsigned adj_visit(AdjMem<ND, SMALL>& w, const AdjArg
 #pragma unroll
       for (int a = 0; a < ND; a++) {
         const int st = a == 0 ? 1 : (a == 1 ? B::PY : B::PZ);
-        if (info_far(f, a, false) && pending_hi(w.lam[ci - 2 * st])) c++;
-        if (info_near(f, a, false) && pending_hi(w.lam[ci - st])) c++;
-        if (info_near(f, a, true) && pending_hi(w.lam[ci + st])) c++;
-        if (info_far(f, a, true) && pending_hi(w.lam[ci + 2 * st])) c++;
+        c += info_far(f, a, false) & pending_hi(w.lam[ci - 2 * st]);
+        c += (info_near(f, a, false) != 0u) & pending_hi(w.lam[ci - st]);
+        c += (info_near(f, a, true) != 0u) & pending_hi(w.lam[ci + st]);
+        c += info_far(f, a, true) & pending_hi(w.lam[ci + 2 * st]);
       }
       if (pend) cnt = c;
       const unsigned rm = __ballot_sync(FULL_WARP, cnt == 0u);
@@ -398,47 +398,35 @@ __device__ __forceinline__ unsigned adj_visit(AdjMem<ND, SMALL>& w, const AdjArg
       double tv[5];
 #pragma unroll
       for (int m = 0; m < 5; m++) tv[m] = fabs(w.t[ci + (m - 2) * st]);
+      // straight-line over the four places a dependant can be (its stencil runs towards this
+      // node, sign sg), the terms of absent ones left out by selection: lanes differ in which
+      // they have, and as branches each place cost its two orders in turn
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        // dependant at offset dl; its stencil runs towards this node (sign sg)
-        const int dl = j < 2 ? j - 2 : j - 1;
-        const double sg = dl > 0 ? -1.0 : 1.0;
-        const int is = dl > 0 ? -1 : 1;
-        const unsigned order = (j == 0 || j == 3) ? (info_far(f, a, j == 3) ? 2u : 0u) : info_near(f, a, j == 2);
-        if (order) {
-          const bool near = j == 1 || j == 2;
-          const int r = 2 + dl;  // index of the dependant in tv
-          double tmp1, J;
-          if (order == 1u) {
-            tmp1 = 0.0 + (sg * k[0]) * tv[r + is];
-            tmp1 += (sg * -k[0]) * tv[r];
-            J = (2.0 * tmp1) * (sg * k[0]);
-          } else {
-            tmp1 = 0.0 + (sg * -k[3]) * tv[r + 2 * is];
-            tmp1 += (sg * k[2]) * tv[r + is];
-            tmp1 += (sg * -k[1]) * tv[r];
-            J = (2.0 * tmp1) * (sg * (near ? k[2] : -k[3]));
-          }
-          sum -= J * w.lam[ci + dl * st];
-        }
+        const int dl = j < 2 ? j - 2 : j - 1, is = dl > 0 ? -1 : 1, r = 2 + dl;  // r: the dependant in tv
+        const double sg = (double)is;
+        const bool far = j == 0 || j == 3;
+        const unsigned order = far ? (info_far(f, a, j == 3) ? 2u : 0u) : info_near(f, a, j == 2);
+        const bool two = far || order == 2u;
+        // 2 (D_a t) of the dependant; a 1st-order one has no third point (0 + x is x)
+        double tmp1 = two ? (sg * -k[3]) * tv[r + 2 * is] : 0.0;
+        tmp1 += (sg * (two ? k[2] : k[0])) * tv[r + is];
+        tmp1 += (sg * (two ? -k[1] : -k[0])) * tv[r];
+        const double J = (2.0 * tmp1) * (sg * (far ? -k[3] : (two ? k[2] : k[0])));
+        const double next = sum - J * w.lam[ci + dl * st];
+        if (order) sum = next;
       }
-      if (cm[a] != 0) {
-        const int ac = cm[a] < 0 ? -cm[a] : cm[a];
-        const double sg = cm[a] > 0 ? -1.0 : 1.0;
-        const double p0 = tv[2], p1 = cm[a] > 0 ? tv[1] : tv[3], p2 = cm[a] > 0 ? tv[0] : tv[4];
-        double tmp1, v;
-        if (ac == 1) {
-          tmp1 = 0.0 + (sg * k[0]) * p1;
-          tmp1 += (sg * -k[0]) * p0;
-          v = (2.0 * tmp1) * (sg * -k[0]);
-        } else {
-          tmp1 = 0.0 + (sg * -k[3]) * p2;
-          tmp1 += (sg * k[2]) * p1;
-          tmp1 += (sg * -k[1]) * p0;
-          v = (2.0 * tmp1) * (sg * -k[1]);
+      {
+        const bool two = cm[a] == 2 || cm[a] == -2, minus = cm[a] > 0;  // the sign of the code against the side
+        const double sg = minus ? -1.0 : 1.0;
+        double tmp1 = two ? (sg * -k[3]) * (minus ? tv[0] : tv[4]) : 0.0;
+        tmp1 += (sg * (two ? k[2] : k[0])) * (minus ? tv[1] : tv[3]);
+        tmp1 += (sg * (two ? -k[1] : -k[0])) * tv[2];
+        const double v = (2.0 * tmp1) * (sg * (two ? -k[1] : -k[0]));
+        if (cm[a] != 0) {
+          dg = first ? v : dg + v;
+          first = false;
         }
-        dg = first ? v : dg + v;
-        first = false;
       }
     }
     if (act) {
@@ -755,7 +743,7 @@ __device__ double fine_diag(const GridDesc& gf, const uint8_t* code, const doubl
 // ready at once and the rest within a few steps; a step costs its chain of L2 reads, which is
 // why a CTA of 512 threads and not a warp: 16 -> 2.0 ms per call at the default window
 // (36^3 fine nodes), whatever the number of sources.
-constexpr int SRCTERM_THREADS = 512;
+constexpr int SRCTERM_THREADS = 1024;
 __global__ void __launch_bounds__(SRCTERM_THREADS) adj_srcterm_kernel(SrcTermArgs sa) {
   const int s = blockIdx.x;
   const int tid = threadIdx.x;

@@ -9,6 +9,7 @@
 // inserts/updates applied by lane 0 in the reference's order. The fine grid is at most
 // ((2*noderadius+2)*downscalefactor+1)^nd nodes (46,656 at the defaults in 3D).
 #include "kernels.cuh"
+#include "node.cuh"
 
 namespace eik {
 
@@ -545,7 +546,7 @@ __device__ __forceinline__ Key fine_key(const CoarseProblem& P, long long l) {
 }
 __device__ __forceinline__ bool key_lt(const Key& a, const Key& b) { return !key_le(b, a); }
 
-constexpr int SEL_THREADS = 256;
+constexpr int SEL_THREADS = 1024;
 
 // Block-wide argmin of keys (ties: smaller node index); idx -1 = none.
 __device__ void block_min_key(Key* k, long long* idx) {
@@ -608,11 +609,7 @@ __global__ void __launch_bounds__(SEL_THREADS) fine_select_kernel(ForwardBatch f
   uint8_t* onh = fb.fine_onh + base;
   int32_t* order = fb.fine_order + base;
   int32_t* tmp = fb.fine_idx + base;
-  auto coords = [&](long long l, int* f) {
-    f[0] = (int)(l % gf.n[0]);
-    f[1] = (int)((l / gf.n[0]) % gf.n[1]);
-    f[2] = (int)(l / ((long long)gf.n[0] * gf.n[1]));
-  };
+  auto coords = [&](long long l, int* f) { node_coords(gf, l, f); };
   auto is_cc = [&](long long l) {
     int f[3];
     coords(l, f);
