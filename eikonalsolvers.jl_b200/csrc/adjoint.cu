@@ -211,9 +211,9 @@ __device__ int seed_index(const ForwardBatch& fb, int s, long long node) {
 }
 
 // One warp per source. The receivers' interpolation runs one receiver a lane; the sums go over
-// the receivers in order (deterministic), a receiver's corners (distinct nodes) one a lane.
+// the receivers in order (deterministic), 32 corners at a time while they are distinct nodes.
 // With one thread per source every read and sum was a dependent round trip: 2.2 ms for 400
-// receivers a source.
+// receivers a source, 0.35 -> 0.23 ms for 100 against one receiver at a time.
 __global__ void __launch_bounds__(32) adj_recv_kernel(RecvArgs ra) {
   const int s = blockIdx.x, lane = threadIdx.x;
   const GridDesc& g = ra.g;
@@ -262,13 +262,26 @@ __global__ void __launch_bounds__(32) adj_recv_kernel(RecvArgs ra) {
     }
     __syncwarp();
     const int m = (int)min(32LL, r1 - rb);
-    for (int i = 0; i < m; i++) {
-      misf += __shfl_sync(0xffffffffu, term, i);
-      const double fi = __shfl_sync(0xffffffffu, fact, i);
-      if (lane < nc) {
-        const long long node = snode[i][lane];
-        if (node >= 0) __stcg(rhs + node, __ldcg(rhs + node) + (-scoef[i][lane]) * fi);
-        else if (node < -1) __stcg(dpsi + (-2 - node), __ldcg(dpsi + (-2 - node)) + scoef[i][lane] * fi);
+    for (int i = 0; i < m; i++) misf += __shfl_sync(0xffffffffu, term, i);
+    auto add = [&](int i, int c, double fi) {
+      const long long node = snode[i][c];
+      if (node >= 0) __stcg(rhs + node, __ldcg(rhs + node) + (-scoef[i][c]) * fi);
+      else if (node < -1) __stcg(dpsi + (-2 - node), __ldcg(dpsi + (-2 - node)) + scoef[i][c] * fi);
+    };
+    // 32 corners at a time; receivers that share a node among them go one after another
+    const int par = 32 / nc;
+    for (int i0 = 0; i0 < m; i0 += par) {
+      const int i = i0 + lane / nc;
+      const double fi = __shfl_sync(0xffffffffu, fact, min(i, 31));
+      const long long node = i < m ? snode[i][lane % nc] : -1;
+      const unsigned same = __match_any_sync(0xffffffffu, node);
+      if (__any_sync(0xffffffffu, node != -1 && (same & (same - 1u)))) {
+        for (int k = 0; k < par; k++) {
+          if (i < m && lane / nc == k) add(i, lane % nc, fi);
+          __syncwarp();
+        }
+      } else if (i < m) {
+        add(i, lane % nc, fi);
       }
       __syncwarp();
     }
@@ -693,21 +706,29 @@ __device__ __forceinline__ unsigned fine_dependants(const GridDesc& gf, const ui
   return dep;
 }
 
+// Jf[r, l] of the dependant r of l in direction k, and r itself.
+__device__ __forceinline__ double fine_term(const GridDesc& gf, const uint8_t* code, const double* fgdt, long long nfmax,
+                                            const int* c, long long l, int k, long long* r) {
+  const int ax = k >> 2, dl = dir_off(k);
+  const long long lr = dir_lin(gf, l, k);
+  int8_t cd[3];
+  unpack_codes(code[lr], cd);
+  const int cc = cd[ax];
+  const int ac = cc < 0 ? -cc : cc, sg = cc > 0 ? -1 : 1;
+  double dh[3];
+  node_dh(gf, c[0] + (ax == 0 ? dl : 0), dh);
+  *r = lr;
+  return fgdt[(long long)ax * nfmax + lr] * ((double)sg * dcoeff(ac, -dl * sg, dh[ax]));
+}
+
 // Σ_r Jf[r, l] λf_r over the dependants of l, in the order of their bits (axis, then offset).
 __device__ __forceinline__ double fine_downsum(const GridDesc& gf, const uint8_t* code, const double* fgdt,
                                                long long nfmax, const double* lamf, const int* c, long long l,
                                                unsigned dep) {
   double sum = 0.0;
   for (; dep; dep &= dep - 1u) {
-    const int k = __ffs(dep) - 1, ax = k >> 2, dl = dir_off(k);
-    const long long lr = dir_lin(gf, l, k);
-    int8_t cd[3];
-    unpack_codes(code[lr], cd);
-    const int cc = cd[ax];
-    const int ac = cc < 0 ? -cc : cc, sg = cc > 0 ? -1 : 1;
-    double dh[3];
-    node_dh(gf, c[0] + (ax == 0 ? dl : 0), dh);
-    const double J = fgdt[(long long)ax * nfmax + lr] * ((double)sg * dcoeff(ac, -dl * sg, dh[ax]));
+    long long lr;
+    const double J = fine_term(gf, code, fgdt, nfmax, c, l, __ffs(dep) - 1, &lr);
     sum += J * __ldcg(lamf + lr);
   }
   return sum;
@@ -738,12 +759,14 @@ __device__ double fine_diag(const GridDesc& gf, const uint8_t* code, const doubl
 // (computestuff_finegrid!, calc_duh_dva_finegrid!, eikmaingrad.jl:540-741). By linearity
 // the same numbers come from ONE fine adjoint solve with right-hand side -z on the
 // coarse-coincident fine nodes, done here in reverse fine FMM order, SRCTERM_THREADS
-// positions at a time: a node is computed once its dependants are (their λ carries the state,
-// LAM_PENDING_BITS before). Consecutive positions lie all over the front, so most of a window is
-// ready at once and the rest within a few steps; a step costs its chain of L2 reads, which is
-// why a CTA of 512 threads and not a warp: 16 -> 2.0 ms per call at the default window
-// (36^3 fine nodes), whatever the number of sources.
+// positions in hand: a node is computed once its dependants are (their λ carries the state,
+// LAM_PENDING_BITS before). Consecutive positions lie all over the front, so most of them are
+// ready at once and the rest within a few tries; what a node costs is its chain of L2 reads,
+// which is why 32 warps that do not wait for one another. Per call at the default window (36^3
+// fine nodes), whatever the number of sources: 16 ms by one warp, 1.5-1.9 ms in windows of 1024
+// positions with a barrier after each try, 0.7-0.8 ms now (128^3 x 1, 64^3 x 32).
 constexpr int SRCTERM_THREADS = 1024;
+constexpr int SRCTERM_POLLS = 1 << 20;  // about a second; a sweep takes about a millisecond
 __global__ void __launch_bounds__(SRCTERM_THREADS) adj_srcterm_kernel(SrcTermArgs sa) {
   const int s = blockIdx.x;
   const int tid = threadIdx.x;
@@ -792,39 +815,47 @@ __global__ void __launch_bounds__(SRCTERM_THREADS) adj_srcterm_kernel(SrcTermArg
   double* lamf = sa.fine_lam + (size_t)s * nfmax;
   double* fgdt = sa.fine_gdt + (size_t)s * g.nd * nfmax;
   const int nacc = o.nacc, nsf = o.nsrcf;
-  // rows of the fine system and the coarse-point numbering (FMM order of the h points)
-  __shared__ int wcount[SRCTERM_THREADS / 32];
+  // rows of the fine system and the coarse-point numbering (FMM order of the h points): a warp
+  // per stretch of positions
+  constexpr int NW = SRCTERM_THREADS / 32;
+  __shared__ int wcount[NW];
   const int lane = tid & 31, warp = tid >> 5;
-  int run = 0;
-  for (int b = 0; b < nacc; b += SRCTERM_THREADS) {
-    const int p = b + tid;
-    long long l = 0;
+  const int per = ((nacc + NW - 1) / NW + 31) & ~31, plo = min(nacc, warp * per), phi = min(nacc, plo + per);
+  int at = 0;
+#pragma unroll 2
+  for (int p = plo + lane; p - lane < phi; p += 32) {
     bool h = false;
-    if (p < nacc) {
-      l = order[p];
+    if (p < phi) {
+      const long long l = order[p];
       lamf[l] = p >= nsf ? __longlong_as_double((long long)LAM_PENDING_BITS) : 0.0;
       for (int a = 0; a < g.nd; a++) fgdt[(long long)a * nfmax + l] = (p >= nsf) ? fine_gdt_of(gf, tt, code, l, a) : 0.0;
       h = onh[l] != 0;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, h);
-    if (lane == 0) wcount[warp] = __popc(m);
-    __syncthreads();
-    int at = run;
-    for (int w = 0; w < SRCTERM_THREADS / 32; w++) {
-      if (w < warp) at += wcount[w];
-      run += wcount[w];
-    }
-    if (p < nacc) hk[l] = h ? at + __popc(m & ((1u << lane) - 1u)) : -1;
-    __syncthreads();
+    at += __popc(__ballot_sync(0xffffffffu, h));
   }
-  // reverse sweep: the largest unfinished position of a window is always ready
-  for (int b = nacc - 1; b >= nsf; b -= SRCTERM_THREADS) {
-    const int p = b - tid;
+  if (lane == 0) wcount[warp] = at;
+  __syncthreads();
+  at = 0;
+  for (int w = 0; w < warp; w++) at += wcount[w];
+#pragma unroll 4
+  for (int p = plo + lane; p - lane < phi; p += 32) {
+    const long long l = p < phi ? order[p] : 0;
+    const bool h = p < phi && onh[l] != 0;
+    const unsigned m = __ballot_sync(0xffffffffu, h);
+    if (p < phi) hk[l] = h ? at + __popc(m & ((1u << lane) - 1u)) : -1;
+    at += __popc(m);
+  }
+  __syncthreads();
+  // Reverse sweep. The warps take the positions from the last down, 32 at a time and without a
+  // barrier between them: a dependant stands at a later position, so it is in a chunk that is
+  // finished or in some warp's hands, and the largest unfinished position never waits.
+  for (int b = nacc - 1 - 32 * warp; b >= nsf; b -= SRCTERM_THREADS) {
+    const int p = b - lane;
     bool done = p < nsf;
-    long long l = 0;
+    long long l = 0, lr = 0;
     int c[3] = {0, 0, 0};
     unsigned dep = 0u;
-    double rhs = 0.0, diag = 1.0;
+    double rhs = 0.0, diag = 1.0, sum = 0.0, J = 0.0;
     if (!done) {
       l = order[p];
       node_coords(gf, l, c);
@@ -832,21 +863,27 @@ __global__ void __launch_bounds__(SRCTERM_THREADS) adj_srcterm_kernel(SrcTermArg
       const int k = hk[l];
       rhs = (k >= 0) ? -(y[k] + dpsi[k]) : 0.0;
       diag = fine_diag(gf, code, fgdt, nfmax, l);
+      if (dep) J = fine_term(gf, code, fgdt, nfmax, c, l, __ffs(dep) - 1, &lr);
     }
-    for (int step = 0; step <= SRCTERM_THREADS; step++) {
-      if (!done) {
-        bool ready = true;
-        for (unsigned m = dep; m && ready; m &= m - 1u)
-          ready = !lam_pending(__ldcg(lamf + dir_lin(gf, l, __ffs(m) - 1)));
-        if (ready) {
-          // nodes of the window are computed from final values only, whenever they see them
-          __stcg(lamf + l, (rhs - fine_downsum(gf, code, fgdt, nfmax, lamf, c, l, dep)) / diag);
-          done = true;
+    int left = SRCTERM_POLLS;
+    while (__any_sync(0xffffffffu, !done) && left-- > 0) {
+      if (done) continue;
+      if (dep) {  // the dependants' terms in the order of their bits, each as soon as its λ is there
+        const double lr_lam = __ldcg(lamf + lr);
+        if (!lam_pending(lr_lam)) {
+          sum += J * lr_lam;
+          dep &= dep - 1u;
+          if (dep) J = fine_term(gf, code, fgdt, nfmax, c, l, __ffs(dep) - 1, &lr);
         }
       }
-      if (__syncthreads_and(done)) break;
+      if (!dep) {
+        __stcg(lamf + l, (rhs - sum) / diag);
+        done = true;
+      }
     }
+    if (left < 0 && !done) atomicOr(fb.err, ERRB_ADJ_NOT_CONVERGED);
   }
+  __syncthreads();
   // per source-box corner: (∂g/∂τ_s)ᵀ λf + H_Aᵀ z
   if (tid < nsf) {
     const long long l = order[tid];
@@ -875,23 +912,29 @@ __global__ void __launch_bounds__(SRCTERM_THREADS) adj_srcterm_kernel(SrcTermArg
       const long long cl = fb.seed_lin[(size_t)s * fb.seedcap + k];
       const int c[3] = {(int)(cl % g.n[0]), (int)((cl / g.n[0]) % g.n[1]), (int)(cl / ((long long)g.n[0] * g.n[1]))};
       int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
-      for (int d = 0; d < g.nd; d++) {
+      for (int d = 0; d < g.nd; d++) {  // the fine nodes nearest to c are a run of each axis
         const int cc = c[d] - o.fine.ijk1[d];
         lo[d] = max(0, (cc - 1) * o.fine.ds);
         hi[d] = min(gf.n[d] - 1, (cc + 1) * o.fine.ds);
+        while (lo[d] <= hi[d] && fine_nn_axis(o.fine, lo[d]) != cc) lo[d]++;
+        while (hi[d] >= lo[d] && fine_nn_axis(o.fine, hi[d]) != cc) hi[d]--;
       }
       double acc = 0.0;
-      for (int fz = lo[2]; fz <= hi[2]; fz++) {
-        if (g.nd == 3 && fine_nn_axis(o.fine, fz) != c[2] - o.fine.ijk1[2]) continue;
-        for (int fy = lo[1]; fy <= hi[1]; fy++) {
-          if (fine_nn_axis(o.fine, fy) != c[1] - o.fine.ijk1[1]) continue;
-          for (int fx = lo[0]; fx <= hi[0]; fx++) {
-            if (fine_nn_axis(o.fine, fx) != c[0] - o.fine.ijk1[0]) continue;
-            const long long lf = lin3(gf, fx, fy, fz);
-            if (st[lf] >= 2) acc += __ldcg(lamf + lf);
+      for (int fz = lo[2]; fz <= hi[2]; fz++)
+        for (int fy = lo[1]; fy <= hi[1]; fy++)
+          for (int f0 = lo[0]; f0 <= hi[0]; f0 += 8) {
+            const long long lf = lin3(gf, f0, fy, fz);
+            bool take[8];
+            double v[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              take[i] = f0 + i <= hi[0] && st[lf + i] >= 2;
+              v[i] = f0 + i <= hi[0] ? __ldcg(lamf + lf + i) : 0.0;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+              if (take[i]) acc += v[i];
           }
-        }
-      }
       gnode[k] = acc;
     }
   }

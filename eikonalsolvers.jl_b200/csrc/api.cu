@@ -163,25 +163,34 @@ int check_extra(eik_ctx* ctx, const eik_extra* ep) {
   return EIK_OK;
 }
 
-__global__ void slowness_kernel(const double* vel, double* slow, long long n, int* nonpos, double* ssum,
-                                unsigned long long* smin) {
-  double acc = 0.0, mn = EIK_INF;
+// Slowness of a model, whether a velocity is not positive, and the smallest slowness. One atomic
+// per CTA: one per thread on a single word held the pass up at any size, 0.31 -> 0.012 ms (128^3).
+constexpr int SLOW_THREADS = 256;
+__global__ void __launch_bounds__(SLOW_THREADS) slowness_kernel(const double* vel, double* slow, long long n, int* nonpos,
+                                                                unsigned long long* smin) {
+  double mn = EIK_INF;
+  bool bad = false;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double v = vel[i];
-    if (!(v > 0.0)) atomicExch(nonpos, 1);
-    slow[i] = 1.0 / v;
-    acc += (v > 0.0) ? 1.0 / v : 0.0;
-    if (v > 0.0) mn = fmin(mn, 1.0 / v);
+    const double v = vel[i], u = 1.0 / v;
+    slow[i] = u;
+    if (v > 0.0) mn = fmin(mn, u);
+    else bad = true;
   }
-  atomicAdd(ssum, acc);
+  if (bad) atomicExch(nonpos, 1);
+  __shared__ double wmin[SLOW_THREADS / 32];
+  for (int o = 16; o; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+  if ((threadIdx.x & 31) == 0) wmin[threadIdx.x >> 5] = mn;
+  __syncthreads();
+  if (threadIdx.x) return;
+  for (int w = 1; w < SLOW_THREADS / 32; w++) mn = fmin(mn, wmin[w]);
   atomicMin(smin, (unsigned long long)__double_as_longlong(mn));  // positive doubles order as integers
 }
 
 void model_refresh(const Model& m, cudaStream_t st) {
-  cudaMemsetAsync(m.dstat, 0, 2 * sizeof(double), st);
-  cudaMemsetAsync(m.dstat + 2, 0x7f, sizeof(double), st);  // a large positive double
-  slowness_kernel<<<592, 256, 0, st>>>(m.vel, m.slow, m.N, reinterpret_cast<int*>(m.dstat), m.dstat + 1,
-                                       reinterpret_cast<unsigned long long*>(m.dstat + 2));
+  cudaMemsetAsync(m.dstat, 0, sizeof(double), st);
+  cudaMemsetAsync(m.dstat + 1, 0x7f, sizeof(double), st);  // a large positive double
+  slowness_kernel<<<592, SLOW_THREADS, 0, st>>>(m.vel, m.slow, m.N, reinterpret_cast<int*>(m.dstat),
+                                                reinterpret_cast<unsigned long long*>(m.dstat + 1));
 }
 
 const void* stage_host(eik_ctx* ctx, const void* src, size_t bytes) {
@@ -224,11 +233,11 @@ int model_create(eik_ctx* ctx, const eik_grid* grd, const double* vel, bool dev,
   CUDA_OK(ctx, cudaMalloc(&m.slow, bytes));
   if (dev) CUDA_OK(ctx, cudaMemcpyAsync(m.vel, vel, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
   else CUDA_OK(ctx, cudaMemcpyAsync(m.vel, vel, bytes, cudaMemcpyHostToDevice, ctx->stream));
-  CUDA_OK(ctx, cudaMalloc(&m.dstat, 3 * sizeof(double)));
+  CUDA_OK(ctx, cudaMalloc(&m.dstat, 2 * sizeof(double)));
   model_refresh(m, ctx->stream);
   int nonpos = 0;
   CUDA_OK(ctx, cudaMemcpyAsync(&nonpos, m.dstat, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CUDA_OK(ctx, cudaMemcpyAsync(&m.smin, m.dstat + 2, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  CUDA_OK(ctx, cudaMemcpyAsync(&m.smin, m.dstat + 1, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_OK(ctx, cudaStreamSynchronize(ctx->stream));
   if (nonpos) {
     cudaFree(m.vel);
@@ -479,7 +488,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
     node_dh(models[i]->g, 0, dh);
     double hmin = dh[0];
     for (int a = 1; a < nd; a++) hmin = std::min(hmin, dh[a]);
-    problem_scale_kernel<<<(int)((ni + 127) / 128), 128, 0, st>>>(dp + src_off[i], (int)ni, models[i]->dstat + 2,
+    problem_scale_kernel<<<(int)((ni + 127) / 128), 128, 0, st>>>(dp + src_off[i], (int)ni, models[i]->dstat + 1,
                                                                   gate, hmin, nd, csmall ? 1 : 0);
     nlaunch += 1;
   }
@@ -497,7 +506,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
     for (int i = 0; i < nmod; i++) {
       const int64_t o = src_off[i];
       if (src_off[i + 1] == o) continue;
-      launch_fine_setup(slice(i), fprobs + o, models[i]->dstat + 2, ctx->gate_for(nd, fsmall), fsmall, fseed_lin + o * 8, fseed_tt + o * 8,
+      launch_fine_setup(slice(i), fprobs + o, models[i]->dstat + 1, ctx->gate_for(nd, fsmall), fsmall, fseed_lin + o * 8, fseed_tt + o * 8,
                         fslow + o * fb.nfmax, fkL + o * fb.nfmax, fkd + o * fb.nfmax, st);
       nlaunch += 2;
     }

@@ -225,7 +225,7 @@ extern "C" int eik_plan_run(eik_plan* p, const double* vel, const double* pickob
   cudaEventRecord(ctx->ev1, st);
   CUDA_OK(ctx, cudaStreamSynchronize(st));
   const int rc = gradient_tail_stats(ctx, p->tail, stats);
-  CUDA_OK(ctx, cudaMemcpy(&m.smin, m.dstat + 2, sizeof(double), cudaMemcpyDeviceToHost));
+  CUDA_OK(ctx, cudaMemcpy(&m.smin, m.dstat + 1, sizeof(double), cudaMemcpyDeviceToHost));
   if (stats) {
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);

@@ -57,7 +57,7 @@ struct Model {
   double* vel = nullptr;   // device
   double* slow = nullptr;  // device, 1.0/vel
   double smin = 0.0;       // smallest slowness of the model (round width of the forward solve)
-  double* dstat = nullptr; // device: [non-positive flag, Σ slowness, smallest slowness]
+  double* dstat = nullptr; // device: [non-positive flag, smallest slowness]
   int plans = 0;           // captured plans that hold this model's buffers
 };
 
