@@ -482,6 +482,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND, SMALL>& w, const Bri
       }
       const bool ev = act && oc == VISIT_NONE;
       double nv, nL;
+      int nd;
       int8_t cd[3] = {0, 0, 0};
       bool done;
       {
@@ -501,12 +502,18 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND, SMALL>& w, const Bri
           }
         }
         int8_t cf[ND];
-        if (!__any_sync(FULL_WARP, ev && sgn < 0)) {
-          done = prefix_rule_fast<ND, false>(t1, t2, t1, t2, c1, c2, slow, &nv, &nL, cf);
-        } else {
-          // special neighbours of some lane: the same with key levels
+        if (ND == 2 || !__any_sync(FULL_WARP, ev && sgn < 0)) {
+          const int d1[ND][2] = {};
+          done = prefix_rule_fast<ND, false>(t1, t2, t1, t2, d1, c1, c2, slow, &nv, &nL, &nd, cf);
+          nd = nL == nv ? 0 : 1;
+          if (ND == 2 && sgn < 0) done = false;
+        } else if constexpr (ND == 3) {
+          // special neighbours of some lane: the same with key levels. In 2D, where that is one
+          // batch in 400, the general rule takes those nodes: the second copy of the fast rule
+          // costs the others more (300x220 x 4 5.5 -> 5.2 ms without it).
           const long long l = (x0[0] + x) + (long long)n[0] * ((x0[1] + y) + (long long)n[1] * (x0[2] + z));
           double L1[ND][2], L2[ND][2];
+          int d1[ND][2];
 #pragma unroll
           for (int a = 0; a < ND; a++) {
             const long long st = a == 0 ? 1LL : (a == 1 ? (long long)n[0] : (long long)n[0] * n[1]);
@@ -515,16 +522,16 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND, SMALL>& w, const Bri
               const long long l1 = s == 0 ? l + st : l - st, l2 = s == 0 ? l1 + st : l1 - st;
               L1[a][s] = sign_set(t1[a][s]) ? __ldcg(kL + l1) : t1[a][s];
               L2[a][s] = sign_set(t2[a][s]) ? __ldcg(kL + l2) : t2[a][s];
+              d1[a][s] = sign_set(t1[a][s]) ? (int)__ldcg(kd + l1) : 0;
               t1[a][s] = fabs(t1[a][s]);
               t2[a][s] = fabs(t2[a][s]);
             }
           }
-          done = prefix_rule_fast<ND, true>(t1, t2, L1, L2, c1, c2, slow, &nv, &nL, cf);
+          done = prefix_rule_fast<ND, true>(t1, t2, L1, L2, d1, c1, c2, slow, &nv, &nL, &nd, cf);
         }
 #pragma unroll
         for (int a = 0; a < ND; a++) cd[a] = cf[a];
       }
-      int nd = nL == nv ? 0 : 1;
       for (unsigned sl = __ballot_sync(FULL_WARP, ev && !done); sl;) {
         // the next 32 / (2*ND) of them, 2*ND lanes each
         constexpr int G = 2 * ND, PAR = 32 / G;

@@ -415,16 +415,18 @@ EIK_HD bool acc2(const NbhdM&, int a, int l, unsigned T) { return (T >> (6 + slo
 // that happens before the node's own acceptance on one axis, the groups from side 0's
 // traveltime on are decided again with the axis' new point.
 //
-// A value not above its group (non-causal) ends the rule: its key is (group, 1, value).
+// A value not above its group (non-causal) ends the rule: its key is (group, one more than the
+// group's depth, value); d1 are the depths of the immediate neighbours, read with levels only.
 //
-// Left to the general rule: a negative discriminant, mixed sides on several axes or with a
-// non-causal value. With levels, also: a non-causal value; source points; an axis with a special key
-// whose other side is accepted before the node; a 2nd-order point accepted after its 1st-order
-// one and before the node.
+// Left to the general rule: a negative discriminant; mixed sides on several axes or with a
+// non-causal value. With levels, also: source points; equal levels under a non-causal value, or one at
+// the depth limit; an axis with a special key that takes the other side's traveltime or 2nd-order
+// point; a 2nd-order point accepted after its 1st-order one and before the node.
 template <int ND, bool LEVELS>
 EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2], const double (&L1)[ND][2],
-                             const double (&L2)[ND][2], const double (&c1)[ND], const double (&c2)[ND], double slow,
-                             double* v_out, double* L_out, int8_t* codes) {
+                             const double (&L2)[ND][2], const int (&d1)[ND][2], const double (&c1)[ND],
+                             const double (&c2)[ND], double slow, double* v_out, double* L_out, int* d_out,
+                             int8_t* codes) {
   const double s2 = slow * slow;
   double m[ND], x[ND], ca[ND], lev[ND], mar = 0.0;
   uint32_t second = 0u, side = 0u, late = 0u, keyed = 0u;
@@ -465,6 +467,7 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
   for (int a = 0; a < ND; a++) codes[a] = 0;
   if (!(first < EIK_INF)) {
     *v_out = *L_out = EIK_INF;
+    *d_out = 0;
     return ok;
   }
   // the axes in the order of their acceptance: group k is the first k of them
@@ -529,22 +532,38 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
   };
   double v;
   ok = root(&v) && ok;
-  if (below && (LEVELS || !(v < tg))) ok = false;
-  const double reach = below ? tg : v;  // neighbours up to here are accepted before the node
+  int depth = below ? 1 : 0;
+  if (LEVELS && below) {
+    double next = EIK_INF;
+    int at = 0;
+#pragma unroll
+    for (int a = 0; a < ND; a++) {
+      if (lev[a] > tg && lev[a] < next) next = lev[a];
+      if (lev[a] == tg) {
+        at++;
+        depth = 1 + (((side >> a) & 1u) ? d1[a][1] : d1[a][0]);
+      }
+    }
+    if (v > tg) {  // above its group after all, by the root's rounding
+      below = false;
+      depth = 0;
+      if (!(v < next)) ok = false;
+    } else if (!(v <= tg) || depth > EIK_MAX_DEPTH) {
+      ok = false;
+    }
+    if (at > 1) ok = false;
+  } else if (below && !(v < tg)) {
+    ok = false;
+  }
+  double reach = below ? tg : v;  // neighbours up to here are accepted before the node
   uint32_t mixed = 0u;
 #pragma unroll
-  for (int a = 0; a < ND; a++) {
-    if ((((side & ~second) >> a) & 1u) && (below ? t1[a][0] <= reach : t1[a][0] < reach) && t2[a][0] <= t1[a][0] &&
-        t2[a][1] > t1[a][0])
+  for (int a = 0; a < ND; a++)
+    if ((((side & ~second & ~keyed) >> a) & 1u) && (below ? t1[a][0] <= reach : t1[a][0] < reach) &&
+        t2[a][0] <= t1[a][0] && t2[a][1] > t1[a][0])
       mixed |= 1u << a;
-    if (LEVELS && ((keyed >> a) & 1u)) {
-      const bool hi = (side >> a) & 1u;
-      if ((hi ? L1[a][0] : L1[a][1]) <= v) ok = false;
-      if (((late >> a) & 1u) && (hi ? L2[a][1] : L2[a][0]) <= v) ok = false;
-    }
-  }
   if (mixed) {
-    if (LEVELS || below || (mixed & (mixed - 1u))) return false;
+    if (below || (mixed & (mixed - 1u))) return false;
     double keep = EIK_INF;  // side 1's own distance-2 node must stay unaccepted up to the last group
 #pragma unroll
     for (int a = 0; a < ND; a++)
@@ -579,9 +598,24 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
     ok = root(&v) && ok;
 #pragma unroll
     for (int a = 0; a < ND; a++) {
-      if ((t1[a][0] < v && t1[a][0] >= keep) || (t1[a][1] < v && t1[a][1] >= keep)) ok = false;
-      if ((((side & ~second & ~mixed) >> a) & 1u) && t1[a][0] < v && t2[a][0] <= t1[a][0] && t2[a][1] > t1[a][0])
+      const double l0 = LEVELS ? L1[a][0] : t1[a][0], l1 = LEVELS ? L1[a][1] : t1[a][1];
+      if ((l0 < v && l0 >= keep) || (l1 < v && l1 >= keep)) ok = false;
+      if ((((side & ~second & ~mixed & ~keyed) >> a) & 1u) && t1[a][0] < v && t2[a][0] <= t1[a][0] && t2[a][1] > t1[a][0])
         ok = false;
+    }
+    reach = v;
+  }
+  if (LEVELS) {
+    // the other side of an axis with a special key, accepted before the node: without effect when
+    // its traveltime is the larger, no 2nd-order point of side 0 stays behind, and no tie decides
+#pragma unroll
+    for (int a = 0; a < ND; a++) {
+      if (!((keyed >> a) & 1u)) continue;
+      const bool hi = (side >> a) & 1u;
+      const double lo = hi ? L1[a][0] : L1[a][1], to = hi ? t1[a][0] : t1[a][1];
+      if (lo <= reach && (lo == reach || (hi ? !(m[a] < to) || (!((second >> a) & 1u) && t2[a][0] <= t1[a][0]) : to < m[a])))
+        ok = false;
+      if (((late >> a) & 1u) && (hi ? L2[a][1] : L2[a][0]) <= reach) ok = false;
     }
   }
 #pragma unroll
@@ -591,6 +625,7 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
   }
   *v_out = v;
   *L_out = below ? tg : v;
+  *d_out = depth;
   return ok;
 }
 

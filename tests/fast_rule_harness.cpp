@@ -50,6 +50,7 @@ static void run(long long cases, unsigned long long seed, bool specials) {
         }
       }
     double t1[ND][2], t2[ND][2], L1[ND][2], L2[ND][2], c1[ND], c2[ND];
+    int d1[ND][2];
     bool special = false;
     for (int a = 0; a < ND; a++) {
       c1[a] = 1.0 / (nb.dh[a] * nb.dh[a]);
@@ -57,6 +58,7 @@ static void run(long long cases, unsigned long long seed, bool specials) {
       for (int l = 0; l < 2; l++) {
         t1[a][l] = nb.t1[a][l];
         t2[a][l] = nb.t2[a][l];
+        d1[a][l] = (int)((nb.d1 >> (4 * slot(a, l))) & 15u);
         L1[a][l] = nb.L1[a][l];
         L2[a][l] = nb.L2[a][l];
         special = special || L1[a][l] != t1[a][l] || L2[a][l] != t2[a][l];
@@ -66,12 +68,13 @@ static void run(long long cases, unsigned long long seed, bool specials) {
     Key key;
     bool neg = false;
     double vf, Lf;
+    int df;
     const double v = prefix_rule<ND>(nb, cr, &key, &neg);
-    const bool ok = special ? prefix_rule_fast<ND, true>(t1, t2, L1, L2, c1, c2, nb.slow, &vf, &Lf, cf)
-                            : prefix_rule_fast<ND, false>(t1, t2, t1, t2, c1, c2, nb.slow, &vf, &Lf, cf);
+    const bool ok = special ? prefix_rule_fast<ND, true>(t1, t2, L1, L2, d1, c1, c2, nb.slow, &vf, &Lf, &df, cf)
+                            : prefix_rule_fast<ND, false>(t1, t2, t1, t2, d1, c1, c2, nb.slow, &vf, &Lf, &df, cf);
     if (!ok) continue;
     decided++;
-    if (std::memcmp(&v, &vf, 8) || std::memcmp(&key.L, &Lf, 8) || key.d != (Lf == vf ? 0 : 1) || neg || std::memcmp(cr, cf, ND)) differing++;
+    if (std::memcmp(&v, &vf, 8) || std::memcmp(&key.L, &Lf, 8) || key.d != df || neg || std::memcmp(cr, cf, ND)) differing++;
   }
   std::printf("%lld %lld\n", decided, differing);
 }
