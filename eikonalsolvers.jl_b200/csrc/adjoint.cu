@@ -1683,7 +1683,10 @@ extern "C" int eik_gradient(eik_ctx* ctx, eik_model_id model, int64_t nsrc, cons
   if (rc) return rc;
   double hm = 0.0;
   CUDA_OK(ctx, cudaMemcpyAsync(&hm, d_m, sizeof(double), cudaMemcpyDeviceToHost, st));
-  if (gradvel && wantvel) CUDA_OK(ctx, cudaMemcpyAsync(gradvel, d_gv, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
+  if (gradvel && wantvel) {
+    rc = copy_out(ctx, gradvel, d_gv, (unsigned long long)N, st);
+    if (rc) return rc;
+  }
   if (gradsrc && wantsrc)
     CUDA_OK(ctx, cudaMemcpyAsync(gradsrc, d_gs, sizeof(double) * nsrc * nd, cudaMemcpyDeviceToHost, st));
   cudaEventRecord(ctx->ev1, st);

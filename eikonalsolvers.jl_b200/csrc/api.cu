@@ -215,7 +215,8 @@ __global__ void problem_scale_kernel(CoarseProblem* dp, int nprob, const double*
   dp[s].din = inner_window(nd, small != 0, hmin * smin);
 }
 
-int model_create(eik_ctx* ctx, const eik_grid* grd, const double* vel, bool dev, eik_model_id* out) {
+enum class VelFrom { host, host_rows, device };
+int model_create(eik_ctx* ctx, const eik_grid* grd, const double* vel, VelFrom from, eik_model_id* out) {
   std::lock_guard<std::mutex> lk(ctx->mu);
   Model m;
   int rc = make_griddesc(ctx, grd, &m.g);
@@ -231,8 +232,13 @@ int model_create(eik_ctx* ctx, const eik_grid* grd, const double* vel, bool dev,
   CUDA_OK(ctx, cudaSetDevice(ctx->device));
   CUDA_OK(ctx, cudaMalloc(&m.vel, bytes));
   CUDA_OK(ctx, cudaMalloc(&m.slow, bytes));
-  if (dev) CUDA_OK(ctx, cudaMemcpyAsync(m.vel, vel, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-  else CUDA_OK(ctx, cudaMemcpyAsync(m.vel, vel, bytes, cudaMemcpyHostToDevice, ctx->stream));
+  if (from == VelFrom::host_rows) {  // by way of the slowness array, which is written afterwards
+    CUDA_OK(ctx, cudaMemcpyAsync(m.slow, vel, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    launch_columns(m.g, m.slow, m.vel, ctx->stream);
+  } else {
+    CUDA_OK(ctx, cudaMemcpyAsync(m.vel, vel, bytes,
+                                 from == VelFrom::device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream));
+  }
   CUDA_OK(ctx, cudaMalloc(&m.dstat, 2 * sizeof(double)));
   model_refresh(m, ctx->stream);
   int nonpos = 0;
@@ -677,6 +683,7 @@ int eik_ctx_destroy(eik_ctx* ctx) {
     cudaFree(kv.second.dstat);
   }
   ctx->scratch.release_all();
+  free_ring(ctx->ring);
   cudaEventDestroy(ctx->ev0);
   cudaEventDestroy(ctx->ev1);
   for (auto& e : ctx->evk) cudaEventDestroy(e);
@@ -790,12 +797,17 @@ const char* eik_last_error(eik_ctx* ctx) {
 
 int eik_model_upload(eik_ctx* ctx, const eik_grid* grd, const double* vel, eik_model_id* out) {
   if (!ctx || !vel || !out) return fail(ctx, EIK_ERR_ASSERT, "NULL argument");
-  return model_create(ctx, grd, vel, false, out);
+  return model_create(ctx, grd, vel, VelFrom::host, out);
+}
+
+int eik_model_upload_rows(eik_ctx* ctx, const eik_grid* grd, const double* vel, eik_model_id* out) {
+  if (!ctx || !vel || !out) return fail(ctx, EIK_ERR_ASSERT, "NULL argument");
+  return model_create(ctx, grd, vel, VelFrom::host_rows, out);
 }
 
 int eik_model_upload_device(eik_ctx* ctx, const eik_grid* grd, const double* vel_dev, eik_model_id* out) {
   if (!ctx || !vel_dev || !out) return fail(ctx, EIK_ERR_ASSERT, "NULL argument");
-  return model_create(ctx, grd, vel_dev, true, out);
+  return model_create(ctx, grd, vel_dev, VelFrom::device, out);
 }
 
 int eik_model_release(eik_ctx* ctx, eik_model_id model) {
@@ -816,9 +828,10 @@ int eik_model_release(eik_ctx* ctx, eik_model_id model) {
   return EIK_OK;
 }
 
-int eik_traveltime(eik_ctx* ctx, eik_model_id model, int64_t nsrc, const double* coordsrc,
-                   const int64_t* rec_off, const double* rec, const eik_extra* ep_in, double* picks,
-                   double* ttgrids, eik_stats* stats) {
+// ttgrids: all grids column-major, one after another; ttrows: one row-major grid per source.
+static int traveltime_call(eik_ctx* ctx, eik_model_id model, int64_t nsrc, const double* coordsrc,
+                           const int64_t* rec_off, const double* rec, const eik_extra* ep_in, double* picks,
+                           double* ttgrids, double* const* ttrows, eik_stats* stats) {
   if (!ctx) return fail(ctx, EIK_ERR_ASSERT, "NULL context");
   std::lock_guard<std::mutex> lk(ctx->mu);
   ctx->scratch.begin_call();
@@ -861,8 +874,9 @@ int eik_traveltime(eik_ctx* ctx, eik_model_id model, int64_t nsrc, const double*
     if (nrec && stats) stats->launches += 1;
     CUDA_OK(ctx, cudaGetLastError());
     if (nrec) CUDA_OK(ctx, cudaMemcpyAsync(picks, d_picks, sizeof(double) * nrec, cudaMemcpyDeviceToHost, st));
-    if (ttgrids)
-      CUDA_OK(ctx, cudaMemcpyAsync(ttgrids, fw.t, sizeof(double) * nsrc * m.N, cudaMemcpyDeviceToHost, st));
+    if (ttgrids) r = copy_out(ctx, ttgrids, fw.t, (unsigned long long)nsrc * m.N, st);
+    if (ttrows) r = copy_rows_out(ctx, ttrows, fw.t, nsrc, m.g, st);
+    if (r) return r;
     cudaEventRecord(ctx->ev1, st);
     return collect_forward_stats(ctx, &fw, stats);
   });
@@ -872,6 +886,20 @@ int eik_traveltime(eik_ctx* ctx, eik_model_id model, int64_t nsrc, const double*
     stats->device_ms = ms;
   }
   return rc;
+}
+
+int eik_traveltime(eik_ctx* ctx, eik_model_id model, int64_t nsrc, const double* coordsrc,
+                   const int64_t* rec_off, const double* rec, const eik_extra* ep, double* picks,
+                   double* ttgrids, eik_stats* stats) {
+  return traveltime_call(ctx, model, nsrc, coordsrc, rec_off, rec, ep, picks, ttgrids, nullptr, stats);
+}
+
+int eik_traveltime_rows(eik_ctx* ctx, eik_model_id model, int64_t nsrc, const double* coordsrc,
+                        const int64_t* rec_off, const double* rec, const eik_extra* ep, double* picks,
+                        double* const* ttgrids, eik_stats* stats) {
+  for (int64_t s = 0; s < nsrc; s++)
+    if (!ttgrids || !ttgrids[s]) return fail(ctx, EIK_ERR_ASSERT, "NULL argument");
+  return traveltime_call(ctx, model, nsrc, coordsrc, rec_off, rec, ep, picks, nullptr, ttgrids, stats);
 }
 
 int eik_traveltime_multi(eik_ctx* ctx, int64_t nmodel, const eik_model_id* model_ids, const int64_t* src_off,

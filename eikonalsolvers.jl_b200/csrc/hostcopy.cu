@@ -1,0 +1,148 @@
+// Large results to pageable host memory, and arrays whose host side is row-major.
+//
+// What bounds such a copy is the host: one thread of the driver copies out of its own pinned
+// buffer and takes the page faults of a fresh destination. Here several threads do, each with
+// two pinned slots of its own, the next chunk crossing the bus while it copies the last one. A
+// row-major destination (the layout of NumPy's default) is gathered by a kernel straight into
+// the slot: the strided reads hit L2, where a transpose on the host reads a cache line per value.
+// Measured with 16 host cores: the 134 MB of a 256^3 gradient 26 -> 5 ms; a 200^3 grid to row-major
+// 41 ms (copy, then NumPy's transpose) -> 5 ms. Slots of 0.5, 1 and 2 MB differ by less than the runs
+// do, and the smallest cost the first call of a context least (3.3, 4.8, 6.7 ms).
+#include <atomic>
+#include <cstring>
+#include <thread>
+
+#include "runtime.hpp"
+
+namespace eik {
+
+constexpr size_t HOST_COPY_MIN = (size_t)8 << 20;
+
+// out[q] = t at row-major position o0 + q (last axis fastest) of a column-major grid.
+__global__ void rows_kernel(const double* t, double* out, int nd, int n0, int n1, int n2, unsigned long long o0,
+                            unsigned cnt) {
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < cnt; q += gridDim.x * blockDim.x) {
+    const unsigned long long o = o0 + q;
+    if (nd == 2) {
+      out[q] = t[o / n1 + (unsigned long long)n0 * (o % n1)];
+    } else {
+      const unsigned long long k = o % n2, r = o / n2;
+      out[q] = t[r / n1 + (unsigned long long)n0 * (r % n1 + (unsigned long long)n1 * k)];
+    }
+  }
+}
+
+// out[l] (column-major) = rows at the same node of a row-major grid.
+__global__ void columns_kernel(const double* rows, double* out, int nd, int n0, int n1, int n2, unsigned long long n) {
+  for (unsigned long long l = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; l < n;
+       l += (unsigned long long)gridDim.x * blockDim.x) {
+    const unsigned long long i = l % n0, r = l / n0;
+    out[l] = nd == 2 ? rows[r + (unsigned long long)n1 * i]
+                     : rows[r / n1 + (unsigned long long)n2 * (r % n1 + (unsigned long long)n1 * i)];
+  }
+}
+
+void launch_columns(const GridDesc& g, const double* rows, double* out, cudaStream_t st) {
+  columns_kernel<<<1184, 256, 0, st>>>(rows, out, g.nd, g.n[0], g.n[1], g.n[2], (unsigned long long)npts(g));
+}
+
+static bool ring_ready(eik_ctx* ctx) {
+  HostRing& h = ctx->ring;
+  if (h.buf) return true;
+  if (cudaMallocHost(&h.buf, HOST_SLOTS * HOST_SLOT) != cudaSuccess) {
+    h.buf = nullptr;
+    cudaGetLastError();
+    return false;
+  }
+  for (auto& e : h.ev)
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+      free_ring(h);
+      cudaGetLastError();
+      return false;
+    }
+  return true;
+}
+
+void free_ring(HostRing& h) {
+  for (auto& e : h.ev) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  }
+  if (h.buf) cudaFreeHost(h.buf);
+  h.buf = nullptr;
+}
+
+// nsrc arrays of n doubles by chunks through the ring; rows: row-major at the destination.
+static int copy_chunks(eik_ctx* ctx, double* const* dst, const double* src, int64_t nsrc, unsigned long long n,
+                       const GridDesc* rows, cudaStream_t st) {
+  CUDA_OK(ctx, cudaStreamSynchronize(st));  // the threads would spin while the solve runs
+  const unsigned long long per = HOST_SLOT / sizeof(double), parts = (n + per - 1) / per, nchunk = parts * nsrc;
+  std::atomic<unsigned long long> next{0};
+  std::atomic<int> bad{(int)cudaSuccess};
+  auto count = [&](unsigned long long c) { return (unsigned)std::min<unsigned long long>(per, n - c % parts * per); };
+  auto work = [&](int w) noexcept {
+    cudaError_t e = cudaSetDevice(ctx->device);
+    bool have = false;
+    unsigned long long last = 0;  // chunk in this worker's other slot, if it has one
+    for (int k = 0; e == cudaSuccess && bad.load() == (int)cudaSuccess; k++) {
+      const unsigned long long c = next.fetch_add(1);
+      const int s = 2 * w + (k & 1);
+      if (c < nchunk) {
+        char* slot = ctx->ring.buf + (size_t)s * HOST_SLOT;
+        const double* from = src + c / parts * n;
+        if (rows)
+          rows_kernel<<<64, 256, 0, st>>>(from, reinterpret_cast<double*>(slot), rows->nd, rows->n[0], rows->n[1],
+                                          rows->n[2], c % parts * per, count(c));
+        else
+          cudaMemcpyAsync(slot, from + c % parts * per, sizeof(double) * count(c), cudaMemcpyDeviceToHost, st);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->ring.ev[s], st);
+      }
+      if (have && e == cudaSuccess) {
+        e = cudaEventSynchronize(ctx->ring.ev[s ^ 1]);
+        if (e == cudaSuccess)
+          std::memcpy(dst[last / parts] + last % parts * per, ctx->ring.buf + (size_t)(s ^ 1) * HOST_SLOT,
+                      sizeof(double) * count(last));
+      }
+      have = c < nchunk;
+      last = c;
+      if (!have) break;
+    }
+    if (e != cudaSuccess) bad.store((int)e);
+  };
+  const int workers = (int)std::min<unsigned long long>(HOST_SLOTS / 2, nchunk);
+  std::thread more[HOST_SLOTS / 2];
+  try {
+    for (int w = 1; w < workers; w++) more[w] = std::thread(work, w);
+  } catch (...) {
+    // no more threads to be had: the ones there are take all chunks
+  }
+  work(0);
+  for (auto& t : more)
+    if (t.joinable()) t.join();
+  CUDA_OK(ctx, cudaStreamSynchronize(st));
+  CUDA_OK(ctx, (cudaError_t)bad.load());
+  return EIK_OK;
+}
+
+int copy_out(eik_ctx* ctx, double* dst, const double* src, unsigned long long n, cudaStream_t st) {
+  const size_t bytes = sizeof(double) * (size_t)n;
+  // small copies: below 8 MB the driver's own takes about 1 ms, less than making the ring costs the first
+  // call; pinned memory takes the copy as it is
+  bool plain = bytes < HOST_COPY_MIN || ctx->capturing;
+  if (!plain) {
+    cudaPointerAttributes at;
+    plain = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type != cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+  }
+  if (!plain && ring_ready(ctx)) return copy_chunks(ctx, &dst, src, 1, n, nullptr, st);
+  CUDA_OK(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
+  return EIK_OK;
+}
+
+int copy_rows_out(eik_ctx* ctx, double* const* dst, const double* src, int64_t nsrc, const GridDesc& g, cudaStream_t st) {
+  if (!ring_ready(ctx)) return fail(ctx, EIK_ERR_CUDA, "cudaMallocHost of the staging ring failed");
+  return copy_chunks(ctx, dst, src, nsrc, (unsigned long long)npts(g), &g, st);
+}
+
+}  // namespace eik

@@ -149,6 +149,18 @@ int gradient_core(eik_ctx* ctx, const Model& m, int64_t nsrc, const double* d_cs
 
 }  // namespace eik
 
+namespace eik {
+// Pinned slots and their events for copy_out (hostcopy.cu): made by the first large copy of a
+// context, bounded, freed with it; used under the context's lock.
+constexpr int HOST_SLOTS = 8;
+constexpr size_t HOST_SLOT = (size_t)512 << 10;
+struct HostRing {
+  char* buf = nullptr;
+  cudaEvent_t ev[HOST_SLOTS] = {};
+};
+void free_ring(HostRing& h);
+}  // namespace eik
+
 struct eik_ctx {
   int device = 0;
   int nsm = 148;
@@ -183,12 +195,21 @@ struct eik_ctx {
   bool capturing = false;                    // the pipeline is being captured into a plan's graph
   std::vector<void*>* stage_arena = nullptr; // pinned host copies made while capturing
   int live_plans = 0;
+  eik::HostRing ring;
   size_t model_bytes = 0;
   eik_model_id next_model = 0;
   std::map<eik_model_id, eik::Model> models;
 };
 
 namespace eik {
+// n doubles from the device to the host, after the stream's work. Returns with the copy enqueued
+// (small or pinned) or done.
+int copy_out(eik_ctx* ctx, double* dst, const double* src, unsigned long long n, cudaStream_t st);
+// nsrc column-major grids, one after another in device memory, to one row-major array each.
+int copy_rows_out(eik_ctx* ctx, double* const* dst, const double* src, int64_t nsrc, const GridDesc& g, cudaStream_t st);
+// A row-major grid in device memory, column-major to out.
+void launch_columns(const GridDesc& g, const double* rows, double* out, cudaStream_t st);
+
 // Runs one pipeline (`call`, which returns an EIK_* code); when its forward solve stopped at
 // the library's automatic round limit (no max_rounds set), runs it once more with wider
 // rounds and the full limit. The solve's result is the fixed point of the order rule, the

@@ -25,7 +25,7 @@ EXPORTED = ["eik_extra_defaults", "eik_ctx_create", "eik_ctx_destroy", "eik_last
             "eik_gradient", "eik_gradient_device", "eik_ctx_stream", "eik_ttimemisfit_noalloc",
             "eik_ctx_set_param", "eik_plan_gradient", "eik_plan_run", "eik_plan_destroy", "eik_tracerays",
             "eik_traveltime_rays", "eik_selftest_wait", "eik_gradient_bytes", "eik_traveltime_multi",
-            "eik_gradient_groups"]
+            "eik_gradient_groups", "eik_model_upload_rows", "eik_traveltime_rows"]
 
 # eik_stats.warn_mask bits and the reference's @warn messages they stand for
 WARNINGS = {
@@ -102,6 +102,9 @@ def load():
         L.eik_model_release.argtypes = [P, C.c_int64]
         L.eik_traveltime.argtypes = [P, C.c_int64, C.c_int64, P, P, P, C.POINTER(eik_extra), P, P,
                                      C.POINTER(eik_stats)]
+        L.eik_model_upload_rows.argtypes = [P, C.POINTER(eik_grid), P, C.POINTER(C.c_int64)]
+        L.eik_traveltime_rows.argtypes = [P, C.c_int64, C.c_int64, P, P, P, C.POINTER(eik_extra), P, P,
+                                          C.POINTER(eik_stats)]
         L.eik_traveltime_multi.argtypes = [P, C.c_int64, P, P, P, P, P, C.POINTER(eik_extra), P, P,
                                            C.POINTER(eik_stats)]
         L.eik_traveltime_multi.restype = C.c_int
@@ -134,7 +137,8 @@ def load():
         for f in ("eik_plan_gradient", "eik_plan_run", "eik_plan_destroy", "eik_tracerays", "eik_traveltime_rays"):
             getattr(L, f).restype = C.c_int
         for f in ("eik_ctx_create", "eik_ctx_destroy", "eik_model_upload", "eik_model_upload_device",
-                  "eik_model_release", "eik_traveltime", "eik_gradient", "eik_gradient_device"):
+                  "eik_model_release", "eik_traveltime", "eik_gradient", "eik_gradient_device",
+                  "eik_model_upload_rows", "eik_traveltime_rows"):
             getattr(L, f).restype = C.c_int
         _lib = L
         return L

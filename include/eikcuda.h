@@ -157,7 +157,9 @@ int eik_selftest_wait(eik_ctx* ctx, double timeout_s);
 /* Uploads a velocity model (host, column-major, FP64) and keeps it resident. Checks
  * all(vel.>0) (eikmainfwd.jl:45). */
 int eik_model_upload(eik_ctx* ctx, const eik_grid* grd, const double* vel, eik_model_id* out);
-/* Same, from a device pointer of this context's device. */
+/* Same, from a row-major host array (last axis fastest): reordered on the device. */
+int eik_model_upload_rows(eik_ctx* ctx, const eik_grid* grd, const double* vel, eik_model_id* out);
+/* As eik_model_upload, from a device pointer of this context's device. */
 int eik_model_upload_device(eik_ctx* ctx, const eik_grid* grd, const double* vel_dev, eik_model_id* out);
 int eik_model_release(eik_ctx* ctx, eik_model_id model);
 
@@ -173,6 +175,12 @@ int eik_gradient_bytes(eik_ctx* ctx, eik_model_id model, int64_t nsrc, int64_t n
 int eik_traveltime(eik_ctx* ctx, eik_model_id model, int64_t nsrc, const double* coordsrc,
                    const int64_t* rec_off, const double* rec, const eik_extra* ep, double* picks,
                    double* ttgrids, eik_stats* stats);
+
+/* eik_traveltime with the traveltime grid of source s at ttgrids[s], in row-major order (last
+ * axis fastest): reordered on the device. */
+int eik_traveltime_rows(eik_ctx* ctx, eik_model_id model, int64_t nsrc, const double* coordsrc,
+                        const int64_t* rec_off, const double* rec, const eik_extra* ep, double* picks,
+                        double* const* ttgrids, eik_stats* stats);
 
 /* No counterpart in the reference as one call: ttforwsomesrc (eikmainfwd.jl:152-199) for the
  * sources of several models of one dimension, whose grids may differ in size, in one
