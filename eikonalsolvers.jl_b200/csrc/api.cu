@@ -540,7 +540,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
       launch_fine_select(slice(i), fprobs + o, ftie + o, st);
       // stops decided by exact ties: the heap is replayed for the flagged sources only, the
       // flags staying on the device (no host round trip between the stages)
-      launch_fine_replay(slice(i), ftie + o, st);
+      launch_fine_replay(slice(i), fprobs + o, ftie + o, st);
       nlaunch += 2;
     }
     CUDA_OK(ctx, cudaGetLastError());
@@ -614,7 +614,7 @@ int collect_forward_stats(eik_ctx* ctx, ForwardState* fw, eik_stats* stats) {
     stats->tile_activations += ctr[2];
     stats->node_evals += ctr[3];
     stats->fwd_rounds += (uint64_t)rounds;
-    for (uint8_t f : tie) stats->fine_replays += f ? 1 : 0;
+    for (uint8_t f : tie) stats->fine_replays += f == 1 ? 1 : 0;
     for (int k = 0; k < 7; k++) stats->fwd_visits[k] += vis[k];
     float a = 0, b = 0;
     cudaEventElapsedTime(&a, ctx->evk[0], ctx->evk[1]);

@@ -76,8 +76,9 @@ struct SmemHeap {
   }
 };
 
-// Neighbourhood of fine node (i,j,k) for the reference's stencil: accepted <=> status==2.
-__device__ __forceinline__ double fine_update(const GridDesc& gf, const double* tt, const uint8_t* st,
+// The reference's update of fine node (i,j,k) from the nodes that `accepted` (of a node index) holds for.
+template <class ACC>
+__device__ __forceinline__ double fine_update(const GridDesc& gf, const double* tt, const ACC& accepted,
                                               double slow, int i, int j, int k, int8_t* codes,
                                               bool* neg) {
   Nbhd nb;
@@ -92,7 +93,7 @@ __device__ __forceinline__ double fine_update(const GridDesc& gf, const double* 
       p[a] += sh;
       if (p[a] < 0 || p[a] >= gf.n[a]) continue;
       const long long pl = lin3(gf, p[0], p[1], p[2]);
-      if (st[pl] == 2) nb_put1(nb, a, l, tt[pl], -EIK_INF, 0);
+      if (accepted(pl)) nb_put1(nb, a, l, tt[pl], -EIK_INF, 0);
       else nb_put1(nb, a, l, EIK_INF, EIK_INF, 0);
       bool ok = true;
       for (int d = 0; d < gf.nd; d++)
@@ -101,7 +102,7 @@ __device__ __forceinline__ double fine_update(const GridDesc& gf, const double* 
         int q[3] = {p[0], p[1], p[2]};
         q[a] += sh;
         const long long ql = lin3(gf, q[0], q[1], q[2]);
-        if (st[ql] == 2) nb_put2(nb, a, l, tt[ql], -EIK_INF, 0);
+        if (accepted(ql)) nb_put2(nb, a, l, tt[ql], -EIK_INF, 0);
         else nb_put2(nb, a, l, EIK_INF, EIK_INF, 0);
       }
     }
@@ -215,15 +216,60 @@ __device__ long long fine_window(const ForwardBatch& fb, const double* src, Fine
   return nfine;
 }
 
+__device__ __forceinline__ Key fine_key(const CoarseProblem& P, long long l) {
+  const double t = P.t[l];
+  const uint8_t cb = P.code[l];
+  if (cb & CODE_SRC_BIT) return Key{P.kL[l], (int)P.kd[l], t};
+  return Key{t, 0, t};
+}
+__device__ __forceinline__ bool key_lt(const Key& a, const Key& b) { return !key_le(b, a); }
+
+// The replay warns of negative discriminants. Where a tied stop needs no replay (fine_select_kernel)
+// the warning comes from the same updates: those of the neighbours of every node accepted before the
+// last batch, from the nodes accepted by then. By threads t0, t0 + dt, ...
+__device__ void fine_warn(const ForwardBatch& fb, const CoarseProblem& P, int s, int t0, int dt) {
+  const GridDesc& gf = P.g;
+  const int32_t* order = fb.fine_order + (size_t)s * fb.nfmax;
+  const Key last = fine_key(P, order[fb.out[s].nacc - 1]);
+  bool any = false;
+  for (int p = t0; p < fb.out[s].nacc; p += dt) {
+    const Key kp = fine_key(P, order[p]);
+    if (p >= fb.out[s].nsrcf && !key_lt(kp, last)) continue;
+    auto accepted = [&](long long r) { return P.t[r] < EIK_INF && key_le(fine_key(P, r), kp); };
+    int f[3];
+    node_coords(gf, order[p], f);
+    for (int k = 0; k < 2 * gf.nd; k++) {
+      int c[3] = {f[0], f[1], f[2]};
+      c[k >> 1] += (k & 1) ? 1 : -1;
+      if (c[k >> 1] < 0 || c[k >> 1] >= gf.n[k >> 1]) continue;
+      const long long cl = lin3(gf, c[0], c[1], c[2]);
+      if (accepted(cl)) continue;
+      int8_t cd[3];
+      bool neg = false;
+      fine_update(gf, P.t, accepted, P.slow[cl], c[0], c[1], c[2], cd, &neg);
+      any = any || neg;
+    }
+  }
+  if (any) atomicOr(&fb.out[s].warn, WARN_NEG_DISCRIMINANT);
+}
+
+enum : uint8_t { TIE_NONE = 0, TIE_REPLAY = 1, TIE_WARN = 2 };
+constexpr int WARN_CTAS = 16;  // per source, of one warp
+
 // ---------------------------------------------------------------- refined start-up --
 constexpr int FINE_THREADS = 32;
 constexpr int MAXPOP = 128;
 
-__global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb, const uint8_t* only) {
+__global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb, const CoarseProblem* fprobs,
+                                                                const uint8_t* tie) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int s = blockIdx.x;
-  if (only && !only[s]) return;  // replay of the flagged sources only
   const int lane = threadIdx.x;
+  if (tie && tie[s] != TIE_REPLAY) {  // replay of the flagged sources only
+    if (tie[s] == TIE_WARN) fine_warn(fb, fprobs[s], s, blockIdx.y * FINE_THREADS + lane, gridDim.y * FINE_THREADS);
+    return;
+  }
+  if (blockIdx.y) return;
   const GridDesc& g = fb.g;
   SrcOut& o = fb.out[s];
   __shared__ FineInfo fi;
@@ -272,6 +318,7 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
   H.Nh = 0;
   const double* slow = fb.slow;
   const double* vel = fb.vel;
+  auto accepted = [&](long long l) { return st[l] == 2; };
   auto velat_f = [&](int i, int j, int k) { return vel[fine_to_coarse(g, fi, i, j, k)]; };
   auto coarse_of = [&](int i, int j, int k, long long* cl) {
     if (i % fi.ds || j % fi.ds || k % fi.ds) return false;
@@ -328,7 +375,7 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
         if (st[cl] == 0) {
           int8_t cd[3];
           bool neg = false;
-          const double v = fine_update(gf, tt, st, slow[fine_to_coarse(g, fi, c[0], c[1], c[2])], c[0],
+          const double v = fine_update(gf, tt, accepted, slow[fine_to_coarse(g, fi, c[0], c[1], c[2])], c[0],
                                        c[1], c[2], cd, &neg);
           if (neg) warn |= WARN_NEG_DISCRIMINANT;
           if (!H.insert(v, (int32_t)(cl + 1))) sh_err |= ERRB_HEAP_OVERFLOW;
@@ -416,7 +463,7 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
       if (st[cl] == 2) continue;
       int8_t cd[3];
       bool neg = false;
-      evv[e] = fine_update(gf, tt, st, slow[fine_to_coarse(g, fi, c[0], c[1], c[2])], c[0], c[1], c[2], cd,
+      evv[e] = fine_update(gf, tt, accepted, slow[fine_to_coarse(g, fi, c[0], c[1], c[2])], c[0], c[1], c[2], cd,
                            &neg);
       evc[e] = pack_codes(cd, nd);
       evneg[e] = neg;
@@ -461,9 +508,12 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
 // on a non-border edge of the window accepted after at least one coarse-coincident node
 // (eikmainfwd.jl:724-754). Acceptance follows the keys of the order rule, so the stop
 // node is the edge node of smallest key above the first coarse-coincident key, and the
-// accepted set is every node of smaller key plus that node. Only when another node has
-// exactly the stop node's traveltime (or an edge node ties with the first coarse-coincident
-// node) does the heap's internal order decide; those sources are replayed exactly.
+// accepted set is every node of smaller key plus that node. Only when another node has exactly the
+// stop node's traveltime and one of them is coarse-coincident, hence perhaps a seed (or an edge
+// node ties with the first coarse-coincident node), does the heap's internal order decide; those
+// sources, and tied ones with seeds of equal times, are replayed exactly. Other ties without a coarse-coincident node are what constant and
+// laterally uniform velocities give for a source off the nodes: replayed they took 205-225 ms of a
+// 210-230 ms call (64^3, 128^3), which now takes 6.7 and 10 ms.
 
 // Window, fine source box, the fine problem of the round solver, its slowness and seeds.
 __global__ void fine_setup_kernel(ForwardBatch fb, CoarseProblem* fprobs, const double* dsmin, double gate, int small,
@@ -538,14 +588,6 @@ __global__ void fine_fill_kernel(ForwardBatch fb, const CoarseProblem* fprobs) {
   }
 }
 
-__device__ __forceinline__ Key fine_key(const CoarseProblem& P, long long l) {
-  const double t = P.t[l];
-  const uint8_t cb = P.code[l];
-  if (cb & CODE_SRC_BIT) return Key{P.kL[l], (int)P.kd[l], t};
-  return Key{t, 0, t};
-}
-__device__ __forceinline__ bool key_lt(const Key& a, const Key& b) { return !key_le(b, a); }
-
 constexpr int SEL_THREADS = 1024;
 
 // Block-wide argmin of keys (ties: smaller node index); idx -1 = none.
@@ -596,7 +638,7 @@ __global__ void __launch_bounds__(SEL_THREADS) fine_select_kernel(ForwardBatch f
   const int tid = threadIdx.x;
   SrcOut& o = fb.out[s];
   if (o.nsrcf == 0) {
-    if (tid == 0) tie[s] = 0;
+    if (tid == 0) tie[s] = TIE_NONE;
     return;
   }
   const CoarseProblem& P = fprobs[s];
@@ -670,16 +712,21 @@ __global__ void __launch_bounds__(SEL_THREADS) fine_select_kernel(ForwardBatch f
   early_edge = __syncthreads_or(early_edge);
   block_min_key(&ks, &is);
   // ties that only the heap's order can settle
-  bool amb = false;
+  bool amb = false, tied = false, tied_cc = is >= 0 && is_cc(is);
   if (ic < 0) amb = true;  // no coarse-coincident node reached: leave it to the replay
   for (long long l = tid; l < n && !amb; l += SEL_THREADS) {
     const double t = P.t[l];
     if (!(t < EIK_INF)) continue;
-    if (is >= 0 && l != is && t == ks.t) amb = true;
+    if (is >= 0 && l != is && t == ks.t) {
+      tied = true;
+      tied_cc = tied_cc || is_cc(l);
+    }
     if (ic >= 0 && kc.L != -EIK_INF && l != ic && is_edge(l) && !is_corner(l) && t == kc.t) amb = true;
   }
-  amb = __syncthreads_or(amb);
-  if (tid == 0) tie[s] = amb ? 1 : 0;
+  tied = __syncthreads_or(tied);
+  tied_cc = __syncthreads_or(tied_cc);
+  amb = __syncthreads_or(amb) || (tied && tied_cc);
+  if (tid == 0) tie[s] = amb ? TIE_REPLAY : TIE_NONE;
   if (amb) return;
   // status and the accepted non-corner nodes (unordered)
   __shared__ unsigned int nlist;
@@ -773,6 +820,19 @@ __global__ void __launch_bounds__(SEL_THREADS) fine_select_kernel(ForwardBatch f
       for (int w = 0; w < SEL_THREADS / 32; w++) carry += wsum[w];
     __syncthreads();
   }
+  if (tied) {
+    // Which of the tied nodes the heap takes before it stops shows nowhere: none is a seed, and in
+    // the last batch none is read by an accepted node, so its adjoint is zero. But seeds of equal
+    // times among themselves are summed in the heap's order: replayed like a tied seed.
+    int first = 0;
+    for (int c = 0; c < nc; c++) first += is_cc(corner[c]);
+    const int ns = min(carry, (int)fb.seedcap);
+    bool equal = false;
+    for (int k = first + tid; k + 1 < ns; k += SEL_THREADS)
+      equal = equal || fb.seed_tt[(size_t)s * fb.seedcap + k] == fb.seed_tt[(size_t)s * fb.seedcap + k + 1];
+    equal = __syncthreads_or(equal);
+    if (tid == 0) tie[s] = equal ? TIE_REPLAY : TIE_WARN;
+  }
   if (tid == 0) {
     o.nseeds = carry < fb.seedcap ? carry : fb.seedcap;
     o.nacc = nacc;
@@ -808,13 +868,13 @@ void launch_fine(const ForwardBatch& fb, cudaStream_t st) {
     cudaFuncSetAttribute(fine_fmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     attr_set = true;
   }
-  fine_fmm_kernel<<<fb.nsrc, FINE_THREADS, sm, st>>>(fb, nullptr);
+  fine_fmm_kernel<<<fb.nsrc, FINE_THREADS, sm, st>>>(fb, nullptr, nullptr);
 }
 
-void launch_fine_replay(const ForwardBatch& fb, const uint8_t* fine_tie, cudaStream_t st) {
+void launch_fine_replay(const ForwardBatch& fb, const CoarseProblem* fprobs, const uint8_t* fine_tie, cudaStream_t st) {
   const size_t sm = fine_smem_bytes(fb.heapcap);
   cudaFuncSetAttribute(fine_fmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  fine_fmm_kernel<<<fb.nsrc, FINE_THREADS, sm, st>>>(fb, fine_tie);
+  fine_fmm_kernel<<<dim3(fb.nsrc, WARN_CTAS), FINE_THREADS, sm, st>>>(fb, fprobs, fine_tie);
 }
 
 }  // namespace eik

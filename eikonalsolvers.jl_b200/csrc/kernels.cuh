@@ -145,12 +145,12 @@ int brick_size(int nd, bool small);
 unsigned long long brick_number(const GridDesc& g, bool small);
 // Refined start-up as a fixed point: window set-up, the fine problems' arrays, the
 // acceptance set at the reference's stop, and the exact heap replay for the sources
-// whose stop is decided by a tie (flags in fine_tie, nonzero = replay needed).
+// whose stop is decided by a tie (flags in fine_tie, 1 = replay needed, 2 = its warning only).
 void launch_fine_setup(const ForwardBatch& fb, CoarseProblem* fprobs, const double* dsmin, double gate, bool small,
                        int32_t* fseed_lin, double* fseed_tt, double* fine_slow, double* fine_kL, uint8_t* fine_kd,
                        cudaStream_t st);
 void launch_fine_select(const ForwardBatch& fb, const CoarseProblem* fprobs, uint8_t* fine_tie, cudaStream_t st);
-void launch_fine_replay(const ForwardBatch& fb, const uint8_t* fine_tie, cudaStream_t st);
+void launch_fine_replay(const ForwardBatch& fb, const CoarseProblem* fprobs, const uint8_t* fine_tie, cudaStream_t st);
 void launch_picks(const GridDesc& g, const double* t, long long N, int nsrc, const long long* recoff,
                   const double* rec, double* picks, cudaStream_t st);
 // Gaussian smoothing of a gradient field (smoothgradkern = l, odd): weights on the host,
