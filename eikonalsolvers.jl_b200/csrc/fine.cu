@@ -52,8 +52,9 @@ struct SmemHeap {
     }
     return true;
   }
-  __device__ void update(double v, int32_t h) {
-    int i = idx[h - 1];
+  // guess: an earlier position of h, right unless a swap has moved it since
+  __device__ void update(double v, int32_t h, int guess) {
+    int i = guess >= 1 && guess <= Nh && hand[guess] == h ? guess : idx[h - 1];
     if (i < 1 || i > Nh) return;  // not in the heap (only after a capacity overflow)
     nodes[i] = v;
     while (i > 1 && nodes[i / 2] > nodes[i]) {
@@ -76,38 +77,37 @@ struct SmemHeap {
   }
 };
 
-// The reference's update of fine node (i,j,k) from the nodes that `accepted` (of a node index) holds for.
-template <class ACC>
+// The reference's update of the fine node l at c from the nodes that `accepted` (of a node index)
+// holds for. Unrolled over axes and sides: the neighbourhood stays in registers and its reads are
+// in flight together, 18 -> 6 us per update.
+template <int ND, class ACC>
 __device__ __forceinline__ double fine_update(const GridDesc& gf, const double* tt, const ACC& accepted,
-                                              double slow, int i, int j, int k, int8_t* codes,
-                                              bool* neg) {
+                                              double slow, const int* c, int l, int8_t* codes, bool* neg) {
   Nbhd nb;
   nb_clear(nb);
-  const int c[3] = {i, j, k};
-  node_dh(gf, i, nb.dh);
+  node_dh(gf, c[0], nb.dh);
   nb.slow = slow;
-  for (int a = 0; a < gf.nd; a++)
-    for (int l = 0; l < 2; l++) {
-      const int sh = l == 0 ? 1 : -1;
-      int p[3] = {c[0], c[1], c[2]};
-      p[a] += sh;
-      if (p[a] < 0 || p[a] >= gf.n[a]) continue;
-      const long long pl = lin3(gf, p[0], p[1], p[2]);
-      if (accepted(pl)) nb_put1(nb, a, l, tt[pl], -EIK_INF, 0);
-      else nb_put1(nb, a, l, EIK_INF, EIK_INF, 0);
-      bool ok = true;
-      for (int d = 0; d < gf.nd; d++)
-        if (p[d] < 1 || p[d] > gf.n[d] - 2) ok = false;
-      if (ok) {
-        int q[3] = {p[0], p[1], p[2]};
-        q[a] += sh;
-        const long long ql = lin3(gf, q[0], q[1], q[2]);
-        if (accepted(ql)) nb_put2(nb, a, l, tt[ql], -EIK_INF, 0);
-        else nb_put2(nb, a, l, EIK_INF, EIK_INF, 0);
+  const int st[3] = {1, gf.n[0], gf.n[0] * gf.n[1]};
+#pragma unroll
+  for (int a = 0; a < ND; a++)
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+      const int sh = s == 0 ? 1 : -1, x = c[a] + sh;
+      if (x < 0 || x >= gf.n[a]) continue;
+      const int pl = l + sh * st[a];
+      if (accepted(pl)) nb_put1(nb, a, s, tt[pl], -EIK_INF, 0);
+      else nb_put1(nb, a, s, EIK_INF, EIK_INF, 0);
+      bool inner = x >= 1 && x <= gf.n[a] - 2;  // 2nd order: the first neighbour is off the border
+#pragma unroll
+      for (int d = 0; d < ND; d++)
+        if (d != a && (c[d] < 1 || c[d] > gf.n[d] - 2)) inner = false;
+      if (inner) {
+        const int ql = pl + sh * st[a];
+        if (accepted(ql)) nb_put2(nb, a, s, tt[ql], -EIK_INF, 0);
+        else nb_put2(nb, a, s, EIK_INF, EIK_INF, 0);
       }
     }
-  const Key T = key_normal(0.0);
-  return gf.nd == 3 ? update_at<3>(nb, T, codes, neg) : update_at<2>(nb, T, codes, neg);
+  return update_at<ND>(nb, key_normal(0.0), codes, neg);
 }
 
 // Fine node -> coarse node used for its velocity (nearest neighbour, eikmainfwd.jl:1035-1051).
@@ -227,6 +227,7 @@ __device__ __forceinline__ bool key_lt(const Key& a, const Key& b) { return !key
 // The replay warns of negative discriminants. Where a tied stop needs no replay (fine_select_kernel)
 // the warning comes from the same updates: those of the neighbours of every node accepted before the
 // last batch, from the nodes accepted by then. By threads t0, t0 + dt, ...
+template <int ND>
 __device__ void fine_warn(const ForwardBatch& fb, const CoarseProblem& P, int s, int t0, int dt) {
   const GridDesc& gf = P.g;
   const int32_t* order = fb.fine_order + (size_t)s * fb.nfmax;
@@ -238,7 +239,7 @@ __device__ void fine_warn(const ForwardBatch& fb, const CoarseProblem& P, int s,
     auto accepted = [&](long long r) { return P.t[r] < EIK_INF && key_le(fine_key(P, r), kp); };
     int f[3];
     node_coords(gf, order[p], f);
-    for (int k = 0; k < 2 * gf.nd; k++) {
+    for (int k = 0; k < 2 * ND; k++) {
       int c[3] = {f[0], f[1], f[2]};
       c[k >> 1] += (k & 1) ? 1 : -1;
       if (c[k >> 1] < 0 || c[k >> 1] >= gf.n[k >> 1]) continue;
@@ -246,7 +247,7 @@ __device__ void fine_warn(const ForwardBatch& fb, const CoarseProblem& P, int s,
       if (accepted(cl)) continue;
       int8_t cd[3];
       bool neg = false;
-      fine_update(gf, P.t, accepted, P.slow[cl], c[0], c[1], c[2], cd, &neg);
+      fine_update<ND>(gf, P.t, accepted, P.slow[cl], c, (int)cl, cd, &neg);
       any = any || neg;
     }
   }
@@ -260,13 +261,14 @@ constexpr int WARN_CTAS = 16;  // per source, of one warp
 constexpr int FINE_THREADS = 32;
 constexpr int MAXPOP = 128;
 
+template <int ND>
 __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb, const CoarseProblem* fprobs,
                                                                 const uint8_t* tie) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int s = blockIdx.x;
   const int lane = threadIdx.x;
   if (tie && tie[s] != TIE_REPLAY) {  // replay of the flagged sources only
-    if (tie[s] == TIE_WARN) fine_warn(fb, fprobs[s], s, blockIdx.y * FINE_THREADS + lane, gridDim.y * FINE_THREADS);
+    if (tie[s] == TIE_WARN) fine_warn<ND>(fb, fprobs[s], s, blockIdx.y * FINE_THREADS + lane, gridDim.y * FINE_THREADS);
     return;
   }
   if (blockIdx.y) return;
@@ -279,6 +281,8 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
   __shared__ double evv[MAXPOP * 6];
   __shared__ uint8_t evc[MAXPOP * 6];
   __shared__ uint8_t evneg[MAXPOP * 6];
+  __shared__ uint8_t evs[MAXPOP * 6];
+  __shared__ int32_t evl[MAXPOP * 6], evp[MAXPOP * 6];
   const double* src = fb.coordsrc + (size_t)s * g.nd;
 
   if (lane == 0) {
@@ -325,8 +329,7 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
     *cl = lin3(g, fi.ijk1[0] + i / fi.ds, fi.ijk1[1] + j / fi.ds, fi.ijk1[2] + k / fi.ds);
     return true;
   };
-  const int nd = g.nd;
-  const int nneigh = 2 * nd;
+  constexpr int nd = ND, nneigh = 2 * ND;
   // neighbour order of ttFMM_core! (eikmainfwd.jl:484-496)
   const int NB2[4][3] = {{1, 0, 0}, {0, 1, 0}, {-1, 0, 0}, {0, -1, 0}};
   const int NB3[6][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {-1, 0, 0}, {0, -1, 0}, {0, 0, -1}};
@@ -375,8 +378,8 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
         if (st[cl] == 0) {
           int8_t cd[3];
           bool neg = false;
-          const double v = fine_update(gf, tt, accepted, slow[fine_to_coarse(g, fi, c[0], c[1], c[2])], c[0],
-                                       c[1], c[2], cd, &neg);
+          const double v = fine_update<ND>(gf, tt, accepted, slow[fine_to_coarse(g, fi, c[0], c[1], c[2])], c,
+                                           (int)cl, cd, &neg);
           if (neg) warn |= WARN_NEG_DISCRIMINANT;
           if (!H.insert(v, (int32_t)(cl + 1))) sh_err |= ERRB_HEAP_OVERFLOW;
           st[cl] = 1;
@@ -406,9 +409,10 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
           st[al] = 2;
           tt[al] = v;
           order[nacc++] = (int32_t)al;
-          const int ai = (int)(al % gf.n[0]);
-          const int aj = (int)((al / gf.n[0]) % gf.n[1]);
-          const int ak = (int)(al / ((long long)gf.n[0] * gf.n[1]));
+          const unsigned ar = (unsigned)al / (unsigned)gf.n[0];
+          const int ai = (int)((unsigned)al - ar * gf.n[0]);
+          const int aj = ND == 3 ? (int)(ar % (unsigned)gf.n[1]) : (int)ar;
+          const int ak = ND == 3 ? (int)(ar / (unsigned)gf.n[1]) : 0;
           long long cl;
           if (coarse_of(ai, aj, ak, &cl)) {
             if (sh_nseed >= fb.seedcap) {
@@ -450,42 +454,46 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
     // ---- all lanes: stencil updates of the popped nodes' neighbours (read-only phase)
     const int nev = sh_npop * nneigh;
     for (int e = lane; e < nev; e += FINE_THREADS) {
-      const long long al = popped[e / nneigh];
+      const unsigned al = (unsigned)popped[e / nneigh], ar = al / (unsigned)gf.n[0];
       const int ne = e % nneigh;
-      int c[3] = {(int)(al % gf.n[0]), (int)((al / gf.n[0]) % gf.n[1]), (int)(al / ((long long)gf.n[0] * gf.n[1]))};
-      for (int d = 0; d < nd; d++) c[d] += (nd == 2 ? NB2[ne][d] : NB3[ne][d]);
+      int c[3] = {(int)(al - ar * gf.n[0]), ND == 3 ? (int)(ar % (unsigned)gf.n[1]) : (int)ar,
+                  ND == 3 ? (int)(ar / (unsigned)gf.n[1]) : 0};
       bool inb = true;
-      for (int d = 0; d < nd; d++)
+#pragma unroll
+      for (int d = 0; d < nd; d++) {
+        c[d] += ne % nd == d ? (ne < nd ? 1 : -1) : 0;  // the neighbour order of NB2, NB3
         if (c[d] < 0 || c[d] >= gf.n[d]) inb = false;
+      }
       evc[e] = 0xff;
       if (!inb) continue;
-      const long long cl = lin3(gf, c[0], c[1], c[2]);
-      if (st[cl] == 2) continue;
+      const int cl = c[0] + gf.n[0] * (c[1] + gf.n[1] * c[2]);
+      const uint8_t sv = st[cl];
+      if (sv == 2) continue;
       int8_t cd[3];
       bool neg = false;
-      evv[e] = fine_update(gf, tt, accepted, slow[fine_to_coarse(g, fi, c[0], c[1], c[2])], c[0], c[1], c[2], cd,
-                           &neg);
+      evl[e] = cl;
+      evs[e] = sv;
+      evp[e] = idxh[cl];
+      evv[e] = fine_update<ND>(gf, tt, accepted, slow[fine_to_coarse(g, fi, c[0], c[1], c[2])], c, cl, cd, &neg);
       evc[e] = pack_codes(cd, nd);
       evneg[e] = neg;
     }
     __syncwarp();
     // ---- lane 0: heap inserts/updates in the reference's order (eikmainfwd.jl:768-813)
     if (lane == 0) {
+      const bool one = sh_npop == 1;  // one node's neighbours are distinct: their status stands
       for (int e = 0; e < nev; e++) {
         if (sh_err) break;
         if (evc[e] == 0xff) continue;
-        const long long al = popped[e / nneigh];
-        const int ne = e % nneigh;
-        int c[3] = {(int)(al % gf.n[0]), (int)((al / gf.n[0]) % gf.n[1]), (int)(al / ((long long)gf.n[0] * gf.n[1]))};
-        for (int d = 0; d < nd; d++) c[d] += (nd == 2 ? NB2[ne][d] : NB3[ne][d]);
-        const long long cl = lin3(gf, c[0], c[1], c[2]);
+        const int cl = evl[e];
         if (evneg[e]) warn |= WARN_NEG_DISCRIMINANT;
-        if (st[cl] == 0) {
-          if (!H.insert(evv[e], (int32_t)(cl + 1))) sh_err |= ERRB_HEAP_OVERFLOW;
+        const uint8_t sv = one ? evs[e] : st[cl];
+        if (sv == 0) {
+          if (!H.insert(evv[e], cl + 1)) sh_err |= ERRB_HEAP_OVERFLOW;
           st[cl] = 1;
           code[cl] = evc[e];
-        } else if (st[cl] == 1) {
-          H.update(evv[e], (int32_t)(cl + 1));
+        } else if (sv == 1) {
+          H.update(evv[e], cl + 1, evp[e]);
           code[cl] = evc[e];
         }
       }
@@ -513,7 +521,7 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
 // node ties with the first coarse-coincident node), does the heap's internal order decide; those
 // sources, and tied ones with seeds of equal times, are replayed exactly. Other ties without a coarse-coincident node are what constant and
 // laterally uniform velocities give for a source off the nodes: replayed they took 205-225 ms of a
-// 210-230 ms call (64^3, 128^3), which now takes 6.7 and 10 ms.
+// 210-230 ms call (64^3, 128^3), which now takes 4.8 and 8.3 ms.
 
 // Window, fine source box, the fine problem of the round solver, its slowness and seeds.
 __global__ void fine_setup_kernel(ForwardBatch fb, CoarseProblem* fprobs, const double* dsmin, double gate, int small,
@@ -861,20 +869,19 @@ void launch_srcbox(const ForwardBatch& fb, cudaStream_t st) {
 
 size_t fine_smem_bytes(int heapcap) { return (sizeof(double) + sizeof(int32_t)) * (size_t)(heapcap + 1); }
 
-void launch_fine(const ForwardBatch& fb, cudaStream_t st) {
+static void launch_fmm(const ForwardBatch& fb, const CoarseProblem* fprobs, const uint8_t* tie, int ctas, cudaStream_t st) {
   const size_t sm = fine_smem_bytes(fb.heapcap);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(fine_fmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr_set = true;
-  }
-  fine_fmm_kernel<<<fb.nsrc, FINE_THREADS, sm, st>>>(fb, nullptr, nullptr);
+  auto go = [&](auto kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    kernel<<<dim3(fb.nsrc, ctas), FINE_THREADS, sm, st>>>(fb, fprobs, tie);
+  };
+  fb.g.nd == 3 ? go(fine_fmm_kernel<3>) : go(fine_fmm_kernel<2>);
 }
 
+void launch_fine(const ForwardBatch& fb, cudaStream_t st) { launch_fmm(fb, nullptr, nullptr, 1, st); }
+
 void launch_fine_replay(const ForwardBatch& fb, const CoarseProblem* fprobs, const uint8_t* fine_tie, cudaStream_t st) {
-  const size_t sm = fine_smem_bytes(fb.heapcap);
-  cudaFuncSetAttribute(fine_fmm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  fine_fmm_kernel<<<dim3(fb.nsrc, WARN_CTAS), FINE_THREADS, sm, st>>>(fb, fprobs, fine_tie);
+  launch_fmm(fb, fprobs, fine_tie, WARN_CTAS, st);
 }
 
 }  // namespace eik
