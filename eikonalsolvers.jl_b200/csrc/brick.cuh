@@ -19,14 +19,15 @@
 // Why this shape: visited one by one from worklists, a node costs ~100 scattered sectors
 // (its neighbours, their codes and stamps, the relisting filter) and a round per layer of the
 // front. A brick visit reads ~10 KB in full sectors for ~200 evaluations and settles several
-// layers, so rounds are fewer (256^3 x 4 sources: 881 instead of 3970) and the evaluation chain
+// layers, so rounds are fewer (256^3 x 4 sources: 857 instead of 3970) and the evaluation chain
 // runs on shared memory. 8^3 nodes with one warp: a front crosses a brick in sheets of about 64
 // nodes, two warp-wide evaluations; larger bricks fill the lanes a little better but leave
 // fewer warps per SM to hide latency. Forward solve, worklists of nodes -> bricks, B200:
-// 256^3 x 4 420 -> 122 ms, 128^3 x 8 123 -> 45 ms, 64^3 x 32 48 -> 16 ms, 128^3 x 1 40 -> 19 ms,
-// 1024x640 x 64 196 -> 44 ms. What bounds it: the longest visit of a round while a round has
-// fewer bricks than the GPU has warps (256^3 x 4: a visit averages 25 us, the longest of a round
-// 90 us); DRAM and the FP64 pipe are idle (below 1 % and 3 %).
+// 256^3 x 4 420 -> 116 ms, 128^3 x 8 123 -> 33 ms, 64^3 x 32 48 -> 14 ms, 128^3 x 1 40 -> 10.4 ms,
+// 1024x640 x 64 196 -> 39 ms (small bricks in the middle three). What bounds it: the longest visit of
+// a round (256^3 x 4: 98 us, a visit averages 30 us, and 68 % of the warps' time is spent at the
+// barrier; 31 % at 256^3 x 32), inside a visit the instructions' latency; DRAM and the FP64 pipe are
+// idle (below 1 % and 3 %).
 #pragma once
 
 #include "kernels.cuh"
@@ -307,10 +308,13 @@ struct VisitTally {
 // Scans (steps of up to two warps of nodes) of a visit before it hands its pending nodes back
 // to the next round of its colour. A visit needs about eight; a few need a hundred and would
 // hold up the round: 256^3 x 4 at 8 / 12 / 16 / 24 / 192 scans: 140 / 126 / 122 / 129 / 150 ms, 64^3 x
-// 32 18.2 / 16.6 / 17.0 / 19.4 / 20.5 ms, 1024x640 x 64 61 / 53 / 49 / 44 / 53 ms. It also ends a visit in
-// which values alternate (the rule's depth limit lets some transient keys do so).
+// 32 18.2 / 16.6 / 17.0 / 19.4 / 20.5 ms, 1024x640 x 64 61 / 53 / 49 / 44 / 53 ms. Small 3D bricks have an
+// eighth of the nodes to settle: 128^3 x 1 at 8 / 11 / 16 scans 10.2 / 10.4 / 11.9 ms, 128^3 x 8 33.7 / 33.2 /
+// 36.0, 64^3 x 32 14.3 / 13.9 / 14.8, spherical 100x90x90 x 12 35.7 / 33.0 / 34.1; small 2D ones (300x220 x 4)
+// 16 / 24 / 32: 8.8 / 5.1 / 5.7 ms. It also ends a visit in which values alternate (the rule's depth limit lets
+// some transient keys do so).
 template <int ND, bool SMALL>
-constexpr int VISIT_MAX_SCANS = ND == 3 ? 16 : 24;
+constexpr int VISIT_MAX_SCANS = ND == 3 ? (SMALL ? 11 : 16) : 24;
 
 // Which steps -2, -1, +1, +2 along an axis stay within [lo, hi) from position p: bits 0..3 of
 // nibble p of the table, for positions 0..15 (low half: 0..7).
