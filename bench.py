@@ -464,7 +464,7 @@ def main_b200(args):
 
     # ---- roofline of the dominant kernel (measured inside the timed region)
     peak, peak_kind = measured_peaks()
-    kern = {"coarse_rounds_kernel": (solve_ms, 16), "adj_rounds_kernel": (adj_ms, 16),
+    kern = {"brick_rounds_kernel": (solve_ms, 16), "adj_rounds_kernel": (adj_ms, 16),
             "fine_fmm_kernel": (fine_ms, 16)}
     top = max(kern, key=lambda k: kern[k][0])
     kms, bpn = kern[top]
@@ -769,7 +769,7 @@ def run_configs_leg(args, device):
                 O.eikgradient(w.vel, w.grd, w.coordsrc[:k], w.coordrec[:k], w.pickobs[:k], w.stdobs[:k], "gradvel",
                               extraparams=cpu_ep, nthreads=min(k, cores))
             tc = time.perf_counter() - t0
-            kern = {"coarse_rounds_kernel": float(st.solve_ms), "adj_rounds_kernel": float(st.adj_ms)}
+            kern = {"brick_rounds_kernel": float(st.solve_ms), "adj_rounds_kernel": float(st.adj_ms)}
             top = max(kern, key=kern.get)
             alg = 16 * N * nsrc
             achieved = alg / (kern[top] / 1000.0) / 1e9 if kern[top] > 0 else None
