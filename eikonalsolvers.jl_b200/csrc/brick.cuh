@@ -310,11 +310,12 @@ struct VisitTally {
 // hold up the round: 256^3 x 4 at 8 / 12 / 16 / 24 / 192 scans: 140 / 126 / 122 / 129 / 150 ms, 64^3 x
 // 32 18.2 / 16.6 / 17.0 / 19.4 / 20.5 ms, 1024x640 x 64 61 / 53 / 49 / 44 / 53 ms. Small 3D bricks have an
 // eighth of the nodes to settle: 128^3 x 1 at 8 / 11 / 16 scans 10.2 / 10.4 / 11.9 ms, 128^3 x 8 33.7 / 33.2 /
-// 36.0, 64^3 x 32 14.3 / 13.9 / 14.8, spherical 100x90x90 x 12 35.7 / 33.0 / 34.1; small 2D ones (300x220 x 4)
-// 16 / 24 / 32: 8.8 / 5.1 / 5.7 ms. It also ends a visit in which values alternate (the rule's depth limit lets
+// 36.0, 64^3 x 32 14.3 / 13.9 / 14.8, spherical 100x90x90 x 12 35.7 / 33.0 / 34.1; small 2D ones, which
+// with wide rounds settle in a few long visits, 24 / 28 / 32 / 40 / 56 at the best width of each: 300x220 x 4
+// 5.2 / 4.6 / 4.0 / 4.0 / 4.0 ms, 517x323 x 4 8.8 / 7.7 / 6.9 / 6.6 / 6.7, 128x80 x 1 2.0 / 1.6 / 1.5 / 1.4 / 1.4. It also ends a visit in which values alternate (the rule's depth limit lets
 // some transient keys do so).
 template <int ND, bool SMALL>
-constexpr int VISIT_MAX_SCANS = ND == 3 ? (SMALL ? 11 : 16) : 24;
+constexpr int VISIT_MAX_SCANS = ND == 3 ? (SMALL ? 11 : 16) : (SMALL ? 40 : 24);
 
 // Which steps -2, -1, +1, +2 along an axis stay within [lo, hi) from position p: bits 0..3 of
 // nibble p of the table, for positions 0..15 (low half: 0..7).

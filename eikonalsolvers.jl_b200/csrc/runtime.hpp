@@ -180,9 +180,10 @@ struct eik_ctx {
   bool fine_replay = false; // refined start-up by exact heap replay for every source (else only on ties)
   // Round width of a call: the value set on the context, else by dimension and brick size (forward
   // solve, 3D small bricks 6 / 8 / 12: 128^3 x 8 37.4 / 36.3 / 36.6 ms; large 4 / 6: 256^3 x 4 127 / 122;
-  // 2D small 16 / 24 / 32: 300x220 x 4 6.1 / 5.3 / 5.0; large 8 / 16 / 24: 1024x640 x 64 44 / 42 / 43).
+  // 2D small 16 / 32 / 48 / 64: 300x220 x 4 6.4 / 4.8 / 4.1 / 3.9, 517x323 x 26 13.2 / 10.5 / 9.6 / 9.8, 1024x640 x
+  // 64 41.8 / 39.0 / 40.8 / -; large 8 / 16 / 24: 1024x640 x 64 44 / 42 / 43).
   double gate_for(int nd, bool small) const {
-    const double g = round_gate > 0.0 ? round_gate : (nd == 2 ? (small ? 24.0 : 16.0) : (small ? 8.0 : 6.0));
+    const double g = round_gate > 0.0 ? round_gate : (nd == 2 ? (small ? 48.0 : 16.0) : (small ? 8.0 : 6.0));
     return retry ? 1.5 * g : g;
   }
   // SMs of a solve over `bricks` bricks: a round visits one colour, so at most half.

@@ -29,7 +29,7 @@ from typing import Dict, Iterable, Optional, Sequence
 
 import numpy as np
 
-DEFAULT_CANDIDATES: Dict[str, Sequence[float]] = {"round_gate": (2.0, 4.0, 6.0, 8.0, 10.0, 12.0, 16.0, 24.0, 32.0), "ctas_per_sm": (0,)}
+DEFAULT_CANDIDATES: Dict[str, Sequence[float]] = {"round_gate": (4.0, 6.0, 8.0, 12.0, 16.0, 24.0, 32.0, 48.0, 64.0), "ctas_per_sm": (0,)}
 SHIPPED_TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuned_b200.json")
 
 
