@@ -528,11 +528,9 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND, SMALL>& w, const Bri
               L1[a][s] = sign_set(t1[a][s]) ? __ldcg(kL + l1) : t1[a][s];
               L2[a][s] = sign_set(t2[a][s]) ? __ldcg(kL + l2) : t2[a][s];
               d1[a][s] = sign_set(t1[a][s]) ? (int)__ldcg(kd + l1) : 0;
-              t1[a][s] = fabs(t1[a][s]);
-              t2[a][s] = fabs(t2[a][s]);
             }
           }
-          done = prefix_rule_fast<ND, true>(t1, t2, L1, L2, d1, c1, c2, slow, &nv, &nL, &nd, cf);
+          done = prefix_rule_signed<ND>(t1, t2, L1, L2, d1, c1, c2, slow, &nv, &nL, &nd, cf);
         }
 #pragma unroll
         for (int a = 0; a < ND; a++) cd[a] = cf[a];

@@ -629,6 +629,28 @@ EIK_HD bool prefix_rule_fast(const double (&t1)[ND][2], const double (&t2)[ND][2
   return ok;
 }
 
+// prefix_rule_fast with levels on a neighbourhood as a brick keeps it: t1 and t2 carry the sign bit of a
+// special key, L1, L2 and d1 the keys (the traveltime and 0 of an ordinary one). A special key whose level
+// equals its traveltime, (t, d >= 1, t), comes after the ordinary (t, 0, t) and before other depths, an order
+// that levels alone do not show: a node beside one goes to the general rule. Exact ties beside a
+// shock make such keys (blocks of round velocity values).
+template <int ND>
+EIK_HD bool prefix_rule_signed(double (&t1)[ND][2], double (&t2)[ND][2], const double (&L1)[ND][2],
+                               const double (&L2)[ND][2], const int (&d1)[ND][2], const double (&c1)[ND],
+                               const double (&c2)[ND], double slow, double* v_out, double* L_out, int* d_out,
+                               int8_t* codes) {
+  bool tied = false;
+#pragma unroll
+  for (int a = 0; a < ND; a++)
+#pragma unroll
+    for (int l = 0; l < 2; l++) {
+      tied = tied || L1[a][l] == -t1[a][l] || L2[a][l] == -t2[a][l];
+      t1[a][l] = fabs(t1[a][l]);
+      t2[a][l] = fabs(t2[a][l]);
+    }
+  return prefix_rule_fast<ND, true>(t1, t2, L1, L2, d1, c1, c2, slow, v_out, L_out, d_out, codes) && !tied;
+}
+
 // Packed derivative codes: one byte per node, (c0+2) + 5*(c1+2) + 25*(c2+2) in the low
 // 7 bits; bit 7 marks a source point (traveltime fixed by the initialisation).
 EIK_HD uint8_t pack_codes(const int8_t* c, int nd) {
