@@ -305,15 +305,21 @@ struct VisitTally {
   }
 };
 
-// Scans (steps of up to two warps of nodes) of a visit before it hands its pending nodes back
-// to the next round of its colour. A visit needs about eight; a few need a hundred and would
+// Scans (steps of up to two warps of nodes) of a visit in which a node changes, before it hands its pending
+// nodes back to the next round of its colour. A visit needs about eight; a few need a hundred and would
 // hold up the round: 256^3 x 4 at 8 / 12 / 16 / 24 / 192 scans: 140 / 126 / 122 / 129 / 150 ms, 64^3 x
 // 32 18.2 / 16.6 / 17.0 / 19.4 / 20.5 ms, 1024x640 x 64 61 / 53 / 49 / 44 / 53 ms. Small 3D bricks have an
 // eighth of the nodes to settle: 128^3 x 1 at 8 / 11 / 16 scans 10.2 / 10.4 / 11.9 ms, 128^3 x 8 33.7 / 33.2 /
 // 36.0, 64^3 x 32 14.3 / 13.9 / 14.8, spherical 100x90x90 x 12 35.7 / 33.0 / 34.1; small 2D ones, which
 // with wide rounds settle in a few long visits, 24 / 28 / 32 / 40 / 56 at the best width of each: 300x220 x 4
-// 5.2 / 4.6 / 4.0 / 4.0 / 4.0 ms, 517x323 x 4 8.8 / 7.7 / 6.9 / 6.6 / 6.7, 128x80 x 1 2.0 / 1.6 / 1.5 / 1.4 / 1.4. It also ends a visit in which values alternate (the rule's depth limit lets
-// some transient keys do so).
+// 5.2 / 4.6 / 4.0 / 4.0 / 4.0 ms, 517x323 x 4 8.8 / 7.7 / 6.9 / 6.6 / 6.7, 128x80 x 1 2.0 / 1.6 / 1.5 / 1.4 / 1.4
+// (all with every scan counted). It also ends a visit in which values alternate (the rule's depth limit lets some
+// transient keys do so). Scans without a change do not count: a visit starts from the nodes' lower
+// bounds, so nodes that wait above the front are evaluated anew by each, and where velocities differ by 30 or
+// more they lie in more inner windows than the bound has scans; counted, they kept every visit from the nodes
+// behind them for good. There are at most as many as nodes (each takes one out of the visit). Times are the
+// same (256^3 x 4 gradient 130.5 -> 130.4 ms, 1024x640 x 64 52.4 -> 52.1), a 64^3 layer of 20 times the velocity
+// 27 ms.
 template <int ND, bool SMALL>
 constexpr int VISIT_MAX_SCANS = ND == 3 ? (SMALL ? 11 : 16) : (SMALL ? 40 : 24);
 
@@ -397,8 +403,9 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND, SMALL>& w, const Bri
   __syncwarp();
   const unsigned Tb = __float_as_uint(T), below = (1u << lane) - 1u;
   unsigned left = PF_NONE, leftmask = 0u;
+  int scans = 0;  // in which a node changed
 #pragma unroll 1
-  for (int it = 0;; it++) {
+  for (;;) {
     unsigned v[B::WORDS];
     unsigned mn = PF_NONE;
 #pragma unroll
@@ -407,7 +414,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND, SMALL>& w, const Bri
       mn = min(mn, v[k]);
     }
     mn = __reduce_min_sync(FULL_WARP, mn);
-    if (mn > Tb || mn == PF_NONE || it >= VISIT_MAX_SCANS<ND, SMALL>) {
+    if (mn > Tb || mn == PF_NONE || scans >= VISIT_MAX_SCANS<ND, SMALL>) {
       left = mn;
 #pragma unroll
       for (int k = 0; k < B::WORDS; k++) {
@@ -430,6 +437,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND, SMALL>& w, const Bri
       cnt += __popc(sel[k]);
     }
     cnt = min(cnt, 64);
+    bool moved = false;
     __syncwarp();
 #pragma unroll 1
     for (int c0 = 0; c0 < cnt; c0 += 32) {
@@ -570,6 +578,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND, SMALL>& w, const Bri
         const bool same = nv == told && nL == Lold && nd == dold;  // +inf equals +inf
         const bool wait = !same && nv > (double)T && nv < EIK_INF && T < 3.402823466e38f;
         changed = !same && !wait;
+        moved = moved || changed;
         oc = same ? (nv < EIK_INF ? VISIT_SAME : VISIT_UNREACHED) : (wait ? VISIT_WAIT : VISIT_CHANGED);
         if (wait) {
           w.pf[q] = front_bits(nv);  // not final yet: the old value stands until the front is there
@@ -635,6 +644,7 @@ __device__ __forceinline__ unsigned visit_brick(WarpMem<ND, SMALL>& w, const Bri
       }
       __syncwarp();
     }
+    scans += __any_sync(FULL_WARP, moved);
   }
   // write back
   double* own = bs.t + b * B::NODES;
