@@ -741,6 +741,12 @@ int eik_ctx_set_param(eik_ctx* ctx, const char* name, double value) {
     ctx->brick_size = (int)value;
     return EIK_OK;
   }
+  if (std::strcmp(name, "host_ring") == 0) {
+    if (!(value == 0.0 || value == 1.0)) return fail(ctx, EIK_ERR_ASSERT, "host_ring must be 0 or 1");
+    ctx->host_ring = value != 0.0;
+    if (!ctx->host_ring) free_ring(ctx->ring);
+    return EIK_OK;
+  }
   if (std::strcmp(name, "max_rounds") == 0) {
     if (!(value >= 0.0 && value <= (double)(1 << 30) && value == (double)(long long)value))
       return fail(ctx, EIK_ERR_ASSERT, "max_rounds must be an integer in [0, 2^30] (0 = the library's limit)");

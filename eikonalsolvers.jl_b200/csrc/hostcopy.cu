@@ -10,6 +10,8 @@
 // do, and the smallest cost the first call of a context least (3.3, 4.8, 6.7 ms).
 #include <atomic>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <thread>
 
 #include "runtime.hpp"
@@ -48,6 +50,7 @@ void launch_columns(const GridDesc& g, const double* rows, double* out, cudaStre
 
 static bool ring_ready(eik_ctx* ctx) {
   HostRing& h = ctx->ring;
+  if (!ctx->host_ring) return false;
   if (h.buf) return true;
   if (cudaMallocHost(&h.buf, HOST_SLOTS * HOST_SLOT) != cudaSuccess) {
     h.buf = nullptr;
@@ -141,8 +144,21 @@ int copy_out(eik_ctx* ctx, double* dst, const double* src, unsigned long long n,
 }
 
 int copy_rows_out(eik_ctx* ctx, double* const* dst, const double* src, int64_t nsrc, const GridDesc& g, cudaStream_t st) {
-  if (!ring_ready(ctx)) return fail(ctx, EIK_ERR_CUDA, "cudaMallocHost of the staging ring failed");
-  return copy_chunks(ctx, dst, src, nsrc, (unsigned long long)npts(g), &g, st);
+  const unsigned long long n = (unsigned long long)npts(g);
+  if (ring_ready(ctx)) return copy_chunks(ctx, dst, src, nsrc, n, &g, st);
+  // no pinned memory to be had: one grid at a time to pageable memory, reordered there
+  std::unique_ptr<double[]> tmp(new (std::nothrow) double[(size_t)n]);
+  if (!tmp) return fail(ctx, EIK_ERR_CUDA, "no host memory to reorder a grid of %llu nodes", n);
+  const size_t n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
+  for (int64_t s = 0; s < nsrc; s++) {
+    CUDA_OK(ctx, cudaMemcpyAsync(tmp.get(), src + (size_t)s * n, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, st));
+    CUDA_OK(ctx, cudaStreamSynchronize(st));
+    double* out = dst[s];
+    for (size_t i = 0; i < n0; i++)
+      for (size_t j = 0; j < n1; j++)
+        for (size_t k = 0; k < n2; k++) *out++ = tmp[i + n0 * (j + n1 * k)];
+  }
+  return EIK_OK;
 }
 
 }  // namespace eik

@@ -143,7 +143,9 @@ void* eik_ctx_stream(eik_ctx* ctx);
  * small forward solve (up to 2^20 node-sources; the refined windows, small grids) resets its
  * state, sets its seeds, solves and stores its results in one launch: 1 (the default) = in 2D, 2 =
  * in any dimension, 0 = never; "brick_size" = bricks of the forward solve and of the adjoint's: 0
- * (the default) = by the call's size, 1 = 4x4x4 / 8x8 nodes, 2 = 8x8x8 / 16x16. Returns EIK_ERR_ASSERT for an unknown name or a value out of
+ * (the default) = by the call's size, 1 = 4x4x4 / 8x8 nodes, 2 = 8x8x8 / 16x16; "host_ring" = 1 (the default) takes
+ * large results to pageable memory by way of 4 MB of pinned slots, 0 by plain copies, as without pinned
+ * memory to be had. Returns EIK_ERR_ASSERT for an unknown name or a value out of
  * range. */
 int eik_ctx_set_param(eik_ctx* ctx, const char* name, double value);
 
