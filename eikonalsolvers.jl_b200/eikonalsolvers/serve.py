@@ -77,27 +77,38 @@ class Request:
         return int(np.atleast_2d(self.coordsrc).shape[0])
 
 
-def request_bytes(grd, nsrc: int, kind: str, extraparams: Optional[ExtraParams] = None) -> int:
-    """Estimated device memory of one batched call: per node and source the forward's fields
-    (traveltime, codes, keys: 18 B) and round-solver state (stamp, cached front, dirty flag,
-    two worklist entries: 29 B), for gradients also the adjoint's (λ, right-hand side and
-    2·(D t) per axis: 16 + 8·ndim B); plus the refined windows ((2r+1)·ds+1 nodes per axis)."""
+def _source_bytes(grds, kind: str, extraparams: Optional[ExtraParams]) -> int:
+    """Device memory of one source of a call whose models have the grids ``grds``: the terms that
+    eik_gradient_bytes counts per source. Per-source arrays are as long as the largest grid, the solves' state
+    as the one with the most bricks; of the two brick sizes the one that takes more."""
     ep = extraparams or ExtraParams()
-    n = int(np.prod(grd.grsize))
-    per = 47 + ((16 + 8 * grd.ndim) if kind == "gradient" else 0)
-    fine = 0
-    if ep.refinearoundsrc:
-        side = (2 * ep.grdrefpars.noderadius + 1) * ep.grdrefpars.downscalefactor + 1
-        fine = side ** grd.ndim * 48
-    return int(nsrc) * (n * per + fine)
+    nd = grds[0].ndim
+    n = max(int(np.prod(g.grsize)) for g in grds)
+    side = (2 * ep.grdrefpars.noderadius + 1) * ep.grdrefpars.downscalefactor + 1 if ep.refinearoundsrc else 0
+    seeds = max((2 * ep.grdrefpars.noderadius + 2) ** nd, 8) if ep.refinearoundsrc else 8
+    fine = side ** nd
+    padded = coarse = bricks = 0  # nodes in whole bricks: of a grid or a refined window, of a grid; bricks
+    for b in (4, 8) if nd == 3 else (8, 16):
+        cb = max(int(np.prod([-(-int(m) // b) for m in g.grsize])) for g in grds)
+        fb = (-(-side // b)) ** nd
+        padded, coarse, bricks = max(padded, max(cb, fb) * b ** nd), max(coarse, cb * b ** nd), max(bricks, cb, fb)
+    # traveltime, codes, keys; brick-ordered traveltime, code and mask; lists; seeds; records; windows
+    per = 18 * n + 9 * padded + padded // 8 + 24 * bricks + 12 * seeds + 1024 + 36 * fine
+    if kind == "gradient":  # the source's field and the call's output; λ and node words; source points; windows
+        per += 16 * n + 12 * coarse + 32 * seeds + (8 + 8 * nd) * fine
+    return per
+
+
+def request_bytes(grd, nsrc: int, kind: str, extraparams: Optional[ExtraParams] = None) -> int:
+    """Estimated device memory of one batched call beside its models, inputs and picks."""
+    return int(nsrc) * _source_bytes([grd], kind, extraparams)
 
 
 def batch_bytes(batch, models) -> int:
-    """Estimated device memory of one merged call: request_bytes at the largest grid of the
-    batch (the per-source arrays of a multi-model call share that stride) for all its sources."""
+    """Estimated device memory of one merged call: all its sources at the largest sizes of its grids
+    (the per-source arrays of a multi-model call share one stride)."""
     grds = [models[r.model][1] for r in batch]
-    big = max(grds, key=lambda g: int(np.prod(g.grsize)))
-    return request_bytes(big, sum(r.nsrc for r in batch), batch[0].kind, batch[0].extraparams)
+    return sum(r.nsrc for r in batch) * _source_bytes(grds, batch[0].kind, batch[0].extraparams)
 
 
 def _ep_key(ep: Optional[ExtraParams]):
