@@ -12,7 +12,9 @@ the forward being most of a gradient call too), checks that every candidate retu
 same picks bit for bit (a live check of the schedule independence the solver relies on:
 a difference raises), sets the fastest pair on the context and remembers it under a key of
 the workload's shape class (dimension, node count and source count rounded up to powers of
-two, refined start-up or not). Later calls with a workload of the same class reuse the
+two, refined start-up or not, small or large bricks, which want different widths). Entries name the solver they
+were measured with: a table kept from another one is read without them, since a width that suited
+nodes in worklists (1 to 3) is a slow one for bricks (300x220 x 4: 9.2 ms at 4, 3.9 at 64). Later calls with a workload of the same class reuse the
 entry without timing. The table can be kept in a JSON file (``path``, or the
 ``EIK_TUNE_CACHE`` environment variable) so that a serving process or a sampler starts
 tuned. Below the caller's table sits the table shipped with the package
@@ -30,6 +32,7 @@ from typing import Dict, Iterable, Optional, Sequence
 import numpy as np
 
 DEFAULT_CANDIDATES: Dict[str, Sequence[float]] = {"round_gate": (4.0, 6.0, 8.0, 12.0, 16.0, 24.0, 32.0, 48.0, 64.0), "ctas_per_sm": (0,)}
+SOLVER = "bricks"
 SHIPPED_TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuned_b200.json")
 
 
@@ -37,10 +40,20 @@ def _pow2(n: int) -> int:
     return 1 << max(0, int(math.ceil(math.log2(max(1, int(n))))))
 
 
+def small_bricks(grd, nsrc: int) -> bool:
+    """Whether the library takes small bricks for this workload (small_bricks in api.cu): by the large bricks
+    that the fronts of all sources touch at a time, about."""
+    n = [float(m) for m in grd.grsize]
+    if len(n) == 3:
+        return int(nsrc) * (n[0] * n[1] + n[1] * n[2] + n[0] * n[2]) / (3.0 * 64.0) < 3000.0
+    return int(nsrc) * (n[0] + n[1]) / 16.0 < 8000.0
+
+
 def workload_key(grd, nsrc: int, extraparams=None) -> str:
     refine = True if extraparams is None else bool(extraparams.refinearoundsrc)
     npts = int(np.prod(grd.grsize))
-    return f"{type(grd).__name__}:n{_pow2(npts)}:s{_pow2(nsrc)}:r{int(refine)}"
+    bricks = "small" if small_bricks(grd, nsrc) else "large"
+    return f"{type(grd).__name__}:n{_pow2(npts)}:s{_pow2(nsrc)}:r{int(refine)}:{bricks}"
 
 
 class Tuner:
@@ -53,20 +66,26 @@ class Tuner:
         self.repeats = max(1, int(repeats))
         self.table: Dict[str, dict] = {}
         self.base: Dict[str, dict] = {}
+        self._foreign: Dict[str, dict] = {}  # another solver's entries, kept in the file
         self._lock = threading.Lock()
         if shipped and os.path.exists(shipped):
-            with open(shipped) as f:
-                self.base = json.load(f)
+            self.base = self._load(shipped)[0]
         if self.path and os.path.exists(self.path):
-            with open(self.path) as f:
-                self.table = json.load(f)
+            self.table, self._foreign = self._load(self.path)
+
+    @staticmethod
+    def _load(path: str):
+        with open(path) as f:
+            t = json.load(f)
+        own = {k: e for k, e in t.items() if e.get("solver") == SOLVER}
+        return own, {k: e for k, e in t.items() if k not in own}
 
     def _save(self):
         if not self.path:
             return
         tmp = self.path + ".tmp"
         with open(tmp, "w") as f:
-            json.dump(self.table, f, indent=1, sort_keys=True)
+            json.dump({**self._foreign, **self.table}, f, indent=1, sort_keys=True)
         os.replace(tmp, self.path)
 
     @staticmethod
@@ -91,7 +110,7 @@ class Tuner:
 
     def tune(self, ctx, model: int, grd, coordsrc, coordrec, extraparams=None, force: bool = False) -> dict:
         """Sets the fastest (round_gate, ctas_per_sm) for this workload on ``ctx`` and returns
-        the table entry: {"round_gate", "ctas_per_sm", "ms", "timings"}."""
+        the table entry: {"round_gate", "ctas_per_sm", "ms", "timings", "solver"}."""
         nsrc = int(np.atleast_2d(coordsrc).shape[0])
         key = workload_key(grd, nsrc, extraparams)
         entry = self._get(key)
@@ -117,7 +136,8 @@ class Tuner:
                 timings.append([float(gate), int(ctas), ms])
                 if best is None or ms < best[2]:
                     best = timings[-1]
-        entry = {"round_gate": best[0], "ctas_per_sm": best[1], "ms": best[2], "timings": timings}
+        entry = {"round_gate": best[0], "ctas_per_sm": best[1], "ms": best[2], "timings": timings,
+                 "solver": SOLVER}
         self.apply(ctx, entry)
         with self._lock:
             self.table[key] = entry
