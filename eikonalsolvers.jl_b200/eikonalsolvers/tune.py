@@ -14,7 +14,7 @@ a difference raises), sets the fastest pair on the context and remembers it unde
 the workload's shape class (dimension, node count and source count rounded up to powers of
 two, refined start-up or not, small or large bricks, which want different widths). Entries name the solver they
 were measured with: a table kept from another one is read without them, since a width that suited
-nodes in worklists (1 to 3) is a slow one for bricks (300x220 x 4: 9.2 ms at 4, 3.9 at 64). Later calls with a workload of the same class reuse the
+nodes in worklists (1 to 3) is a slow one for bricks (300x220 x 4, a call: 9.3 ms at 4, 5.3 at 64). Later calls with a workload of the same class reuse the
 entry without timing. The table can be kept in a JSON file (``path``, or the
 ``EIK_TUNE_CACHE`` environment variable) so that a serving process or a sampler starts
 tuned. Below the caller's table sits the table shipped with the package
