@@ -519,8 +519,8 @@ __global__ void __launch_bounds__(FINE_THREADS) fine_fmm_kernel(ForwardBatch fb,
 // accepted set is every node of smaller key plus that node. Only when another node has exactly the
 // stop node's traveltime and one of them is coarse-coincident, hence perhaps a seed (or an edge
 // node ties with the first coarse-coincident node), does the heap's internal order decide; those
-// sources, and tied ones with seeds of equal times, are replayed exactly. Other ties without a coarse-coincident node are what constant and
-// laterally uniform velocities give for a source off the nodes: replayed they took 205-225 ms of a
+// sources, and tied ones with seeds of equal times or keys of depth 2, are replayed exactly. Other ties without a
+// coarse-coincident node are what constant and laterally uniform velocities give for a source off the nodes: replayed they took 205-225 ms of a
 // 210-230 ms call (64^3, 128^3), which now takes 4.8 and 8.3 ms.
 
 // Window, fine source box, the fine problem of the round solver, its slowness and seeds.
@@ -734,6 +734,15 @@ __global__ void __launch_bounds__(SEL_THREADS) fine_select_kernel(ForwardBatch f
   tied = __syncthreads_or(tied);
   tied_cc = __syncthreads_or(tied_cc);
   amb = __syncthreads_or(amb) || (tied && tied_cc);
+  if (tied && !amb) {
+    // Keys order accepted nodes as the heap does up to depth 1; a chain of non-causal acceptances may be
+    // interleaved with others by value (of 927 windows with layers of contrast 1.5 to 20, 60 differed from the
+    // heap, all among the 105 that hold a key of depth 2 or more). Tied windows that hold one are replayed.
+    bool deep = false;
+    for (long long l = tid; l < n; l += SEL_THREADS)
+      if ((P.code[l] & CODE_SRC_BIT) && P.t[l] < EIK_INF && P.kd[l] >= 2 && !key_lt(ks, fine_key(P, l))) deep = true;
+    amb = __syncthreads_or(deep);
+  }
   if (tid == 0) tie[s] = amb ? TIE_REPLAY : TIE_NONE;
   if (amb) return;
   // status and the accepted non-corner nodes (unordered)
