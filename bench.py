@@ -465,7 +465,7 @@ def main_b200(args):
     # ---- roofline of the dominant kernel (measured inside the timed region)
     peak, peak_kind = measured_peaks()
     kern = {"brick_rounds_kernel": (solve_ms, 16), "adj_rounds_kernel": (adj_ms, 16),
-            "fine_fmm_kernel": (fine_ms, 16)}
+            "refined start-up": (fine_ms, 16)}
     top = max(kern, key=lambda k: kern[k][0])
     kms, bpn = kern[top]
     per_launch_ms = kms / args.steps

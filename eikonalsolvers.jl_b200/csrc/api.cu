@@ -202,7 +202,7 @@ const void* stage_host(eik_ctx* ctx, const void* src, size_t bytes) {
   return p;
 }
 
-// Round width and lower-bound increment of every coarse problem from the model's smallest
+// Round width and least increment of every coarse problem from the model's smallest
 // slowness, read on the device (the expressions and their order are the host's).
 __global__ void problem_scale_kernel(CoarseProblem* dp, int nprob, const double* dsmin, double gate, double hmin,
                                      int nd, int small) {
@@ -210,7 +210,6 @@ __global__ void problem_scale_kernel(CoarseProblem* dp, int nprob, const double*
   if (s >= nprob) return;
   const double smin = *dsmin;
   dp[s].delta = gate * hmin * smin;
-  dp[s].incmin = 0.999 * (2.0 / 3.0) * hmin * smin / sqrt((double)nd);
   dp[s].linc = 0.999 * (2.0 / 3.0) * hmin / sqrt((double)nd);
   dp[s].din = inner_window(nd, small != 0, hmin * smin);
 }
@@ -287,9 +286,9 @@ static double front_bricks(const GridDesc& g) {
 // Small bricks for solves whose rounds leave most of the GPU's warps without a large brick: a
 // round then lasts as long as its longest visit, which a small brick shortens. Large ones cost
 // less per node once the rounds fill the GPU. Small / large bricks, forward solve, by front:
-// 64 (64^3 x 1) 4.6 / 7.5 ms, 256 (128^3 x 1) 12.9 / 19.0, 1024 (256^3 x 1) 48 / 59, 2048 (64^3 x 32)
-// 15.0 / 16.0, 2048 (128^3 x 8) 37 / 45, 4096 (256^3 x 4) 138 / 127; 2D 130 (300x220 x 4) 6.0 / 7.3,
-// 6656 (1024x640 x 64) 38 / 42.
+// 64 (64^3 x 1) 3.6 / 6.2 ms, 256 (128^3 x 1) 10.0 / 16.0, 1024 (256^3 x 1) 38 / 48, 2048 (64^3 x 32)
+// 13.5 / 14.3, 2048 (128^3 x 8) 33 / 38, 4096 (256^3 x 4) 121 / 108, 32768 (256^3 x 32) 670 / 525; 2D 130
+// (300x220 x 4) 5.3 / 7.2, 6656 (1024x640 x 64) 41.2 / 41.3.
 static bool small_bricks(const eik_ctx* ctx, int nd, double front) {
   if (ctx->brick_size > 0) return ctx->brick_size == 1;
   return front < (nd == 3 ? 3000.0 : 8000.0);
@@ -370,7 +369,7 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
       P.code = code + s * N;
       P.kL = kL + s * N;
       P.kd = kd + s * N;
-      P.delta = P.incmin = P.linc = 0.0;  // set on the device from the model's smallest slowness
+      P.delta = P.linc = 0.0;  // set on the device from the model's smallest slowness
       P.din = 0.0f;
       uniform_coeffs(P.g, &P.c1u, &P.c2u);
     }
@@ -442,7 +441,6 @@ int forward_multi(eik_ctx* ctx, int nmod, const Model* const* models, const int6
   const bool fuse = ctx->cluster_solve == 2 || (ctx->cluster_solve == 1 && nd == 2);
   sa.err = fb.err;
   sa.probs = dp;
-  sa.max_activations = ~0ull;
   sa.timeout_ns = 20LL * 1000 * 1000 * 1000;
   // refined windows: one more round-solver problem per source
   CoarseProblem* fprobs = nullptr;

@@ -225,7 +225,6 @@ __device__ __noinline__ RuleOut rule_slow(const CoarseProblem& P, const double* 
   o.key.L = __shfl_sync(FULL_WARP, mine.L, from);
   o.key.d = __shfl_sync(FULL_WARP, mine.d, from);
   const int pc = __shfl_sync(FULL_WARP, packed, from);
-  o.neg = false;
   if (pick < 0) {
     o.v = EIK_INF;
     o.key.L = EIK_INF;

@@ -573,7 +573,6 @@ __global__ void fine_setup_kernel(ForwardBatch fb, CoarseProblem* fprobs, const 
   const double smin = *dsmin;
   uniform_coeffs(gf, &P.c1u, &P.c2u);
   P.delta = gate * hmin * smin;
-  P.incmin = 0.999 * (2.0 / 3.0) * hmin * smin / sqrt((double)gf.nd);
   P.linc = 0.999 * (2.0 / 3.0) * hmin / sqrt((double)gf.nd);
   P.din = inner_window(gf.nd, small != 0, hmin * smin);
 }

@@ -62,8 +62,8 @@ struct CoarseProblem {
   double* kL;      // key level of special nodes (-inf for source points)
   uint8_t* kd;     // key depth of special nodes
   double delta;    // round width of the forward solve (traveltime units)
-  double incmin;   // smallest increment of the local update over a neighbour: (2/3) h s_min / sqrt(nd)
-  double linc;     // the same per unit of slowness: (2/3) h / sqrt(nd), h the smallest spacing
+  double linc;     // least increment of the local update over a neighbour per unit of slowness: (2/3) h / sqrt(nd),
+                   // h the smallest spacing
   float din;       // inner window of a brick visit (traveltime units)
   double c1u, c2u; // Cartesian grids: the local solver's coefficients 1/h^2 and 9/(4h^2); 0 otherwise
 };
@@ -116,7 +116,6 @@ struct SolveArgs {
   int32_t nprob;
   int32_t nd;
   unsigned long long* activations;  // list entries visited
-  unsigned long long max_activations;
   unsigned long long* node_evals;
   uint32_t* err;
   int32_t* abort_flag;

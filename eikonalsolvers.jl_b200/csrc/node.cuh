@@ -23,11 +23,9 @@ struct RuleOut {
   double v;
   Key key;
   int8_t cd[3];
-  bool neg;
 };
 
-// Neighbour directions of a node: k = 4*axis + {0: -2, 1: -1, 2: +1, 3: +2}; bit 12 = itself.
-constexpr int DIR_SELF = 12;
+// Neighbour directions of a node: k = 4*axis + {0: -2, 1: -1, 2: +1, 3: +2}.
 __device__ __forceinline__ int dir_off(int k) { return (k & 3) < 2 ? (k & 3) - 2 : (k & 3) - 1; }
 // Grid coordinates of node l. A problem has fewer than 2^32 nodes (a launch numbers its
 // node-sources in 32 bits), so 32-bit division is exact and far cheaper than 64-bit.
@@ -38,11 +36,10 @@ __device__ __forceinline__ void node_coords(const GridDesc& g, long long l, int*
   c[1] = (int)(q % n1);
   c[2] = (int)(q / n1);
 }
-// Linear index of the node in direction k (or DIR_SELF) of node l, which the direction must
+// Linear index of the node in direction k of node l, which the direction must
 // keep in the grid: the grid is column-major (lin3), so a step along an axis adds that axis's
 // stride. Arithmetic only: an array indexed by the loop's axis would live in local memory.
 __device__ __forceinline__ long long dir_lin(const GridDesc& g, long long l, int k) {
-  if (k == DIR_SELF) return l;
   const int ax = k >> 2;
   const long long st = ax == 0 ? 1LL : (ax == 1 ? (long long)g.n[0] : (long long)g.n[0] * g.n[1]);
   return l + dir_off(k) * st;
