@@ -176,6 +176,7 @@ struct eik_ctx {
   int retry = 0;             // a pipeline run again after the automatic round limit: wider rounds, limit 2^24
   int auto_round_limit = 0;  // the automatic round limit of a first run (0 = by the grid's diameter)
   double sm_fraction = 0.0; // share of the SMs the persistent (cooperative) solves use; 0 = by size
+  unsigned long long rows_bytes = 0;  // row-major results so far (hostcopy.cu)
   bool host_ring = true;     // large results by way of the pinned ring (hostcopy.cu); false: plain copies
   double ray_room = 3.0;     // room of a ray in its first tracing pass, in straight-line lengths
   bool fine_replay = false; // refined start-up by exact heap replay for every source (else only on ties)

@@ -34,9 +34,9 @@ def _warn(st) -> None:
         warnings.warn(msg, EikonalWarning, stacklevel=3)
 
 
-# Traveltime grids of at least this many bytes in all are put in row-major order on the device,
-# smaller ones by NumPy: 2 MB take 0.3 ms beyond the solve against 0.9 ms, 7 MB 0.7 against 4.9 ms, 64 MB
-# 5 against 41 ms, but the first such call of a context pays 3 ms for its pinned slots.
+# Traveltime grids of at least this many bytes in all are put in row-major order by the library, on the device once
+# its pinned slots exist (they are made when a context has brought back 8 MB), smaller ones by NumPy: 2 MB take
+# 0.3 ms beyond the solve against 0.9 ms, 7 MB 0.7 against 4.9 ms, 64 MB 5 against 41 ms.
 ROWS_MIN_BYTES = 1 << 22
 
 

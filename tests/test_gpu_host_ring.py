@@ -46,10 +46,12 @@ def test_many_small_grids(monkeypatch, n, nsrc):
     ctx = Context(0)
     try:
         mid = ctx.upload(vel, grd)
-        rows = ctx.traveltime(mid, grd, cs, rec, returntt=True, extraparams=ep)[1]
-        assert 8 * rows[0].size * nsrc >= api.ROWS_MIN_BYTES
+        # the first results by plain copies, the later ones through the ring
+        rows = [ctx.traveltime(mid, grd, cs, rec, returntt=True, extraparams=ep)[1] for _ in range(3)]
+        assert 8 * rows[0][0].size * nsrc >= api.ROWS_MIN_BYTES
         monkeypatch.setattr(api, "ROWS_MIN_BYTES", 1 << 62)  # column-major, put in order by NumPy
         cols = ctx.traveltime(mid, grd, cs, rec, returntt=True, extraparams=ep)[1]
     finally:
         ctx.close()
-    assert all(np.array_equal(a, b) for a, b in zip(rows, cols))
+    for r in rows:
+        assert all(np.array_equal(a, b) for a, b in zip(r, cols))
